@@ -430,6 +430,7 @@ tmvg_status tmvg_destroy(tmvg_handle h)
     if (c->work2) cudaFree(c->work2);
     if (c->work3) cudaFree(c->work3);
     if (c->io) cudaFree(c->io);
+    if (c->pool) cudaMemPoolDestroy(c->pool);
     if (c->perm_lists) cudaFree(c->perm_lists);
     if (c->trsv_flags) cudaFree(c->trsv_flags);
     if (c->trsv_pub) cudaFree(c->trsv_pub);

@@ -85,6 +85,8 @@ struct Context {
     // Third grow-only workspace: operand copies of the tensor-core update.
     void* work3 = nullptr;
     size_t work3_bytes = 0;
+    // Stream-ordered scratch of the sliced products (created on first use).
+    cudaMemPool_t pool = nullptr;
     // Device copies of the host entry points' operands (grow-only).
     void* io = nullptr;
     size_t io_bytes = 0;

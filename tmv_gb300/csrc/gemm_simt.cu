@@ -12,8 +12,10 @@
 // src/TMV_MultMM.cpp:447-448).  Each thread owns a TM x TN block of C whose
 // rows are consecutive, so a warp stores 16*TM consecutive rows per column.
 #include "gemm.cuh"
+#include "gemm_sliced.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace tmvg {
 
@@ -216,6 +218,13 @@ tmvg_status gemm(Context* c, int64_t m, int64_t n, int64_t k, T alpha,
     int64_t lda = 0, ldb = 0;
     if (!classify(m, k, A.si, A.sj, arm, lda) || !classify(k, n, B.si, B.sj, brm, ldb))
         return set_error(c, TMVG_BAD_ARG, "gemm: A and B must be column- or row-major");
+    if constexpr (std::is_same<T, double>::value) {
+        if (sliced_wanted(c, m, n, k)) {
+            const tmvg_status st = sliced_gemm(c, m, n, k, alpha, Mat<const double>{A.p, arm ? lda : 1, arm ? 1 : lda},
+                                               Mat<const double>{B.p, brm ? ldb : 1, brm ? 1 : ldb}, beta, C.p, ldc);
+            if (st != TMVG_UNSUPPORTED) return st;
+        }
+    }
     if (arm) {
         if (brm) return launch_gemm<T, true, true>(c, m, n, k, alpha, A.p, lda, B.p, ldb, beta, C.p, ldc);
         return launch_gemm<T, true, false>(c, m, n, k, alpha, A.p, lda, B.p, ldb, beta, C.p, ldc);

@@ -1,0 +1,725 @@
+// gemm_sliced.cu -- FP64 products on the tcgen05 tensor cores.
+//
+// GB300 issues 2 FP64 FMAs per SM per clock (1.25 TFLOP/s on the device) and
+// 4096 BF16 FMAs.  The product is therefore taken apart into exact integer
+// products (the error-free splitting of Ozaki, Ogita, Oishi and Rump, "Error-
+// free transformations of matrix multiplication", Numer. Algorithms 2012):
+// every row of A and every column of B is scaled by a power of two and cut
+// into kSlices = 8 signed digits of 8 bits, |digit| <= 128, stored as BF16
+// (exact).  Digit products are integers up to 2^14, so an FP32 accumulator in
+// tensor memory holds the sum of up to 1024 of them exactly: the (at most 8)
+// digit pairs (i, j) with i + j = d over a chunk of 128 in K share one
+// accumulator, d = 0..7, and pairs with i + j > 7 (below 2^-64 of the largest
+// product) are left out: 36 of 64.  The epilogue adds the eight accumulators
+// into a 96-bit integer per element of C and rounds to FP64 once.
+//
+// Accuracy: an element's error is about 2^-64 sqrt(K) times (row maximum of A
+// x column maximum of B), against 2^-54 of sum |a||b| for a chain of FMAs.
+// That is smaller unless the row's and the column's large entries do not
+// meet, so the slicing kernel counts, per vector, the entries within 2^-4 of
+// the largest; where the fewest of a tile's rows and columns cannot overlap
+// in 1.75 sqrt(K) places (pigeonhole), or an entry is not finite or its
+// vector's scale is extreme, the tile's CTA takes the FP64 pipe instead, on
+// the unsliced operands, with the FMA chain of gemm_simt_kernel.
+//
+// Data flow per CTA (persistent over 128 x 64 tiles of C): one thread loads
+// stages of K = 32 (8 digits x (128 + 64) rows x 64 bytes = 96 KB, two
+// stages) by TMA into 64-byte-swizzled shared memory; one thread multiplies
+// digit i of A with digits 0..7-i of B at once (they lie behind one another
+// in shared memory, and so do their accumulators in the 512 TMEM columns:
+// N = 64 (8 - i), in pieces of up to 256, so that A is read once per 256
+// columns); eight warps drain the accumulators after every K = 128.
+// All waits are bounded; on a timeout the kernel records kDevTimeout.
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
+#include "async.cuh"
+#include "gemm_sliced.cuh"
+
+#include <algorithm>
+#include <climits>
+#include <cmath>
+
+namespace tmvg {
+
+constexpr int kSlices = 8;
+constexpr int kSlM = 128, kSlN = 64;    // tile of C
+constexpr int kSlK = 32;                // K per stage: 64 bytes of BF16
+constexpr int kSlChunk = 4;             // stages per accumulation chunk (K = 128)
+constexpr int kSlStages = 2;
+constexpr int kSlABytes = kSlices * kSlM * kSlK * 2;
+constexpr int kSlBBytes = kSlices * kSlN * kSlK * 2;
+constexpr int kSlStageBytes = kSlABytes + kSlBBytes;
+constexpr size_t kSlSmem = (size_t)kSlStages * kSlStageBytes + 1024;
+constexpr int kSlEpiWarps = 8;
+constexpr int kSlThreads = 32 * (kSlEpiWarps + 2);
+constexpr int kSlCols = kSlN / 2;       // columns of C per epilogue thread
+constexpr int kFillBad = -(1 << 29);    // fill count of a group that cannot be sliced
+constexpr int kFillRange = 4;           // entries within 2^-4 of the vector's largest count
+constexpr int kExpLimit = 450;          // |scale exponent| beyond this takes the FP64 pipe
+
+size_t sliced_bytes(int64_t rows, int64_t K)
+{
+    const int64_t Kp = ceil_div(K, (int64_t)kSlK) * kSlK;
+    return (size_t)kSlices * rows * Kp * 2 + 8 * ((size_t)rows + 64) + 512;
+}
+
+SlicedOperand sliced_layout(void* buf, int64_t rows, int64_t K)
+{
+    SlicedOperand s;
+    s.rows = rows;
+    s.Kp = ceil_div(K, (int64_t)kSlK) * kSlK;
+    s.group = K <= kSlK ? 64 : 16;
+    s.digits = static_cast<uint16_t*>(buf);
+    s.exps = reinterpret_cast<int*>(s.digits + (size_t)kSlices * rows * s.Kp);
+    s.fill = s.exps + rows;
+    return s;
+}
+
+// ---------------------------------------------------------------------
+// Slicing.  A CTA takes R vectors; the first pass over them finds the largest
+// exponent, the second (from L2) cuts the digits with integer operations
+// only (the FP64 pipe would take 2 elements per SM per clock).  Bound: 8
+// bytes read and 16 written per element.
+// ---------------------------------------------------------------------
+constexpr int kSplitThreads = 256;
+
+struct SplitSide {
+    const double* p;
+    int64_t sr, sk;   // element (vector r, place k) at p[r*sr + k*sk]
+    uint16_t* digits;
+    int* exps;
+    int* fill;
+    int64_t rows, Kp;
+};
+
+// value = (-1)^s X 2^(E - 63) with E the vector's scale, as 8 balanced bytes
+__device__ __forceinline__ unsigned long long fixed63(double v, int emax)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const int ef = (int)((b >> 52) & 0x7ff);
+    unsigned long long x = (b & 0x000fffffffffffffull) | 0x0010000000000000ull;
+    const int sh = 10 - (emax - ef);
+    if (ef == 0 || sh < -53) x = 0;  // zero, subnormal, or below the last digit
+    else if (sh >= 0) x <<= sh;
+    else x = (x + (1ull << (-sh - 1))) >> (-sh);
+    return (b >> 63) ? 0ull - x : x;
+}
+
+template <int R>
+__global__ void __launch_bounds__(kSplitThreads)
+sliced_split_kernel(SplitSide sa, SplitSide sb, int64_t groups_a, int64_t K)
+{
+    constexpr int G = kSplitThreads / R;  // threads sharing a vector
+    const bool is_b = (int64_t)blockIdx.x >= groups_a;
+    const SplitSide s = is_b ? sb : sa;
+    const int64_t grp = is_b ? blockIdx.x - groups_a : blockIdx.x;
+    __shared__ int s_emax[R], s_big[R];
+    __shared__ int s_min;
+    const int tid = threadIdx.x;
+    const bool kc = s.sk == 1;  // K contiguous: neighbouring threads take neighbouring k
+    const int r = kc ? tid / G : tid % R;
+    const int g = kc ? tid % G : tid / R;
+    const int64_t row = grp * R + r;
+    const bool have = row < s.rows;
+    const double* p = s.p + row * s.sr;
+    if (tid < R) {
+        s_emax[tid] = 0;
+        s_big[tid] = 0;
+    }
+    if (tid == 0) s_min = INT_MAX;
+    __syncthreads();
+    if (have) {
+        int e = 0;
+#pragma unroll 8
+        for (int64_t k = g; k < K; k += G)
+            e = max(e, (int)((unsigned)__double2hiint(p[k * s.sk]) >> 20 & 0x7ff));
+        atomicMax(&s_emax[r], e);
+    }
+    __syncthreads();
+    const int emax = s_emax[r];
+    int big = 0;
+    if (have) {
+        const size_t slice = (size_t)s.rows * s.Kp;
+        for (int64_t k0 = (int64_t)g * 8; k0 < s.Kp; k0 += G * 8) {
+            double v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = k0 + q < K ? p[(k0 + q) * s.sk] : 0.0;
+            uint32_t w[kSlices][4];
+#pragma unroll
+            for (int q = 0; q < 8; q += 2) {
+                uint32_t lo[2], hi[2], top[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int ef = (int)((unsigned)__double2hiint(v[q + h]) >> 20 & 0x7ff);
+                    big += ef != 0 && ef >= emax - kFillRange;
+                    const unsigned long long x = fixed63(v[q + h], emax);
+                    // adding 128 to every byte below the top one makes each an
+                    // unsigned digit + 128, with the carries resolved
+                    const unsigned long long y = (x & 0x00ffffffffffffffull) + 0x0080808080808080ull;
+                    lo[h] = (uint32_t)y;
+                    hi[h] = (uint32_t)(y >> 32);
+                    top[h] = (uint32_t)((int)((long long)x >> 56) + (int)(hi[h] >> 24) + 128);
+                }
+                // byte b -> the BF16 of b - 128: 2^23 + b, less 2^23 + 128, is exact
+                auto bf = [](uint32_t byte) {
+                    return __float_as_uint(__uint_as_float(0x4b000000u | byte) - 8388736.0f);
+                };
+                w[0][q / 2] = __byte_perm(bf(top[0]), bf(top[1]), 0x7632);
+#pragma unroll
+                for (int d = 1; d < kSlices; ++d) {
+                    const int at = 7 - d;  // byte of y
+                    const uint32_t b0 = ((at < 4 ? lo[0] : hi[0]) >> (8 * (at & 3))) & 0xff;
+                    const uint32_t b1 = ((at < 4 ? lo[1] : hi[1]) >> (8 * (at & 3))) & 0xff;
+                    w[d][q / 2] = __byte_perm(bf(b0), bf(b1), 0x7632);
+                }
+            }
+            uint16_t* dst = s.digits + (size_t)row * s.Kp + k0;
+#pragma unroll
+            for (int d = 0; d < kSlices; ++d)
+                *reinterpret_cast<uint4*>(dst + d * slice) = make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
+        }
+        atomicAdd(&s_big[r], big);
+    }
+    __syncthreads();
+    if (tid < R && grp * R + tid < s.rows) {
+        const int ee = s_emax[tid];  // exponent field: |entries| < 2^(ee - 1022)
+        int b = s_big[tid];
+        const int sc = ee == 0 ? 0 : ee - 1022;
+        if (ee == 0x7ff || sc > kExpLimit || sc < -kExpLimit) b = kFillBad;
+        else if (ee == 0) b = INT_MAX / 4;  // a zero vector: every product is exactly zero (see below)
+        s.exps[grp * R + tid] = sc;
+        atomicMin(&s_min, b);
+    }
+    // a vector of subnormals only would be sliced as zero: it takes the FP64 pipe
+    if (have && s_emax[r] == 0) {
+        bool sub = false;
+        for (int64_t k = g; k < K; k += G) sub |= (__double_as_longlong(p[k * s.sk]) << 1) != 0;
+        if (sub) atomicMin(&s_min, kFillBad);
+    }
+    __syncthreads();
+    if (tid == 0) s.fill[grp] = s_min;
+}
+
+tmvg_status sliced_split(Context* c, int64_t K, Mat<const double> A, const SlicedOperand& sa,
+                         Mat<const double> B, const SlicedOperand& sb)
+{
+    const int R = sa.rows ? sa.group : sb.group;
+    const SplitSide a{A.p, A.si, A.sj, sa.digits, sa.exps, sa.fill, sa.rows, sa.Kp};
+    const SplitSide b{B.p, B.sj, B.si, sb.digits, sb.exps, sb.fill, sb.rows, sb.Kp};
+    const int64_t ga = ceil_div(sa.rows, (int64_t)R), gb = ceil_div(sb.rows, (int64_t)R);
+    if (ga + gb == 0) return TMVG_OK;
+    if (R == 64)
+        sliced_split_kernel<64><<<(unsigned)(ga + gb), kSplitThreads, 0, c->stream>>>(a, b, ga, K);
+    else
+        sliced_split_kernel<16><<<(unsigned)(ga + gb), kSplitThreads, 0, c->stream>>>(a, b, ga, K);
+    ++c->launches;
+    return check_cuda(c, cudaGetLastError(), "sliced split launch");
+}
+
+// ---------------------------------------------------------------------
+// The product.
+// ---------------------------------------------------------------------
+__device__ __forceinline__ void sl_tma_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+            smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(0)
+        : "memory");
+}
+
+__device__ __forceinline__ void sl_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void sl_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+// Shared-memory matrix descriptor: K-major, 64-byte swizzle, rows of 64 bytes
+// in 8-row (512-byte) groups.
+__device__ __forceinline__ uint64_t sw64_desc(uint32_t addr)
+{
+    uint64_t d = (addr >> 4) & 0x3FFFull;
+    d |= 1ull << 16;
+    d |= (uint64_t)(512 >> 4) << 32;
+    d |= 1ull << 46;
+    d |= 4ull << 61;
+    return d;
+}
+
+// Instruction descriptor: D FP32, A and B BF16, both K-major, M = 128.
+__device__ __forceinline__ uint32_t bf16_idesc(int n)
+{
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kSlM >> 4) << 24);
+}
+
+__device__ __forceinline__ void sl_umma(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+__device__ __forceinline__ void sl_commit(uint64_t* bar)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                     smem_u32(bar))
+                 : "memory");
+}
+
+__device__ __forceinline__ void sl_ld4(uint32_t taddr, uint32_t (&v)[4])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(taddr)
+                 : "memory");
+}
+
+__device__ __forceinline__ void sl_arrive(uint64_t* bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// One chunk's eight accumulators of an element as p 2^32 + q in units of
+// 2^-62: p = a0 2^16 + a1 2^8 + a2, q = a3 2^24 + a4 2^16 + a5 2^8 + a6 +
+// a7 2^-8.  The accumulators are integers: |a_d| <= (d + 1) 2^21, so a0 and
+// a1 (up to 2^22) convert by one FP32 addition of 1.5 2^23, whose mantissa
+// then holds the integer; a2..a5 take the converter (16 per SM per clock);
+// a6 + a7 2^-8 is rounded to a multiple of 4 (2^-60) by the same addition.
+__device__ __forceinline__ void sl_combine(const uint32_t (&a)[kSlices], long long& p, long long& q)
+{
+    constexpr float kMagic = 12582912.0f;  // 1.5 2^23
+    constexpr uint32_t kBits = 0x4b400000u;
+    const uint32_t b0 = __float_as_uint(__uint_as_float(a[0]) + kMagic);
+    const uint32_t b1 = __float_as_uint(__uint_as_float(a[1]) + kMagic);
+    const int s = (int)(b0 * 256u + b1 - (kBits * 257u));
+    const int i2 = __float2int_rn(__uint_as_float(a[2]));
+    const int i3 = __float2int_rn(__uint_as_float(a[3]));
+    const int i4 = __float2int_rn(__uint_as_float(a[4]));
+    const int i5 = __float2int_rn(__uint_as_float(a[5]));
+    const float f = fmaf(__uint_as_float(a[7]), 0.00390625f, __uint_as_float(a[6]));
+    const int i6 = (int)(__float_as_uint(fmaf(f, 0.25f, kMagic)) - kBits);
+    p = (long long)s * 256 + i2;
+    q = (long long)i3 * 16777216 + ((long long)i4 * 65536 + ((long long)i5 * 256 + (long long)i6 * 4));
+}
+
+// The 96-bit integer (w2:w1:w0) 2^(e - 62) rounded to FP64 (nearest; a tie
+// goes away from zero).
+__device__ __forceinline__ double sl_to_double(uint32_t w0, uint32_t w1, uint32_t w2, int e)
+{
+    const uint32_t sgn = (uint32_t)((int)w2 >> 31);
+    unsigned long long lo = ((unsigned long long)w1 << 32) | w0;
+    lo = (lo ^ (((unsigned long long)sgn << 32) | sgn)) + (sgn & 1u);
+    uint32_t hi = (w2 ^ sgn) + ((sgn && lo == 0ull) ? 1u : 0u);
+    // left-align the top 64 bits
+    unsigned long long top;
+    int msb;  // position of the leading bit
+    if (hi) {
+        const int lz = __clz(hi);
+        msb = 95 - lz;
+        top = ((unsigned long long)hi << 32) | (lo >> 32);
+        if (lz) top = (top << lz) | ((uint32_t)lo >> (32 - lz));
+    } else {
+        if (lo == 0ull) return 0.0;
+        const int lz = __clzll((long long)lo);
+        msb = 63 - lz;
+        top = lo << lz;
+    }
+    const unsigned long long mant = (top >> 11) + ((top >> 10) & 1ull);
+    const unsigned long long bits = ((unsigned long long)(msb + e - 62 + 1023 - 1) << 52) + mant;
+    return __longlong_as_double((long long)(bits | ((unsigned long long)(sgn & 0x80000000u) << 32)));
+}
+
+struct SlicedArgs {
+    int64_t M, N, K;
+    double alpha;
+    int add;                         // beta
+    int unit;                        // alpha: 1 or -1, or 0 for any other value
+    const double *A, *B;             // the operands themselves (FP64 tiles)
+    int64_t asi, asj, bsi, bsj;
+    const int *ea, *eb, *fa, *fb;
+    int ga, gb;                      // vectors per fill group
+    int need;                        // overlap that a sliced tile needs
+    double* C;
+    int64_t ldc;
+    int64_t mt, nt;                  // tiles
+};
+
+// Tile t of the persistent order: columns of 16 tile rows, so that the tiles
+// in flight together share their operands in L2.
+__device__ __forceinline__ void sl_tile(const SlicedArgs& g, int64_t t, int64_t& mi, int64_t& ni)
+{
+    constexpr int64_t GM = 16;
+    const int64_t per = GM * g.nt, band = t / per, rem = t - band * per;
+    const int64_t h = min(GM, g.mt - band * GM);
+    mi = band * GM + rem % h;
+    ni = rem / h;
+}
+
+// Whether the tile's operands may be sliced (every caller gets one answer).
+__device__ __forceinline__ bool sl_ok(const SlicedArgs& g, int64_t mi, int64_t ni)
+{
+    int a = INT_MAX / 4, b = INT_MAX / 4;
+    const int64_t a1 = min((g.M - 1) / g.ga, (mi * kSlM + kSlM - 1) / g.ga);
+    const int64_t b1 = min((g.N - 1) / g.gb, (ni * kSlN + kSlN - 1) / g.gb);
+    for (int64_t i = mi * kSlM / g.ga; i <= a1; ++i) a = min(a, __ldg(&g.fa[i]));
+    for (int64_t i = ni * kSlN / g.gb; i <= b1; ++i) b = min(b, __ldg(&g.fb[i]));
+    return (int64_t)a + b - g.K >= g.need;
+}
+
+// ONE: K fits one accumulation chunk, so nothing is carried between chunks.
+template <bool ONE>
+__global__ void __launch_bounds__(kSlThreads, 1)
+sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB,
+                   const __grid_constant__ SlicedArgs g, int* err)
+{
+    extern __shared__ uint8_t sl_smem_raw[];
+    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(sl_smem_raw) + 1023) &
+                                               ~static_cast<uintptr_t>(1023));
+    __shared__ __align__(8) uint64_t full[kSlStages], empty[kSlStages], acc_full, acc_empty;
+    __shared__ uint32_t s_tmem;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+    if (warp == kSlEpiWarps) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
+                     "r"(512u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int s = 0; s < kSlStages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(&acc_full, 1);
+        mbar_init(&acc_empty, kSlEpiWarps);
+        mbar_fence_init();
+    }
+    sl_fence_before();
+    __syncthreads();
+    sl_fence_after();
+    const uint32_t tmem = s_tmem;
+    const int nst = (int)((g.K + kSlK - 1) / kSlK);
+    const int64_t tiles = g.mt * g.nt;
+
+    if (warp == kSlEpiWarps) {
+        // operands by TMA
+        if (lane == 0) {
+            uint32_t it = 0;
+            bool ok = true;
+            for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+                int64_t mi, ni;
+                sl_tile(g, t, mi, ni);
+                if (!sl_ok(g, mi, ni)) continue;
+                for (int s = 0; s < nst; ++s, ++it) {
+                    const uint32_t slot = it % kSlStages;
+                    if (it >= kSlStages && !mbar_wait(&empty[slot], (it / kSlStages - 1) & 1)) {
+                        ok = false;
+                        break;
+                    }
+                    uint8_t* st = base + slot * kSlStageBytes;
+                    mbar_expect_tx(&full[slot], (uint32_t)kSlStageBytes);
+                    sl_tma_3d(st, &mA, &full[slot], s * kSlK, (int)(mi * kSlM));
+                    sl_tma_3d(st + kSlABytes, &mB, &full[slot], s * kSlK, (int)(ni * kSlN));
+                }
+            }
+            if (!ok) atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
+            // the last loads must have landed before the CTA leaves
+            for (uint32_t q = it > kSlStages ? it - kSlStages : 0; q < it; ++q)
+                mbar_wait(&full[q % kSlStages], (q / kSlStages) & 1);
+        }
+    } else if (warp == kSlEpiWarps + 1) {
+        // products
+        if (lane == 0) {
+            uint32_t it = 0, ch = 0;
+            bool ok = true;
+            for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+                int64_t mi, ni;
+                sl_tile(g, t, mi, ni);
+                if (!sl_ok(g, mi, ni)) continue;
+                for (int s = 0; s < nst && ok; ++s, ++it) {
+                    const bool first = s % kSlChunk == 0;
+                    if (first && ch > 0) ok = mbar_wait(&acc_empty, (ch - 1) & 1);
+                    const uint32_t slot = it % kSlStages;
+                    ok = ok && mbar_wait(&full[slot], (it / kSlStages) & 1);
+                    if (!ok) break;
+                    sl_fence_after();
+                    const uint32_t a0 = smem_u32(base + slot * kSlStageBytes), b0 = a0 + kSlABytes;
+#pragma unroll
+                    for (int kk = 0; kk < kSlK / 16; ++kk) {
+                        const uint64_t bd = sw64_desc(b0 + kk * 32);
+#pragma unroll
+                        for (int i = 0; i < kSlices; ++i) {
+                            const uint64_t ad = sw64_desc(a0 + i * (kSlM * kSlK * 2) + kk * 32);
+                            const int cols = kSlN * (kSlices - i);
+                            const uint32_t acc = (first && kk == 0 && i == 0) ? 0u : 1u;
+                            const int n0 = cols < 256 ? cols : 256;
+                            sl_umma(tmem + kSlN * i, ad, bd, bf16_idesc(n0), acc);
+                            if (cols > 256)
+                                sl_umma(tmem + kSlN * i + 256, ad, bd + ((256 * kSlK * 2) >> 4),
+                                        bf16_idesc(cols - 256), acc);
+                        }
+                    }
+                    sl_commit(&empty[slot]);
+                    if (s % kSlChunk == kSlChunk - 1 || s == nst - 1) {
+                        sl_commit(&acc_full);
+                        ++ch;
+                    }
+                }
+            }
+            if (!ok) atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
+            // every product must be done before the tensor memory goes back
+            else if (ch > 0) mbar_wait(&acc_full, (ch - 1) & 1);
+        }
+    } else {
+        // eight warps: warp w drains lanes 32 (w % 4).. (rows of the tile) and
+        // columns 32 (w / 4).. of every accumulator
+        const int rl = (warp & 3) * 32 + lane, ch0 = (warp >> 2) * kSlCols;
+        const uint32_t tb = tmem + ((uint32_t)((warp & 3) * 32) << 16) + ch0;
+        uint32_t ch = 0;
+        bool ok = true;
+        for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+            int64_t mi, ni;
+            sl_tile(g, t, mi, ni);
+            const int64_t r = mi * kSlM + rl, col0 = ni * kSlN + ch0;
+            const bool in = r < g.M;
+            const int nc = (int)max((int64_t)0, min((int64_t)kSlCols, g.N - col0));
+            double* Cp = g.C + r + col0 * g.ldc;
+            if (!sl_ok(g, mi, ni)) {
+                // the FP64 pipe: a row and 8 columns of C at a time
+                for (int j0 = 0; in && j0 < nc; j0 += 8) {
+                    double acc[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) acc[q] = 0.0;
+                    for (int64_t k = 0; k < g.K; ++k) {
+                        const double av = g.A[r * g.asi + k * g.asj];
+#pragma unroll
+                        for (int q = 0; q < 8; ++q)
+                            if (j0 + q < nc) acc[q] = fma(av, __ldg(&g.B[k * g.bsi + (col0 + j0 + q) * g.bsj]), acc[q]);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (j0 + q < nc) {
+                            const double v = g.alpha * acc[q];
+                            double* cp = Cp + (j0 + q) * g.ldc;
+                            *cp = g.add ? v + *cp : v;
+                        }
+                }
+                __syncwarp();
+                continue;
+            }
+            const int ea = in ? __ldg(&g.ea[r]) : 0;
+            uint32_t t0[ONE ? 1 : kSlCols], t1[ONE ? 1 : kSlCols], t2[ONE ? 1 : kSlCols];
+            if constexpr (!ONE) {
+#pragma unroll
+                for (int j = 0; j < kSlCols; ++j) t0[j] = t1[j] = t2[j] = 0u;
+            }
+            auto store = [&](int j, uint32_t w0, uint32_t w1, uint32_t w2, double cold) {
+                const double v = sl_to_double(w0, w1, w2, ea + __ldg(&g.eb[col0 + j]));
+                double o;
+                // (a comparison of doubles would take the FP64 pipe)
+                if (!g.add) o = g.unit == 1 ? v : g.alpha * v;
+                else o = g.unit == 1 ? cold + v : g.unit == -1 ? cold - v : fma(g.alpha, v, cold);
+                Cp[j * g.ldc] = o;
+            };
+            for (int s = 0; s < nst; s += kSlChunk, ++ch) {
+                double cold[ONE ? kSlCols : 1];
+                if constexpr (ONE) {
+                    // C on its way while the products run
+#pragma unroll
+                    for (int j = 0; j < kSlCols; ++j)
+                        cold[j] = (in && j < nc && g.add) ? Cp[j * g.ldc] : 0.0;
+                }
+                ok = __all_sync(0xffffffffu, mbar_wait(&acc_full, ch & 1));
+                if (!ok) break;
+                sl_fence_after();
+#pragma unroll
+                for (int j = 0; j < kSlCols; j += 4) {
+                    uint32_t v[kSlices][4];
+                    __syncwarp();
+#pragma unroll
+                    for (int d = 0; d < kSlices; ++d) sl_ld4(tb + d * kSlN + j, v[d]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (j + 4 == kSlCols) {
+                        sl_fence_before();
+                        __syncwarp();
+                        if (lane == 0) sl_arrive(&acc_empty);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        uint32_t a[kSlices];
+#pragma unroll
+                        for (int d = 0; d < kSlices; ++d) a[d] = v[d][e];
+                        long long p, q;
+                        sl_combine(a, p, q);
+                        // (q) + (p << 32) into the 96-bit sum
+                        const uint32_t q0 = (uint32_t)q, q1 = (uint32_t)((unsigned long long)q >> 32);
+                        const uint32_t q2 = (uint32_t)((int)q1 >> 31);
+                        const uint32_t p0 = (uint32_t)p, p1 = (uint32_t)((unsigned long long)p >> 32);
+                        if constexpr (ONE) {
+                            uint32_t w1, w2;
+                            asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, %4, %5;" : "=r"(w1), "=r"(w2) : "r"(q1), "r"(p0), "r"(q2), "r"(p1));
+                            if (in && j + e < nc) store(j + e, q0, w1, w2, cold[j + e]);
+                        } else {
+                            asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
+                                : "+r"(t0[j + e]), "+r"(t1[j + e]), "+r"(t2[j + e])
+                                : "r"(q0), "r"(q1), "r"(q2));
+                            asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, %3;"
+                                : "+r"(t1[j + e]), "+r"(t2[j + e])
+                                : "r"(p0), "r"(p1));
+                        }
+                    }
+                }
+            }
+            if constexpr (!ONE) {
+                if (ok && in) {
+#pragma unroll
+                    for (int j = 0; j < kSlCols; ++j)
+                        if (j < nc) store(j, t0[j], t1[j], t2[j], g.add ? Cp[j * g.ldc] : 0.0);
+                }
+            }
+            __syncwarp();
+        }
+        if (!ok && lane == 0) atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
+    }
+    sl_fence_before();
+    __syncthreads();
+    if (warp == kSlEpiWarps) {
+        sl_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+
+static PFN_cuTensorMapEncodeTiled_v12000 sl_encode_fn()
+{
+    static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
+                cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+        cudaGetLastError();
+        return (PFN_cuTensorMapEncodeTiled_v12000) nullptr;
+    }();
+    return fn;
+}
+
+static bool sl_map(CUtensorMap* map, const SlicedOperand& s, int box_rows)
+{
+    auto fn = sl_encode_fn();
+    if (!fn) return false;
+    cuuint64_t dims[3] = {(cuuint64_t)s.Kp, (cuuint64_t)s.rows, (cuuint64_t)kSlices};
+    cuuint64_t strides[2] = {(cuuint64_t)s.Kp * 2, (cuuint64_t)s.rows * s.Kp * 2};
+    cuuint32_t box[3] = {(cuuint32_t)kSlK, (cuuint32_t)box_rows, (cuuint32_t)kSlices};
+    cuuint32_t estr[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, s.digits, dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+tmvg_status sliced_apply(Context* c, int64_t M, int64_t N, int64_t K, double alpha, Mat<const double> A,
+                         const SlicedOperand& sa, Mat<const double> B, const SlicedOperand& sb, double beta,
+                         double* C, int64_t ldc, int max_ctas)
+{
+    if (M <= 0 || N <= 0 || K <= 0) return TMVG_OK;
+    CUtensorMap mA, mB;
+    if (!sl_map(&mA, sa, kSlM) || !sl_map(&mB, sb, kSlN))
+        return set_error(c, TMVG_CUDA_ERROR, "sliced product: tensor map encoding failed");
+    SlicedArgs g;
+    g.M = M, g.N = N, g.K = K, g.alpha = alpha, g.add = beta != 0.0, g.unit = alpha == 1.0 ? 1 : alpha == -1.0 ? -1 : 0;
+    g.A = A.p, g.asi = A.si, g.asj = A.sj;
+    g.B = B.p, g.bsi = B.si, g.bsj = B.sj;
+    g.ea = sa.exps, g.eb = sb.exps, g.fa = sa.fill, g.fb = sb.fill, g.ga = sa.group, g.gb = sb.group;
+    g.need = (int)std::ceil(1.75 * std::sqrt((double)K));
+    g.C = C, g.ldc = ldc;
+    g.mt = ceil_div(M, (int64_t)kSlM), g.nt = ceil_div(N, (int64_t)kSlN);
+    const int64_t cap = max_ctas > 0 ? max_ctas : c->num_sms;
+    const unsigned grid = (unsigned)std::min<int64_t>(g.mt * g.nt, cap);
+    auto kern = ceil_div(K, (int64_t)kSlK) <= kSlChunk ? sliced_gemm_kernel<true> : sliced_gemm_kernel<false>;
+    tmvg_status st = check_cuda(
+        c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlSmem), "sliced product");
+    if (st) return st;
+    kern<<<grid, kSlThreads, kSlSmem, c->stream>>>(mA, mB, g, c->dflags);
+    ++c->launches;
+    return check_cuda(c, cudaGetLastError(), "sliced product launch");
+}
+
+void* scratch_alloc(Context* c, size_t bytes, cudaStream_t s)
+{
+    if (!c->pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = c->device;
+        if (cudaMemPoolCreate(&c->pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            c->pool = nullptr;
+            return nullptr;
+        }
+        uint64_t keep = 1ull << 30;
+        cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    void* p = nullptr;
+    if (cudaMallocFromPoolAsync(&p, bytes, c->pool, s) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return p;
+}
+
+void scratch_free(void* p, cudaStream_t s)
+{
+    if (p && cudaFreeAsync(p, s) != cudaSuccess) cudaGetLastError();
+}
+
+bool sliced_wanted(Context* c, int64_t M, int64_t N, int64_t K)
+{
+    if (M < 64 || N < 48 || K < 24 || M > INT_MAX / 2 || N > INT_MAX / 2) return false;
+    if ((double)M * (double)N * (double)K < 1.2e7) return false;
+    if (!sl_encode_fn()) return false;
+    // a captured stream keeps the FP64 pipe: its graph would hold scratch of
+    // the pool
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return cap == cudaStreamCaptureStatusNone;
+}
+
+tmvg_status sliced_gemm(Context* c, int64_t M, int64_t N, int64_t K, double alpha, Mat<const double> A,
+                        Mat<const double> B, double beta, double* C, int64_t ldc)
+{
+    // blocks of at most 256 MiB of digits per operand
+    constexpr int64_t kMaxK = 16384;
+    const int64_t kb = std::min(K, kMaxK);
+    const int64_t cap = std::max<int64_t>(kSlM, (((int64_t)1 << 28) / (2 * kSlices * (kb + kSlK))) / kSlM * kSlM);
+    const int64_t mb = std::min(M, cap), nb = std::min(N, cap);
+    const size_t ba = (sliced_bytes(mb, kb) + 255) & ~size_t(255);
+    unsigned char* ws = (unsigned char*)scratch_alloc(c, ba + sliced_bytes(nb, kb), c->stream);
+    if (!ws) return TMVG_UNSUPPORTED;
+    tmvg_status st = TMVG_OK;
+    for (int64_t k0 = 0; k0 < K && !st; k0 += kb) {
+        const int64_t k = std::min(kb, K - k0);
+        for (int64_t i0 = 0; i0 < M && !st; i0 += mb) {
+            const int64_t m = std::min(mb, M - i0);
+            const Mat<const double> a{A.p + i0 * A.si + k0 * A.sj, A.si, A.sj};
+            const SlicedOperand sa = sliced_layout(ws, m, k);
+            for (int64_t j0 = 0; j0 < N && !st; j0 += nb) {
+                const int64_t n = std::min(nb, N - j0);
+                const Mat<const double> b{B.p + k0 * B.si + j0 * B.sj, B.si, B.sj};
+                const SlicedOperand sb = sliced_layout(ws + ba, n, k);
+                SlicedOperand one = sa;
+                if (j0 > 0) one.rows = 0;  // A's block is sliced already
+                st = sliced_split(c, k, a, one, b, sb);
+                if (!st)
+                    st = sliced_apply(c, m, n, k, alpha, a, sa, b, sb, k0 > 0 ? 1.0 : beta, C + i0 + j0 * ldc, ldc);
+            }
+        }
+    }
+    scratch_free(ws, c->stream);
+    return st;
+}
+
+}  // namespace tmvg

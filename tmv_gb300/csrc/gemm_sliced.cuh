@@ -1,0 +1,48 @@
+// gemm_sliced.cuh -- FP64 products on the tcgen05 tensor cores from exact
+// 8-bit slices of the operands (gemm_sliced.cu).
+#pragma once
+
+#include "gemm.cuh"
+
+namespace tmvg {
+
+// One sliced operand: `rows` vectors of length K (the rows of A, or the
+// columns of B), each scaled by its own power of two.
+struct SlicedOperand {
+    uint16_t* digits = nullptr;  // [kSlices][rows][Kp] bf16 integers, K contiguous
+    int* exps = nullptr;         // per vector: every |entry| < 2^exps
+    int* fill = nullptr;         // per group of vectors: fewest entries within 2^-4 of the largest
+    int64_t rows = 0, Kp = 0;
+    int group = 16;              // vectors per fill group
+};
+
+// Bytes of a sliced operand and its layout in a buffer of that size.
+size_t sliced_bytes(int64_t rows, int64_t K);
+SlicedOperand sliced_layout(void* buf, int64_t rows, int64_t K);
+
+// Slices the rows of A (M x K) and the columns of B (K x N) in one launch on
+// c->stream; either may be left out (rows == 0).
+tmvg_status sliced_split(Context* c, int64_t K, Mat<const double> A, const SlicedOperand& sa,
+                         Mat<const double> B, const SlicedOperand& sb);
+
+// C (M x N, column-major) = alpha A B + beta C (beta 0 or 1) from the slices;
+// A and B themselves are read only where a tile's range of magnitudes needs
+// the FP64 pipe.  `max_ctas` bounds the persistent grid (0: one per SM).
+tmvg_status sliced_apply(Context* c, int64_t M, int64_t N, int64_t K, double alpha, Mat<const double> A,
+                         const SlicedOperand& sa, Mat<const double> B, const SlicedOperand& sb, double beta,
+                         double* C, int64_t ldc, int max_ctas = 0);
+
+// Whether a product of this size is faster sliced than on the FP64 pipe.
+bool sliced_wanted(Context* c, int64_t M, int64_t N, int64_t K);
+
+// The whole product; TMVG_UNSUPPORTED (with nothing launched) where the
+// workspace or the tensor-map encoder is not to be had.
+tmvg_status sliced_gemm(Context* c, int64_t M, int64_t N, int64_t K, double alpha, Mat<const double> A,
+                        Mat<const double> B, double beta, double* C, int64_t ldc);
+
+// Stream-ordered scratch from the context's own pool (bounded: what a
+// synchronisation finds unused above 1 GiB goes back to the device).
+void* scratch_alloc(Context* c, size_t bytes, cudaStream_t s);
+void scratch_free(void* p, cudaStream_t s);
+
+}  // namespace tmvg
