@@ -7,8 +7,8 @@ digit pairs left out and the digits' last rounding are below K (7 + 2) 2^-64 of
 the product of the row's and the column's scale (powers of two above their
 largest entries), i.e. K 2^-60, and the result is rounded once (2^-53 of it),
 with a rounding for alpha and one for the sum with C.  A tile (128 x 64) whose
-rows and columns cannot be shown to overlap in their large entries runs as a
-chain of FMAs: K 2^-53 |A||B|; which tiles those are is worked out here."""
+rows and columns do not overlap in their large entries runs as a chain of FMAs:
+K 2^-53 |A||B|; the tiles that certainly do overlap are worked out here."""
 import numpy as np
 import pytest
 
@@ -75,7 +75,7 @@ def test_exact_integers(dev, m, n, k, la, lb, lc, spread):
         got = _run(dev, a.astype(float), b.astype(float), c0, add, alpha, la, lb, lc)[np.ix_(pick_r, pick_c)]
         want = exact.astype(float) * alpha + (c0[np.ix_(pick_r, pick_c)] if add else 0.0)
         size = np.abs(exact.astype(float)) + (np.abs(c0[np.ix_(pick_r, pick_c)]) if add else 0.0)
-        tol = np.where(tile, k * 2.0 ** -60 * scale, chain) + 2.0 ** -51 * size
+        tol = np.where(tile, k * 2.0 ** -60 * scale, np.maximum(chain, k * 2.0 ** -60 * scale)) + 2.0 ** -51 * size
         assert (np.abs(got - want) <= tol).all()
 
 
@@ -95,6 +95,12 @@ def test_special_operands(dev, k):
     assert np.array_equal(got[~fin & ~np.isnan(want)], want[~fin & ~np.isnan(want)])
     lim = k * 2.0 ** -52 * (np.abs(np.nan_to_num(a, posinf=0, neginf=0)) @ np.abs(np.nan_to_num(b, posinf=0, neginf=0)))
     assert (np.abs(got - want)[fin] <= lim[fin]).all()
+    # zero rows and columns among ordinary ones are exactly zero
+    x, y = rng.standard_normal((m, k)), rng.standard_normal((k, n))
+    x[130:135], y[:, 70] = 0.0, 0.0
+    got = _run(dev, x, y, np.zeros((m, n)), False, 1.0, "F", "F", "F")
+    assert (got[130:135] == 0).all() and (got[:, 70] == 0).all()
+    assert (np.abs(got - x @ y) <= k * 2.0 ** -52 * (np.abs(x) @ np.abs(y))).all()
     # graded against each other: every product is about 1, each entry's own
     # size from 1 to 2^40 of its vector's largest; and a sparse pair; both to
     # the componentwise bound of an FMA chain, K 2^-53 |A||B|

@@ -16,11 +16,16 @@
 // Accuracy: an element's error is about 2^-64 sqrt(K) times (row maximum of A
 // x column maximum of B), against 2^-54 of sum |a||b| for a chain of FMAs.
 // That is smaller unless the row's and the column's large entries do not
-// meet, so the slicing kernel counts, per vector, the entries within 2^-4 of
-// the largest; where the fewest of a tile's rows and columns cannot overlap
-// in 1.75 sqrt(K) places (pigeonhole), or an entry is not finite or its
-// vector's scale is extreme, the tile's CTA takes the FP64 pipe instead, on
-// the unsliced operands, with the FMA chain of gemm_simt_kernel.
+// meet, i.e. unless sum |a||b| < 2^-9 sqrt(K) of that product of maxima.  Two
+// looks decide that before a tile is multiplied: the slicing kernel counts,
+// per vector, the entries within 2^-4 of the largest, and where the fewest of
+// the tile's rows and columns must overlap in 1.75 sqrt(K) places (pigeonhole)
+// the tile is good; otherwise the CTA sums the products of the leading digits'
+// moduli, which ends as soon as every element has passed.  A tile that fails
+// both, or has an entry that is not finite or a vector of extreme scale, takes
+// the FP64 pipe on the unsliced operands, with the FMA chain of
+// gemm_simt_kernel (65 us for K = 32 against 5: the second look keeps tiles of
+// ordinary data, of which one in some thousand fails the first, off it).
 //
 // Data flow per CTA (persistent over 128 x 64 tiles of C): one thread loads
 // stages of K = 32 (8 digits x (128 + 64) rows x 64 bytes = 96 KB, two
@@ -28,7 +33,7 @@
 // digit i of A with digits 0..7-i of B at once (they lie behind one another
 // in shared memory, and so do their accumulators in the 512 TMEM columns:
 // N = 64 (8 - i), in pieces of up to 256, so that A is read once per 256
-// columns); eight warps drain the accumulators after every K = 128.
+// columns); sixteen warps drain the accumulators after every K = 128.
 // All waits are bounded; on a timeout the kernel records kDevTimeout.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -51,11 +56,14 @@ constexpr int kSlABytes = kSlices * kSlM * kSlK * 2;
 constexpr int kSlBBytes = kSlices * kSlN * kSlK * 2;
 constexpr int kSlStageBytes = kSlABytes + kSlBBytes;
 constexpr size_t kSlSmem = (size_t)kSlStages * kSlStageBytes + 1024;
-constexpr int kSlEpiWarps = 8;
+constexpr int kSlEpiWarps = 16;  // 4 per scheduler: the epilogue is bound by latencies
 constexpr int kSlThreads = 32 * (kSlEpiWarps + 2);
-constexpr int kSlCols = kSlN / 2;       // columns of C per epilogue thread
+static_assert(kSlM / 16 * kSlN == 32 * kSlEpiWarps, "a prefetch per epilogue thread");
+constexpr int kSlCols = kSlN / (kSlEpiWarps / 4);  // columns of C per epilogue thread
 constexpr int kFillBad = -(1 << 29);    // fill count of a group that cannot be sliced
 constexpr int kFillRange = 4;           // entries within 2^-4 of the vector's largest count
+constexpr int kZeroExp = -(1 << 20);    // scale exponent of a zero vector
+constexpr int kMaxTilesPerCta = 16384;
 constexpr int kExpLimit = 450;          // |scale exponent| beyond this takes the FP64 pipe
 
 size_t sliced_bytes(int64_t rows, int64_t K)
@@ -185,9 +193,9 @@ sliced_split_kernel(SplitSide sa, SplitSide sb, int64_t groups_a, int64_t K)
     if (tid < R && grp * R + tid < s.rows) {
         const int ee = s_emax[tid];  // exponent field: |entries| < 2^(ee - 1022)
         int b = s_big[tid];
-        const int sc = ee == 0 ? 0 : ee - 1022;
-        if (ee == 0x7ff || sc > kExpLimit || sc < -kExpLimit) b = kFillBad;
-        else if (ee == 0) b = INT_MAX / 4;  // a zero vector: every product is exactly zero (see below)
+        const int sc = ee == 0 ? kZeroExp : ee - 1022;
+        if (ee == 0) b = INT_MAX / 4;  // a zero vector: every product is exactly zero (but see below)
+        else if (ee == 0x7ff || sc > kExpLimit || sc < -kExpLimit) b = kFillBad;
         s.exps[grp * R + tid] = sc;
         atomicMin(&s_min, b);
     }
@@ -304,30 +312,31 @@ __device__ __forceinline__ void sl_combine(const uint32_t (&a)[kSlices], long lo
 }
 
 // The 96-bit integer (w2:w1:w0) 2^(e - 62) rounded to FP64 (nearest; a tie
-// goes away from zero).
+// goes away from zero), on the integer pipe and without branches.
 __device__ __forceinline__ double sl_to_double(uint32_t w0, uint32_t w1, uint32_t w2, int e)
 {
     const uint32_t sgn = (uint32_t)((int)w2 >> 31);
-    unsigned long long lo = ((unsigned long long)w1 << 32) | w0;
-    lo = (lo ^ (((unsigned long long)sgn << 32) | sgn)) + (sgn & 1u);
-    uint32_t hi = (w2 ^ sgn) + ((sgn && lo == 0ull) ? 1u : 0u);
-    // left-align the top 64 bits
-    unsigned long long top;
-    int msb;  // position of the leading bit
-    if (hi) {
-        const int lz = __clz(hi);
-        msb = 95 - lz;
-        top = ((unsigned long long)hi << 32) | (lo >> 32);
-        if (lz) top = (top << lz) | ((uint32_t)lo >> (32 - lz));
-    } else {
-        if (lo == 0ull) return 0.0;
-        const int lz = __clzll((long long)lo);
-        msb = 63 - lz;
-        top = lo << lz;
+    uint32_t a, m, l;  // |w|
+    asm("sub.cc.u32 %0, %3, %6;\n\tsubc.cc.u32 %1, %4, %6;\n\tsubc.u32 %2, %5, %6;"
+        : "=r"(l), "=r"(m), "=r"(a)
+        : "r"(w0 ^ sgn), "r"(w1 ^ sgn), "r"(w2 ^ sgn), "r"(sgn));
+    int msb = 95;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {  // the leading word into a
+        const bool z = a == 0u;
+        a = z ? m : a;
+        m = z ? l : m;
+        l = z ? 0u : l;
+        msb -= z ? 32 : 0;
     }
-    const unsigned long long mant = (top >> 11) + ((top >> 10) & 1ull);
-    const unsigned long long bits = ((unsigned long long)(msb + e - 62 + 1023 - 1) << 52) + mant;
-    return __longlong_as_double((long long)(bits | ((unsigned long long)(sgn & 0x80000000u) << 32)));
+    const int lz = __clz((int)a);
+    const uint32_t hi = __funnelshift_l(m, a, lz), lo = __funnelshift_l(l, m, lz);
+    msb -= lz;
+    const unsigned long long top = ((unsigned long long)hi << 32) | lo;
+    const unsigned long long mant = (top >> 11) + ((lo >> 10) & 1u);
+    const unsigned long long bits = ((unsigned long long)(uint32_t)(msb + e - 62 + 1023 - 1) << 52) + mant;
+    const unsigned long long r = bits | ((unsigned long long)(sgn & 0x80000000u) << 32);
+    return __longlong_as_double((long long)(a ? r : 0ull));
 }
 
 struct SlicedArgs {
@@ -339,7 +348,10 @@ struct SlicedArgs {
     int64_t asi, asj, bsi, bsj;
     const int *ea, *eb, *fa, *fb;
     int ga, gb;                      // vectors per fill group
-    int need;                        // overlap that a sliced tile needs
+    int need;                        // first look: overlap that a sliced tile needs
+    float need_sum;                  // second look: sum of leading digits' products
+    const uint16_t *da, *db;         // leading digits, K contiguous (stride Kp)
+    int64_t Kp;
     double* C;
     int64_t ldc;
     int64_t mt, nt;                  // tiles
@@ -356,19 +368,57 @@ __device__ __forceinline__ void sl_tile(const SlicedArgs& g, int64_t t, int64_t&
     ni = rem / h;
 }
 
-// Whether the tile's operands may be sliced (every caller gets one answer).
-__device__ __forceinline__ bool sl_ok(const SlicedArgs& g, int64_t mi, int64_t ni)
+// First look at a tile: 1 good, 0 undecided, -1 for the FP64 pipe.
+__device__ __forceinline__ int sl_look(const SlicedArgs& g, int64_t mi, int64_t ni)
 {
     int a = INT_MAX / 4, b = INT_MAX / 4;
     const int64_t a1 = min((g.M - 1) / g.ga, (mi * kSlM + kSlM - 1) / g.ga);
     const int64_t b1 = min((g.N - 1) / g.gb, (ni * kSlN + kSlN - 1) / g.gb);
     for (int64_t i = mi * kSlM / g.ga; i <= a1; ++i) a = min(a, __ldg(&g.fa[i]));
     for (int64_t i = ni * kSlN / g.gb; i <= b1; ++i) b = min(b, __ldg(&g.fb[i]));
-    return (int64_t)a + b - g.K >= g.need;
+    if (a < 0 || b < 0) return -1;
+    return (int64_t)a + b - g.K >= g.need ? 1 : 0;
 }
 
-// ONE: K fits one accumulation chunk, so nothing is carried between chunks.
-template <bool ONE>
+// Second look (the whole CTA): the sum of |leading digit of a| |leading digit
+// of b| over K reaches need_sum for every element, or the element's row or
+// column is zero.
+__device__ __noinline__ bool sl_look_again(const SlicedArgs& g, int64_t mi, int64_t ni)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool work = warp < kSlEpiWarps;
+    const int64_t r = mi * kSlM + (warp & 3) * 32 + lane;
+    const int64_t c0 = ni * kSlN + (int64_t)(warp >> 2) * kSlCols;
+    const int nc = work ? (int)max((int64_t)0, min((int64_t)kSlCols, g.N - c0)) : 0;
+    bool pass = !work || r >= g.M || __ldg(&g.ea[r]) == kZeroExp;
+    unsigned todo = pass ? 0u : (1u << nc) - 1u;
+    float sum[kSlCols];
+#pragma unroll
+    for (int j = 0; j < kSlCols; ++j) sum[j] = 0.0f;
+    for (int64_t k = 0; k < g.Kp; k += 8) {
+        if (todo) {
+            const uint4 av = *reinterpret_cast<const uint4*>(g.da + r * g.Kp + k);
+            const uint32_t aw[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+            for (int j = 0; j < kSlCols; ++j) {
+                if (j < nc) {
+                    const uint4 bv = *reinterpret_cast<const uint4*>(g.db + (c0 + j) * g.Kp + k);
+                    const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        sum[j] = fmaf(__uint_as_float((aw[q] << 16) & 0x7fffffffu),
+                                      __uint_as_float((bw[q] << 16) & 0x7fffffffu), sum[j]);
+                        sum[j] = fmaf(__uint_as_float(aw[q] & 0x7fff0000u), __uint_as_float(bw[q] & 0x7fff0000u), sum[j]);
+                    }
+                    if (sum[j] >= g.need_sum || __ldg(&g.eb[c0 + j]) == kZeroExp) todo &= ~(1u << j);
+                }
+            }
+        }
+        if (__syncthreads_and(todo == 0u)) return true;
+    }
+    return false;
+}
+
 __global__ void __launch_bounds__(kSlThreads, 1)
 sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB,
                    const __grid_constant__ SlicedArgs g, int* err)
@@ -378,6 +428,8 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
                                                ~static_cast<uintptr_t>(1023));
     __shared__ __align__(8) uint64_t full[kSlStages], empty[kSlStages], acc_full, acc_empty;
     __shared__ uint32_t s_tmem;
+    __shared__ uint32_t s_ok[kMaxTilesPerCta / 32];
+    __shared__ int s_open;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
     if (warp == kSlEpiWarps) {
@@ -391,6 +443,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
+        s_open = 0;
         mbar_init(&acc_full, 1);
         mbar_init(&acc_empty, kSlEpiWarps);
         mbar_fence_init();
@@ -402,15 +455,44 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
     const int nst = (int)((g.K + kSlK - 1) / kSlK);
     const int64_t tiles = g.mt * g.nt;
 
+    // which of this CTA's tiles are sliced, before the warps part
+    const int mine = (int)((tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
+    for (int i0 = warp * 32; i0 < mine; i0 += kSlThreads) {
+        int64_t mi, ni;
+        int look = 1;
+        if (i0 + lane < mine) {
+            sl_tile(g, blockIdx.x + (int64_t)(i0 + lane) * gridDim.x, mi, ni);
+            look = sl_look(g, mi, ni);
+        }
+        const unsigned good = __ballot_sync(0xffffffffu, look == 1), open = __ballot_sync(0xffffffffu, look == 0);
+        if (lane == 0) {
+            s_ok[i0 >> 5] = good;
+            if (open) s_open = 1;
+        }
+    }
+    __syncthreads();
+    if (s_open) {
+        for (int i = 0; i < mine; ++i) {
+            if ((s_ok[i >> 5] >> (i & 31)) & 1u) continue;
+            int64_t mi, ni;
+            sl_tile(g, blockIdx.x + (int64_t)i * gridDim.x, mi, ni);
+            const bool again = sl_look(g, mi, ni) == 0 && sl_look_again(g, mi, ni);
+            __syncthreads();  // every thread has read the word
+            if (again && tid == 0) s_ok[i >> 5] |= 1u << (i & 31);
+            __syncthreads();
+        }
+    }
+    auto sliced = [&](int i) { return ((s_ok[i >> 5] >> (i & 31)) & 1u) != 0u; };
+
     if (warp == kSlEpiWarps) {
         // operands by TMA
         if (lane == 0) {
             uint32_t it = 0;
             bool ok = true;
-            for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+            for (int i = 0; i < mine && ok; ++i) {
+                if (!sliced(i)) continue;
                 int64_t mi, ni;
-                sl_tile(g, t, mi, ni);
-                if (!sl_ok(g, mi, ni)) continue;
+                sl_tile(g, blockIdx.x + (int64_t)i * gridDim.x, mi, ni);
                 for (int s = 0; s < nst; ++s, ++it) {
                     const uint32_t slot = it % kSlStages;
                     if (it >= kSlStages && !mbar_wait(&empty[slot], (it / kSlStages - 1) & 1)) {
@@ -433,10 +515,10 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
         if (lane == 0) {
             uint32_t it = 0, ch = 0;
             bool ok = true;
-            for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+            for (int i = 0; i < mine && ok; ++i) {
+                if (!sliced(i)) continue;
                 int64_t mi, ni;
-                sl_tile(g, t, mi, ni);
-                if (!sl_ok(g, mi, ni)) continue;
+                sl_tile(g, blockIdx.x + (int64_t)i * gridDim.x, mi, ni);
                 for (int s = 0; s < nst && ok; ++s, ++it) {
                     const bool first = s % kSlChunk == 0;
                     if (first && ch > 0) ok = mbar_wait(&acc_empty, (ch - 1) & 1);
@@ -449,14 +531,14 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
                     for (int kk = 0; kk < kSlK / 16; ++kk) {
                         const uint64_t bd = sw64_desc(b0 + kk * 32);
 #pragma unroll
-                        for (int i = 0; i < kSlices; ++i) {
-                            const uint64_t ad = sw64_desc(a0 + i * (kSlM * kSlK * 2) + kk * 32);
-                            const int cols = kSlN * (kSlices - i);
-                            const uint32_t acc = (first && kk == 0 && i == 0) ? 0u : 1u;
+                        for (int d = 0; d < kSlices; ++d) {
+                            const uint64_t ad = sw64_desc(a0 + d * (kSlM * kSlK * 2) + kk * 32);
+                            const int cols = kSlN * (kSlices - d);
+                            const uint32_t acc = (first && kk == 0 && d == 0) ? 0u : 1u;
                             const int n0 = cols < 256 ? cols : 256;
-                            sl_umma(tmem + kSlN * i, ad, bd, bf16_idesc(n0), acc);
+                            sl_umma(tmem + kSlN * d, ad, bd, bf16_idesc(n0), acc);
                             if (cols > 256)
-                                sl_umma(tmem + kSlN * i + 256, ad, bd + ((256 * kSlK * 2) >> 4),
+                                sl_umma(tmem + kSlN * d + 256, ad, bd + ((256 * kSlK * 2) >> 4),
                                         bf16_idesc(cols - 256), acc);
                         }
                     }
@@ -472,20 +554,20 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
             else if (ch > 0) mbar_wait(&acc_full, (ch - 1) & 1);
         }
     } else {
-        // eight warps: warp w drains lanes 32 (w % 4).. (rows of the tile) and
-        // columns 32 (w / 4).. of every accumulator
+        // sixteen warps: warp w drains lanes 32 (w % 4).. (rows of the tile) and
+        // columns 16 (w / 4).. of every accumulator
         const int rl = (warp & 3) * 32 + lane, ch0 = (warp >> 2) * kSlCols;
         const uint32_t tb = tmem + ((uint32_t)((warp & 3) * 32) << 16) + ch0;
         uint32_t ch = 0;
         bool ok = true;
-        for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+        for (int i = 0; i < mine && ok; ++i) {
             int64_t mi, ni;
-            sl_tile(g, t, mi, ni);
+            sl_tile(g, blockIdx.x + (int64_t)i * gridDim.x, mi, ni);
             const int64_t r = mi * kSlM + rl, col0 = ni * kSlN + ch0;
             const bool in = r < g.M;
             const int nc = (int)max((int64_t)0, min((int64_t)kSlCols, g.N - col0));
             double* Cp = g.C + r + col0 * g.ldc;
-            if (!sl_ok(g, mi, ni)) {
+            if (!sliced(i)) {
                 // the FP64 pipe: a row and 8 columns of C at a time
                 for (int j0 = 0; in && j0 < nc; j0 += 8) {
                     double acc[8];
@@ -508,28 +590,27 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
                 __syncwarp();
                 continue;
             }
+            // this row's scale, and a column's per lane; C's first columns on
+            // their way while the products run
             const int ea = in ? __ldg(&g.ea[r]) : 0;
-            uint32_t t0[ONE ? 1 : kSlCols], t1[ONE ? 1 : kSlCols], t2[ONE ? 1 : kSlCols];
-            if constexpr (!ONE) {
+            const int ebl = lane < nc ? __ldg(&g.eb[col0 + lane]) : 0;
+            constexpr int CB = 8;
+            double cold[CB];
+            const bool add = g.add != 0;
 #pragma unroll
-                for (int j = 0; j < kSlCols; ++j) t0[j] = t1[j] = t2[j] = 0u;
+            for (int q = 0; q < CB; ++q) cold[q] = (add && in && q < nc) ? Cp[q * g.ldc] : 0.0;
+            if (add && i + 1 < mine) {
+                // the next tile of C into L2: a line of 16 rows per thread
+                int64_t mx, nx;
+                sl_tile(g, blockIdx.x + (int64_t)(i + 1) * gridDim.x, mx, nx);
+                const int64_t rx = mx * kSlM + 16 * (tid & 7), cx = nx * kSlN + (tid >> 3);
+                if (rx < g.M && cx < g.N)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(g.C + rx + cx * g.ldc));
             }
-            auto store = [&](int j, uint32_t w0, uint32_t w1, uint32_t w2, double cold) {
-                const double v = sl_to_double(w0, w1, w2, ea + __ldg(&g.eb[col0 + j]));
-                double o;
-                // (a comparison of doubles would take the FP64 pipe)
-                if (!g.add) o = g.unit == 1 ? v : g.alpha * v;
-                else o = g.unit == 1 ? cold + v : g.unit == -1 ? cold - v : fma(g.alpha, v, cold);
-                Cp[j * g.ldc] = o;
-            };
-            for (int s = 0; s < nst; s += kSlChunk, ++ch) {
-                double cold[ONE ? kSlCols : 1];
-                if constexpr (ONE) {
-                    // C on its way while the products run
+            uint32_t t0[kSlCols], t1[kSlCols], t2[kSlCols];
 #pragma unroll
-                    for (int j = 0; j < kSlCols; ++j)
-                        cold[j] = (in && j < nc && g.add) ? Cp[j * g.ldc] : 0.0;
-                }
+            for (int j = 0; j < kSlCols; ++j) t0[j] = t1[j] = t2[j] = 0u;
+            for (int s = 0; s < nst; s += kSlChunk, ++ch) {
                 ok = __all_sync(0xffffffffu, mbar_wait(&acc_full, ch & 1));
                 if (!ok) break;
                 sl_fence_after();
@@ -541,6 +622,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
                     for (int d = 0; d < kSlices; ++d) sl_ld4(tb + d * kSlN + j, v[d]);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (j + 4 == kSlCols) {
+                        // drained: the next products may start
                         sl_fence_before();
                         __syncwarp();
                         if (lane == 0) sl_arrive(&acc_empty);
@@ -552,31 +634,40 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
                         for (int d = 0; d < kSlices; ++d) a[d] = v[d][e];
                         long long p, q;
                         sl_combine(a, p, q);
-                        // (q) + (p << 32) into the 96-bit sum
+                        // q + (p << 32) into the 96-bit sum
                         const uint32_t q0 = (uint32_t)q, q1 = (uint32_t)((unsigned long long)q >> 32);
-                        const uint32_t q2 = (uint32_t)((int)q1 >> 31);
                         const uint32_t p0 = (uint32_t)p, p1 = (uint32_t)((unsigned long long)p >> 32);
-                        if constexpr (ONE) {
-                            uint32_t w1, w2;
-                            asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, %4, %5;" : "=r"(w1), "=r"(w2) : "r"(q1), "r"(p0), "r"(q2), "r"(p1));
-                            if (in && j + e < nc) store(j + e, q0, w1, w2, cold[j + e]);
-                        } else {
-                            asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
-                                : "+r"(t0[j + e]), "+r"(t1[j + e]), "+r"(t2[j + e])
-                                : "r"(q0), "r"(q1), "r"(q2));
-                            asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, %3;"
-                                : "+r"(t1[j + e]), "+r"(t2[j + e])
-                                : "r"(p0), "r"(p1));
-                        }
+                        asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
+                            : "+r"(t0[j + e]), "+r"(t1[j + e]), "+r"(t2[j + e])
+                            : "r"(q0), "r"(q1), "r"((uint32_t)((int)q1 >> 31)));
+                        asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, %3;"
+                            : "+r"(t1[j + e]), "+r"(t2[j + e])
+                            : "r"(p0), "r"(p1));
                     }
                 }
             }
-            if constexpr (!ONE) {
-                if (ok && in) {
+            if (!ok) break;
+            // rounded and into C, the next columns of C loaded ahead
 #pragma unroll
-                    for (int j = 0; j < kSlCols; ++j)
-                        if (j < nc) store(j, t0[j], t1[j], t2[j], g.add ? Cp[j * g.ldc] : 0.0);
+            for (int j0 = 0; j0 < kSlCols; j0 += CB) {
+                double next[CB];
+                if (j0 + CB < kSlCols) {
+#pragma unroll
+                    for (int q = 0; q < CB; ++q)
+                        next[q] = (add && in && j0 + CB + q < nc) ? Cp[(j0 + CB + q) * g.ldc] : 0.0;
                 }
+#pragma unroll
+                for (int q = 0; q < CB; ++q) {
+                    const int j = j0 + q;
+                    const double v = sl_to_double(t0[j], t1[j], t2[j], ea + __shfl_sync(0xffffffffu, ebl, j));
+                    double o;
+                    // (a comparison of doubles would take the FP64 pipe)
+                    if (!add) o = g.unit == 1 ? v : g.alpha * v;
+                    else o = g.unit == 1 ? cold[q] + v : g.unit == -1 ? cold[q] - v : fma(g.alpha, v, cold[q]);
+                    if (in && j < nc) Cp[j * g.ldc] = o;
+                }
+#pragma unroll
+                for (int q = 0; q < CB; ++q) cold[q] = next[q];
             }
             __syncwarp();
         }
@@ -631,16 +722,21 @@ tmvg_status sliced_apply(Context* c, int64_t M, int64_t N, int64_t K, double alp
     g.A = A.p, g.asi = A.si, g.asj = A.sj;
     g.B = B.p, g.bsi = B.si, g.bsj = B.sj;
     g.ea = sa.exps, g.eb = sb.exps, g.fa = sa.fill, g.fb = sb.fill, g.ga = sa.group, g.gb = sb.group;
+    // sum |a||b| of at least 2^-9.2 sqrt(K) of the product of the scales: an
+    // entry within 2^-4 of its vector's largest is at least 2^-5 of the scale;
+    // a leading digit d (of 2^7) stands for at least d / 2
     g.need = (int)std::ceil(1.75 * std::sqrt((double)K));
+    g.need_sum = (float)(112.0 * std::sqrt((double)K));
+    g.da = sa.digits, g.db = sb.digits, g.Kp = sa.Kp;
     g.C = C, g.ldc = ldc;
     g.mt = ceil_div(M, (int64_t)kSlM), g.nt = ceil_div(N, (int64_t)kSlN);
     const int64_t cap = max_ctas > 0 ? max_ctas : c->num_sms;
     const unsigned grid = (unsigned)std::min<int64_t>(g.mt * g.nt, cap);
-    auto kern = ceil_div(K, (int64_t)kSlK) <= kSlChunk ? sliced_gemm_kernel<true> : sliced_gemm_kernel<false>;
     tmvg_status st = check_cuda(
-        c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlSmem), "sliced product");
+        c, cudaFuncSetAttribute(sliced_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlSmem),
+        "sliced product");
     if (st) return st;
-    kern<<<grid, kSlThreads, kSlSmem, c->stream>>>(mA, mB, g, c->dflags);
+    sliced_gemm_kernel<<<grid, kSlThreads, kSlSmem, c->stream>>>(mA, mB, g, c->dflags);
     ++c->launches;
     return check_cuda(c, cudaGetLastError(), "sliced product launch");
 }
@@ -689,13 +785,15 @@ bool sliced_wanted(Context* c, int64_t M, int64_t N, int64_t K)
 }
 
 tmvg_status sliced_gemm(Context* c, int64_t M, int64_t N, int64_t K, double alpha, Mat<const double> A,
-                        Mat<const double> B, double beta, double* C, int64_t ldc)
+                        Mat<const double> B, double beta, double* C, int64_t ldc, int max_ctas)
 {
     // blocks of at most 256 MiB of digits per operand
     constexpr int64_t kMaxK = 16384;
     const int64_t kb = std::min(K, kMaxK);
     const int64_t cap = std::max<int64_t>(kSlM, (((int64_t)1 << 28) / (2 * kSlices * (kb + kSlK))) / kSlM * kSlM);
-    const int64_t mb = std::min(M, cap), nb = std::min(N, cap);
+    const int64_t mb = std::min(M, cap);
+    const int64_t nb = std::min(std::min(N, cap), std::max<int64_t>(1, kMaxTilesPerCta / ceil_div(mb, (int64_t)kSlM)) *
+                                                      kSlN * (max_ctas > 0 ? max_ctas : c->num_sms));
     const size_t ba = (sliced_bytes(mb, kb) + 255) & ~size_t(255);
     unsigned char* ws = (unsigned char*)scratch_alloc(c, ba + sliced_bytes(nb, kb), c->stream);
     if (!ws) return TMVG_UNSUPPORTED;
@@ -714,7 +812,8 @@ tmvg_status sliced_gemm(Context* c, int64_t M, int64_t N, int64_t K, double alph
                 if (j0 > 0) one.rows = 0;  // A's block is sliced already
                 st = sliced_split(c, k, a, one, b, sb);
                 if (!st)
-                    st = sliced_apply(c, m, n, k, alpha, a, sa, b, sb, k0 > 0 ? 1.0 : beta, C + i0 + j0 * ldc, ldc);
+                    st = sliced_apply(c, m, n, k, alpha, a, sa, b, sb, k0 > 0 ? 1.0 : beta, C + i0 + j0 * ldc, ldc,
+                                      max_ctas);
             }
         }
     }

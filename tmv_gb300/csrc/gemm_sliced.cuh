@@ -38,7 +38,7 @@ bool sliced_wanted(Context* c, int64_t M, int64_t N, int64_t K);
 // The whole product; TMVG_UNSUPPORTED (with nothing launched) where the
 // workspace or the tensor-map encoder is not to be had.
 tmvg_status sliced_gemm(Context* c, int64_t M, int64_t N, int64_t K, double alpha, Mat<const double> A,
-                        Mat<const double> B, double beta, double* C, int64_t ldc);
+                        Mat<const double> B, double beta, double* C, int64_t ldc, int max_ctas = 0);
 
 // Stream-ordered scratch from the context's own pool (bounded: what a
 // synchronisation finds unused above 1 GiB goes back to the device).
