@@ -19,6 +19,7 @@
 // The L column is scaled by the reciprocal of the pivot, as TMV's v /= x does
 // (include/tmv/TMV_VectorArith.h:104-106).
 #include "async.cuh"
+#include "gemm_sliced.cuh"
 #include "gemm_tc.cuh"
 #include "lu.cuh"
 #include "pivots.cuh"
@@ -433,6 +434,39 @@ __device__ __forceinline__ void reg_key_reduce(unsigned long long& key, int& idx
     }
 }
 
+// The lane that wins the same order over the warp (the lowest of the lanes
+// that tie in key and index); key and idx become the winner's.  FP64: one
+// redux.sync and a ballot decide unless keys tie in their upper 32 bits (three
+// redux.sync took 400 clocks on the chain of every column).
+template <typename T>
+__device__ __forceinline__ int reg_key_winner(unsigned long long& key, int& idx)
+{
+    if constexpr (sizeof(T) == 4) {
+        const unsigned k0 = (unsigned)key;
+        const int i0 = idx;
+        reg_key_reduce<T>(key, idx);
+        return __ffs(__ballot_sync(0xffffffffu, k0 == (unsigned)key && i0 == idx)) - 1;
+    } else {
+        const unsigned hi = (unsigned)(key >> 32);
+        const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+        bool in = hi == mhi;
+        unsigned m = __ballot_sync(0xffffffffu, in);
+        if (m & (m - 1)) {
+            const unsigned lo = in ? (unsigned)key : 0u;
+            const unsigned mlo = __reduce_max_sync(0xffffffffu, lo);  // (every lane takes part)
+            in = in && lo == mlo;
+            const unsigned i = in ? (unsigned)idx : 0xffffffffu;
+            const unsigned mi = __reduce_min_sync(0xffffffffu, i);
+            in = in && i == mi;
+            m = __ballot_sync(0xffffffffu, in);
+        }
+        const int w = __ffs(m) - 1;
+        key = ((unsigned long long)mhi << 32) | __shfl_sync(0xffffffffu, (unsigned)key, w);
+        idx = __shfl_sync(0xffffffffu, idx, w);
+        return w;
+    }
+}
+
 // 16-byte vectors of a row held in registers (4 floats or 2 doubles).
 template <typename T>
 struct Vec16;
@@ -806,12 +840,27 @@ constexpr int kLeaf = 8;
 constexpr int kLeafThreads = 512;
 constexpr int kLeafWarps = kLeafThreads / 32;
 
+// What a candidate row sends.  FP32: its leaf part with the owed update
+// applied.  FP64: its leaf part as it stands and the multiplier it owes (a
+// DFMA takes its sub-partition 64 clocks whatever the lanes, so the seven of
+// the owed update would sit on the chain in every warp; the receiver's warp 0
+// applies them in one).
 template <typename T>
-struct LeafMsg {
+struct LeafMsg;
+template <>
+struct LeafMsg<float> {
     unsigned long long key;
     int pos;
     int loc;  // cta << 16 | thread
-    T leaf[kLeaf];
+    float leaf[kLeaf];
+};
+template <>
+struct LeafMsg<double> {
+    unsigned long long key;
+    int pos;
+    int loc;
+    double leaf[kLeaf];
+    double owed, pad;
 };
 
 template <typename T, int NB>
@@ -916,6 +965,27 @@ __device__ __forceinline__ void leaf_send_row(const T (&x)[NB], int rot, int pw,
         bulk_s2cluster(cluster_addr(dst_row, d), stage, (uint32_t)(pw * sizeof(T)), cluster_addr(bar, d));
 }
 
+// The winner's leaf part into s_urow[u] (warp 0).  FP64: positions 1..7-u
+// still owe step u-1's update, one per lane; and the pivot's reciprocal.
+template <typename T>
+__device__ __forceinline__ void leaf_pivot_row(const T* sent, T (*s_urow)[kLeaf], int u, bool owe_u, int lane, T* rcp)
+{
+    if constexpr (sizeof(T) == 8) {
+        const T r = recip_rn(sent[0]);
+        if (lane < kLeaf) {
+            T v = sent[lane];
+            if (owe_u && lane >= 1 && lane <= kLeaf - 1 - u)
+                v = fma(-sent[kLeaf], s_urow[u - 1][lane + 1 < kLeaf ? lane + 1 : lane], v);
+            s_urow[u][lane] = v;
+        }
+        if (lane == 0) *rcp = r;
+    } else {
+        using V = Vec16<T>;
+        if (lane < kLeaf / V::E)
+            reinterpret_cast<typename V::type*>(s_urow[u])[lane] = reinterpret_cast<const typename V::type*>(sent)[lane];
+    }
+}
+
 template <typename T, int NB>
 __global__ void __launch_bounds__(kLeafThreads, 1)
 lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int nb,
@@ -929,13 +999,15 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
     constexpr int kMsgVecs = (int)(sizeof(LeafMsg<T>) / 16);
     static_assert(sizeof(LeafMsg<T>) % 16 == 0, "message in 16-byte pieces");
     constexpr int kLast = kLeaf - 1;
+    constexpr bool kRaw = sizeof(T) == 8;  // candidates travel without their owed update
+    constexpr int kSent = (int)((sizeof(LeafMsg<T>) - 16) / sizeof(T));
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
 
     __shared__ unsigned long long s_key[kLeafWarps];
     __shared__ int s_idx[kLeafWarps];
     __shared__ int s_loc[kLeafWarps];
-    __shared__ __align__(16) T warp_leaf[kLeafWarps][kLeaf];     // each warp's candidate's leaf part
+    __shared__ __align__(16) T warp_leaf[kLeafWarps][kSent];     // each warp's candidate's leaf part
     __shared__ __align__(16) LeafMsg<T> msg[2][kClusterCtas];   // messages, by column parity
     __shared__ __align__(16) T s_urow[kLeaf][kLeaf];             // the leaf's pivot rows, leaf part
     __shared__ __align__(16) T s_rem[2][kLeaf][NB];              // pivot rows, then U (by leaf parity)
@@ -943,6 +1015,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
     __shared__ __align__(8) uint64_t mbar[2];
     __shared__ __align__(8) uint64_t mbar_leaf;
     __shared__ unsigned long long s_wk;
+    __shared__ T s_rcp;  // FP64: the pivot's reciprocal, taken once (a chain of DFMAs)
     __shared__ int s_wi, s_wloc;
     __shared__ unsigned char s_mode[kPanelMax];
     __shared__ int s_piv[kPanelMax];
@@ -956,6 +1029,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
     const int r0 = cta * rows_per_cta;
     const int nr = max(0, min(rows_per_cta, m - r0));
     const bool have = tid < nr;
+    const int nthr = (int)blockDim.x, nwarp = nthr >> 5;
     T* Ap = A + k + k * lda;
 
     if (tid == 0) {
@@ -966,7 +1040,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
         s_npairs = 0;
         mbar_fence_init();
     }
-    for (int j = tid; j < nb; j += kLeafThreads) s_mode[j] = modes[j];
+    for (int j = tid; j < nb; j += nthr) s_mode[j] = modes[j];
     const T* Xp = Sp ? Sp : Ap;
     const int64_t ldx = Sp ? lds : lda;
     T x[NB];
@@ -993,6 +1067,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
         unsigned ufmask = 0;
         T lprev = T(0);       // the previous step's multiplier, owed on positions > step + 1
         bool owe = false;
+        bool owe_u = false;   // whether the rows still active owe it (the same in every thread)
 #pragma unroll 1
         for (int u = 0; u < steps; ++u) {
             // the leaf's registers are rotated one position per step:
@@ -1003,17 +1078,30 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             // 1. this warp's candidate; the winner's leaf part with the owed update applied
             unsigned long long bk = act ? reg_pivot_key(x[0], pos == j, r2) : 0ull;
             int bi = act ? pos : INT_MAX;
-            reg_key_reduce<T>(bk, bi);
-            if (act && pos == bi) {
-                // (in position order; positions 1..7-u owe step u-1's update,
-                // whose pivot row s_urow[u-1] is in step u-1's position order)
-                T lp[kLeaf];
+            bool win;
+            if constexpr (kRaw) {
+                win = lane == reg_key_winner<T>(bk, bi);
+            } else {
+                reg_key_reduce<T>(bk, bi);
+                win = act && pos == bi;
+            }
+            if (win) {
+                if constexpr (kRaw) {
 #pragma unroll
-                for (int q = 0; q < kLeaf; ++q)
-                    lp[q] = (owe && q >= 1 && q <= kLast - u) ? fma(-lprev, s_urow[u - 1][q + 1 < kLeaf ? q + 1 : q], x[q]) : x[q];
+                    for (int q = 0; q < kLeaf / V::E; ++q)
+                        reinterpret_cast<typename V::type*>(warp_leaf[warp])[q] = V::make(&x[q * V::E]);
+                    warp_leaf[warp][kLeaf] = lprev;
+                } else {
+                    // (in position order; positions 1..7-u owe step u-1's update,
+                    // whose pivot row s_urow[u-1] is in step u-1's position order)
+                    T lp[kLeaf];
 #pragma unroll
-                for (int q = 0; q < kLeaf / V::E; ++q)
-                    reinterpret_cast<typename V::type*>(warp_leaf[warp])[q] = V::make(&lp[q * V::E]);
+                    for (int q = 0; q < kLeaf; ++q)
+                        lp[q] = (owe && q >= 1 && q <= kLast - u) ? fma(-lprev, s_urow[u - 1][q + 1 < kLeaf ? q + 1 : q], x[q]) : x[q];
+#pragma unroll
+                    for (int q = 0; q < kLeaf / V::E; ++q)
+                        reinterpret_cast<typename V::type*>(warp_leaf[warp])[q] = V::make(&lp[q * V::E]);
+                }
                 s_loc[warp] = loc;
             }
             if (lane == 0) {
@@ -1023,20 +1111,18 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             __syncthreads();
             if (warp == 0) {
                 // 2. this CTA's candidate; with a cluster, one message into every CTA
-                bk = lane < kLeafWarps ? s_key[lane] : 0ull;
-                bi = lane < kLeafWarps ? s_idx[lane] : INT_MAX;
-                reg_key_reduce<T>(bk, bi);
-                const unsigned wm = __ballot_sync(0xffffffffu, lane < kLeafWarps && bi != INT_MAX && s_idx[lane] == bi);
-                const int ww = wm ? __ffs(wm) - 1 : -1;
+                // (s_idx INT_MAX: a warp without candidates)
+                bk = lane < nwarp ? s_key[lane] : 0ull;
+                bi = lane < nwarp ? s_idx[lane] : INT_MAX;
+                const int wn = reg_key_winner<T>(bk, bi);
+                const int ww = bi != INT_MAX ? wn : -1;
                 if (G == 1) {
                     if (lane == 0) {
                         s_wk = bk;
                         s_wi = bi;
                         s_wloc = ww >= 0 ? s_loc[ww] : -1;
                     }
-                    if (ww >= 0 && lane < kLeaf / V::E)
-                        reinterpret_cast<typename V::type*>(s_urow[u])[lane] =
-                            reinterpret_cast<const typename V::type*>(warp_leaf[ww])[lane];
+                    if (ww >= 0) leaf_pivot_row<T>(warp_leaf[ww], s_urow, u, owe_u, lane, &s_rcp);
                 } else {
                     if (lane == 0) mbar_expect_tx(&mbar[par], (uint32_t)(G * sizeof(LeafMsg<T>)));
                     if (lane < G) {
@@ -1075,17 +1161,14 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
                 } else {
                     unsigned long long wk = lane < G ? msg[par][lane].key : 0ull;
                     int wi = lane < G ? msg[par][lane].pos : INT_MAX;
-                    reg_key_reduce<T>(wk, wi);
-                    const unsigned om = __ballot_sync(0xffffffffu, lane < G && wi != INT_MAX && msg[par][lane].pos == wi);
-                    const int wo = om ? __ffs(om) - 1 : -1;
+                    const int wn = reg_key_winner<T>(wk, wi);
+                    const int wo = wi != INT_MAX ? wn : -1;
                     if (lane == 0) {
                         s_wk = wk;
                         s_wi = wi;
                         s_wloc = wo >= 0 ? msg[par][wo].loc : -1;
                     }
-                    if (wo >= 0 && lane < kLeaf / V::E)
-                        reinterpret_cast<typename V::type*>(s_urow[u])[lane] =
-                            reinterpret_cast<const typename V::type*>(msg[par][wo].leaf)[lane];
+                    if (wo >= 0) leaf_pivot_row<T>(msg[par][wo].leaf, s_urow, u, owe_u, lane, &s_rcp);
                 }
             }
             __syncthreads();
@@ -1093,6 +1176,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             // 5. the decision: bookkeeping, the column's scaling and the next column
             const bool uf = reg_key_underflows<T>(s_wk);
             bool own;
+            owe_u = !uf && u + 2 < kLeaf;
             if (uf) {
                 own = act && pos == j;
                 if (act) x[0] = T(0);
@@ -1114,7 +1198,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             }
             if (!uf && act) {
                 // TMV scales the column by the reciprocal of the pivot
-                const T l = x[0] * recip_rn(s_urow[u][0]);
+                const T l = x[0] * (kRaw ? s_rcp : recip_rn(s_urow[u][0]));
                 x[0] = l;
                 if (u < kLast) x[1] = fma(-l, s_urow[u][1], x[1]);
                 if (u + 2 < kLeaf) {
@@ -1144,7 +1228,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             __syncthreads();
             if (s_abort) break;
             T(*Ur)[NB] = s_rem[lpar];
-            for (int p = kLeaf + tid; p < pw; p += kLeafThreads) {
+            for (int p = kLeaf + tid; p < pw; p += nthr) {
                 T uc[kLeaf];
 #pragma unroll
                 for (int t = 0; t < kLeaf; ++t) uc[t] = Ur[t][p];
@@ -1187,7 +1271,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             }
         }
         if (cta == 0)
-            for (int j = tid; j < nb; j += kLeafThreads) P[k + j] = s_piv[j];
+            for (int j = tid; j < nb; j += nthr) P[k + j] = s_piv[j];
     }
     cluster.sync();  // no CTA leaves while another may still store into it
     if (cta == 0 && tid == 0 && !s_abort) pairs[0] = s_npairs;
@@ -1418,7 +1502,7 @@ u12_reg_kernel(int nb, const T* __restrict__ L, int64_t lda, T* __restrict__ A12
 // ---------------------------------------------------------------------
 constexpr int kNarrowRows = 64;
 constexpr int kNarrowThreads = 256;
-constexpr int kNarrowNB = 64;  // the step's width: the FP32 register panel's
+constexpr int kNarrowNB = RegPanel<float>::NB;  // the step's width
 constexpr int kNarrowXP = kNarrowNB + 4;
 constexpr size_t kNarrowSmem =
     sizeof(float) * ((size_t)kNarrowNB * kNarrowNB + (size_t)kNarrowNB * kNarrowXP + (size_t)kNarrowRows * (kNarrowNB + 1));
@@ -1562,6 +1646,146 @@ narrow_update_f32_kernel(const float* __restrict__ A, int64_t lda, int64_t n, in
             const int r = rg + 32 * q, cc = 8 * cg + e;
             if (r < R && cc < nc) S[(r0 + r - k) + cc * lds] = acc[q][e];
         }
+}
+
+// ---------------------------------------------------------------------
+// FP64 register path.  A DFMA occupies its sub-partition for 64 clocks
+// whatever the number of active lanes, so a substitution by one thread per
+// column (496 dependent-issue DFMAs) took 16 us at any width; here its
+// entries are spread over the lanes.
+//
+// U12 = L11^-1 A12 of many columns: a warp takes 8 columns, 4 lanes each (lane
+// s holds rows 4q + s): 143 DFMAs per 8 columns.  Same operations in the same
+// order per entry as u12_reg_kernel.
+// ---------------------------------------------------------------------
+constexpr int kU12F64Warps = 4;  // one per sub-partition
+
+__global__ void __launch_bounds__(32 * kU12F64Warps)
+u12_f64_kernel(int nb, const double* __restrict__ L, int64_t lda, double* __restrict__ A12, int64_t ncols)
+{
+    constexpr int NB = RegPanel<double>::NB;
+    __shared__ double LsT[NB][NB];  // LsT[j][i] = L(i, j) for i > j, else 0
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int s = lane & 3;
+    const int64_t col = ((int64_t)blockIdx.x * kU12F64Warps + warp) * 8 + (lane >> 2);
+    double* a = A12 + col * lda;
+    double x[NB / 4];
+#pragma unroll
+    for (int q = 0; q < NB / 4; ++q) x[q] = (col < ncols && 4 * q + s < nb) ? a[4 * q + s] : 0.0;
+    for (int t = tid; t < NB * NB; t += 32 * kU12F64Warps) {
+        const int i = t % NB, j = t / NB;
+        LsT[j][i] = (i < nb && i > j) ? L[i + (int64_t)j * lda] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < NB - 1; ++j) {
+        const double xj = __shfl_sync(0xffffffffu, x[j >> 2], (lane & ~3) | (j & 3));
+#pragma unroll
+        for (int q = j >> 2; q < NB / 4; ++q) {
+            const double r = fma(-LsT[j][4 * q + s], xj, x[q]);
+            if (4 * q + s > j) x[q] = r;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NB / 4; ++q)
+        if (col < ncols && 4 * q + s < nb) a[4 * q + s] = x[q];
+}
+
+// The next panel's columns [c0, c0+nc) with step k (the "narrow" update), out
+// of place like narrow_update_f32_kernel: row interchanges by gather, U12, and
+// the rank-32 update of kNarrow64Rows rows per CTA, into the scratch panel S.
+// A cluster of 8 CTAs solves U12 together (4 columns each, a warp per column,
+// a lane per row: 31 steps of one DFMA and a shuffle, 1.5 us) and shares it
+// through DSMEM.  Bound: rest * 32 * 32 DFMAs on the FP64 pipe (7 us at
+// rest = 4096, less a launch).
+constexpr int kNarrow64Rows = 16;
+constexpr int kNarrow64Threads = 256;
+constexpr int kNarrow64Ctas = 8;
+
+__global__ void __cluster_dims__(kNarrow64Ctas, 1, 1) __launch_bounds__(kNarrow64Threads)
+narrow_update_f64_kernel(const double* __restrict__ A, int64_t lda, int64_t n, int64_t k, int64_t c0, int nc,
+                         const int* __restrict__ pairs, double* __restrict__ S, int64_t lds)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr int NB = RegPanel<double>::NB, R = kNarrow64Rows;
+    static_assert(NB == 32 && NB == kNarrow64Ctas * 4 && kNarrow64Threads == 16 * R, "shape");
+    __shared__ __align__(16) double UT[NB][NB];  // UT[t][c] = U12(t, c)
+    __shared__ double Ls[R][NB + 1];
+    __shared__ int s_dst[2 * NB], s_src[2 * NB], map_blk[NB], map_row[R];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = (int)cluster.block_rank();
+    const int64_t r0 = k + NB + (int64_t)blockIdx.x * R;
+    const int rows = (int)max((int64_t)0, min((int64_t)R, n - r0));
+    // loads that need no row map
+    double l[NB - 1];
+    if (warp < 4) {
+#pragma unroll
+        for (int j = 0; j < NB - 1; ++j) l[j] = lane > j ? A[(k + lane) + (k + j) * lda] : 0.0;
+    } else {
+        for (int t = tid - 128; t < R * NB; t += 128) {
+            const int r = t % R, j = t / R;
+            Ls[r][j] = r < rows ? A[(r0 + r) + (k + j) * lda] : 0.0;
+        }
+    }
+    const int np = min(pairs[0], 2 * NB);
+    if (tid < np) {
+        s_dst[tid] = pairs[1 + tid];
+        s_src[tid] = pairs[1 + kMaxPairs + tid];
+    }
+    if (tid < NB) map_blk[tid] = (int)(k + tid);
+    if (tid < R) map_row[tid] = (int)(r0 + tid);
+    __syncthreads();
+    if (tid < np) {
+        const int64_t d = s_dst[tid];
+        if (d >= k && d < k + NB) map_blk[d - k] = s_src[tid];
+        else if (d >= r0 && d < r0 + rows) map_row[d - r0] = s_src[tid];
+    }
+    __syncthreads();
+    const int rr = tid % R, cc = 2 * (tid / R);
+    double old[2], acc[2] = {0.0, 0.0};
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+        old[e] = (rr < rows && cc + e < nc) ? A[map_row[rr] + (c0 + cc + e) * lda] : 0.0;
+    if (warp < 4) {
+        const int c = 4 * rank + warp;
+        double x = c < nc ? A[map_blk[lane] + (c0 + c) * lda] : 0.0;
+#pragma unroll
+        for (int j = 0; j < NB - 1; ++j) {
+            const double r = fma(-l[j], __shfl_sync(0xffffffffu, x, j), x);
+            if (lane > j) x = r;
+        }
+#pragma unroll
+        for (int d = 0; d < kNarrow64Ctas; ++d) *cluster.map_shared_rank(&UT[lane][c], d) = x;
+    }
+    cluster.sync();
+    if (blockIdx.x == 0) {
+        for (int t = tid; t < NB * nc; t += kNarrow64Threads) S[t % NB + (int64_t)(t / NB) * lds] = UT[t % NB][t / NB];
+    }
+#pragma unroll 8
+    for (int t = 0; t < NB; ++t) {
+        const double lv = Ls[rr][t];
+        const double2 u = *reinterpret_cast<const double2*>(&UT[t][cc]);
+        acc[0] = fma(lv, u.x, acc[0]);
+        acc[1] = fma(lv, u.y, acc[1]);
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+        if (rr < rows && cc + e < nc) S[(r0 + rr - k) + (cc + e) * lds] = old[e] - acc[e];
+}
+
+static tmvg_status narrow_update_f64(Context* c, const double* A, int64_t lda, int64_t n, int64_t k, int64_t c0,
+                                     int nc, const int* pairs, double* S, int64_t lds)
+{
+    constexpr int NB = RegPanel<double>::NB;
+    const int64_t rest = n - k - NB;
+    const double fr = (double)rest, fc = (double)nc;
+    ScopedTimer timer(c, kClsTrailingUpdate, sizeof(double) * (2.0 * fr * fc + fr * NB + NB * fc), 2.0 * fr * fc * NB);
+    const unsigned clusters = (unsigned)std::max<int64_t>(1, ceil_div(rest, kNarrow64Rows * kNarrow64Ctas));
+    narrow_update_f64_kernel<<<clusters * kNarrow64Ctas, kNarrow64Threads, 0, c->stream>>>(A, lda, n, k, c0, nc, pairs,
+                                                                                         S, lds);
+    ++c->launches;
+    return check_cuda(c, cudaGetLastError(), "lu: narrow update launch");
 }
 
 static tmvg_status narrow_update_f32(Context* c, const float* A, int64_t lda, int64_t n, int64_t k, int64_t c0,
@@ -1914,6 +2138,9 @@ static tmvg_status update_columns(Context* c, int64_t n, T* A, int64_t lda, int6
             else
                 u12_reg_kernel<T, NB, false, kU12NarrowCols><<<grid, kU12RegBlock, 0, c->stream>>>(
                     nb, L11, lda, A12, nc, nullptr, nullptr, sp, k);
+        } else if constexpr (std::is_same<T, double>::value) {
+            u12_f64_kernel<<<(unsigned)ceil_div(nc, 8 * kU12F64Warps), 32 * kU12F64Warps, 0, c->stream>>>(
+                nb, L11, lda, A12, nc);
         } else {
             const unsigned grid = (unsigned)ceil_div(nc, kU12RegThreads);
             if (tc)
@@ -1944,6 +2171,16 @@ static tmvg_status update_columns(Context* c, int64_t n, T* A, int64_t lda, int6
     if constexpr (std::is_same<T, float>::value) {
         // FP32 factor: 3xTF32 on the tensor cores keeps FP32 accuracy
         if (tc) return tf32x3_apply(c, rest, nc, nb, bc, A + (k + nb) + c0 * lda, lda);
+    } else {
+        // the sliced product is persistent, one CTA per SM: it leaves the next
+        // panel's cluster its SMs, or that cluster's share of the tiles would
+        // wait for the panel (n = 4096: 32.3 ms with all SMs)
+        if (sliced_wanted(c, rest, nc, nb)) {
+            st = sliced_gemm(c, rest, nc, nb, -1.0, Mat<const double>{A + (k + nb) + k * lda, 1, lda},
+                             Mat<const double>{A12, 1, lda}, 1.0, A + (k + nb) + c0 * lda, lda,
+                             std::max(1, c->num_sms - kClusterCtas));
+            if (st != TMVG_UNSUPPORTED) return st;
+        }
     }
     return gemm<T>(c, rest, nc, nb, T(-1), Mat<const T>{A + (k + nb) + k * lda, 1, lda},
                    Mat<const T>{A12, 1, lda}, T(1), Mat<T>{A + (k + nb) + c0 * lda, 1, lda});
@@ -2089,12 +2326,12 @@ static tmvg_status launch_panel_cluster_reg(Context* c, cudaStream_t s, T* A, in
     // two-rows-per-thread panel keeps 16 CTAs (a panel of at most 512 rows in
     // one CTA).
     const int64_t m = n - k;
-    int G = m <= 2 * kReg2Threads ? 1 : kClusterCtas;
+    int G = c->panel_reg2 && m <= 2 * kReg2Threads ? 1 : kClusterCtas;
     if (!c->panel_reg2) {
         if (sizeof(T) == 4)
             while (G > 1 && (int64_t)(G / 2) * kLeafThreads >= m) G /= 2;
         else
-            G = m <= 128 ? 1 : kClusterCtas;
+            while (G > 1 && (int64_t)(G / 2) * 128 >= m) G /= 2;
     }
     const int rpc = (int)ceil_div(m, G);
     cudaLaunchConfig_t cfg = {};
@@ -2104,7 +2341,9 @@ static tmvg_status launch_panel_cluster_reg(Context* c, cudaStream_t s, T* A, in
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(G);
-    cfg.blockDim = dim3(c->panel_reg2 ? kReg2Threads : kLeafThreads);
+    // the leaf panel launches no warps without rows (at least two: warp 0 also
+    // decides)
+    cfg.blockDim = dim3(c->panel_reg2 ? kReg2Threads : std::max(64, (int)ceil_div(rpc, 32) * 32));
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
     cfg.attrs = attr;
@@ -2190,15 +2429,14 @@ tmvg_status lu_factor(Context* c, int64_t n, T* A, int64_t lda, int64_t* P)
         // step s+1 writes its L21 split while step s's update still reads.
         bool tc_any = false;
         Tf32x3Buffers arena[2] = {};
-        // FP32 register path: the narrow update writes the next panel's
-        // columns into a scratch panel (n x 64, double-buffered by step
-        // parity) that the panel kernel reads
+        // register path: the narrow update writes the next panel's columns
+        // into a scratch panel (n x nbmax, double-buffered by step parity)
+        // that the panel kernel reads
         T* Sbuf[2] = {nullptr, nullptr};
-        if constexpr (std::is_same<T, float>::value) {
-            const bool tc = n - nbmax >= kTcMinRest && tf32x3_supported(nbmax);
-            const bool fused = reg && nbmax == kNarrowNB;
-            const size_t part = ((size_t)n * nbmax * sizeof(float) + 255) & ~size_t(255);
-            const int nparts = (tc ? 6 : 0) + (fused ? 2 : 0);
+        {
+            const bool tc = std::is_same<T, float>::value && n - nbmax >= kTcMinRest && tf32x3_supported(nbmax);
+            const size_t part = ((size_t)n * nbmax * sizeof(T) + 255) & ~size_t(255);
+            const int nparts = (tc ? 6 : 0) + (reg ? 2 : 0);
             if (nparts > 0) {
                 unsigned char* w3 = (unsigned char*)workspace3(c, nparts * part);
                 if (!w3) return TMVG_OOM;
@@ -2211,7 +2449,7 @@ tmvg_status lu_factor(Context* c, int64_t n, T* A, int64_t lda, int64_t* P)
                     }
                     tc_any = true;
                 }
-                if (fused) {
+                if (reg) {
                     Sbuf[0] = (T*)(w3 + (nparts - 2) * part);
                     Sbuf[1] = (T*)(w3 + (nparts - 1) * part);
                 }
@@ -2271,16 +2509,18 @@ tmvg_status lu_factor(Context* c, int64_t n, T* A, int64_t lda, int64_t* P)
             // update, event ev_wide), then the next panel
             if (step > 0) st = check_cuda(c, cudaStreamWaitEvent(side, c->ev_wide, 0), "lu: wide wait");
             c->stream = side;
-            // the fused narrow update (FP32 register path, 64-wide step) writes
-            // the next panel's columns into Sp; otherwise they are updated in A
+            // the fused narrow update (register path; nb == nbmax here) writes
+            // the next panel's columns into Sk; otherwise they are updated in A
             T* Sk = Sbuf[step & 1];
-            const bool fused = Sk != nullptr && nb == kNarrowNB;
+            const bool fused = Sk != nullptr;
             if constexpr (std::is_same<T, float>::value) {
                 // the L21 split here when the narrow update reads it; with the
                 // fused narrow update (exact FP32) only the wide update does,
                 // and the main stream makes it
                 if (!st && tc && !fused) st = tf32x3_split_a(c, rest, nb, A + (k + nb) + k * lda, lda, b);
                 if (!st && fused) st = narrow_update_f32(c, A, lda, n, k, k + nb, nb2, pk, Sk, n);
+            } else {
+                if (!st && fused) st = narrow_update_f64(c, A, lda, n, k, k + nb, nb2, pk, Sk, n);
             }
             if (!st && !fused) st = update_columns<T>(c, n, A, lda, k, nb, k + nb, nb2, tc, b, pk);
             c->stream = main_stream;
