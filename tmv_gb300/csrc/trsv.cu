@@ -28,11 +28,9 @@ namespace tmvg {
 
 constexpr int kTrsvBlock = 64;
 constexpr int kTrsvThreads = 256;
-// right-hand sides per launch of the multi-column variant (keeps the static
-// shared memory of the FP64 instance under 48 KB)
+// columns solved without inverted diagonal blocks
 template <typename T>
-constexpr int kTrsvMaxRhs = sizeof(T) == 8 ? 4 : 8;
-
+constexpr int64_t kTrsvFewRhs = sizeof(T) == 8 ? 8 : 16;
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
 {
     unsigned v;
@@ -46,57 +44,103 @@ __device__ __forceinline__ void st_release(unsigned* p, unsigned v)
 }
 
 // Inverse of each 64 x 64 lower diagonal block (an upper triangle arrives
-// index-reversed), for the many-column solve: one CTA per block, thread j
-// builds column j by forward substitution with the diagonal's reciprocals
-// (taken once per block).  dinv[b] is row-major 64 x 64; sing[b] = 1 when
-// the block has a zero diagonal (that block keeps the substitution, with
-// TMV's zero-skipping and singular semantics).
+// index-reversed), for the many-column solve, by forward substitution with
+// the diagonal's reciprocals (taken once per block).  dinv[b] is row-major 64 x
+// 64; sing[b] = 1 when the block has a zero diagonal (that block keeps the
+// substitution, with TMV's zero-skipping and singular semantics).
+//
+// A DFMA holds its sub-partition for 64 clocks whatever its active lanes, so
+// the columns are spread: four CTAs per block, four warps each, a warp four
+// columns with eight lanes per column (lane s holds rows 8q + s).  One thread
+// per column took 65 us, this 9.
+constexpr int kInvCtas = 4;
+constexpr int kInvThreads = 128;
+
 template <typename T>
-__global__ void __launch_bounds__(kTrsvBlock)
+__global__ void __launch_bounds__(kInvThreads)
 tri_inv64_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t tsj, bool unit,
                  T* __restrict__ dinv, int* __restrict__ sing)
 {
-    // dynamic shared memory: D and X, each kTrsvBlock x (kTrsvBlock + 1)
-    extern __shared__ __align__(16) unsigned char inv_smem[];
-    T(*D)[kTrsvBlock + 1] = reinterpret_cast<T(*)[kTrsvBlock + 1]>(inv_smem);
-    T(*X)[kTrsvBlock + 1] = D + kTrsvBlock;
+    __shared__ T D[kTrsvBlock][kTrsvBlock + 1];  // D[j][i] = D(i, j)
     __shared__ T rd[kTrsvBlock];
-    __shared__ int s_sing;
-    const int tid = threadIdx.x;
-    const int64_t b = blockIdx.x, r0 = b * kTrsvBlock;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t b = blockIdx.x / kInvCtas, r0 = b * kTrsvBlock;
+    const int part = blockIdx.x % kInvCtas;
     const int rows = (int)min((int64_t)kTrsvBlock, n - r0);
-    if (tid == 0) s_sing = 0;
-    for (int t = tid; t < kTrsvBlock * kTrsvBlock; t += kTrsvBlock) {
+    for (int t = tid; t < kTrsvBlock * kTrsvBlock; t += kInvThreads) {
         const int rr = t % kTrsvBlock, cc = t / kTrsvBlock;
-        D[rr][cc] = (rr < rows && cc <= rr) ? tri[(r0 + rr) * tsi + (r0 + cc) * tsj] : T(0);
+        D[cc][rr] = (rr < rows && cc <= rr) ? tri[(r0 + rr) * tsi + (r0 + cc) * tsj] : T(0);
     }
     __syncthreads();
-    if (!unit && tid < rows) {
-        if (D[tid][tid] == T(0)) s_sing = 1;
-        else rd[tid] = T(1) / D[tid][tid];
+    bool zero = false;
+    if (tid < kTrsvBlock) {
+        zero = !unit && tid < rows && D[tid][tid] == T(0);
+        rd[tid] = unit || tid >= rows || zero ? T(1) : T(1) / D[tid][tid];
     }
-    __syncthreads();
-    if (tid == 0) sing[b] = s_sing;
-    if (s_sing) return;
-    const int j = tid;
-    for (int i = 0; i < kTrsvBlock; ++i) {
-        T v = T(0);
-        if (i < rows && j < rows && i >= j) {
-            T acc = i == j ? T(1) : T(0);
-            for (int k = j; k < i; ++k) acc -= D[i][k] * X[k][j];
-            v = unit ? acc : acc * rd[i];
+    const bool any = __syncthreads_or(zero);
+    if (tid == 0 && part == 0) sing[b] = any;
+    if (any) return;
+    const int s = lane & 7, col = part * 16 + warp * 4 + (lane >> 3);
+    const int first = part * 16 + warp * 4;  // rows above a warp's first column stay zero
+    T x[kTrsvBlock / 8];
+#pragma unroll
+    for (int q = 0; q < kTrsvBlock / 8; ++q) x[q] = (8 * q + s == col && col < rows) ? T(1) : T(0);
+#pragma unroll
+    for (int j = 0; j < kTrsvBlock; ++j) {
+        if (j < first) continue;
+        T v = __shfl_sync(0xffffffffu, x[j >> 3], (lane & ~7) | (j & 7));
+        if (!unit) v *= rd[j];
+        if (s == (j & 7)) x[j >> 3] = v;
+#pragma unroll
+        for (int q = j >> 3; q < kTrsvBlock / 8; ++q) {
+            const T r = fma(-D[j][8 * q + s], v, x[q]);
+            if (8 * q + s > j) x[q] = r;
         }
-        X[i][j] = v;
     }
-    __syncthreads();
     T* out = dinv + b * kTrsvBlock * kTrsvBlock;
-    for (int t = tid; t < kTrsvBlock * kTrsvBlock; t += kTrsvBlock) out[t] = X[t / kTrsvBlock][t % kTrsvBlock];
+#pragma unroll
+    for (int q = 0; q < kTrsvBlock / 8; ++q) out[(8 * q + s) * kTrsvBlock + col] = x[q];
+}
+
+// v / d from r, the correctly rounded reciprocal of d: v r and one correction
+// by the remainder (Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", 1990) -- three dependent FP64 operations on the
+// chain of a substitution instead of a division; the division itself where a
+// magnitude is too near the ends of the range for the remainder to be exact.
+template <typename T>
+__device__ __forceinline__ T quotient(T v, T d, T r)
+{
+    if constexpr (sizeof(T) == 8) {
+        const T q0 = v * r;
+        const T q = fma(fma(-q0, d, v), r, q0);
+        auto mid = [](double x) { return (((unsigned)__double2hiint(x) >> 20) & 0x7ff) - 100u < 1846u; };
+        return mid(q) && mid(v) && mid(d) && mid(r) ? q : v / d;
+    } else {
+        return v / d;
+    }
+}
+
+template <typename T>
+__device__ __forceinline__ bool nonzero(T v)
+{
+    // (a comparison of doubles would take the FP64 pipe)
+    if constexpr (sizeof(T) == 8) return (__double_as_longlong(v) << 1) != 0;
+    else return v != T(0);
 }
 
 // One CTA per (row block, group of NR right-hand sides); tickets hand the
 // pairs out block by block (all groups of block b before block b+1), and a
 // CTA waits only on earlier blocks of its own group, so every wait is on a
 // ticket already handed out.  flags[g * nblk + b] publishes (b, g).
+//
+// Bound: the chain of n/64 blocks.  On it per block: the wait and the read of
+// x of the block before (two L2 round trips), its 64 x 64 x NR product (NR us
+// on one SM's FP64 pipe, so few columns per CTA), and the diagonal block: a
+// substitution in registers, one warp per column with a lane per two rows
+// (per row a shuffle and a DFMA, and three more for the quotient: 4 and 11 us
+// for the unit and the other triangle), or a product with the inverse.
+// n = 4096, one column, both triangles: 3.2 ms with the substitution through
+// shared memory and a division per row (25 us a block).
 template <typename T, int NR>
 __global__ void __launch_bounds__(kTrsvThreads)
 trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t tsj, bool unit,
@@ -105,19 +149,17 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
                       unsigned long long tbase, unsigned spin_limit, int* err,
                       const T* __restrict__ dinv, const int* __restrict__ dinv_sing)
 {
+    static_assert(NR <= kTrsvThreads / 64, "a thread per entry of a block's solution");
     __shared__ long long s_tk;
-    __shared__ T xs[kTrsvBlock][NR];
-    __shared__ T xj[kTrsvBlock][NR];
+    __shared__ T xs[NR][kTrsvBlock];
+    __shared__ T xj[2][kTrsvBlock][NR];
     __shared__ T Td[kTrsvBlock][kTrsvBlock + 1];
-    __shared__ T part[4][kTrsvBlock][NR];
-    __shared__ int s_abort;
+    __shared__ T rd[kTrsvBlock];
+    __shared__ T part[4][NR][kTrsvBlock];
 
     const int tid = threadIdx.x;
     const int i = tid & 63, g = tid >> 6;
-    if (tid == 0) {
-        s_tk = (long long)(atomicAdd(ticket, 1ull) - tbase);
-        s_abort = 0;
-    }
+    if (tid == 0) s_tk = (long long)(atomicAdd(ticket, 1ull) - tbase);
     __syncthreads();
     const int64_t nblk = (n + kTrsvBlock - 1) / kTrsvBlock;
     if (s_tk < 0 || s_tk >= nblk * groups) return;
@@ -128,6 +170,7 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
     flags += (int64_t)grp * nblk;
     const int64_t r0 = b * kTrsvBlock;
     const int rows = (int)min((int64_t)kTrsvBlock, n - r0);
+    const bool mine = tid < kTrsvBlock * NR && g < nr;  // this thread holds entry (i, g)
 
     // diagonal block (or its inverse) and right-hand side
     const bool use_inv = dinv != nullptr && dinv_sing[b] == 0;
@@ -140,11 +183,10 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
             const int rr = t % kTrsvBlock, cc = t / kTrsvBlock;
             Td[rr][cc] = (rr < rows && cc <= rr) ? tri[(r0 + rr) * tsi + (r0 + cc) * tsj] : T(0);
         }
+        __syncthreads();
+        if (tid < kTrsvBlock) rd[tid] = unit ? T(1) : T(1) / Td[tid][tid];
     }
-    for (int t = tid; t < kTrsvBlock * NR; t += kTrsvThreads) {
-        const int rr = t % kTrsvBlock, q = t / kTrsvBlock;
-        xs[rr][q] = (rr < rows && q < nr) ? B[(r0 + rr) * bsi + q * bsj] : T(0);
-    }
+    T x = (mine && i < rows) ? B[(r0 + i) * bsi + g * bsj] : T(0);
 
     T acc[NR];
 #pragma unroll
@@ -156,93 +198,90 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
 #pragma unroll
         for (int c = 0; c < 16; ++c)
             a[c] = (i < rows) ? tri[(r0 + i) * tsi + (c0 + g * 16 + c) * tsj] : T(0);
-        if (tid == 0) {
+        bool late = false;
+        if (tid < kTrsvBlock * NR) {
             unsigned spins = 0;
             while (ld_acquire(flags + j) != epoch) {
                 if (++spins > spin_limit || *((volatile int*)err) == kDevTimeout) {
                     atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
-                    s_abort = 1;
+                    late = true;
                     break;
                 }
                 if (spins > 32) __nanosleep(32);
             }
+            xj[j & 1][i][g] = g < nr ? __ldcg(&B[(c0 + i) * bsi + g * bsj]) : T(0);
         }
-        __syncthreads();
-        if (s_abort) return;
-        for (int t = tid; t < kTrsvBlock * NR; t += kTrsvThreads) {
-            const int rr = t % kTrsvBlock, q = t / kTrsvBlock;
-            xj[rr][q] = (q < nr) ? __ldcg(&B[(c0 + rr) * bsi + q * bsj]) : T(0);
-        }
-        __syncthreads();
+        // (the other parity's buffer is read before this barrier and written after it)
+        if (__syncthreads_or(late)) return;
 #pragma unroll
         for (int c = 0; c < 16; ++c)
 #pragma unroll
-            for (int q = 0; q < NR; ++q) acc[q] -= a[c] * xj[g * 16 + c][q];
-        __syncthreads();
+            for (int q = 0; q < NR; ++q) acc[q] -= a[c] * xj[j & 1][g * 16 + c][q];
     }
 #pragma unroll
-    for (int q = 0; q < NR; ++q) part[g][i][q] = acc[q];
+    for (int q = 0; q < NR; ++q) part[g][q][i] = acc[q];
     __syncthreads();
-    for (int t = tid; t < kTrsvBlock * NR; t += kTrsvThreads) {
-        const int rr = t % kTrsvBlock, q = t / kTrsvBlock;
-        xs[rr][q] += ((part[0][rr][q] + part[1][rr][q]) + part[2][rr][q]) + part[3][rr][q];
+    if (tid < kTrsvBlock * NR) {
+        x += ((part[0][g][i] + part[1][g][i]) + part[2][g][i]) + part[3][g][i];
+        xs[g][i] = x;
     }
     __syncthreads();
 
-    // diagonal block: x_b = D_b^-1 x_b as a product (thread (i, q) one entry),
-    // or warp q substitutes right-hand side q (2 rows per lane)
-    const int warp = tid >> 5, lane = tid & 31;
-    bool sing = false;
+    // diagonal block
     if (use_inv) {
-        constexpr int PER = (NR * kTrsvBlock + kTrsvThreads - 1) / kTrsvThreads;
-        T v[PER];
+        // a quarter of each row's product per thread
+        T v[NR];
 #pragma unroll
-        for (int u = 0; u < PER; ++u) {
-            const int t = tid + u * kTrsvThreads, ii = t % kTrsvBlock, q = t / kTrsvBlock;
-            v[u] = T(0);
-            if (q < nr && ii < rows)
-                for (int kk = 0; kk <= ii; ++kk) v[u] += Td[ii][kk] * xs[kk][q];
-        }
+        for (int q = 0; q < NR; ++q) v[q] = T(0);
+#pragma unroll
+        for (int c = 0; c < 16; ++c)
+#pragma unroll
+            for (int q = 0; q < NR; ++q) v[q] += Td[i][g * 16 + c] * xs[q][g * 16 + c];
+#pragma unroll
+        for (int q = 0; q < NR; ++q) part[g][q][i] = v[q];
         __syncthreads();
-#pragma unroll
-        for (int u = 0; u < PER; ++u) {
-            const int t = tid + u * kTrsvThreads, ii = t % kTrsvBlock, q = t / kTrsvBlock;
-            if (q < nr && ii < rows) xs[ii][q] = v[u];
-        }
-    }
-    for (int q = warp; q < nr && !use_inv; q += kTrsvThreads / 32) {
-        for (int jj = 0; jj < rows; ++jj) {
-            __syncwarp();
-            T v = xs[jj][q];
-            if (!unit) {
-                const T d = Td[jj][jj];
-                if (skip_zero) {
-                    if (v != T(0)) {
-                        if (d == T(0)) sing = true;
-                        else v = v / d;
+        if (tid < kTrsvBlock * NR)
+            x = ((part[0][g][i] + part[1][g][i]) + part[2][g][i]) + part[3][g][i];
+    } else {
+        const int warp = tid >> 5, lane = tid & 31;
+        bool sing = false;
+        if (warp < nr) {
+            T lo = xs[warp][lane], hi = xs[warp][lane + 32];
+#pragma unroll 4
+            for (int jj = 0; jj < rows; ++jj) {
+                T v = __shfl_sync(0xffffffffu, jj < 32 ? lo : hi, jj & 31);
+                const T tl = Td[lane][jj], th = Td[lane + 32][jj];
+                if (!unit) {
+                    const T d = Td[jj][jj], r = rd[jj];
+                    if (skip_zero) {
+                        if (nonzero(v)) {
+                            if (!nonzero(d)) sing = true;
+                            else v = quotient(v, d, r);
+                        }
+                    } else {
+                        if (!nonzero(d)) sing = true;
+                        else v = v * r;
                     }
-                } else {
-                    if (d == T(0)) sing = true;
-                    else v = v * (T(1) / d);
+                    if (lane == (jj & 31)) (jj < 32 ? lo : hi) = v;
+                }
+                if (!skip_zero || nonzero(v)) {
+                    if (jj < 32) {
+                        const T u = lo - tl * v;
+                        if (lane > jj) lo = u;
+                    }
+                    const T u = hi - th * v;
+                    if (lane + 32 > jj) hi = u;
                 }
             }
-            __syncwarp();
-            if (lane == 0) xs[jj][q] = v;
-            if (v != T(0) || !skip_zero) {
-                const int k1 = lane, k2 = lane + 32;
-                if (k1 > jj && k1 < rows) xs[k1][q] -= Td[k1][jj] * v;
-                if (k2 > jj && k2 < rows) xs[k2][q] -= Td[k2][jj] * v;
-            }
+            xs[warp][lane] = lo;
+            xs[warp][lane + 32] = hi;
         }
+        if (sing) atomicCAS(err, (int)kDevOk, (int)kDevSingular);
+        __syncthreads();
+        if (tid < kTrsvBlock * NR) x = xs[g][i];
     }
-    if (sing) atomicCAS(err, (int)kDevOk, (int)kDevSingular);
-    __syncthreads();
-    for (int t = tid; t < kTrsvBlock * NR; t += kTrsvThreads) {
-        const int rr = t % kTrsvBlock, q = t / kTrsvBlock;
-        if (rr < rows && q < nr) B[(r0 + rr) * bsi + q * bsj] = xs[rr][q];
-    }
-    __threadfence();
-    __syncthreads();
+    if (mine && i < rows) B[(r0 + i) * bsi + g * bsj] = x;
+    __syncthreads();  // (the release below is cumulative over these writes)
     if (tid == 0) st_release(flags + b, epoch);
 }
 
@@ -261,8 +300,11 @@ tmvg_status trsm_sync_free(Context* c, int64_t n, const T* tri, int64_t tsi, int
         bsi = -bsi;
     }
     const int64_t nblk = ceil_div(n, kTrsvBlock);
-    constexpr int NRM = kTrsvMaxRhs<T>;
-    const int64_t groups = nrhs == 1 ? 1 : ceil_div(nrhs, NRM);
+    // Columns per CTA: one up to kTrsvFewRhs, where the chain of blocks is
+    // the bound; two beyond (half the reads of the triangle), four where the
+    // flags would not suffice.
+    const int NR = nrhs <= kTrsvFewRhs<T> ? 1 : nblk * ceil_div(nrhs, (int64_t)2) <= (int64_t)kTrsvFlagCap ? 2 : 4;
+    const int64_t groups = ceil_div(nrhs, (int64_t)NR);
     if (nblk * groups > (int64_t)kTrsvFlagCap)
         return set_error(c, TMVG_UNSUPPORTED, "trsv: n x nrhs too large for the flag array");
     const unsigned epoch = ++c->trsv_epoch;
@@ -281,37 +323,28 @@ tmvg_status trsm_sync_free(Context* c, int64_t n, const T* tri, int64_t tsi, int
     }
     const unsigned limit = c->poll_limit ? c->poll_limit : kSpinLimit;
     const unsigned grid = (unsigned)(nblk * groups);
-    // Beyond two groups (more than 2 NR columns) the diagonal blocks are
-    // inverted first, so that a block's step on the chain is a short product
-    // instead of a 64-step substitution with a division per step.
+    // Beyond kTrsvFewRhs columns the diagonal blocks are inverted first, so
+    // that a block's step on the chain is a short product instead of a 64-step
+    // substitution.
     const T* dinv = nullptr;
     const int* dsing = nullptr;
-    if (groups > 2) {
+    if (nrhs > kTrsvFewRhs<T>) {
         const size_t ib = sizeof(T) * (size_t)nblk * kTrsvBlock * kTrsvBlock;
         unsigned char* w = (unsigned char*)trsv_dinv_buffer(c, ib + sizeof(int) * (size_t)nblk);
         if (!w) return set_error(c, TMVG_OOM, "trsv: inverse blocks");
         T* dv = (T*)w;
         int* ds = (int*)(w + ib);
-        const size_t smem = sizeof(T) * 2 * kTrsvBlock * (kTrsvBlock + 1);
-        st = check_cuda(c, cudaFuncSetAttribute(tri_inv64_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)smem),
-                        "trsv inverse blocks: smem attribute");
-        if (st) return st;
-        tri_inv64_kernel<T><<<(unsigned)nblk, kTrsvBlock, smem, c->stream>>>(n, tri, tsi, tsj, unit, dv, ds);
+        tri_inv64_kernel<T><<<(unsigned)nblk * kInvCtas, kInvThreads, 0, c->stream>>>(n, tri, tsi, tsj, unit, dv, ds);
         ++c->launches;
         st = check_cuda(c, cudaGetLastError(), "trsv inverse blocks");
         if (st) return st;
         dinv = dv;
         dsing = ds;
     }
-    if (nrhs == 1)
-        trsm_sync_free_kernel<T, 1><<<grid, kTrsvThreads, 0, c->stream>>>(
-            n, tri, tsi, tsj, unit, nrhs, 1, B, bsi, bsj, skip_zero, c->trsv_flags, epoch,
-            c->trsv_ticket, tbase, limit, c->dflags, nullptr, nullptr);
-    else
-        trsm_sync_free_kernel<T, NRM><<<grid, kTrsvThreads, 0, c->stream>>>(
-            n, tri, tsi, tsj, unit, nrhs, (int)groups, B, bsi, bsj, skip_zero, c->trsv_flags, epoch,
-            c->trsv_ticket, tbase, limit, c->dflags, dinv, dsing);
+    auto kern = NR == 1 ? trsm_sync_free_kernel<T, 1> : NR == 2 ? trsm_sync_free_kernel<T, 2> : trsm_sync_free_kernel<T, 4>;
+    kern<<<grid, kTrsvThreads, 0, c->stream>>>(n, tri, tsi, tsj, unit, nrhs, (int)groups, B, bsi, bsj, skip_zero,
+                                               c->trsv_flags, epoch, c->trsv_ticket, tbase, limit, c->dflags, dinv,
+                                               dsing);
     ++c->launches;
     return check_cuda(c, cudaGetLastError(), "trsv launch");
 }
