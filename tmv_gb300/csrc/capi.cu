@@ -57,6 +57,20 @@ void* workspace2(Context* c, size_t bytes) { return grow(c, c->work2, c->work2_b
 void* workspace3(Context* c, size_t bytes) { return grow(c, c->work3, c->work3_bytes, bytes); }
 void* perm_lists_buffer(Context* c, size_t bytes) { return grow(c, c->perm_lists, c->perm_lists_bytes, bytes); }
 void* trsv_dinv_buffer(Context* c, size_t bytes) { return grow(c, c->trsv_dinv, c->trsv_dinv_bytes, bytes); }
+void* trsv_words_buffer(Context* c, size_t bytes)
+{
+    const size_t had = c->trsv_words_bytes;
+    void* p = grow(c, c->trsv_words, c->trsv_words_bytes, bytes);
+    // no word may hold an epoch before it is published
+    if (p && c->trsv_words_bytes != had && cudaMemsetAsync(p, 0, c->trsv_words_bytes, c->stream) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(c->trsv_words);
+        c->trsv_words = nullptr;
+        c->trsv_words_bytes = 0;
+        return nullptr;
+    }
+    return p;
+}
 
 static cudaEvent_t pooled_event(Context* c)
 {
@@ -435,6 +449,7 @@ tmvg_status tmvg_destroy(tmvg_handle h)
     if (c->trsv_flags) cudaFree(c->trsv_flags);
     if (c->trsv_pub) cudaFree(c->trsv_pub);
     if (c->trsv_dinv) cudaFree(c->trsv_dinv);
+    if (c->trsv_words) cudaFree(c->trsv_words);
     if (c->dflags) cudaFree(c->dflags);
     if (c->hflags) cudaFreeHost(c->hflags);
     for (const TimedSpan& sp : c->spans) {

@@ -71,6 +71,10 @@ struct Context {
     // word (epoch << 32 | value bits); grow-only, never needs clearing.
     unsigned long long* trsv_pub = nullptr;
     size_t trsv_pub_len = 0;
+    // Published solution entries of the sync-free solves: 16-byte words
+    // (value, epoch), grow-only, zeroed when allocated.
+    void* trsv_words = nullptr;
+    size_t trsv_words_bytes = 0;
     // Inverted 64 x 64 diagonal blocks of the many-column sync-free solve
     // (grow-only) and their per-block zero-diagonal flags.
     void* trsv_dinv = nullptr;
@@ -156,6 +160,7 @@ void* workspace2(Context* c, size_t bytes);
 void* workspace3(Context* c, size_t bytes);
 void* perm_lists_buffer(Context* c, size_t bytes);
 void* trsv_dinv_buffer(Context* c, size_t bytes);
+void* trsv_words_buffer(Context* c, size_t bytes);
 // Reads and clears the device error word (synchronises the stream).
 tmvg_status collect_device_error(Context* c, const char* what);
 

@@ -8,9 +8,8 @@
 //   1. for every earlier block j, loads the 64x64 tile T[b, j] into registers
 //      (independent of x), waits (bounded) until block j publishes its
 //      solution, and accumulates T[b, j] x_j;
-//   2. substitutes through the diagonal block with one warp per right-hand
-//      side;
-//   3. writes x_b and publishes it (release store of the launch's epoch).
+//   2. solves the diagonal block, by its inverse or by substitution;
+//   3. writes x_b and publishes it (entries tagged with the launch's epoch).
 // An upper-triangular solve is the same lower solve on index-reversed views
 // (negative strides), so the sums are taken in the order of TMV's
 // column-oriented vector solve (src/TMV_TriDiv_V.cpp:148-236, 322-398):
@@ -128,26 +127,71 @@ __device__ __forceinline__ bool nonzero(T v)
     else return v != T(0);
 }
 
+// A published entry of the solution and the launch's epoch in one word that
+// is stored and loaded whole, so a consumer polls the value itself: no flag,
+// no fence, one L2 round trip.
+__device__ __forceinline__ void pub_store(void* words, int64_t at, double v, unsigned epoch)
+{
+    asm volatile(
+        "{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(
+            static_cast<char*>(words) + 16 * at),
+        "l"(__double_as_longlong(v)), "l"((long long)epoch)
+        : "memory");
+}
+__device__ __forceinline__ bool pub_load(const void* words, int64_t at, unsigned epoch, double& v)
+{
+    long long x, e;
+    asm volatile(
+        "{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+        : "=l"(x), "=l"(e)
+        : "l"(static_cast<const char*>(words) + 16 * at)
+        : "memory");
+    v = __longlong_as_double(x);
+    return e == (long long)epoch;
+}
+__device__ __forceinline__ void pub_store(void* words, int64_t at, float v, unsigned epoch)
+{
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(static_cast<char*>(words) + 16 * at),
+                 "l"(((unsigned long long)epoch << 32) | __float_as_uint(v))
+                 : "memory");
+}
+__device__ __forceinline__ bool pub_load(const void* words, int64_t at, unsigned epoch, float& v)
+{
+    unsigned long long x;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];"
+                 : "=l"(x)
+                 : "l"(static_cast<const char*>(words) + 16 * at)
+                 : "memory");
+    v = __uint_as_float((unsigned)x);
+    return (unsigned)(x >> 32) == epoch;
+}
+
+__device__ __forceinline__ bool finite(double v) { return ((unsigned)__double2hiint(v) & 0x7ff00000u) != 0x7ff00000u; }
+__device__ __forceinline__ bool finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+
 // One CTA per (row block, group of NR right-hand sides); tickets hand the
 // pairs out block by block (all groups of block b before block b+1), and a
 // CTA waits only on earlier blocks of its own group, so every wait is on a
-// ticket already handed out.  flags[g * nblk + b] publishes (b, g).
+// ticket already handed out.  pub[q * n + i] publishes entry i of column q.
 //
-// Bound: the chain of n/64 blocks.  On it per block: the wait and the read of
-// x of the block before (two L2 round trips), its 64 x 64 x NR product (NR us
-// on one SM's FP64 pipe, so few columns per CTA), and the diagonal block: a
-// substitution in registers, one warp per column with a lane per two rows
-// (per row a shuffle and a DFMA, and three more for the quotient: 4 and 11 us
-// for the unit and the other triangle), or a product with the inverse.
-// n = 4096, one column, both triangles: 3.2 ms with the substitution through
-// shared memory and a division per row (25 us a block).
+// Bound: the chain of n/64 blocks.  On it per block: the published words' way
+// through L2, the 64 x 64 x NR product with the block before (NR us on one
+// SM's FP64 pipe, so few columns per CTA), and the diagonal block.  Its
+// inverse takes one product of the same size.  For few columns (refine) the
+// product is corrected once, x = y + D^-1 (b - D y) with y = D^-1 b, which
+// gives the substitution's accuracy also where the block is ill-conditioned,
+// in 3.3 us against 7 (unit) and 21 us for the substitution (per row a
+// shuffle and a DFMA, and three more for the quotient).  The substitution
+// remains for a block with a zero diagonal, for n <= 64, and where the
+// corrected product is not finite.  n = 4096, one column: 0.82 / 1.72 ms with
+// the substitution and published flags.
 template <typename T, int NR>
 __global__ void __launch_bounds__(kTrsvThreads)
 trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t tsj, bool unit,
                       int64_t nrhs, int groups, T* B, int64_t bsi, int64_t bsj, bool skip_zero,
-                      unsigned* flags, unsigned epoch, unsigned long long* ticket,
+                      void* pub, unsigned epoch, unsigned long long* ticket,
                       unsigned long long tbase, unsigned spin_limit, int* err,
-                      const T* __restrict__ dinv, const int* __restrict__ dinv_sing)
+                      const T* __restrict__ dinv, const int* __restrict__ dinv_sing, bool refine)
 {
     static_assert(NR <= kTrsvThreads / 64, "a thread per entry of a block's solution");
     __shared__ long long s_tk;
@@ -167,26 +211,29 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
     const int grp = (int)(s_tk % groups);
     const int nr = (int)min((int64_t)NR, nrhs - (int64_t)grp * NR);
     B += (int64_t)grp * NR * bsj;
-    flags += (int64_t)grp * nblk;
+    const int64_t pub0 = (int64_t)grp * NR * n;
     const int64_t r0 = b * kTrsvBlock;
     const int rows = (int)min((int64_t)kTrsvBlock, n - r0);
-    const bool mine = tid < kTrsvBlock * NR && g < nr;  // this thread holds entry (i, g)
+    const bool holds = tid < kTrsvBlock * NR;              // this thread holds entry (i, g)
+    const bool mine = holds && g < nr && i < rows;
 
     // diagonal block (or its inverse) and right-hand side
-    const bool use_inv = dinv != nullptr && dinv_sing[b] == 0;
+    bool use_inv = dinv != nullptr && dinv_sing[b] == 0;
+    T dg[16];  // D(i, 16 g ..), for the correction
+#pragma unroll
+    for (int c = 0; c < 16; ++c)
+        dg[c] = (!use_inv || refine) && i < rows && g * 16 + c <= i ? tri[(r0 + i) * tsi + (r0 + g * 16 + c) * tsj] : T(0);
+    if (unit && i >= g * 16 && i < g * 16 + 16) {
+#pragma unroll
+        for (int c = 0; c < 16; ++c)
+            if (g * 16 + c == i) dg[c] = T(1);
+    }
     if (use_inv) {
         const T* di = dinv + b * kTrsvBlock * kTrsvBlock;
         for (int t = tid; t < kTrsvBlock * kTrsvBlock; t += kTrsvThreads)
             Td[t / kTrsvBlock][t % kTrsvBlock] = di[t];
-    } else {
-        for (int t = tid; t < kTrsvBlock * kTrsvBlock; t += kTrsvThreads) {
-            const int rr = t % kTrsvBlock, cc = t / kTrsvBlock;
-            Td[rr][cc] = (rr < rows && cc <= rr) ? tri[(r0 + rr) * tsi + (r0 + cc) * tsj] : T(0);
-        }
-        __syncthreads();
-        if (tid < kTrsvBlock) rd[tid] = unit ? T(1) : T(1) / Td[tid][tid];
     }
-    T x = (mine && i < rows) ? B[(r0 + i) * bsi + g * bsj] : T(0);
+    T x = mine ? B[(r0 + i) * bsi + g * bsj] : T(0);
 
     T acc[NR];
 #pragma unroll
@@ -199,17 +246,20 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
         for (int c = 0; c < 16; ++c)
             a[c] = (i < rows) ? tri[(r0 + i) * tsi + (c0 + g * 16 + c) * tsj] : T(0);
         bool late = false;
-        if (tid < kTrsvBlock * NR) {
-            unsigned spins = 0;
-            while (ld_acquire(flags + j) != epoch) {
-                if (++spins > spin_limit || *((volatile int*)err) == kDevTimeout) {
-                    atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
-                    late = true;
-                    break;
+        if (holds) {
+            T v = T(0);
+            if (g < nr) {
+                unsigned spins = 0;
+                while (!pub_load(pub, pub0 + (int64_t)g * n + c0 + i, epoch, v)) {
+                    if (++spins > spin_limit || (spins % 64 == 0 && *((volatile int*)err) == kDevTimeout)) {
+                        atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
+                        late = true;
+                        break;
+                    }
+                    if (spins > 64) __nanosleep(32);
                 }
-                if (spins > 32) __nanosleep(32);
             }
-            xj[j & 1][i][g] = g < nr ? __ldcg(&B[(c0 + i) * bsi + g * bsj]) : T(0);
+            xj[j & 1][i][g] = v;
         }
         // (the other parity's buffer is read before this barrier and written after it)
         if (__syncthreads_or(late)) return;
@@ -218,31 +268,65 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
 #pragma unroll
             for (int q = 0; q < NR; ++q) acc[q] -= a[c] * xj[j & 1][g * 16 + c][q];
     }
-#pragma unroll
-    for (int q = 0; q < NR; ++q) part[g][q][i] = acc[q];
-    __syncthreads();
-    if (tid < kTrsvBlock * NR) {
-        x += ((part[0][g][i] + part[1][g][i]) + part[2][g][i]) + part[3][g][i];
-        xs[g][i] = x;
-    }
-    __syncthreads();
-
-    // diagonal block
-    if (use_inv) {
-        // a quarter of each row's product per thread
-        T v[NR];
-#pragma unroll
-        for (int q = 0; q < NR; ++q) v[q] = T(0);
-#pragma unroll
-        for (int c = 0; c < 16; ++c)
-#pragma unroll
-            for (int q = 0; q < NR; ++q) v[q] += Td[i][g * 16 + c] * xs[q][g * 16 + c];
+    // the quarters of a row's sums, added by the entry's holder (the result
+    // is the holder's only)
+    auto gather = [&](const T(&v)[NR]) {
 #pragma unroll
         for (int q = 0; q < NR; ++q) part[g][q][i] = v[q];
         __syncthreads();
-        if (tid < kTrsvBlock * NR)
-            x = ((part[0][g][i] + part[1][g][i]) + part[2][g][i]) + part[3][g][i];
-    } else {
+        return holds ? ((part[0][g][i] + part[1][g][i]) + part[2][g][i]) + part[3][g][i] : T(0);
+    };
+    auto share = [&](T v) {
+        if (holds) xs[g][i] = v;
+        __syncthreads();
+    };
+    x += gather(acc);
+    share(x);
+
+    // diagonal block
+    if (use_inv) {
+        // (entries above the diagonal take no part, whatever x holds there)
+        auto inverse_times_xs = [&](T(&v)[NR]) {
+#pragma unroll
+            for (int q = 0; q < NR; ++q) v[q] = T(0);
+#pragma unroll
+            for (int c = 0; c < 16; ++c)
+#pragma unroll
+                for (int q = 0; q < NR; ++q)
+                    if (g * 16 + c <= i) v[q] += Td[i][g * 16 + c] * xs[q][g * 16 + c];
+        };
+        T v[NR];
+        inverse_times_xs(v);
+        const T y = gather(v);
+        if (!refine) {
+            x = y;
+        } else {
+            share(y);
+#pragma unroll
+            for (int q = 0; q < NR; ++q) v[q] = T(0);
+#pragma unroll
+            for (int c = 0; c < 16; ++c)
+#pragma unroll
+                for (int q = 0; q < NR; ++q)
+                    if (g * 16 + c <= i) v[q] += dg[c] * xs[q][g * 16 + c];
+            const T r = x - gather(v);
+            share(r);
+            inverse_times_xs(v);
+            const T z = y + gather(v);
+            if (__syncthreads_or(!finite(z))) {
+                use_inv = false;  // the substitution decides
+                share(x);
+            } else {
+                x = z;
+            }
+        }
+    }
+    if (!use_inv) {
+#pragma unroll
+        for (int c = 0; c < 16; ++c) Td[i][g * 16 + c] = dg[c];
+        __syncthreads();
+        if (tid < kTrsvBlock) rd[tid] = unit ? T(1) : T(1) / Td[tid][tid];
+        __syncthreads();
         const int warp = tid >> 5, lane = tid & 31;
         bool sing = false;
         if (warp < nr) {
@@ -278,11 +362,12 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
         }
         if (sing) atomicCAS(err, (int)kDevOk, (int)kDevSingular);
         __syncthreads();
-        if (tid < kTrsvBlock * NR) x = xs[g][i];
+        if (holds) x = xs[g][i];
     }
-    if (mine && i < rows) B[(r0 + i) * bsi + g * bsj] = x;
-    __syncthreads();  // (the release below is cumulative over these writes)
-    if (tid == 0) st_release(flags + b, epoch);
+    if (mine) {
+        pub_store(pub, pub0 + (int64_t)g * n + r0 + i, x, epoch);
+        B[(r0 + i) * bsi + g * bsj] = x;
+    }
 }
 
 template <typename T>
@@ -307,7 +392,8 @@ tmvg_status trsm_sync_free(Context* c, int64_t n, const T* tri, int64_t tsi, int
     const int64_t groups = ceil_div(nrhs, (int64_t)NR);
     if (nblk * groups > (int64_t)kTrsvFlagCap)
         return set_error(c, TMVG_UNSUPPORTED, "trsv: n x nrhs too large for the flag array");
-    const unsigned epoch = ++c->trsv_epoch;
+    if (++c->trsv_epoch == 0) ++c->trsv_epoch;  // 0 is the cleared words' tag
+    const unsigned epoch = c->trsv_epoch;
     // tickets restart at 0 for every launch
     tmvg_status st = check_cuda(
         c, cudaMemsetAsync(c->trsv_ticket, 0, sizeof(unsigned long long), c->stream),
@@ -323,12 +409,13 @@ tmvg_status trsm_sync_free(Context* c, int64_t n, const T* tri, int64_t tsi, int
     }
     const unsigned limit = c->poll_limit ? c->poll_limit : kSpinLimit;
     const unsigned grid = (unsigned)(nblk * groups);
-    // Beyond kTrsvFewRhs columns the diagonal blocks are inverted first, so
-    // that a block's step on the chain is a short product instead of a 64-step
-    // substitution.
+    void* pub = trsv_words_buffer(c, 16 * (size_t)n * (size_t)(groups * NR));
+    if (!pub) return set_error(c, TMVG_OOM, "trsv: published words");
+    // The diagonal blocks are inverted first (all but the only one).
+    const bool few = nrhs <= kTrsvFewRhs<T>;
     const T* dinv = nullptr;
     const int* dsing = nullptr;
-    if (nrhs > kTrsvFewRhs<T>) {
+    if (nblk > 1 || !few) {
         const size_t ib = sizeof(T) * (size_t)nblk * kTrsvBlock * kTrsvBlock;
         unsigned char* w = (unsigned char*)trsv_dinv_buffer(c, ib + sizeof(int) * (size_t)nblk);
         if (!w) return set_error(c, TMVG_OOM, "trsv: inverse blocks");
@@ -342,9 +429,8 @@ tmvg_status trsm_sync_free(Context* c, int64_t n, const T* tri, int64_t tsi, int
         dsing = ds;
     }
     auto kern = NR == 1 ? trsm_sync_free_kernel<T, 1> : NR == 2 ? trsm_sync_free_kernel<T, 2> : trsm_sync_free_kernel<T, 4>;
-    kern<<<grid, kTrsvThreads, 0, c->stream>>>(n, tri, tsi, tsj, unit, nrhs, (int)groups, B, bsi, bsj, skip_zero,
-                                               c->trsv_flags, epoch, c->trsv_ticket, tbase, limit, c->dflags, dinv,
-                                               dsing);
+    kern<<<grid, kTrsvThreads, 0, c->stream>>>(n, tri, tsi, tsj, unit, nrhs, (int)groups, B, bsi, bsj, skip_zero, pub,
+                                               epoch, c->trsv_ticket, tbase, limit, c->dflags, dinv, dsing, few);
     ++c->launches;
     return check_cuda(c, cudaGetLastError(), "trsv launch");
 }
