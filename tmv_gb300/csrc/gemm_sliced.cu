@@ -92,6 +92,15 @@ SlicedOperand sliced_layout(void* buf, int64_t rows, int64_t K)
 // ---------------------------------------------------------------------
 constexpr int kSplitThreads = 256;
 
+// Element (r, k) of an operand; Z: of a complex matrix's real form.
+template <bool Z>
+__device__ __forceinline__ double sl_at(const double* __restrict__ p, int64_t sr, int64_t sk, int64_t r, int64_t k)
+{
+    if constexpr (!Z) return __ldg(p + r * sr + k * sk);
+    const double v = __ldg(p + 2 * ((r >> 1) * sr + (k >> 1) * sk) + ((r ^ k) & 1));
+    return (r & 1) < (k & 1) ? -v : v;
+}
+
 struct SplitSide {
     const double* p;
     int64_t sr, sk;   // element (vector r, place k) at p[r*sr + k*sk]
@@ -114,14 +123,10 @@ __device__ __forceinline__ unsigned long long fixed63(double v, int emax)
     return (b >> 63) ? 0ull - x : x;
 }
 
-template <int R>
-__global__ void __launch_bounds__(kSplitThreads)
-sliced_split_kernel(SplitSide sa, SplitSide sb, int64_t groups_a, int64_t K)
+template <int R, bool Z>
+__device__ __forceinline__ void split_vectors(const SplitSide& s, int64_t grp, int64_t K)
 {
     constexpr int G = kSplitThreads / R;  // threads sharing a vector
-    const bool is_b = (int64_t)blockIdx.x >= groups_a;
-    const SplitSide s = is_b ? sb : sa;
-    const int64_t grp = is_b ? blockIdx.x - groups_a : blockIdx.x;
     __shared__ int s_emax[R], s_big[R];
     __shared__ int s_min;
     const int tid = threadIdx.x;
@@ -130,7 +135,8 @@ sliced_split_kernel(SplitSide sa, SplitSide sb, int64_t groups_a, int64_t K)
     const int g = kc ? tid % G : tid / R;
     const int64_t row = grp * R + r;
     const bool have = row < s.rows;
-    const double* p = s.p + row * s.sr;
+    const double* p = Z ? s.p : s.p + row * s.sr;
+    const int64_t zr = Z ? row : 0;
     if (tid < R) {
         s_emax[tid] = 0;
         s_big[tid] = 0;
@@ -141,7 +147,7 @@ sliced_split_kernel(SplitSide sa, SplitSide sb, int64_t groups_a, int64_t K)
         int e = 0;
 #pragma unroll 8
         for (int64_t k = g; k < K; k += G)
-            e = max(e, (int)((unsigned)__double2hiint(p[k * s.sk]) >> 20 & 0x7ff));
+            e = max(e, (int)((unsigned)__double2hiint(sl_at<Z>(p, s.sr, s.sk, zr, k)) >> 20 & 0x7ff));
         atomicMax(&s_emax[r], e);
     }
     __syncthreads();
@@ -152,7 +158,7 @@ sliced_split_kernel(SplitSide sa, SplitSide sb, int64_t groups_a, int64_t K)
         for (int64_t k0 = (int64_t)g * 8; k0 < s.Kp; k0 += G * 8) {
             double v[8];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) v[q] = k0 + q < K ? p[(k0 + q) * s.sk] : 0.0;
+            for (int q = 0; q < 8; ++q) v[q] = k0 + q < K ? sl_at<Z>(p, s.sr, s.sk, zr, k0 + q) : 0.0;
             uint32_t w[kSlices][4];
 #pragma unroll
             for (int q = 0; q < 8; q += 2) {
@@ -202,25 +208,33 @@ sliced_split_kernel(SplitSide sa, SplitSide sb, int64_t groups_a, int64_t K)
     // a vector of subnormals only would be sliced as zero: it takes the FP64 pipe
     if (have && s_emax[r] == 0) {
         bool sub = false;
-        for (int64_t k = g; k < K; k += G) sub |= (__double_as_longlong(p[k * s.sk]) << 1) != 0;
+        for (int64_t k = g; k < K; k += G) sub |= (__double_as_longlong(sl_at<Z>(p, s.sr, s.sk, zr, k)) << 1) != 0;
         if (sub) atomicMin(&s_min, kFillBad);
     }
     __syncthreads();
     if (tid == 0) s.fill[grp] = s_min;
 }
 
+// Both operands in one launch: groups_a CTAs for A, the rest for B.
+template <int R, bool ZLEFT>
+__global__ void __launch_bounds__(kSplitThreads)
+sliced_split_kernel(SplitSide sa, SplitSide sb, int64_t groups_a, int64_t K)
+{
+    if ((int64_t)blockIdx.x < groups_a) split_vectors<R, ZLEFT>(sa, blockIdx.x, K);
+    else split_vectors<R, false>(sb, blockIdx.x - groups_a, K);
+}
+
 tmvg_status sliced_split(Context* c, int64_t K, Mat<const double> A, const SlicedOperand& sa,
-                         Mat<const double> B, const SlicedOperand& sb)
+                         Mat<const double> B, const SlicedOperand& sb, bool zleft)
 {
     const int R = sa.rows ? sa.group : sb.group;
     const SplitSide a{A.p, A.si, A.sj, sa.digits, sa.exps, sa.fill, sa.rows, sa.Kp};
     const SplitSide b{B.p, B.sj, B.si, sb.digits, sb.exps, sb.fill, sb.rows, sb.Kp};
     const int64_t ga = ceil_div(sa.rows, (int64_t)R), gb = ceil_div(sb.rows, (int64_t)R);
     if (ga + gb == 0) return TMVG_OK;
-    if (R == 64)
-        sliced_split_kernel<64><<<(unsigned)(ga + gb), kSplitThreads, 0, c->stream>>>(a, b, ga, K);
-    else
-        sliced_split_kernel<16><<<(unsigned)(ga + gb), kSplitThreads, 0, c->stream>>>(a, b, ga, K);
+    auto kern = R == 64 ? (zleft ? sliced_split_kernel<64, true> : sliced_split_kernel<64, false>)
+                        : (zleft ? sliced_split_kernel<16, true> : sliced_split_kernel<16, false>);
+    kern<<<(unsigned)(ga + gb), kSplitThreads, 0, c->stream>>>(a, b, ga, K);
     ++c->launches;
     return check_cuda(c, cudaGetLastError(), "sliced split launch");
 }
@@ -346,6 +360,7 @@ struct SlicedArgs {
     int unit;                        // alpha: 1 or -1, or 0 for any other value
     const double *A, *B;             // the operands themselves (FP64 tiles)
     int64_t asi, asj, bsi, bsj;
+    bool zleft;
     const int *ea, *eb, *fa, *fb;
     int ga, gb;                      // vectors per fill group
     int need;                        // first look: overlap that a sliced tile needs
@@ -574,7 +589,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
 #pragma unroll
                     for (int q = 0; q < 8; ++q) acc[q] = 0.0;
                     for (int64_t k = 0; k < g.K; ++k) {
-                        const double av = g.A[r * g.asi + k * g.asj];
+                        const double av = g.zleft ? sl_at<true>(g.A, g.asi, g.asj, r, k) : sl_at<false>(g.A, g.asi, g.asj, r, k);
 #pragma unroll
                         for (int q = 0; q < 8; ++q)
                             if (j0 + q < nc) acc[q] = fma(av, __ldg(&g.B[k * g.bsi + (col0 + j0 + q) * g.bsj]), acc[q]);
@@ -711,7 +726,7 @@ static bool sl_map(CUtensorMap* map, const SlicedOperand& s, int box_rows)
 
 tmvg_status sliced_apply(Context* c, int64_t M, int64_t N, int64_t K, double alpha, Mat<const double> A,
                          const SlicedOperand& sa, Mat<const double> B, const SlicedOperand& sb, double beta,
-                         double* C, int64_t ldc, int max_ctas)
+                         double* C, int64_t ldc, int max_ctas, bool zleft)
 {
     if (M <= 0 || N <= 0 || K <= 0) return TMVG_OK;
     CUtensorMap mA, mB;
@@ -719,7 +734,7 @@ tmvg_status sliced_apply(Context* c, int64_t M, int64_t N, int64_t K, double alp
         return set_error(c, TMVG_CUDA_ERROR, "sliced product: tensor map encoding failed");
     SlicedArgs g;
     g.M = M, g.N = N, g.K = K, g.alpha = alpha, g.add = beta != 0.0, g.unit = alpha == 1.0 ? 1 : alpha == -1.0 ? -1 : 0;
-    g.A = A.p, g.asi = A.si, g.asj = A.sj;
+    g.A = A.p, g.asi = A.si, g.asj = A.sj, g.zleft = zleft;
     g.B = B.p, g.bsi = B.si, g.bsj = B.sj;
     g.ea = sa.exps, g.eb = sb.exps, g.fa = sa.fill, g.fb = sb.fill, g.ga = sa.group, g.gb = sb.group;
     // sum |a||b| of at least 2^-9.2 sqrt(K) of the product of the scales: an
@@ -785,7 +800,8 @@ bool sliced_wanted(Context* c, int64_t M, int64_t N, int64_t K)
 }
 
 tmvg_status sliced_gemm(Context* c, int64_t M, int64_t N, int64_t K, double alpha, Mat<const double> A,
-                        Mat<const double> B, double beta, double* C, int64_t ldc, int max_ctas)
+                        Mat<const double> B, double beta, double* C, int64_t ldc, int max_ctas,
+                        bool zleft)
 {
     // blocks of at most 256 MiB of digits per operand
     constexpr int64_t kMaxK = 16384;
@@ -802,6 +818,7 @@ tmvg_status sliced_gemm(Context* c, int64_t M, int64_t N, int64_t K, double alph
         const int64_t k = std::min(kb, K - k0);
         for (int64_t i0 = 0; i0 < M && !st; i0 += mb) {
             const int64_t m = std::min(mb, M - i0);
+            // (i0 and k0 are even: the real form's offsets are the same)
             const Mat<const double> a{A.p + i0 * A.si + k0 * A.sj, A.si, A.sj};
             const SlicedOperand sa = sliced_layout(ws, m, k);
             for (int64_t j0 = 0; j0 < N && !st; j0 += nb) {
@@ -810,10 +827,10 @@ tmvg_status sliced_gemm(Context* c, int64_t M, int64_t N, int64_t K, double alph
                 const SlicedOperand sb = sliced_layout(ws + ba, n, k);
                 SlicedOperand one = sa;
                 if (j0 > 0) one.rows = 0;  // A's block is sliced already
-                st = sliced_split(c, k, a, one, b, sb);
+                st = sliced_split(c, k, a, one, b, sb, zleft);
                 if (!st)
                     st = sliced_apply(c, m, n, k, alpha, a, sa, b, sb, k0 > 0 ? 1.0 : beta, C + i0 + j0 * ldc, ldc,
-                                      max_ctas);
+                                      max_ctas, zleft);
             }
         }
     }

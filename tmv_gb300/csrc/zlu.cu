@@ -24,6 +24,7 @@
 // Values agree with TMV's recursive factorisation to rounding; pivots are
 // TMV's wherever rounding does not decide a tie.
 #include "zlu.cuh"
+#include "gemm_sliced.cuh"
 #include "trsv.cuh"
 
 #include <cooperative_groups.h>
@@ -437,22 +438,41 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
     cluster.sync();  // no CTA leaves while another may still read its shared memory
 }
 
-// The panel's interchanges P[k..k+kb) applied in order to the columns
-// [c0, c1), one column per thread.
-__global__ void zlu_swap_rest_kernel(int64_t c0, int64_t c1, double2* A, int64_t lda, int64_t k, int kb,
-                                     const int64_t* __restrict__ P)
+// The panel's interchanges P[k..k+kb) (kb <= 32) applied in order to the
+// columns [c0, c1): a warp per column, lane l holding row k + l and the row
+// P[k + l] (its first lane, where several name one row); the interchanges are
+// replayed on the registers by shuffles and every row is read and written
+// once.  (A column per thread replayed them through memory: 25 us, on the
+// look-ahead chain.)
+constexpr int kZSwapWarps = 4;
+__global__ void __launch_bounds__(32 * kZSwapWarps)
+zlu_swap_rest_kernel(int64_t c0, int64_t c1, double2* A, int64_t lda, int64_t k, int kb,
+                     const int64_t* __restrict__ P)
 {
-    const int64_t col = c0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const int64_t col = c0 + blockIdx.x * (int64_t)kZSwapWarps + (threadIdx.x >> 5);
     if (col >= c1) return;
     double2* a = A + col * lda;
-    for (int jj = 0; jj < kb; ++jj) {
-        const int64_t j = k + jj, p = P[j];
-        if (p != j) {
-            const double2 x = a[j];
-            a[j] = a[p];
-            a[p] = x;
-        }
+    const bool act = lane < kb;
+    const int64_t p = act ? P[k + lane] : k + lane;
+    const int q = (int)(p - k);                                  // >= lane
+    const unsigned same = __match_any_sync(0xffffffffu, q);
+    const int first = __ffs(same) - 1;
+    const bool below = act && q >= kb;                           // P's row lies below the block
+    double2 x = act ? a[k + lane] : make_double2(0.0, 0.0);
+    double2 y = below && first == lane ? a[p] : make_double2(0.0, 0.0);
+    for (int j = 0; j < kb; ++j) {
+        const int qj = __shfl_sync(0xffffffffu, q, j);
+        if (qj == j) continue;
+        const int src = qj < kb ? qj : __shfl_sync(0xffffffffu, first, j);  // the other row's lane
+        const double2 v = qj < kb ? x : y;
+        const double ox = __shfl_sync(0xffffffffu, v.x, src), oy = __shfl_sync(0xffffffffu, v.y, src);
+        const double jx = __shfl_sync(0xffffffffu, x.x, j), jy = __shfl_sync(0xffffffffu, x.y, j);
+        if (lane == src) (qj < kb ? x : y) = make_double2(jx, jy);
+        if (lane == j) x = make_double2(ox, oy);
     }
+    if (act) a[k + lane] = x;
+    if (below && first == lane) a[p] = y;
 }
 
 // U12 = L11^-1 A12 (L11 unit lower, KB x KB) for the columns [c0, c1): a
@@ -555,6 +575,50 @@ zlu_gemm_kernel(int64_t n, double2* A, int64_t lda, int64_t k, int64_t cbeg, int
     }
 }
 
+// The same for at most KB columns (the next panel's, on the look-ahead chain):
+// 8 rows x KB columns per CTA, so that every SM takes part (64 x 64 tiles gave
+// 32 CTAs of half-empty tiles at n = 2048: 139 us; this 18).  Bound: 4 DFMAs
+// per complex product on the FP64 pipe.
+constexpr int kZNarrowRows = 8;
+template <int KB>
+__global__ void __launch_bounds__(kZNarrowRows * KB / 2)
+zlu_narrow_kernel(int64_t n, double2* A, int64_t lda, int64_t k, int64_t cbeg, int64_t cend)
+{
+    constexpr int R = kZNarrowRows, T = R * KB / 2;
+    __shared__ double2 s_l[R][KB + 1], s_u[KB][KB + 1];
+    const int tid = threadIdx.x, r = tid % R, cc = tid / R;  // columns cc and cc + KB/2
+    const int64_t r0 = k + KB + (int64_t)blockIdx.x * R;
+    double2 old[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int64_t j = cbeg + cc + e * (KB / 2);
+        old[e] = r0 + r < n && j < cend ? A[r0 + r + j * lda] : make_double2(0.0, 0.0);
+    }
+    for (int t = tid; t < R * KB; t += T)
+        s_l[t % R][t / R] = r0 + t % R < n ? A[r0 + t % R + (k + t / R) * lda] : make_double2(0.0, 0.0);
+    for (int t = tid; t < KB * KB; t += T)
+        s_u[t % KB][t / KB] = cbeg + t / KB < cend ? A[k + t % KB + (cbeg + t / KB) * lda] : make_double2(0.0, 0.0);
+    __syncthreads();
+    double2 acc[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+#pragma unroll 8
+    for (int q = 0; q < KB; ++q) {
+        const double2 l = s_l[r][q];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const double2 u = s_u[q][cc + e * (KB / 2)];
+            acc[e].x = fma(l.x, u.x, acc[e].x);
+            acc[e].x = fma(-l.y, u.y, acc[e].x);
+            acc[e].y = fma(l.x, u.y, acc[e].y);
+            acc[e].y = fma(l.y, u.x, acc[e].y);
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int64_t j = cbeg + cc + e * (KB / 2);
+        if (r0 + r < n && j < cend) A[r0 + r + j * lda] = make_double2(old[e].x - acc[e].x, old[e].y - acc[e].y);
+    }
+}
+
 // The panel width for n: 32 where ceil(n/16) rows of 33 entries fit the
 // shared memory, else 16; 0 (column path) beyond.
 static int zpanel_width(int64_t n)
@@ -633,17 +697,35 @@ static tmvg_status zlu_factor_blocked(Context* c, int64_t n, double2* A, int64_t
     };
     auto swap = [&](int64_t c0, int64_t c1, int64_t k, int kb) {
         if (c1 <= c0) return;
-        zlu_swap_rest_kernel<<<(unsigned)ceil_div(c1 - c0, 128), 128, 0, c->stream>>>(c0, c1, A, lda, k, kb, P);
+        zlu_swap_rest_kernel<<<(unsigned)ceil_div(c1 - c0, kZSwapWarps), 32 * kZSwapWarps, 0, c->stream>>>(c0, c1, A, lda, k, kb, P);
         ++c->launches;
     };
     // step k's U12 and product for the columns [c0, c1) (k + KB <= c0)
-    auto update = [&](int64_t k, int64_t c0, int64_t c1) {
-        if (c1 <= c0 || k + KB >= n) return;
+    auto update = [&](int64_t k, int64_t c0, int64_t c1) -> tmvg_status {
+        if (c1 <= c0 || k + KB >= n) return TMVG_OK;
         zlu_trsm_kernel<KB><<<(unsigned)ceil_div(c1 - c0, kZTrsmWarps), 32 * kZTrsmWarps, 0, c->stream>>>(
             c1, A, lda, k, c0);
-        const dim3 grid((unsigned)ceil_div(n - k - KB, kZgBM), (unsigned)ceil_div(c1 - c0, kZgBN));
+        ++c->launches;
+        const int64_t m = n - k - KB, nc = c1 - c0;
+        if (nc <= KB) {
+            zlu_narrow_kernel<KB><<<(unsigned)ceil_div(m, kZNarrowRows), kZNarrowRows * KB / 2, 0, c->stream>>>(
+                n, A, lda, k, c0, c1);
+            ++c->launches;
+            return TMVG_OK;
+        }
+        // as a real product on the tensor cores, leaving the panel's cluster
+        // its SMs
+        if (sliced_wanted(c, 2 * m, nc, 2 * KB)) {
+            const tmvg_status s2 = sliced_gemm(
+                c, 2 * m, nc, 2 * KB, -1.0, Mat<const double>{(const double*)(A + (k + KB) + k * lda), 1, lda},
+                Mat<const double>{(const double*)(A + k + c0 * lda), 1, 2 * lda}, 1.0,
+                (double*)(A + (k + KB) + c0 * lda), 2 * lda, std::max(1, c->num_sms - kZPanelCtas), true);
+            if (s2 != TMVG_UNSUPPORTED) return s2;
+        }
+        const dim3 grid((unsigned)ceil_div(m, kZgBM), (unsigned)ceil_div(nc, kZgBN));
         zlu_gemm_kernel<KB><<<grid, 256, 0, c->stream>>>(n, A, lda, k, c0, c1);
-        c->launches += 2;
+        ++c->launches;
+        return TMVG_OK;
     };
     if ((st = check_cuda(c, cudaEventRecord(c->ev_fork, c->stream), "lu_z: fork"))) return st;
     if ((st = check_cuda(c, cudaStreamWaitEvent(c->side, c->ev_fork, 0), "lu_z: fork wait"))) return st;
@@ -656,7 +738,7 @@ static tmvg_status zlu_factor_blocked(Context* c, int64_t n, double2* A, int64_t
         if (kn < n) {
             // narrow: the next panel's columns, then that panel on the side stream
             swap(kn, kn1, k, kb);
-            update(k, kn, kn1);
+            if ((st = update(k, kn, kn1))) return st;
             if ((st = check_cuda(c, cudaGetLastError(), "lu_z: narrow update"))) return st;
             if ((st = check_cuda(c, cudaEventRecord(c->ev_wide, c->stream), "lu_z: narrow event"))) return st;
             if ((st = check_cuda(c, cudaStreamWaitEvent(c->side, c->ev_wide, 0), "lu_z: narrow wait"))) return st;
@@ -667,7 +749,7 @@ static tmvg_status zlu_factor_blocked(Context* c, int64_t n, double2* A, int64_t
         // the next panel
         swap(0, k, k, kb);
         swap(kn1, n, k, kb);
-        update(k, kn1, n);
+        if ((st = update(k, kn1, n))) return st;
         if ((st = check_cuda(c, cudaGetLastError(), "lu_z: wide update"))) return st;
     }
     return TMVG_OK;
