@@ -19,21 +19,22 @@
 
 namespace tmvg {
 
-template <typename T, int TM, int TN, int BK, bool ARM, bool BRM>
-__global__ void __launch_bounds__(256)
+// NX x NY threads.
+template <typename T, int TM, int TN, int BK, bool ARM, bool BRM, int NX = 16, int NY = 16>
+__global__ void __launch_bounds__(NX * NY)
 gemm_simt_kernel(int64_t M, int64_t N, int64_t K, T alpha,
                  const T* __restrict__ A, int64_t lda,
                  const T* __restrict__ B, int64_t ldb, T beta,
                  T* __restrict__ C, int64_t ldc)
 {
-    constexpr int BM = 16 * TM, BN = 16 * TN;
-    constexpr int NA = BM * BK / 256, NB = BN * BK / 256;
-    static_assert(NA * 256 == BM * BK && NB * 256 == BN * BK, "tile");
+    constexpr int BM = NX * TM, BN = NY * TN, NT = NX * NY;
+    constexpr int NA = BM * BK / NT, NB = BN * BK / NT;
+    static_assert(NA * NT == BM * BK && NB * NT == BN * BK, "tile");
     __shared__ T As[BK][BM + 1];
     __shared__ T Bs[BK][BN + 1];
 
     const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
+    const int tx = tid % NX, ty = tid / NX;
     const int64_t i0 = (int64_t)blockIdx.x * BM;
     const int64_t j0 = (int64_t)blockIdx.y * BN;
 
@@ -47,7 +48,7 @@ gemm_simt_kernel(int64_t M, int64_t N, int64_t K, T alpha,
     auto load = [&](int64_t k0) {
 #pragma unroll
         for (int t = 0; t < NA; ++t) {
-            const int idx = tid + t * 256;
+            const int idx = tid + t * NT;
             int ii, kk;
             if (ARM) { ii = idx / BK; kk = idx % BK; }
             else { ii = idx % BM; kk = idx / BM; }
@@ -58,7 +59,7 @@ gemm_simt_kernel(int64_t M, int64_t N, int64_t K, T alpha,
         }
 #pragma unroll
         for (int t = 0; t < NB; ++t) {
-            const int idx = tid + t * 256;
+            const int idx = tid + t * NT;
             int jj, kk;
             if (BRM) { jj = idx % BN; kk = idx / BN; }
             else { jj = idx / BK; kk = idx % BK; }
@@ -71,7 +72,7 @@ gemm_simt_kernel(int64_t M, int64_t N, int64_t K, T alpha,
     auto store = [&]() {
 #pragma unroll
         for (int t = 0; t < NA; ++t) {
-            const int idx = tid + t * 256;
+            const int idx = tid + t * NT;
             int ii, kk;
             if (ARM) { ii = idx / BK; kk = idx % BK; }
             else { ii = idx % BM; kk = idx / BM; }
@@ -79,7 +80,7 @@ gemm_simt_kernel(int64_t M, int64_t N, int64_t K, T alpha,
         }
 #pragma unroll
         for (int t = 0; t < NB; ++t) {
-            const int idx = tid + t * 256;
+            const int idx = tid + t * NT;
             int jj, kk;
             if (BRM) { jj = idx % BN; kk = idx / BN; }
             else { jj = idx / BK; kk = idx % BK; }
@@ -140,6 +141,13 @@ struct SimtSmallTile<double> { static constexpr int TM = 2, TN = 2, BK = 16; };
 template <>
 struct SimtSmallTile<float> { static constexpr int TM = 4, TN = 4, BK = 8; };
 
+// FP64 products whose half-size tiles still leave most sub-partitions idle
+// (a DFMA holds its sub-partition for 64 clocks whatever its lanes, so the
+// time is K x 64 clocks x warps per sub-partition x entries per thread): one
+// entry per thread in 8 x 8 tiles, two warps, while those number at most two
+// per SM.  65 x 33 x 97: 28 us with 32 x 32 tiles (6 CTAs), 8 with these.
+constexpr int kTinyTile = 8, kTinyBK = 32;
+
 template <typename T, bool ARM, bool BRM>
 static tmvg_status launch_gemm(Context* c, int64_t m, int64_t n, int64_t k, T alpha,
                                const T* A, int64_t lda, const T* B, int64_t ldb,
@@ -147,6 +155,15 @@ static tmvg_status launch_gemm(Context* c, int64_t m, int64_t n, int64_t k, T al
 {
     constexpr int TM = SimtTile<T>::TM, TN = SimtTile<T>::TN, BK = SimtTile<T>::BK;
     dim3 grid((unsigned)ceil_div(m, 16 * TM), (unsigned)ceil_div(n, 16 * TN));
+    if constexpr (std::is_same<T, double>::value) {
+        const dim3 g3((unsigned)ceil_div(m, kTinyTile), (unsigned)ceil_div(n, kTinyTile));
+        if (g3.y <= 65535 && (int64_t)g3.x * g3.y <= 2 * c->num_sms) {
+            gemm_simt_kernel<T, 1, 1, kTinyBK, ARM, BRM, kTinyTile, kTinyTile>
+                <<<g3, kTinyTile * kTinyTile, 0, c->stream>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
+            ++c->launches;
+            return check_cuda(c, cudaGetLastError(), "gemm launch");
+        }
+    }
     if ((int64_t)grid.x * grid.y < c->num_sms) {
         constexpr int STM = SimtSmallTile<T>::TM, STN = SimtSmallTile<T>::TN, SBK = SimtSmallTile<T>::BK;
         dim3 g2((unsigned)ceil_div(m, 16 * STM), (unsigned)ceil_div(n, 16 * STN));

@@ -2130,7 +2130,10 @@ static tmvg_status update_columns(Context* c, int64_t n, T* A, int64_t lda, int6
         // a few columns (the next panel's): spread over more CTAs, since
         // each one's latency is staging L11 and the substitution chain
         const int* sp = fuse_swaps ? pairs : nullptr;
-        if (nc <= NB) {
+        if (std::is_same<T, double>::value && !sp) {
+            u12_f64_kernel<<<(unsigned)ceil_div(nc, 8 * kU12F64Warps), 32 * kU12F64Warps, 0, c->stream>>>(
+                nb, (const double*)L11, lda, (double*)A12, nc);
+        } else if (nc <= NB) {
             const unsigned grid = (unsigned)ceil_div(nc, kU12NarrowCols);
             if (tc)
                 u12_reg_kernel<T, NB, true, kU12NarrowCols><<<grid, kU12RegBlock, 0, c->stream>>>(
@@ -2138,9 +2141,6 @@ static tmvg_status update_columns(Context* c, int64_t n, T* A, int64_t lda, int6
             else
                 u12_reg_kernel<T, NB, false, kU12NarrowCols><<<grid, kU12RegBlock, 0, c->stream>>>(
                     nb, L11, lda, A12, nc, nullptr, nullptr, sp, k);
-        } else if constexpr (std::is_same<T, double>::value) {
-            u12_f64_kernel<<<(unsigned)ceil_div(nc, 8 * kU12F64Warps), 32 * kU12F64Warps, 0, c->stream>>>(
-                nb, L11, lda, A12, nc);
         } else {
             const unsigned grid = (unsigned)ceil_div(nc, kU12RegThreads);
             if (tc)

@@ -49,11 +49,12 @@ __device__ __forceinline__ void st_release(unsigned* p, unsigned v)
 // substitution, with TMV's zero-skipping and singular semantics).
 //
 // A DFMA holds its sub-partition for 64 clocks whatever its active lanes, so
-// the columns are spread: four CTAs per block, four warps each, a warp four
-// columns with eight lanes per column (lane s holds rows 8q + s).  One thread
-// per column took 65 us, this 9.
-constexpr int kInvCtas = 4;
+// the columns are spread: eight CTAs per block, four warps each, a warp two
+// columns with sixteen lanes per column (lane s holds rows 16q + s).  One
+// thread per column took 65 us, this 12.
+constexpr int kInvCtas = 8;
 constexpr int kInvThreads = 128;
+constexpr int kInvLanes = 16;
 
 template <typename T>
 __global__ void __launch_bounds__(kInvThreads)
@@ -79,26 +80,28 @@ tri_inv64_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t tsj,
     const bool any = __syncthreads_or(zero);
     if (tid == 0 && part == 0) sing[b] = any;
     if (any) return;
-    const int s = lane & 7, col = part * 16 + warp * 4 + (lane >> 3);
-    const int first = part * 16 + warp * 4;  // rows above a warp's first column stay zero
-    T x[kTrsvBlock / 8];
+    constexpr int NL = kInvLanes, NQ = kTrsvBlock / NL;
+    static_assert(kInvCtas * (kInvThreads / NL) == kTrsvBlock, "a column per group of lanes");
+    const int first = part * (kTrsvBlock / kInvCtas) + warp * (32 / NL);  // rows above a warp's columns stay zero
+    const int s = lane % NL, col = first + lane / NL;
+    T x[NQ];
 #pragma unroll
-    for (int q = 0; q < kTrsvBlock / 8; ++q) x[q] = (8 * q + s == col && col < rows) ? T(1) : T(0);
+    for (int q = 0; q < NQ; ++q) x[q] = (NL * q + s == col && col < rows) ? T(1) : T(0);
 #pragma unroll
     for (int j = 0; j < kTrsvBlock; ++j) {
         if (j < first) continue;
-        T v = __shfl_sync(0xffffffffu, x[j >> 3], (lane & ~7) | (j & 7));
+        T v = __shfl_sync(0xffffffffu, x[j / NL], (lane & ~(NL - 1)) | (j % NL));
         if (!unit) v *= rd[j];
-        if (s == (j & 7)) x[j >> 3] = v;
+        if (s == j % NL) x[j / NL] = v;
 #pragma unroll
-        for (int q = j >> 3; q < kTrsvBlock / 8; ++q) {
-            const T r = fma(-D[j][8 * q + s], v, x[q]);
-            if (8 * q + s > j) x[q] = r;
+        for (int q = j / NL; q < NQ; ++q) {
+            const T r = fma(-D[j][NL * q + s], v, x[q]);
+            if (NL * q + s > j) x[q] = r;
         }
     }
     T* out = dinv + b * kTrsvBlock * kTrsvBlock;
 #pragma unroll
-    for (int q = 0; q < kTrsvBlock / 8; ++q) out[(8 * q + s) * kTrsvBlock + col] = x[q];
+    for (int q = 0; q < NQ; ++q) out[(NL * q + s) * kTrsvBlock + col] = x[q];
 }
 
 // v / d from r, the correctly rounded reciprocal of d: v r and one correction
