@@ -145,7 +145,8 @@ struct SimtSmallTile<float> { static constexpr int TM = 4, TN = 4, BK = 8; };
 // (a DFMA holds its sub-partition for 64 clocks whatever its lanes, so the
 // time is K x 64 clocks x warps per sub-partition x entries per thread): one
 // entry per thread in 8 x 8 tiles, two warps, while those number at most two
-// per SM.  65 x 33 x 97: 28 us with 32 x 32 tiles (6 CTAs), 8 with these.
+// per SM.  65 x 33 x 97: 28 us with 32 x 32 tiles (6 CTAs), 8 with these.  One
+// entry per thread in 16 x 16 tiles up to four of those per SM.
 constexpr int kTinyTile = 8, kTinyBK = 32;
 
 template <typename T, bool ARM, bool BRM>
@@ -160,6 +161,13 @@ static tmvg_status launch_gemm(Context* c, int64_t m, int64_t n, int64_t k, T al
         if (g3.y <= 65535 && (int64_t)g3.x * g3.y <= 2 * c->num_sms) {
             gemm_simt_kernel<T, 1, 1, kTinyBK, ARM, BRM, kTinyTile, kTinyTile>
                 <<<g3, kTinyTile * kTinyTile, 0, c->stream>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
+            ++c->launches;
+            return check_cuda(c, cudaGetLastError(), "gemm launch");
+        }
+        const dim3 g4((unsigned)ceil_div(m, 16), (unsigned)ceil_div(n, 16));
+        if (g4.y <= 65535 && (int64_t)g4.x * g4.y <= 4 * c->num_sms) {
+            gemm_simt_kernel<T, 1, 1, 16, ARM, BRM><<<g4, 256, 0, c->stream>>>(m, n, k, alpha, A, lda, B, ldb, beta, C,
+                                                                              ldc);
             ++c->launches;
             return check_cuda(c, cudaGetLastError(), "gemm launch");
         }
@@ -195,7 +203,7 @@ __global__ void scale_kernel(int64_t m, int64_t n, T* C, int64_t si, int64_t sj,
 
 template <typename T>
 tmvg_status gemm(Context* c, int64_t m, int64_t n, int64_t k, T alpha,
-                 Mat<const T> A, Mat<const T> B, T beta, Mat<T> C)
+                 Mat<const T> A, Mat<const T> B, T beta, Mat<T> C, bool fma_pipe)
 {
     if (m < 0 || n < 0 || k < 0) return set_error(c, TMVG_BAD_ARG, "gemm: negative size");
     if (m == 0 || n == 0) return TMVG_OK;
@@ -212,7 +220,7 @@ tmvg_status gemm(Context* c, int64_t m, int64_t n, int64_t k, T alpha,
         if (!(C.sj == 1 || n == 1))
             return set_error(c, TMVG_BAD_ARG, "gemm: C must be column- or row-major");
         return gemm<T>(c, n, m, k, alpha, Mat<const T>{B.p, B.sj, B.si},
-                       Mat<const T>{A.p, A.sj, A.si}, beta, Mat<T>{C.p, C.sj, C.si});
+                       Mat<const T>{A.p, A.sj, A.si}, beta, Mat<T>{C.p, C.sj, C.si}, fma_pipe);
     }
     const int64_t ldc = (n == 1) ? std::max<int64_t>(m, 1) : C.sj;
     // Operand classification: column-major usable when stepi == 1 (or one
@@ -236,7 +244,7 @@ tmvg_status gemm(Context* c, int64_t m, int64_t n, int64_t k, T alpha,
     if (!classify(m, k, A.si, A.sj, arm, lda) || !classify(k, n, B.si, B.sj, brm, ldb))
         return set_error(c, TMVG_BAD_ARG, "gemm: A and B must be column- or row-major");
     if constexpr (std::is_same<T, double>::value) {
-        if (sliced_wanted(c, m, n, k)) {
+        if (!fma_pipe && sliced_wanted(c, m, n, k)) {
             const tmvg_status st = sliced_gemm(c, m, n, k, alpha, Mat<const double>{A.p, arm ? lda : 1, arm ? 1 : lda},
                                                Mat<const double>{B.p, brm ? ldb : 1, brm ? 1 : ldb}, beta, C.p, ldc);
             if (st != TMVG_UNSUPPORTED) return st;
@@ -251,8 +259,8 @@ tmvg_status gemm(Context* c, int64_t m, int64_t n, int64_t k, T alpha,
 }
 
 template tmvg_status gemm<double>(Context*, int64_t, int64_t, int64_t, double, Mat<const double>,
-                                  Mat<const double>, double, Mat<double>);
+                                  Mat<const double>, double, Mat<double>, bool);
 template tmvg_status gemm<float>(Context*, int64_t, int64_t, int64_t, float, Mat<const float>,
-                                 Mat<const float>, float, Mat<float>);
+                                 Mat<const float>, float, Mat<float>, bool);
 
 }  // namespace tmvg

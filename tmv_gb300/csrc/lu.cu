@@ -2704,6 +2704,13 @@ __global__ void scatter_cols_kernel(int64_t n, const int* __restrict__ perm, con
 // zero above row block c, so block step kb solves and updates only the
 // columns [0, kb + w) (n^3/3 flops); U^-1 (L^-1) is the dense upper solve
 // (n^3 flops).  A zero U(j,j) is reported as singular.
+//
+// FP64: the diagonal blocks by their inverses (one launch for all of them, then
+// a product per step; TMV inverts its triangles by blocks too); a 64-step
+// substitution took 80 us of every step.  The block column of the identity
+// stays on the FP64 pipe: it is triangular, and its tiles would not be sliced.
+// Pairs of upper blocks share one update of K = 128, whose time is that of
+// K = 64 (n = 1501: inverse 8.1 -> 2.7 ms).
 template <typename T>
 static tmvg_status inverse_unpermuted(Context* c, int64_t n, const T* LU, int64_t lda, T* Y)
 {
@@ -2711,16 +2718,53 @@ static tmvg_status inverse_unpermuted(Context* c, int64_t n, const T* LU, int64_
     identity_kernel<T><<<blocks, 256, 0, c->stream>>>(n, Y, n);
     ++c->launches;
     tmvg_status st = check_cuda(c, cudaGetLastError(), "inverse: identity launch");
-    for (int64_t kb = 0; kb < n && !st; kb += kTriBlock) {
-        const int w = (int)std::min<int64_t>(kTriBlock, n - kb);
-        const int64_t cols = kb + w;
-        st = launch_tri_diag<T>(c, w, LU + kb + kb * lda, 1, lda, false, true, cols, Y + kb, 1, n, false);
-        if (!st && kb + w < n)
-            st = gemm<T>(c, n - kb - w, cols, w, T(-1), Mat<const T>{LU + (kb + w) + kb * lda, 1, lda},
-                         Mat<const T>{Y + kb, 1, n}, T(1), Mat<T>{Y + kb + w, 1, n});
+    if constexpr (std::is_same<T, double>::value) {
+        constexpr int64_t W = kTriBlock;
+        double *dl = nullptr, *du = nullptr;
+        if (!st) st = lu_inv64(c, n, LU, lda, &dl, &du);
+        auto below = [&](int64_t kb, int w, int64_t c0, int64_t nc, bool fma_pipe) {
+            return gemm<T>(c, n - kb - w, nc, w, T(-1), Mat<const T>{LU + (kb + w) + kb * lda, 1, lda},
+                           Mat<const T>{Y + kb + c0 * n, 1, n}, T(1), Mat<T>{Y + kb + w + c0 * n, 1, n}, fma_pipe);
+        };
+        for (int64_t kb = 0; kb < n && !st; kb += W) {
+            const int w = (int)std::min<int64_t>(W, n - kb);
+            // (the unit lower blocks are corrected up to 8 of them: beyond, the
+            // exact trailing products leave the residual below the
+            // substitution's without it, 3.4e-16 against 4.4e-16 at n = 513)
+            st = apply_inv64(c, w, kb + w, dl + kb * W, false, n <= 8 * W ? LU + kb + kb * lda : nullptr, lda, Y + kb,
+                             n);
+            if (kb + w >= n) break;
+            if (!st && kb > 0) st = below(kb, w, 0, kb, false);
+            if (!st) st = below(kb, w, kb, w, true);
+        }
+        // rows [r0, r1) of Y less U(r0:r1, k0:k1) X(k0:k1, :)
+        auto above = [&](int64_t r0, int64_t r1, int64_t k0, int64_t k1) {
+            return gemm<T>(c, r1 - r0, n, k1 - k0, T(-1), Mat<const T>{LU + r0 + k0 * lda, 1, lda},
+                           Mat<const T>{Y + k0, 1, n}, T(1), Mat<T>{Y + r0, 1, n});
+        };
+        for (int64_t hi = n; hi > 0 && !st;) {
+            const int64_t kb = (hi - 1) / W * W, lo = std::max<int64_t>(kb - W, 0);
+            st = apply_inv64(c, (int)(hi - kb), n, du + kb * W, true, LU + kb + kb * lda, lda, Y + kb, n);
+            if (!st && lo < kb) {
+                st = above(lo, kb, kb, hi);
+                if (!st) st = apply_inv64(c, (int)(kb - lo), n, du + lo * W, true, LU + lo + lo * lda, lda, Y + lo, n);
+            }
+            if (!st && lo > 0) st = above(0, lo, lo, hi);
+            hi = lo;
+        }
+        return st;
+    } else {
+        for (int64_t kb = 0; kb < n && !st; kb += kTriBlock) {
+            const int w = (int)std::min<int64_t>(kTriBlock, n - kb);
+            const int64_t cols = kb + w;
+            st = launch_tri_diag<T>(c, w, LU + kb + kb * lda, 1, lda, false, true, cols, Y + kb, 1, n, false);
+            if (!st && kb + w < n)
+                st = gemm<T>(c, n - kb - w, cols, w, T(-1), Mat<const T>{LU + (kb + w) + kb * lda, 1, lda},
+                             Mat<const T>{Y + kb, 1, n}, T(1), Mat<T>{Y + kb + w, 1, n});
+        }
+        if (!st) st = tri_solve<T>(c, n, LU, 1, lda, true, false, n, Y, 1, n, false);
+        return st;
     }
-    if (!st) st = tri_solve<T>(c, n, LU, 1, lda, true, false, n, Y, 1, n, false);
-    return st;
 }
 
 template <typename T>

@@ -56,20 +56,19 @@ constexpr int kInvCtas = 8;
 constexpr int kInvThreads = 128;
 constexpr int kInvLanes = 16;
 
-template <typename T>
-__global__ void __launch_bounds__(kInvThreads)
-tri_inv64_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t tsj, bool unit,
-                 T* __restrict__ dinv, int* __restrict__ sing)
+// CTA `part` of a block: load(i, j) gives entry (i, j) of the lower triangle
+// (i >= j, i < rows), store(i, j, v) takes an entry of the inverse (64 x 64,
+// zero above the diagonal).  Returns whether the diagonal has a zero (nothing
+// is stored then).
+template <typename T, typename Load, typename Store>
+__device__ __forceinline__ bool inv64(int part, int rows, bool unit, Load load, Store store)
 {
     __shared__ T D[kTrsvBlock][kTrsvBlock + 1];  // D[j][i] = D(i, j)
     __shared__ T rd[kTrsvBlock];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t b = blockIdx.x / kInvCtas, r0 = b * kTrsvBlock;
-    const int part = blockIdx.x % kInvCtas;
-    const int rows = (int)min((int64_t)kTrsvBlock, n - r0);
     for (int t = tid; t < kTrsvBlock * kTrsvBlock; t += kInvThreads) {
         const int rr = t % kTrsvBlock, cc = t / kTrsvBlock;
-        D[cc][rr] = (rr < rows && cc <= rr) ? tri[(r0 + rr) * tsi + (r0 + cc) * tsj] : T(0);
+        D[cc][rr] = (rr < rows && cc <= rr) ? load(rr, cc) : T(0);
     }
     __syncthreads();
     bool zero = false;
@@ -77,9 +76,7 @@ tri_inv64_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t tsj,
         zero = !unit && tid < rows && D[tid][tid] == T(0);
         rd[tid] = unit || tid >= rows || zero ? T(1) : T(1) / D[tid][tid];
     }
-    const bool any = __syncthreads_or(zero);
-    if (tid == 0 && part == 0) sing[b] = any;
-    if (any) return;
+    if (__syncthreads_or(zero)) return true;
     constexpr int NL = kInvLanes, NQ = kTrsvBlock / NL;
     static_assert(kInvCtas * (kInvThreads / NL) == kTrsvBlock, "a column per group of lanes");
     const int first = part * (kTrsvBlock / kInvCtas) + warp * (32 / NL);  // rows above a warp's columns stay zero
@@ -99,9 +96,138 @@ tri_inv64_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t tsj,
             if (NL * q + s > j) x[q] = r;
         }
     }
-    T* out = dinv + b * kTrsvBlock * kTrsvBlock;
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) out[(NL * q + s) * kTrsvBlock + col] = x[q];
+    for (int q = 0; q < NQ; ++q) store(NL * q + s, col, x[q]);
+    return false;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kInvThreads)
+tri_inv64_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t tsj, bool unit,
+                 T* __restrict__ dinv, int* __restrict__ sing)
+{
+    const int64_t b = blockIdx.x / kInvCtas, r0 = b * kTrsvBlock;
+    const int part = blockIdx.x % kInvCtas;
+    T* out = dinv + b * kTrsvBlock * kTrsvBlock;
+    const bool zero = inv64<T>(
+        part, (int)min((int64_t)kTrsvBlock, n - r0), unit,
+        [&](int i, int j) { return tri[(r0 + i) * tsi + (r0 + j) * tsj]; },
+        [&](int i, int j, T v) { out[i * kTrsvBlock + j] = v; });
+    if (threadIdx.x == 0 && part == 0) sing[b] = zero;
+}
+
+// The inverted 64-row diagonal blocks of both triangles of a packed LU
+// factor, for the inverse: unit lower blocks into dl, upper ones into du (64 x
+// 64 row-major each, in the matrix's own order).  A zero U(j,j) is singular.
+__global__ void __launch_bounds__(kInvThreads)
+lu_inv64_kernel(int64_t n, const double* __restrict__ LU, int64_t ld, double* __restrict__ dl,
+                double* __restrict__ du, int* err)
+{
+    const int64_t nblk = (n + kTrsvBlock - 1) / kTrsvBlock;
+    const int64_t bb = blockIdx.x / kInvCtas;
+    const bool up = bb >= nblk;
+    const int64_t b = up ? bb - nblk : bb, r0 = b * kTrsvBlock;
+    const int part = blockIdx.x % kInvCtas, rows = (int)min((int64_t)kTrsvBlock, n - r0);
+    const double* d = LU + r0 + r0 * ld;
+    double* out = (up ? du : dl) + b * kTrsvBlock * kTrsvBlock;
+    // an upper block is the lower one of its reversed indices
+    const bool zero = inv64<double>(
+        part, rows, !up, [&](int i, int j) { return up ? d[rows - 1 - i + (rows - 1 - j) * ld] : d[i + j * ld]; },
+        [&](int i, int j, double v) {
+            if (!up) out[i * kTrsvBlock + j] = v;
+            else if (i < rows && j < rows) out[(rows - 1 - i) * kTrsvBlock + (rows - 1 - j)] = v;
+        });
+    if (zero && threadIdx.x == 0) atomicCAS(err, (int)kDevOk, (int)kDevSingular);
+}
+
+tmvg_status lu_inv64(Context* c, int64_t n, const double* LU, int64_t ld, double** dl, double** du)
+{
+    const int64_t nblk = ceil_div(n, kTrsvBlock);
+    const size_t part = (size_t)nblk * kTrsvBlock * kTrsvBlock;
+    double* w = (double*)trsv_dinv_buffer(c, sizeof(double) * 2 * part);
+    if (!w) return set_error(c, TMVG_OOM, "inverse blocks");
+    *dl = w;
+    *du = w + part;
+    lu_inv64_kernel<<<(unsigned)(2 * nblk) * kInvCtas, kInvThreads, 0, c->stream>>>(n, LU, ld, *dl, *du, c->dflags);
+    ++c->launches;
+    return check_cuda(c, cudaGetLastError(), "inverse blocks");
+}
+
+// Y (w x cols, leading dimension ld) := D^-1 Y for one diagonal block from its
+// inverse: 64 rows x 8 columns per CTA, two entries per thread, corrected once,
+// y + D^-1 (b - D y) with y = D^-1 b, so that an ill-conditioned block costs no
+// accuracy (without it the residual of the inverse of a 65 x 65 matrix of
+// condition 1e10 grew 7-fold).  t is the block in the matrix: upper, or unit
+// lower; null: no correction.  Bound: the FP64 pipe.
+constexpr int kApplyCols = 8;
+__global__ void __launch_bounds__(256)
+apply_inv64_kernel(int w, int64_t cols, const double* __restrict__ dinv, bool upper, const double* __restrict__ t,
+                   int64_t ldt, double* Y, int64_t ld)
+{
+    __shared__ double D[kTrsvBlock][kTrsvBlock + 1];
+    __shared__ double y[kTrsvBlock][kApplyCols];
+    const int tid = threadIdx.x, i = tid & 63, g = tid >> 6;
+    const int64_t c0 = (int64_t)blockIdx.x * kApplyCols;
+    for (int q = tid; q < kTrsvBlock * kTrsvBlock; q += 256) {
+        const int rr = q / kTrsvBlock, cc = q % kTrsvBlock;
+        D[rr][cc] = rr < w && cc < w ? dinv[q] : 0.0;
+    }
+    double b[2], v[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        b[e] = i < w && c0 + g + 4 * e < cols ? Y[i + (c0 + g + 4 * e) * ld] : 0.0;
+        y[i][g + 4 * e] = b[e];
+    }
+    __syncthreads();
+    // entries beyond the diagonal take no part, whatever y holds there
+    const int k0 = upper ? i & ~31 : 0, k1 = upper ? kTrsvBlock : (i | 31) + 1;
+    auto times_inverse = [&] {
+        v[0] = v[1] = 0.0;
+#pragma unroll 8
+        for (int k = k0; k < k1; ++k) {
+            if (upper ? k < i : k > i) continue;
+            const double d = D[i][k];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) v[e] = fma(d, y[k][g + 4 * e], v[e]);
+        }
+    };
+    auto share = [&](const double(&x)[2]) {
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 2; ++e) y[i][g + 4 * e] = x[e];
+        __syncthreads();
+    };
+    times_inverse();
+    if (t) {
+        const double first[2] = {v[0], v[1]};
+        share(first);
+        double r[2] = {0.0, 0.0};
+#pragma unroll 8
+        for (int k = k0; k < k1; ++k) {
+            if ((upper ? k < i : k > i) || k >= w || i >= w) continue;
+            const double d = !upper && k == i ? 1.0 : __ldg(&t[i + k * ldt]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) r[e] = fma(d, y[k][g + 4 * e], r[e]);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) r[e] = b[e] - r[e];
+        share(r);
+        times_inverse();
+#pragma unroll
+        for (int e = 0; e < 2; ++e) v[e] += first[e];
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+        if (i < w && c0 + g + 4 * e < cols) Y[i + (c0 + g + 4 * e) * ld] = v[e];
+}
+
+tmvg_status apply_inv64(Context* c, int w, int64_t cols, const double* dinv, bool upper, const double* t, int64_t ldt,
+                        double* Y, int64_t ld)
+{
+    apply_inv64_kernel<<<(unsigned)ceil_div(cols, (int64_t)kApplyCols), 256, 0, c->stream>>>(w, cols, dinv, upper, t,
+                                                                                           ldt, Y, ld);
+    ++c->launches;
+    return check_cuda(c, cudaGetLastError(), "inverse block product");
 }
 
 // v / d from r, the correctly rounded reciprocal of d: v r and one correction
