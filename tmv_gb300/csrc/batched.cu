@@ -108,19 +108,58 @@ constexpr bool kStageU12 = sizeof(T) == 4;
 __device__ __forceinline__ bool nz(double x) { return (__double_as_longlong(x) << 1) != 0; }
 __device__ __forceinline__ bool nz(float x) { return (__float_as_uint(x) << 1) != 0u; }
 
+// Pivot keys as ordered integers: a float's in its own 32 bits (a conversion
+// to double would take the FP64 pipe).
+__device__ __forceinline__ long long batch_ikey(double v, bool first, bool r2) { return pivot_ikey(v, first, r2); }
+__device__ __forceinline__ long long batch_ikey(float v, bool first, bool r2)
+{
+    const unsigned b = __float_as_uint(v) & 0x7fffffffu;
+    if (b > 0x7f800000u) return first ? (r2 ? 0LL : 0x7f800000LL) : -1LL;
+    return (long long)b;
+}
+template <typename T>
+constexpr long long kKeyMin = sizeof(T) == 8 ? 0x0010000000000000LL : 0x00800000LL;  // the smallest normal's
+
+// The lane that holds the warp's winner (largest key, lowest index): one
+// redux.sync of the keys' upper halves and a ballot, more only where those tie.
+__device__ __forceinline__ int batch_winner(long long key, int idx)
+{
+    // keys are >= -1 or LLONG_MIN (no candidate): their signed upper halves order them
+    const int hi = (int)(key >> 32);
+    const int mhi = __reduce_max_sync(0xffffffffu, hi);
+    bool in = hi == mhi;
+    unsigned m = __ballot_sync(0xffffffffu, in);
+    if (m & (m - 1)) {
+        const unsigned lo = in ? (unsigned)key : 0u;
+        const unsigned mlo = __reduce_max_sync(0xffffffffu, lo);  // (every lane takes part)
+        in = in && lo == mlo;
+        const unsigned i = in ? (unsigned)idx : 0xffffffffu;
+        const unsigned mi = __reduce_min_sync(0xffffffffu, i);
+        in = in && i == mi;
+        m = __ballot_sync(0xffffffffu, in);
+    }
+    return __ffs(m) - 1;
+}
+
+// Shared words of one CTA's factorisation (one set for every instance).
+constexpr int kBatchPairs = 32;  // row pairs of a panel: 2 PW
+struct BatchScratch {
+    long long key[kBatchThreads / 32];
+    int idx[kBatchThreads / 32];
+    double val[kBatchThreads / 32];
+    double inv;
+    int piv[kBatchPairs / 2];
+    int pairs[1 + 2 * kBatchPairs];
+};
+
 template <typename T, int PW>
 __device__ void factor_one(int64_t n, int64_t r, T* __restrict__ A, T* __restrict__ B,
-                           int64_t* __restrict__ P, T* smem)
+                           int64_t* __restrict__ P, T* smem, BatchScratch& sc)
 {
     constexpr int LDP = PW + 1;
     T* pan = smem;  // [256][LDP]
     T* u12s = smem + kBatchMaxN * LDP;  // FP32 only: U12 rows [PW][256]
-    __shared__ long long s_key[kBatchThreads / 32];
-    __shared__ long long s_idx[kBatchThreads / 32];
-    __shared__ long long w_key;
-    __shared__ long long w_idx;
-    __shared__ int s_piv[PW];
-    __shared__ int s_pairs[1 + 2 * kMaxPairs];
+    int* s_piv = sc.piv;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     bool prev_uf = false;
@@ -146,24 +185,39 @@ __device__ void factor_one(int64_t n, int64_t r, T* __restrict__ A, T* __restric
         for (int j = 0; j < w; ++j) {
             const bool r2 = r2_column(n, k0 + j) && !prev_uf;
             long long bk = LLONG_MIN;
-            long long bi = LLONG_MAX;
-            for (int rr = j + tid; rr < m; rr += kBatchThreads)
-                pivot_icombine(bk, bi, pivot_ikey(pan[rr * LDP + j], rr == j, r2), (long long)rr);
-            warp_pivot_ireduce(bk, bi);
-            if (lane == 0) { s_key[warp] = bk; s_idx[warp] = bi; }
-            __syncthreads();
-            if (warp == 0) {
-                bk = lane < kBatchThreads / 32 ? s_key[lane] : LLONG_MIN;
-                bi = lane < kBatchThreads / 32 ? s_idx[lane] : LLONG_MAX;
-                warp_pivot_ireduce(bk, bi);
-                if (lane == 0) { w_key = bk; w_idx = bi; }
+            int bi = INT_MAX;
+            T bv = T(0);
+            for (int rr = j + tid; rr < m; rr += kBatchThreads) {
+                const T v = pan[rr * LDP + j];
+                const long long key = batch_ikey(v, rr == j, r2);
+                if (key > bk) {  // (rows ascend: ties keep the first)
+                    bk = key;
+                    bi = rr;
+                    bv = v;
+                }
+            }
+            if (lane == batch_winner(bk, bi)) {
+                sc.key[warp] = bk;
+                sc.idx[warp] = bi;
+                if constexpr (sizeof(T) == 8) sc.val[warp] = bv;
             }
             __syncthreads();
-            const int wi = (int)w_idx;
-            // the winning key is the bits of |pivot| (0 or inf bits for a NaN
-            // first element): TMV_Underflow is a comparison of bit patterns
-            if (w_key < __double_as_longlong(std::is_same<T, double>::value ? 2.2250738585072014e-308
-                                                                            : 1.1754943508222875e-38)) {
+            // every thread takes the winner of the four warps
+            long long wk = sc.key[0];
+            int wi = sc.idx[0], ww = 0;
+#pragma unroll
+            for (int q = 1; q < kBatchThreads / 32; ++q) {
+                const long long k2 = sc.key[q];
+                const int i2 = sc.idx[q];
+                if (k2 > wk || (k2 == wk && i2 < wi)) {
+                    wk = k2;
+                    wi = i2;
+                    ww = q;
+                }
+            }
+            // TMV_Underflow is a comparison of bit patterns (a NaN first
+            // element counts as 0 or infinity)
+            if (wk < kKeyMin<T>) {
                 if (tid == 0) s_piv[j] = (int)(k0 + j);
                 for (int rr = j + tid; rr < m; rr += kBatchThreads) pan[rr * LDP + j] = T(0);
                 prev_uf = true;
@@ -175,8 +229,14 @@ __device__ void factor_one(int64_t n, int64_t r, T* __restrict__ A, T* __restric
                     pan[j * LDP + tid] = pan[wi * LDP + tid];
                     pan[wi * LDP + tid] = t;
                 }
+                // the reciprocal by one warp (an FP64 one is about seven
+                // operations of 64 clocks for each warp that takes it)
+                if (sizeof(T) == 8 && warp == 1) {
+                    const double inv1 = 1.0 / sc.val[ww];
+                    if (lane == 0) sc.inv = inv1;
+                }
                 __syncthreads();
-                const T inv = T(1) / pan[j * LDP + j];
+                const T inv = sizeof(T) == 8 ? (T)sc.inv : T(1) / pan[j * LDP + j];
                 for (int rr = j + 1 + tid; rr < m; rr += kBatchThreads) {
                     T* row = pan + rr * LDP;
                     const T l = row[j] * inv;
@@ -193,14 +253,14 @@ __device__ void factor_one(int64_t n, int64_t r, T* __restrict__ A, T* __restric
         for (int j = tid; j < w; j += kBatchThreads) P[k0 + j] = s_piv[j];
         // interchanges on the other columns of A and on B: the panel's swaps
         // as (dst, src) row pairs, applied per column as one gather
-        if (warp == 0) panel_row_pairs(k0, w, s_piv, s_pairs);
+        if (warp == 0) panel_row_pairs<kBatchPairs / 2, kBatchPairs>(k0, w, s_piv, sc.pairs);
         __syncthreads();
         {
-            const int np = s_pairs[0];
-            const int* dst = s_pairs + 1;
-            const int* src = s_pairs + 1 + kMaxPairs;
+            const int np = sc.pairs[0];
+            const int* dst = sc.pairs + 1;
+            const int* src = sc.pairs + 1 + kBatchPairs;
             // a warp per column, a lane per pair: at most 2 PW <= 32 rows move
-            static_assert(2 * PW <= 32, "one lane per row pair");
+            static_assert(2 * PW <= kBatchPairs && kBatchPairs <= 32, "one lane per row pair");
             for (int64_t col = warp; col < n + r; col += kBatchThreads / 32) {
                 if (col >= k0 && col < k0 + w) continue;
                 T* p = col < n ? A + col * n : B + (col - n) * n;
@@ -320,6 +380,11 @@ __device__ void lu_solve_staged(int64_t n, int64_t r, const T* __restrict__ LU, 
     // factor entries a thread loads ahead of their (zero-skipping) use
     constexpr int PF = sizeof(T) == 8 ? 8 : 16;
     static_assert(kSolveBlock % PF == 0, "whole prefetch groups");
+    // the diagonal blocks: lane (dl, dq) takes right-hand side dq and every
+    // dgrp-th row, so that few right-hand sides still fill the warp
+    int dcols = 1;
+    while (dcols < r) dcols *= 2;
+    const int dgrp = 32 / dcols, dq = lane % dcols, dl = lane / dcols;
     // the diagonal block into dg, eight loads in flight per thread
     auto stage = [&](int j0, int jb) {
         for (int t0 = tid; t0 < jb * jb; t0 += kBatchThreads * 8) {
@@ -341,12 +406,13 @@ __device__ void lu_solve_staged(int64_t n, int64_t r, const T* __restrict__ LU, 
             const int jb = (int)min((int64_t)kSolveBlock, n - j0);
             stage(j0, jb);
             __syncthreads();
-            if (warp == 0 && lane < r) {
-                T* xq = xs + lane * XS + j0;
+            if (warp == 0) {
+                T* xq = xs + dq * XS + j0;
                 for (int k = 0; k < jb; ++k) {
-                    const T xk = xq[k];
+                    const T xk = dq < r ? xq[k] : T(0);
                     if (nz(xk))
-                        for (int i = k + 1; i < jb; ++i) xq[i] -= dg[i * DS + k] * xk;
+                        for (int i = k + 1 + dl; i < jb; i += dgrp) xq[i] -= dg[i * DS + k] * xk;
+                    __syncwarp();
                 }
             }
             __syncthreads();
@@ -375,17 +441,26 @@ __device__ void lu_solve_staged(int64_t n, int64_t r, const T* __restrict__ LU, 
             const int j0 = max(0, j1 - kSolveBlock), jb = j1 - j0;
             stage(j0, jb);
             __syncthreads();
-            if (warp == 0 && lane < r) {
-                T* xq = xs + lane * XS + j0;
+            if (warp == 0) {
+                T* xq = xs + dq * XS + j0;
+                // the diagonal's reciprocals at once, a lane each
+                const T rd = T(1) / (lane < jb ? dg[lane * DS + lane] : T(1));
                 for (int k = jb - 1; k >= 0; --k) {
-                    T v = xq[k];
+                    T v = dq < r ? xq[k] : T(0);
+                    const T rk = __shfl_sync(0xffffffffu, rd, k);
+                    __syncwarp();  // every lane has read x_k
                     if (nz(v)) {
                         const T d = dg[k * DS + k];
-                        if (!nz(d)) *sing = 1;
-                        else xq[k] = v = v / d;
+                        if (!nz(d)) {
+                            *sing = 1;
+                        } else {
+                            v = quotient(v, d, rk);
+                            if (dl == 0) xq[k] = v;
+                        }
                     }
                     if (nz(v))
-                        for (int i = 0; i < k; ++i) xq[i] -= dg[i * DS + k] * v;
+                        for (int i = dl; i < k; i += dgrp) xq[i] -= dg[i * DS + k] * v;
+                    __syncwarp();
                 }
             }
             __syncthreads();
@@ -418,12 +493,12 @@ __device__ void lu_solve_staged(int64_t n, int64_t r, const T* __restrict__ LU, 
 
 template <int PW>
 __device__ void factor_solve_one(int64_t n, int64_t r, double* __restrict__ A, double* __restrict__ B,
-                                 int64_t* __restrict__ P, int* __restrict__ status, double* smem)
+                                 int64_t* __restrict__ P, int* __restrict__ status, double* smem, BatchScratch& sc,
+                                 int& s_sing)
 {
-    __shared__ int s_sing;
     const int tid = threadIdx.x;
     if (tid == 0) s_sing = 0;
-    factor_one<double, PW>(n, r, A, B, P, smem);
+    factor_one<double, PW>(n, r, A, B, P, smem, sc);
 
     // Solve: B holds P B; L (unit) then U (lu_solve_staged)
     if (r > 0) {
@@ -449,7 +524,8 @@ __global__ void __launch_bounds__(kBatchThreads, 4)
 batched_lu_kernel(const BatchDev* __restrict__ args, unsigned* queue)
 {
     extern __shared__ __align__(16) double bsmem[];
-    __shared__ int s_item;
+    __shared__ int s_item, s_sing;
+    __shared__ BatchScratch sc;
     const BatchDev& a = *args;
     for (;;) {
         if (threadIdx.x == 0) s_item = (int)atomicAdd(queue, 1u);
@@ -463,8 +539,8 @@ batched_lu_kernel(const BatchDev* __restrict__ args, unsigned* queue)
         double* B = a.B + a.b_off[s];
         int64_t* P = a.P + a.p_off[s];
         int* st = a.status + s;
-        if (a.pw[size_class(n)] == 8) factor_solve_one<8>(n, r, A, B, P, st, bsmem);
-        else factor_solve_one<16>(n, r, A, B, P, st, bsmem);
+        if (a.pw[size_class(n)] == 8) factor_solve_one<8>(n, r, A, B, P, st, bsmem, sc, s_sing);
+        else factor_solve_one<16>(n, r, A, B, P, st, bsmem, sc, s_sing);
         __syncthreads();
     }
 }
@@ -496,16 +572,23 @@ __device__ __forceinline__ double nan_max_abs(double a, double b)
     return (x != x || y != y) ? __longlong_as_double(0x7ff8000000000000LL) : fmax(x, y);
 }
 
+// Its shared words, likewise one set: two instances' own took the memory of
+// the fourth CTA per SM.
+struct MixedScratch {
+    unsigned long long anorm;
+    unsigned long long bn[kBatchMaxRhs], rn[kBatchMaxRhs], xn[kBatchMaxRhs];
+    int inv[kBatchMaxN];  // row i of r goes to position inv[i] of P r
+    int sing, done;
+};
+
 template <int PW>
-__device__ void mixed_one(const BatchDev& d, int s, unsigned char* smem_raw)
+__device__ void mixed_one(const BatchDev& d, int s, unsigned char* smem_raw, BatchScratch& sc, MixedScratch& ms)
 {
     constexpr int XS = kBatchMaxN + 1;
     constexpr int RPT = kBatchMaxN / kBatchThreads;  // rows per thread in the residual
     static_assert(RPT == 2, "the residual loop handles two row blocks");
-    __shared__ unsigned long long s_anorm;
-    __shared__ unsigned long long s_bn[kBatchMaxRhs], s_rn[kBatchMaxRhs], s_xn[kBatchMaxRhs];
-    __shared__ int s_inv[kBatchMaxN];  // row i of r goes to position s_inv[i] of P r
-    __shared__ int s_sing, s_done;
+    unsigned long long &s_anorm = ms.anorm, *s_bn = ms.bn, *s_rn = ms.rn, *s_xn = ms.xn;
+    int *s_inv = ms.inv, &s_sing = ms.sing, &s_done = ms.done;
 
     const int tid = threadIdx.x;
     const int64_t n = d.n[s], r = d.nrhs[s];
@@ -528,7 +611,7 @@ __device__ void mixed_one(const BatchDev& d, int s, unsigned char* smem_raw)
     }
     __syncthreads();
     // 2. FP32 factorisation (interchanges on As only: b stays in place)
-    factor_one<float, PW>(n, 0, As, nullptr, P, reinterpret_cast<float*>(smem_raw));
+    factor_one<float, PW>(n, 0, As, nullptr, P, reinterpret_cast<float*>(smem_raw), sc);
     __syncthreads();
     // the gather of P r: apply the interchanges to the identity, invert
     if (tid == 0) {
@@ -662,6 +745,8 @@ batched_mixed_kernel(const BatchDev* __restrict__ args, unsigned* queue)
 {
     extern __shared__ __align__(16) unsigned char bsmem_mixed[];
     __shared__ int s_item;
+    __shared__ BatchScratch sc;
+    __shared__ MixedScratch ms;
     const BatchDev& a = *args;
     for (;;) {
         if (threadIdx.x == 0) s_item = (int)atomicAdd(queue, 1u);
@@ -670,8 +755,8 @@ batched_mixed_kernel(const BatchDev* __restrict__ args, unsigned* queue)
         __syncthreads();
         if (item >= a.count) return;
         const int s = a.order[item];
-        if (a.pw[size_class(a.n[s])] == 8) mixed_one<8>(a, s, bsmem_mixed);
-        else mixed_one<16>(a, s, bsmem_mixed);
+        if (a.pw[size_class(a.n[s])] == 8) mixed_one<8>(a, s, bsmem_mixed, sc, ms);
+        else mixed_one<16>(a, s, bsmem_mixed, sc, ms);
     }
 }
 

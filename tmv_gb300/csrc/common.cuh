@@ -247,6 +247,32 @@ __device__ __forceinline__ bool underflows<double>(double a) { return a < 2.2250
 template <>
 __device__ __forceinline__ bool underflows<float>(double a) { return a < 1.1754943508222875e-38; }
 
+// v / d from r, the correctly rounded reciprocal of d: v r and one correction
+// by the remainder (Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", 1990) -- three dependent FP64 operations on the
+// chain of a substitution instead of a division; the division itself where a
+// magnitude is too near the ends of the range for the remainder to be exact.
+template <typename T>
+__device__ __forceinline__ T quotient(T v, T d, T r)
+{
+    if constexpr (sizeof(T) == 8) {
+        const T q0 = v * r;
+        const T q = fma(fma(-q0, d, v), r, q0);
+        auto mid = [](double x) { return (((unsigned)__double2hiint(x) >> 20) & 0x7ff) - 100u < 1846u; };
+        return mid(q) && mid(v) && mid(d) && mid(r) ? q : v / d;
+    } else {
+        return v / d;
+    }
+}
+
+template <typename T>
+__device__ __forceinline__ bool nonzero(T v)
+{
+    // (a comparison of doubles would take the FP64 pipe)
+    if constexpr (sizeof(T) == 8) return (__double_as_longlong(v) << 1) != 0;
+    else return v != T(0);
+}
+
 // ---------------------------------------------------------------------
 // Grid barrier for cooperative launches (all CTAs co-resident).
 // `counter` is a monotonically increasing word zeroed before the launch; the

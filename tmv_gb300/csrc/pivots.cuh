@@ -23,10 +23,12 @@ constexpr int kPairsPanelMax = 128;
 // ---------------------------------------------------------------------
 constexpr int kMaxPairs = 2 * kPairsPanelMax;
 
+// (CAP: largest nb; MAXP: distance of the dst and src arrays)
+template <int CAP = kPairsPanelMax, int MAXP = kMaxPairs>
 __device__ inline void panel_row_pairs(int64_t k, int nb, const int* piv, int* pairs)
 {
-    __shared__ int lab[2 * kPairsPanelMax];  // the row whose content each slot holds
-    __shared__ short slot[kPairsPanelMax];   // the slot step t exchanges with slot t
+    __shared__ int lab[2 * CAP];  // the row whose content each slot holds
+    __shared__ short slot[CAP];   // the slot step t exchanges with slot t
     const int lane = threadIdx.x & 31;
     for (int t = lane; t < nb; t += 32) {
         const int p = piv[t];
@@ -61,7 +63,7 @@ __device__ inline void panel_row_pairs(int64_t k, int nb, const int* piv, int* p
         if (moved) {
             const int q = np + __popc(m & ((1u << lane) - 1u));
             pairs[1 + q] = row;
-            pairs[1 + kMaxPairs + q] = lab[s];
+            pairs[1 + MAXP + q] = lab[s];
         }
         np += __popc(m);
     }

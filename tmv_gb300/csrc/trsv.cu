@@ -230,32 +230,6 @@ tmvg_status apply_inv64(Context* c, int w, int64_t cols, const double* dinv, boo
     return check_cuda(c, cudaGetLastError(), "inverse block product");
 }
 
-// v / d from r, the correctly rounded reciprocal of d: v r and one correction
-// by the remainder (Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000 processor", 1990) -- three dependent FP64 operations on the
-// chain of a substitution instead of a division; the division itself where a
-// magnitude is too near the ends of the range for the remainder to be exact.
-template <typename T>
-__device__ __forceinline__ T quotient(T v, T d, T r)
-{
-    if constexpr (sizeof(T) == 8) {
-        const T q0 = v * r;
-        const T q = fma(fma(-q0, d, v), r, q0);
-        auto mid = [](double x) { return (((unsigned)__double2hiint(x) >> 20) & 0x7ff) - 100u < 1846u; };
-        return mid(q) && mid(v) && mid(d) && mid(r) ? q : v / d;
-    } else {
-        return v / d;
-    }
-}
-
-template <typename T>
-__device__ __forceinline__ bool nonzero(T v)
-{
-    // (a comparison of doubles would take the FP64 pipe)
-    if constexpr (sizeof(T) == 8) return (__double_as_longlong(v) << 1) != 0;
-    else return v != T(0);
-}
-
 // A published entry of the solution and the launch's epoch in one word that
 // is stored and loaded whole, so a consumer polls the value itself: no flag,
 // no fence, one L2 round trip.
