@@ -9,7 +9,7 @@
 // src/TMV_LUDiv.cpp:186).  status[s] = 1 when a zero U(j,j) met a nonzero
 // (TMV's SingularUpperTriMatrix), else 0.
 //
-// Kernel: grid = SMs x resident CTAs (128 threads, four per SM, so that one
+// Kernel: grid = SMs x resident CTAs (128 threads, five per SM, so that one
 // CTA's barrier-bound phases overlap another's FMA work); each CTA repeatedly takes the next
 // system from an atomic queue over `order` (largest n first, so the tail of
 // the launch holds the small systems) and runs, for n <= 256:
@@ -520,7 +520,7 @@ __device__ void factor_solve_one(int64_t n, int64_t r, double* __restrict__ A, d
     if (tid == 0) *status = s_sing;
 }
 
-__global__ void __launch_bounds__(kBatchThreads, 4)
+__global__ void __launch_bounds__(kBatchThreads, 5)
 batched_lu_kernel(const BatchDev* __restrict__ args, unsigned* queue)
 {
     extern __shared__ __align__(16) double bsmem[];
@@ -558,19 +558,14 @@ batched_lu_kernel(const BatchDev* __restrict__ args, unsigned* queue)
 // converged, 1 a zero U(j,j) of the FP32 factors met a nonzero, 2 not
 // converged within max_iter corrections (B holds the last iterate).
 // ---------------------------------------------------------------------
-__device__ __forceinline__ void smem_max_abs(unsigned long long* slot, double v)
+// |v| as an ordered integer: non-negative doubles order like their bit
+// patterns, and a NaN's lie above infinity's, so a NaN is kept by a maximum
+// (which so takes no FP64 issue slots).
+__device__ __forceinline__ unsigned long long abs_bits(double v)
 {
-    // non-negative doubles order like their bit patterns; a NaN is kept as NaN
-    const double a = fabs(v);
-    atomicMax(slot, (unsigned long long)__double_as_longlong(a != a ? __longlong_as_double(0x7ff8000000000000LL) : a));
+    return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
 }
-
-// max(|a|, |b|) with a NaN kept
-__device__ __forceinline__ double nan_max_abs(double a, double b)
-{
-    const double x = fabs(a), y = fabs(b);
-    return (x != x || y != y) ? __longlong_as_double(0x7ff8000000000000LL) : fmax(x, y);
-}
+__device__ __forceinline__ void smem_max_abs(unsigned long long* slot, double v) { atomicMax(slot, abs_bits(v)); }
 
 // Its shared words, likewise one set: two instances' own took the memory of
 // the fourth CTA per SM.
@@ -682,23 +677,23 @@ __device__ void mixed_one(const BatchDev& d, int s, unsigned char* smem_raw, Bat
 #pragma unroll
         for (int q = 0; q < kBatchMaxRhs; ++q) {
             if (q >= r) break;
-            double rm = 0.0, xm = 0.0;
+            unsigned long long rm = 0ull, xm = 0ull;
 #pragma unroll
             for (int u = 0; u < RPT; ++u) {
                 const int i = tid + u * kBatchThreads;
                 if (i >= n) continue;
                 ds[q * XS + s_inv[i]] = (float)acc[u][q];
-                rm = nan_max_abs(rm, acc[u][q]);
-                xm = nan_max_abs(xm, xs[q * XS + i]);
+                rm = max(rm, abs_bits(acc[u][q]));
+                xm = max(xm, abs_bits(xs[q * XS + i]));
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
-                rm = nan_max_abs(rm, __shfl_xor_sync(0xffffffffu, rm, o));
-                xm = nan_max_abs(xm, __shfl_xor_sync(0xffffffffu, xm, o));
+                rm = max(rm, __shfl_xor_sync(0xffffffffu, rm, o));
+                xm = max(xm, __shfl_xor_sync(0xffffffffu, xm, o));
             }
             if ((tid & 31) == 0) {
-                smem_max_abs(&s_rn[q], rm);
-                smem_max_abs(&s_xn[q], xm);
+                atomicMax(&s_rn[q], rm);
+                atomicMax(&s_xn[q], xm);
             }
         }
         __syncthreads();
