@@ -153,7 +153,7 @@ static tmvg_status drain_spans(Context* c)
     return TMVG_OK;
 }
 
-tmvg_status collect_device_error(Context* c, const char* what)
+tmvg_status collect_device_error(Context* c, const char* what, bool* retry)
 {
     tmvg_status st = check_cuda(
         c, cudaMemcpyAsync(c->hflags, c->dflags, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream),
@@ -165,6 +165,10 @@ tmvg_status collect_device_error(Context* c, const char* what)
     if (code == kDevOk) return TMVG_OK;
     cudaMemsetAsync(c->dflags, 0, 2 * sizeof(int), c->stream);
     cudaStreamSynchronize(c->stream);
+    if (code == kDevRetry && retry) {
+        *retry = true;
+        return TMVG_OK;
+    }
     if (code == kDevSingular)
         return set_error(c, TMVG_SINGULAR, std::string(what) + ": singular triangular factor");
     if (code == kDevTimeout)

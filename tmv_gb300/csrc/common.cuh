@@ -24,6 +24,7 @@ enum DevError : int {
     kDevOk = 0,
     kDevTimeout = 1,
     kDevSingular = 2,
+    kDevRetry = 3,  // the caller solves again another way
 };
 
 // Kernel classes timed by tmvg_timing_enable (the TMVG_KCLASS_* values).
@@ -162,7 +163,8 @@ void* perm_lists_buffer(Context* c, size_t bytes);
 void* trsv_dinv_buffer(Context* c, size_t bytes);
 void* trsv_words_buffer(Context* c, size_t bytes);
 // Reads and clears the device error word (synchronises the stream).
-tmvg_status collect_device_error(Context* c, const char* what);
+// With `retry`, kDevRetry is no error but sets it.
+tmvg_status collect_device_error(Context* c, const char* what, bool* retry = nullptr);
 
 // ---------------------------------------------------------------------
 // Pivot search keys.

@@ -230,6 +230,14 @@ tmvg_status apply_inv64(Context* c, int w, int64_t cols, const double* dinv, boo
     return check_cuda(c, cudaGetLastError(), "inverse block product");
 }
 
+// Entry (r, c) of the real form of complex data (see the solve kernel).
+template <typename T>
+__device__ __forceinline__ T real_form(const T* __restrict__ z, int64_t si, int64_t sj, T zsgn, int64_t r, int64_t c)
+{
+    const T* e = z + 2 * ((r >> 1) * si + (c >> 1) * sj);
+    return ((r ^ c) & 1) == 0 ? e[0] : (r & 1) ? zsgn * e[1] : -zsgn * e[1];
+}
+
 // A published entry of the solution and the launch's epoch in one word that
 // is stored and loaded whole, so a consumer polls the value itself: no flag,
 // no fence, one L2 round trip.
@@ -288,9 +296,15 @@ __device__ __forceinline__ bool finite(float v) { return (__float_as_uint(v) & 0
 // remains for a block with a zero diagonal, for n <= 64, and where the
 // corrected product is not finite.  n = 4096, one column: 0.82 / 1.72 ms with
 // the substitution and published flags.
-template <typename T, int NR>
+//
+// Z: a complex triangle in its real form, 2 x 2 blocks (re, -im; im, re), so
+// that n, B and the words are the interleaved parts; tsi and tsj are strides of
+// complex entries, zsgn is -1 for an index-reversed triangle (each pair is then
+// (im, re)).  Such a block has no substitution here: where it would be needed
+// the launch records kDevRetry and the caller takes another solve.
+template <typename T, int NR, bool Z>
 __global__ void __launch_bounds__(kTrsvThreads)
-trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t tsj, bool unit,
+trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t tsj, T zsgn, bool unit,
                       int64_t nrhs, int groups, T* B, int64_t bsi, int64_t bsj, bool skip_zero,
                       void* pub, unsigned epoch, unsigned long long* ticket,
                       unsigned long long tbase, unsigned spin_limit, int* err,
@@ -306,6 +320,11 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
 
     const int tid = threadIdx.x;
     const int i = tid & 63, g = tid >> 6;
+    const int last = Z ? i | 1 : i;  // the last column of row i in a diagonal block
+    auto at = [&](int64_t r, int64_t c) {
+        if constexpr (Z) return real_form(tri, tsi, tsj, zsgn, r, c);
+        else return tri[r * tsi + c * tsj];
+    };
     if (tid == 0) s_tk = (long long)(atomicAdd(ticket, 1ull) - tbase);
     __syncthreads();
     const int64_t nblk = (n + kTrsvBlock - 1) / kTrsvBlock;
@@ -325,11 +344,13 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
     T dg[16];  // D(i, 16 g ..), for the correction
 #pragma unroll
     for (int c = 0; c < 16; ++c)
-        dg[c] = (!use_inv || refine) && i < rows && g * 16 + c <= i ? tri[(r0 + i) * tsi + (r0 + g * 16 + c) * tsj] : T(0);
-    if (unit && i >= g * 16 && i < g * 16 + 16) {
+        dg[c] = (!use_inv || refine) && i < rows && g * 16 + c <= last ? at(r0 + i, r0 + g * 16 + c) : T(0);
+    if (unit) {
 #pragma unroll
-        for (int c = 0; c < 16; ++c)
-            if (g * 16 + c == i) dg[c] = T(1);
+        for (int c = 0; c < 16; ++c) {
+            const int k = g * 16 + c;
+            if (Z ? k >> 1 == i >> 1 : k == i) dg[c] = k == i ? T(1) : T(0);
+        }
     }
     if (use_inv) {
         const T* di = dinv + b * kTrsvBlock * kTrsvBlock;
@@ -347,7 +368,7 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
         T a[16];
 #pragma unroll
         for (int c = 0; c < 16; ++c)
-            a[c] = (i < rows) ? tri[(r0 + i) * tsi + (c0 + g * 16 + c) * tsj] : T(0);
+            a[c] = (i < rows) ? at(r0 + i, c0 + g * 16 + c) : T(0);
         bool late = false;
         if (holds) {
             T v = T(0);
@@ -396,7 +417,7 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
             for (int c = 0; c < 16; ++c)
 #pragma unroll
                 for (int q = 0; q < NR; ++q)
-                    if (g * 16 + c <= i) v[q] += Td[i][g * 16 + c] * xs[q][g * 16 + c];
+                    if (g * 16 + c <= last) v[q] += Td[i][g * 16 + c] * xs[q][g * 16 + c];
         };
         T v[NR];
         inverse_times_xs(v);
@@ -411,7 +432,7 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
             for (int c = 0; c < 16; ++c)
 #pragma unroll
                 for (int q = 0; q < NR; ++q)
-                    if (g * 16 + c <= i) v[q] += dg[c] * xs[q][g * 16 + c];
+                    if (g * 16 + c <= last) v[q] += dg[c] * xs[q][g * 16 + c];
             const T r = x - gather(v);
             share(r);
             inverse_times_xs(v);
@@ -424,7 +445,9 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
             }
         }
     }
-    if (!use_inv) {
+    if (Z) {
+        if (!use_inv && tid == 0) atomicCAS(err, (int)kDevOk, (int)kDevRetry);
+    } else if (!use_inv) {
 #pragma unroll
         for (int c = 0; c < 16; ++c) Td[i][g * 16 + c] = dg[c];
         __syncthreads();
@@ -473,28 +496,21 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
     }
 }
 
-template <typename T>
-tmvg_status trsm_sync_free(Context* c, int64_t n, const T* tri, int64_t tsi, int64_t tsj,
-                           bool upper, bool unit, int64_t nrhs, T* B, int64_t bsi, int64_t bsj,
-                           bool skip_zero)
+// One launch of the solve for an index-lower triangle (n rows; of its real
+// form when Z), from the inverted blocks dinv (null: substitution only).
+template <typename T, bool Z>
+static tmvg_status launch_trsm(Context* c, int64_t n, const T* tri, int64_t tsi, int64_t tsj, T zsgn, bool unit,
+                               int64_t nrhs, T* B, int64_t bsi, int64_t bsj, bool skip_zero, const T* dinv,
+                               const int* dsing, bool refine)
 {
-    if (n <= 0 || nrhs <= 0) return TMVG_OK;
-    if (upper) {
-        // reverse both index orders: U(n-1-i, n-1-j) is lower in (i, j)
-        tri = tri + (n - 1) * (tsi + tsj);
-        tsi = -tsi;
-        tsj = -tsj;
-        B = B + (n - 1) * bsi;
-        bsi = -bsi;
-    }
     const int64_t nblk = ceil_div(n, kTrsvBlock);
     // Columns per CTA: one up to kTrsvFewRhs, where the chain of blocks is
-    // the bound; two beyond (half the reads of the triangle), four where the
-    // flags would not suffice.
+    // the bound; two beyond (half the reads of the triangle), four where there
+    // would be too many CTAs.
     const int NR = nrhs <= kTrsvFewRhs<T> ? 1 : nblk * ceil_div(nrhs, (int64_t)2) <= (int64_t)kTrsvFlagCap ? 2 : 4;
     const int64_t groups = ceil_div(nrhs, (int64_t)NR);
     if (nblk * groups > (int64_t)kTrsvFlagCap)
-        return set_error(c, TMVG_UNSUPPORTED, "trsv: n x nrhs too large for the flag array");
+        return set_error(c, TMVG_UNSUPPORTED, "trsv: n x nrhs too large for one launch");
     if (++c->trsv_epoch == 0) ++c->trsv_epoch;  // 0 is the cleared words' tag
     const unsigned epoch = c->trsv_epoch;
     // tickets restart at 0 for every launch
@@ -514,28 +530,129 @@ tmvg_status trsm_sync_free(Context* c, int64_t n, const T* tri, int64_t tsi, int
     const unsigned grid = (unsigned)(nblk * groups);
     void* pub = trsv_words_buffer(c, 16 * (size_t)n * (size_t)(groups * NR));
     if (!pub) return set_error(c, TMVG_OOM, "trsv: published words");
+    auto kern = NR == 1   ? trsm_sync_free_kernel<T, 1, Z>
+                : NR == 2 ? trsm_sync_free_kernel<T, 2, Z>
+                          : trsm_sync_free_kernel<T, 4, Z>;
+    kern<<<grid, kTrsvThreads, 0, c->stream>>>(n, tri, tsi, tsj, zsgn, unit, nrhs, (int)groups, B, bsi, bsj, skip_zero,
+                                               pub, epoch, c->trsv_ticket, tbase, limit, c->dflags, dinv, dsing,
+                                               refine);
+    ++c->launches;
+    return check_cuda(c, cudaGetLastError(), "trsv launch");
+}
+
+// The buffer of the inverted blocks: their entries, then a flag per block.
+template <typename T>
+static tmvg_status inverse_blocks_buffer(Context* c, int64_t nblk, T** dinv, int** sing)
+{
+    const size_t ib = sizeof(T) * (size_t)nblk * kTrsvBlock * kTrsvBlock;
+    unsigned char* w = (unsigned char*)trsv_dinv_buffer(c, ib + sizeof(int) * (size_t)nblk);
+    if (!w) return set_error(c, TMVG_OOM, "trsv: inverse blocks");
+    *dinv = (T*)w;
+    *sing = (int*)(w + ib);
+    return TMVG_OK;
+}
+
+template <typename T>
+tmvg_status trsm_sync_free(Context* c, int64_t n, const T* tri, int64_t tsi, int64_t tsj,
+                           bool upper, bool unit, int64_t nrhs, T* B, int64_t bsi, int64_t bsj,
+                           bool skip_zero)
+{
+    if (n <= 0 || nrhs <= 0) return TMVG_OK;
+    if (upper) {
+        // reverse both index orders: U(n-1-i, n-1-j) is lower in (i, j)
+        tri = tri + (n - 1) * (tsi + tsj);
+        tsi = -tsi;
+        tsj = -tsj;
+        B = B + (n - 1) * bsi;
+        bsi = -bsi;
+    }
     // The diagonal blocks are inverted first (all but the only one).
+    const int64_t nblk = ceil_div(n, kTrsvBlock);
     const bool few = nrhs <= kTrsvFewRhs<T>;
-    const T* dinv = nullptr;
-    const int* dsing = nullptr;
+    T* dinv = nullptr;
+    int* dsing = nullptr;
     if (nblk > 1 || !few) {
-        const size_t ib = sizeof(T) * (size_t)nblk * kTrsvBlock * kTrsvBlock;
-        unsigned char* w = (unsigned char*)trsv_dinv_buffer(c, ib + sizeof(int) * (size_t)nblk);
-        if (!w) return set_error(c, TMVG_OOM, "trsv: inverse blocks");
-        T* dv = (T*)w;
-        int* ds = (int*)(w + ib);
-        tri_inv64_kernel<T><<<(unsigned)nblk * kInvCtas, kInvThreads, 0, c->stream>>>(n, tri, tsi, tsj, unit, dv, ds);
+        tmvg_status st = inverse_blocks_buffer(c, nblk, &dinv, &dsing);
+        if (st) return st;
+        tri_inv64_kernel<T><<<(unsigned)nblk * kInvCtas, kInvThreads, 0, c->stream>>>(n, tri, tsi, tsj, unit, dinv,
+                                                                                   dsing);
         ++c->launches;
         st = check_cuda(c, cudaGetLastError(), "trsv inverse blocks");
         if (st) return st;
-        dinv = dv;
-        dsing = ds;
     }
-    auto kern = NR == 1 ? trsm_sync_free_kernel<T, 1> : NR == 2 ? trsm_sync_free_kernel<T, 2> : trsm_sync_free_kernel<T, 4>;
-    kern<<<grid, kTrsvThreads, 0, c->stream>>>(n, tri, tsi, tsj, unit, nrhs, (int)groups, B, bsi, bsj, skip_zero, pub,
-                                               epoch, c->trsv_ticket, tbase, limit, c->dflags, dinv, dsing, few);
+    return launch_trsm<T, false>(c, n, tri, tsi, tsj, T(1), unit, nrhs, B, bsi, bsj, skip_zero, dinv, dsing, few);
+}
+
+// The inverted diagonal blocks of a complex triangle's real form: 32 complex
+// rows each.  With d the block's diagonal the block is diag(d) (I + N), N
+// strictly lower, whose real form is unit lower: its inverse, and then the
+// columns of pair k by the real form of 1 / d_k.
+__global__ void __launch_bounds__(kInvThreads)
+ztri_inv64_kernel(int64_t n, const double* __restrict__ z, int64_t tsi, int64_t tsj, double zsgn, bool unit,
+                  const double2* __restrict__ recip, int64_t rstep, double* __restrict__ dinv, int* __restrict__ sing)
+{
+    const int64_t b = blockIdx.x / kInvCtas, r0 = b * kTrsvBlock;
+    const int part = blockIdx.x % kInvCtas, rows = (int)min((int64_t)kTrsvBlock, n - r0);
+    double* out = dinv + b * kTrsvBlock * kTrsvBlock;
+    __shared__ double2 s_r[kTrsvBlock / 2];  // 1 / d, as the real form's pairs read it
+    bool zero = false;
+    if (threadIdx.x < kTrsvBlock / 2) {
+        double2 r = make_double2(1.0, 0.0);
+        if (!unit && (int)(2 * threadIdx.x) < rows) {
+            r = recip[(r0 / 2 + threadIdx.x) * rstep];
+            zero = r.x == 0.0 && r.y == 0.0;
+            r.y *= zsgn;
+        }
+        s_r[threadIdx.x] = r;
+    }
+    const bool any = __syncthreads_or(zero);
+    if (threadIdx.x == 0 && part == 0) sing[b] = any;
+    if (any) return;
+    inv64<double>(
+        part, rows, true,
+        [&](int i, int j) {
+            if (i >> 1 == j >> 1) return i == j ? 1.0 : 0.0;
+            // row pair i of 1/d times the block's column j
+            const double re = real_form(z, tsi, tsj, zsgn, r0 + (i & ~1), r0 + j);
+            const double im = real_form(z, tsi, tsj, zsgn, r0 + (i | 1), r0 + j);
+            const double2 r = s_r[i >> 1];
+            return (i & 1) ? r.x * im + r.y * re : r.x * re - r.y * im;
+        },
+        [&](int i, int j, double v) {
+            // the pair's other column is 16 lanes away
+            const double w = __shfl_xor_sync(0xffffffffu, v, kInvLanes);
+            const double2 r = s_r[j >> 1];
+            out[i * kTrsvBlock + j] = (j & 1) ? v * r.x - w * r.y : v * r.x + w * r.y;
+        });
+}
+
+tmvg_status ztrsm_sync_free(Context* c, int64_t n, const double* z, int64_t ld, bool upper, int64_t nrhs, double* X,
+                            const double2* recip)
+{
+    const int64_t N = 2 * n, nblk = ceil_div(N, kTrsvBlock);
+    double* dinv = nullptr;
+    int* dsing = nullptr;
+    tmvg_status st = inverse_blocks_buffer(c, nblk, &dinv, &dsing);
+    if (st) return st;
+    const double* tri = z;
+    int64_t si = 1, sj = ld, bsi = 1, rstep = 1;
+    double sgn = 1.0;
+    if (upper) {
+        tri = z + 2 * (n - 1) * (1 + ld);
+        si = -1;
+        sj = -ld;
+        X += N - 1;
+        bsi = -1;
+        recip += n - 1;
+        rstep = -1;
+        sgn = -1.0;
+    }
+    ztri_inv64_kernel<<<(unsigned)nblk * kInvCtas, kInvThreads, 0, c->stream>>>(N, tri, si, sj, sgn, !upper, recip, rstep,
+                                                                             dinv, dsing);
     ++c->launches;
-    return check_cuda(c, cudaGetLastError(), "trsv launch");
+    st = check_cuda(c, cudaGetLastError(), "trsv inverse blocks");
+    if (st) return st;
+    return launch_trsm<double, true>(c, N, tri, si, sj, sgn, !upper, nrhs, X, bsi, N, true, dinv, dsing, true);
 }
 
 // ---------------------------------------------------------------------
