@@ -308,7 +308,7 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
                       int64_t nrhs, int groups, T* B, int64_t bsi, int64_t bsj, bool skip_zero,
                       void* pub, unsigned epoch, unsigned long long* ticket,
                       unsigned long long tbase, unsigned spin_limit, int* err,
-                      const T* __restrict__ dinv, const int* __restrict__ dinv_sing, bool refine)
+                      const T* __restrict__ dinv, const int* __restrict__ dinv_sing, bool refine, int vec)
 {
     static_assert(NR <= kTrsvThreads / 64, "a thread per entry of a block's solution");
     __shared__ long long s_tk;
@@ -366,9 +366,21 @@ trsm_sync_free_kernel(int64_t n, const T* __restrict__ tri, int64_t tsi, int64_t
     for (int64_t j = 0; j < b; ++j) {
         const int64_t c0 = j * kTrsvBlock;
         T a[16];
+        if (!Z && sizeof(T) == 8 && vec) {
+            // rows contiguous: 16 bytes at a time (a sector is then read in
+            // two loads, not four; the CTAs of an SM leave little L1)
+            const T* p = tri + (r0 + i) * tsi + (c0 + g * 16) * tsj;
 #pragma unroll
-        for (int c = 0; c < 16; ++c)
-            a[c] = (i < rows) ? at(r0 + i, c0 + g * 16 + c) : T(0);
+            for (int u = 0; u < 8; ++u) {
+                double2 v = make_double2(0.0, 0.0);
+                if (i < rows) v = *reinterpret_cast<const double2*>(vec > 0 ? p + 2 * u : p - 2 * u - 1);
+                a[2 * u] = vec > 0 ? v.x : v.y;
+                a[2 * u + 1] = vec > 0 ? v.y : v.x;
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 16; ++c) a[c] = (i < rows) ? at(r0 + i, c0 + g * 16 + c) : T(0);
+        }
         bool late = false;
         if (holds) {
             T v = T(0);
@@ -533,9 +545,13 @@ static tmvg_status launch_trsm(Context* c, int64_t n, const T* tri, int64_t tsi,
     auto kern = NR == 1   ? trsm_sync_free_kernel<T, 1, Z>
                 : NR == 2 ? trsm_sync_free_kernel<T, 2, Z>
                           : trsm_sync_free_kernel<T, 4, Z>;
+    // 16-byte loads along contiguous rows, where every row's tiles are aligned
+    const T* lowest = tsj == -1 ? tri - 1 : tri;
+    const bool aligned = sizeof(T) == 8 && (reinterpret_cast<uintptr_t>(lowest) & 15) == 0 && tsi % 2 == 0;
+    const int vec = !Z && aligned && (tsj == 1 || tsj == -1) && tsi != 1 && tsi != -1 ? (int)tsj : 0;
     kern<<<grid, kTrsvThreads, 0, c->stream>>>(n, tri, tsi, tsj, zsgn, unit, nrhs, (int)groups, B, bsi, bsj, skip_zero,
                                                pub, epoch, c->trsv_ticket, tbase, limit, c->dflags, dinv, dsing,
-                                               refine);
+                                               refine, vec);
     ++c->launches;
     return check_cuda(c, cudaGetLastError(), "trsv launch");
 }

@@ -181,10 +181,13 @@ zlu_update_kernel(int64_t n, double2* A, int64_t lda, int64_t k)
 // root) is evaluated only where it can decide: a proxy key per row, the bits
 // of |z|^2 computed after scaling z by a power of two (two FP64 operations,
 // relative error below 2^-51), selects the rows within 256 ulps of |z|^2 of
-// the CTA's largest key; those get TMV_ABS and the largest TMV_ABS (lowest
-// row on ties) is the CTA's candidate.  TMV_ABS differs from |z| by at most a few
-// ulps, so no row outside the margin can hold the maximum.  Infinite and NaN
-// entries follow TMV_ABS (NaN): chosen only as the column's first entry.
+// the cluster's largest key.  TMV_ABS differs from |z| by at most a few ulps, so
+// no row outside the margin can hold the maximum: a single row within it is
+// the pivot, and every CTA takes TMV_InverseOf of its entry while the pivot row
+// travels.  Otherwise (rows that tie, a zero column, infinities, NaN) a second
+// exchange follows: the rows near each CTA's largest key get TMV_ABS, and the
+// largest of those (lowest row on ties) is the pivot.  Infinite and NaN entries
+// follow TMV_ABS (NaN): chosen only as the column's first entry.
 // ---------------------------------------------------------------------------
 constexpr int kZPanelCtas = 16;
 constexpr int kZPanelThreads = 512;
@@ -255,6 +258,10 @@ __device__ __forceinline__ long long zabs_key(double raw, bool first)
 
 template <int KB>
 struct ZPanelShared {
+    long long prox_key[2];     // this CTA's largest proxy key (LLONG_MIN: no row)
+    long long prox_row[2];     // its global row
+    double2 prox_z[2];         // its entry
+    int prox_near[2];          // rows of the CTA within the margin of it
     long long cand_key[2];     // this CTA's candidate: zabs_key (-2: none)
     double cand_abs[2];        // its TMV_ABS (NaN kept)
     long long cand_row[2];     // its global row (LLONG_MAX: none)
@@ -267,6 +274,52 @@ struct ZPanelShared {
     long long wkey[kZPanelThreads / 32];
     int wrow[kZPanelThreads / 32];
 };
+
+// The warp's winner (largest key, lowest index): one redux.sync and a ballot
+// unless the keys' upper halves tie.
+__device__ __forceinline__ int zkey_winner(long long key, int idx)
+{
+    const int hi = (int)(key >> 32);
+    const int mhi = __reduce_max_sync(0xffffffffu, hi);
+    bool in = hi == mhi;
+    unsigned m = __ballot_sync(0xffffffffu, in);
+    if (m & (m - 1)) {
+        const unsigned lo = in ? (unsigned)key : 0u;
+        const unsigned mlo = __reduce_max_sync(0xffffffffu, lo);  // (every lane takes part)
+        in = in && lo == mlo;
+        const unsigned i = in ? (unsigned)idx : 0xffffffffu;
+        const unsigned mi = __reduce_min_sync(0xffffffffu, i);
+        in = in && i == mi;
+        m = __ballot_sync(0xffffffffu, in);
+    }
+    return __ffs(m) - 1;
+}
+
+// Column j = k + jj of this CTA's rows below j scaled by the pivot's inverse,
+// the panel's later columns updated.
+template <int KB>
+__device__ __forceinline__ void zpanel_update(int64_t n, int64_t k, int kb, int jj, int rpc, int cta, int r0,
+                                              double2* s_rows, const double2* prow, double2 inv, bool under)
+{
+    for (int r = r0 + (int)threadIdx.x; r < rpc; r += kZPanelThreads) {
+        const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
+        if (i >= n) break;
+        if (i == k + jj) continue;
+        double2* row = &s_rows[r * (KB + 1)];
+        const double2 l = under ? make_double2(0.0, 0.0) : zmul(row[jj], inv);
+        row[jj] = l;
+#pragma unroll 4
+        for (int c = jj + 1; c < kb; ++c) {
+            const double2 u = prow[c];
+            double2 a = row[c];
+            a.x = fma(-l.x, u.x, a.x);
+            a.x = fma(l.y, u.y, a.x);
+            a.y = fma(-l.x, u.y, a.y);
+            a.y = fma(-l.y, u.x, a.y);
+            row[c] = a;
+        }
+    }
+}
 
 template <int KB>
 __global__ void __launch_bounds__(kZPanelThreads)
@@ -296,23 +349,97 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         const int lj = (d0 >= 0 && d0 % kZPanelCtas == 0) ? (int)(d0 / kZPanelCtas) : -1;
         // stage 1: largest proxy key (the first row's key kept for stage 2)
         long long bk = LLONG_MIN, key0 = LLONG_MIN;
+        int bp = INT_MAX;
         for (int r = r0 + tid; r < rpc; r += kZPanelThreads) {
             const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
             if (i >= n) break;
             const long long key = zproxy_key(s_rows[r * RS + jj], i == j);
             if (r == r0 + tid) key0 = key;
-            bk = key > bk ? key : bk;
+            if (key > bk) {
+                bk = key;
+                bp = r;
+            }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const long long ok = __shfl_xor_sync(0xffffffffu, bk, o);
-            bk = ok > bk ? ok : bk;
+        if (lane == zkey_winner(bk, bp)) {
+            sh.wkey[warp] = bk;
+            sh.wrow[warp] = bp;
         }
-        if (lane == 0) sh.wkey[warp] = bk;
         __syncthreads();
         long long mk = sh.wkey[0];
+        int mr = sh.wrow[0];
 #pragma unroll
-        for (int w = 1; w < kZPanelThreads / 32; ++w) mk = sh.wkey[w] > mk ? sh.wkey[w] : mk;
+        for (int w = 1; w < kZPanelThreads / 32; ++w)
+            if (sh.wkey[w] > mk) {
+                mk = sh.wkey[w];
+                mr = sh.wrow[w];
+            }
+        // the cluster's largest, and how many rows lie within the margin
+        int near = 0;
+        for (int r = r0 + tid; r < rpc; r += kZPanelThreads) {
+            if (k + cta + (int64_t)kZPanelCtas * r >= n) break;
+            const long long key =
+                r == r0 + tid ? key0 : zproxy_key(s_rows[r * RS + jj], k + cta + (int64_t)kZPanelCtas * r == j);
+            near += mk != LLONG_MIN && key >= mk - 64;
+        }
+        const int several = rpc > kZPanelThreads ? __syncthreads_or(near > 1) : 0;
+        near = __syncthreads_count(near > 0) + (several ? 1 : 0);
+        if (tid < kb) {
+            if (mr != INT_MAX) sh.cand_rowv[par][tid] = s_rows[mr * RS + tid];
+            if (lj >= 0) sh.diag_rowv[par][tid] = s_rows[lj * RS + tid];
+        }
+        if (tid == 0) {
+            sh.prox_key[par] = mk;
+            sh.prox_row[par] = mr == INT_MAX ? LLONG_MAX : k + cta + (long long)kZPanelCtas * mr;
+            sh.prox_z[par] = mr != INT_MAX ? s_rows[mr * RS + jj] : make_double2(0.0, 0.0);
+            sh.prox_near[par] = near;
+        }
+        cluster.sync();
+        const int owner_j = (int)((j - k) % kZPanelCtas);
+        {
+            long long ck = LLONG_MIN, cr = LLONG_MAX;
+            double2 cz = make_double2(0.0, 0.0);
+            int cn = 0;
+            if (lane < kZPanelCtas) {
+                ZPanelShared<KB>* o = cluster.map_shared_rank(&sh, lane);
+                ck = o->prox_key[par];
+                cr = o->prox_row[par];
+                cz = o->prox_z[par];
+                cn = o->prox_near[par];
+            }
+            const int wc = zkey_winner(ck, lane);
+            const long long gk = __shfl_sync(0xffffffffu, ck, wc);
+            const unsigned close = __ballot_sync(0xffffffffu, ck != LLONG_MIN && ck >= gk - 64);
+            const int gn = __shfl_sync(0xffffffffu, cn, wc);
+            // an ordinary key (neither zero nor not finite), alone in the margin
+            if (gk > kZKeyZero && gk < kZKeyNaNFirst && close == 1u << wc && gn == 1) {
+                const long long wr = __shfl_sync(0xffffffffu, cr, wc);
+                const double2 z = make_double2(__shfl_sync(0xffffffffu, cz.x, wc), __shfl_sync(0xffffffffu, cz.y, wc));
+                // (every warp of every CTA decides alike) below the normal
+                // range only if both parts are
+                const long long big = max(__double_as_longlong(z.x) & kZAbsBits, __double_as_longlong(z.y) & kZAbsBits);
+                if (big >= __double_as_longlong(4.0 * DBL_MIN)) {
+                    if (warp == 1) {
+                        const double2 inv1 = tmv_inverse_of(z);
+                        if (lane == 0) {
+                            sh.inv = inv1;
+                            sh.under = 0;
+                            if (cta == 0) P[j] = wr;
+                        }
+                    }
+                    if (tid < kb) {
+                        const double2 v = cluster.map_shared_rank(&sh, wc)->cand_rowv[par][tid];
+                        sh.prow[tid] = v;
+                        if (lj >= 0) s_rows[lj * RS + tid] = v;
+                        if (wr != j && (int)((wr - k) % kZPanelCtas) == cta)
+                            s_rows[(int)((wr - k) / kZPanelCtas) * RS + tid] =
+                                cluster.map_shared_rank(&sh.diag_rowv[par][0], owner_j)[tid];
+                    }
+                    __syncthreads();
+                    zpanel_update<KB>(n, k, kb, jj, rpc, cta, r0, s_rows, sh.prow, sh.inv, false);
+                    continue;
+                }
+            }
+        }
         // stage 2: TMV_ABS (and TMV_InverseOf) of the rows within 64 key units
         // (256 ulps of |z|^2) of the largest
         const long long thr = mk <= LLONG_MIN + 64 ? LLONG_MIN + 1 : mk - 64;
@@ -349,11 +476,8 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         for (int w = 1; w < kZPanelThreads / 32; ++w)
             if (sh.wkey[w] > ba || (sh.wkey[w] == ba && sh.wrow[w] < br)) { ba = sh.wkey[w]; br = sh.wrow[w]; }
         // stage the candidate (its owner thread writes its TMV_ABS and
-        // inverse) and, where owned, row j
-        if (tid < kb) {
-            if (br != INT_MAX) sh.cand_rowv[par][tid] = s_rows[br * RS + tid];
-            if (lj >= 0) sh.diag_rowv[par][tid] = s_rows[lj * RS + tid];
-        }
+        // inverse); row j is staged already
+        if (tid < kb && br != INT_MAX) sh.cand_rowv[par][tid] = s_rows[br * RS + tid];
         if (br != INT_MAX && (br - r0) % kZPanelThreads == tid && br >= r0) {
             sh.cand_abs[par] = braw;
             sh.cand_inv[par] = binv;
@@ -379,7 +503,6 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
             const int oc = __shfl_xor_sync(0xffffffffu, wc, o);
             if (oa > wa || (oa == wa && orow < wr)) { wa = oa; wr = orow; wc = oc; }
         }
-        const int owner_j = (int)((j - k) % kZPanelCtas);
         // U's row j: the pivot row (or row j with its column zeroed)
         if (tid < kb) {
             ZPanelShared<KB>* w = cluster.map_shared_rank(&sh, wc);
@@ -406,26 +529,7 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
             }
         }
         __syncthreads();
-        // scale and update this CTA's rows below j
-        const double2 inv = sh.inv;
-        const bool und = sh.under != 0;
-        for (int r = r0 + tid; r < rpc; r += kZPanelThreads) {
-            const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
-            if (i >= n) break;
-            if (i == j) continue;
-            double2* row = &s_rows[r * RS];
-            const double2 l = und ? make_double2(0.0, 0.0) : zmul(row[jj], inv);
-            row[jj] = l;
-            for (int c = jj + 1; c < kb; ++c) {
-                const double2 u = sh.prow[c];
-                double2 a = row[c];
-                a.x = fma(-l.x, u.x, a.x);
-                a.x = fma(l.y, u.y, a.x);
-                a.y = fma(-l.x, u.y, a.y);
-                a.y = fma(-l.y, u.x, a.y);
-                row[c] = a;
-            }
-        }
+        zpanel_update<KB>(n, k, kb, jj, rpc, cta, r0, s_rows, sh.prow, sh.inv, sh.under != 0);
         // (the next column reads only this thread's rows until its first
         // __syncthreads; sh.prow is rewritten only after the next cluster.sync)
     }
