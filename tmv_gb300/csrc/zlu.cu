@@ -24,6 +24,7 @@
 // Values agree with TMV's recursive factorisation to rounding; pivots are
 // TMV's wherever rounding does not decide a tie.
 #include "zlu.cuh"
+#include "async.cuh"
 #include "gemm_sliced.cuh"
 #include "trsv.cuh"
 
@@ -256,21 +257,35 @@ __device__ __forceinline__ long long zabs_key(double raw, bool first)
     return b;
 }
 
+// A CTA's candidate of one column, as sent to every CTA.
+struct __align__(16) ZMsg {
+    long long key;  // its largest proxy key (LLONG_MIN: no row)
+    long long row;  // the global row
+    int near;       // rows of the CTA within the margin of it
+    int pad[3];
+};
+
 template <int KB>
 struct ZPanelShared {
-    long long prox_key[2];     // this CTA's largest proxy key (LLONG_MIN: no row)
-    long long prox_row[2];     // its global row
-    double2 prox_z[2];         // its entry
-    int prox_near[2];          // rows of the CTA within the margin of it
-    long long cand_key[2];     // this CTA's candidate: zabs_key (-2: none)
-    double cand_abs[2];        // its TMV_ABS (NaN kept)
-    long long cand_row[2];     // its global row (LLONG_MAX: none)
-    double2 cand_inv[2];       // TMV_InverseOf of its entry
-    double2 cand_rowv[2][KB];  // its row's panel entries
-    double2 diag_rowv[2][KB];  // row j's panel entries (the CTA owning row j)
-    double2 prow[KB];          // the pivot row after the interchange: U's row j
+    // messages of the column, by its parity: every CTA's candidate and that
+    // row, and row j (from the CTA that holds it)
+    ZMsg msg[2][kZPanelCtas];
+    double2 rowv[2][kZPanelCtas][KB];
+    double2 diagv[2][KB];
+    double2 stage[2][2][KB];   // this CTA's rows on their way (candidate, row j)
+    double2 prow[2][KB];       // the pivot row after the interchange: U's row j
+    uint64_t mbar[2];
+    // the second exchange
+    long long cand_key;        // this CTA's candidate: zabs_key (-2: none)
+    double cand_abs;           // its TMV_ABS (NaN kept)
+    long long cand_row;        // its global row (LLONG_MAX: none)
+    double2 cand_inv;          // TMV_InverseOf of its entry
+    double2 cand_rowv[KB];     // its row's panel entries
+    double2 diag_rowv[KB];     // row j's panel entries (the CTA owning row j)
     double2 inv;
-    int under;
+    long long piv;             // the pivot's global row
+    int from;                  // the CTA it comes from; -1: the second exchange decides
+    int under, abort;
     long long wkey[kZPanelThreads / 32];
     int wrow[kZPanelThreads / 32];
 };
@@ -295,59 +310,65 @@ __device__ __forceinline__ int zkey_winner(long long key, int idx)
     return __ffs(m) - 1;
 }
 
-// Column j = k + jj of this CTA's rows below j scaled by the pivot's inverse,
-// the panel's later columns updated.
-template <int KB>
-__device__ __forceinline__ void zpanel_update(int64_t n, int64_t k, int kb, int jj, int rpc, int cta, int r0,
-                                              double2* s_rows, const double2* prow, double2 inv, bool under)
+// a - l u
+__device__ __forceinline__ double2 zfms(double2 a, double2 l, double2 u)
 {
-    for (int r = r0 + (int)threadIdx.x; r < rpc; r += kZPanelThreads) {
-        const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
-        if (i >= n) break;
-        if (i == k + jj) continue;
-        double2* row = &s_rows[r * (KB + 1)];
-        const double2 l = under ? make_double2(0.0, 0.0) : zmul(row[jj], inv);
-        row[jj] = l;
-#pragma unroll 4
-        for (int c = jj + 1; c < kb; ++c) {
-            const double2 u = prow[c];
-            double2 a = row[c];
-            a.x = fma(-l.x, u.x, a.x);
-            a.x = fma(l.y, u.y, a.x);
-            a.y = fma(-l.x, u.y, a.y);
-            a.y = fma(-l.y, u.x, a.y);
-            row[c] = a;
-        }
-    }
+    a.x = fma(-l.x, u.x, a.x);
+    a.x = fma(l.y, u.y, a.x);
+    a.y = fma(-l.x, u.y, a.y);
+    a.y = fma(-l.y, u.x, a.y);
+    return a;
 }
 
+// One column's chain carries only what the next pivot decision needs.  After
+// a decision a row is scaled and takes the update of the next column; the rest
+// of the step's rank-1 update (its multiplier is the row's own entry of column
+// j) is owed and paid while the next column's messages travel.  A candidate's
+// row is therefore sent as it stands, and the receiver applies what it owes, a
+// column per lane.  The exchange is one message per CTA and destination (the
+// key by st.async, the row by a bulk copy) on the receiver's mbarrier; only the
+// second exchange uses cluster barriers.  Messages are double-buffered by
+// column parity: a CTA sends for column j + 1 after all its threads are done
+// with column j, so when every message of j + 1 is in, j's buffers are free.
+// Waits are bounded; a CTA that gives up records kDevTimeout and the others
+// time out in turn.  Per column at m = 2048 (clocks): 17500 with cluster
+// barriers, remote reads by every warp and the whole update on the chain.
 template <int KB>
 __global__ void __launch_bounds__(kZPanelThreads)
 zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k, int kb, int64_t* __restrict__ P,
-                      int rpc)
+                      int rpc, int* err)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ double2 s_rows[];  // rpc rows, stride KB + 1
-    __shared__ ZPanelShared<KB> sh;
+    __shared__ __align__(16) ZPanelShared<KB> sh;
     constexpr int RS = KB + 1;
     const int cta = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        mbar_init(&sh.mbar[0], 1u);
+        mbar_init(&sh.mbar[1], 1u);
+        sh.abort = 0;
+        mbar_fence_init();
+    }
     // local row r is global row k + cta + 16 r
     for (int t = tid; t < rpc * kb; t += kZPanelThreads) {
         const int r = t % rpc, c = t / rpc;
         const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
         s_rows[r * RS + c] = i < n ? A[i + (k + c) * lda] : make_double2(0.0, 0.0);
     }
-    __syncthreads();
+    cluster.sync();  // every CTA's mbarriers are initialised before any message
     for (int jj = 0; jj < kb; ++jj) {
         const int par = jj & 1;
         const int64_t j = k + jj;
+        const int owner_j = jj % kZPanelCtas;
         // rows of this CTA at or below j: r >= r0
         const int64_t d0 = j - k - cta;
         const int r0 = d0 <= 0 ? 0 : (int)((d0 + kZPanelCtas - 1) / kZPanelCtas);
-        const int lj = (d0 >= 0 && d0 % kZPanelCtas == 0) ? (int)(d0 / kZPanelCtas) : -1;
-        // stage 1: largest proxy key (the first row's key kept for stage 2)
+        const int lj = cta == owner_j ? jj / kZPanelCtas : -1;
+        const double2* pold = sh.prow[par ^ 1];
+        double2* pnew = sh.prow[par];
+        // stage 1: largest proxy key (the first row's key kept)
         long long bk = LLONG_MIN, key0 = LLONG_MIN;
         int bp = INT_MAX;
         for (int r = r0 + tid; r < rpc; r += kZPanelThreads) {
@@ -368,170 +389,216 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         long long mk = sh.wkey[0];
         int mr = sh.wrow[0];
 #pragma unroll
-        for (int w = 1; w < kZPanelThreads / 32; ++w)
-            if (sh.wkey[w] > mk) {
-                mk = sh.wkey[w];
-                mr = sh.wrow[w];
+        for (int w = 1; w < kZPanelThreads / 32; ++w) {
+            const long long wk = sh.wkey[w];
+            const int wr = sh.wrow[w];
+            if (wk > mk || (wk == mk && wr < mr)) {
+                mk = wk;
+                mr = wr;
             }
-        // the cluster's largest, and how many rows lie within the margin
+        }
+        // how many of its rows lie within the margin
         int near = 0;
         for (int r = r0 + tid; r < rpc; r += kZPanelThreads) {
-            if (k + cta + (int64_t)kZPanelCtas * r >= n) break;
-            const long long key =
-                r == r0 + tid ? key0 : zproxy_key(s_rows[r * RS + jj], k + cta + (int64_t)kZPanelCtas * r == j);
+            const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
+            if (i >= n) break;
+            const long long key = r == r0 + tid ? key0 : zproxy_key(s_rows[r * RS + jj], i == j);
             near += mk != LLONG_MIN && key >= mk - 64;
         }
         const int several = rpc > kZPanelThreads ? __syncthreads_or(near > 1) : 0;
         near = __syncthreads_count(near > 0) + (several ? 1 : 0);
-        if (tid < kb) {
-            if (mr != INT_MAX) sh.cand_rowv[par][tid] = s_rows[mr * RS + tid];
-            if (lj >= 0) sh.diag_rowv[par][tid] = s_rows[lj * RS + tid];
-        }
-        if (tid == 0) {
-            sh.prox_key[par] = mk;
-            sh.prox_row[par] = mr == INT_MAX ? LLONG_MAX : k + cta + (long long)kZPanelCtas * mr;
-            sh.prox_z[par] = mr != INT_MAX ? s_rows[mr * RS + jj] : make_double2(0.0, 0.0);
-            sh.prox_near[par] = near;
-        }
-        cluster.sync();
-        const int owner_j = (int)((j - k) % kZPanelCtas);
-        {
-            long long ck = LLONG_MIN, cr = LLONG_MAX;
-            double2 cz = make_double2(0.0, 0.0);
-            int cn = 0;
-            if (lane < kZPanelCtas) {
-                ZPanelShared<KB>* o = cluster.map_shared_rank(&sh, lane);
-                ck = o->prox_key[par];
-                cr = o->prox_row[par];
-                cz = o->prox_z[par];
-                cn = o->prox_near[par];
+        if (warp == 0) {
+            // the rows as they stand, and the message into every CTA
+            if (lane < kb) {
+                sh.stage[par][0][lane] = mr != INT_MAX ? s_rows[mr * RS + lane] : make_double2(0.0, 0.0);
+                if (lj >= 0) sh.stage[par][1][lane] = s_rows[lj * RS + lane];
             }
-            const int wc = zkey_winner(ck, lane);
-            const long long gk = __shfl_sync(0xffffffffu, ck, wc);
-            const unsigned close = __ballot_sync(0xffffffffu, ck != LLONG_MIN && ck >= gk - 64);
-            const int gn = __shfl_sync(0xffffffffu, cn, wc);
-            // an ordinary key (neither zero nor not finite), alone in the margin
-            if (gk > kZKeyZero && gk < kZKeyNaNFirst && close == 1u << wc && gn == 1) {
-                const long long wr = __shfl_sync(0xffffffffu, cr, wc);
-                const double2 z = make_double2(__shfl_sync(0xffffffffu, cz.x, wc), __shfl_sync(0xffffffffu, cz.y, wc));
-                // (every warp of every CTA decides alike) below the normal
-                // range only if both parts are
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0)
+                mbar_expect_tx(&sh.mbar[par], (uint32_t)(kZPanelCtas * (sizeof(ZMsg) + KB * sizeof(double2)) +
+                                                         KB * sizeof(double2)));
+            if (lane < kZPanelCtas) {
+                const uint32_t bar = cluster_addr(&sh.mbar[par], lane);
+                const uint32_t dst = cluster_addr(&sh.msg[par][cta], lane);
+                const long long row = mr == INT_MAX ? LLONG_MAX : k + cta + (long long)kZPanelCtas * mr;
+                st_async16(dst, make_uint4((unsigned)mk, (unsigned)(mk >> 32), (unsigned)row, (unsigned)(row >> 32)), bar);
+                st_async16(dst + 16, make_uint4((unsigned)near, 0u, 0u, 0u), bar);
+                bulk_s2cluster(cluster_addr(sh.rowv[par][cta], lane), sh.stage[par][0], KB * sizeof(double2), bar);
+                if (lj >= 0)
+                    bulk_s2cluster(cluster_addr(sh.diagv[par], lane), sh.stage[par][1], KB * sizeof(double2), bar);
+            }
+        }
+        // the shadow: what step j - 1 still owes (rows below j - 1, columns
+        // beyond j); every warp, warp 0 after it has sent
+        if (jj > 0) {
+            for (int r = r0 + tid; r < rpc; r += kZPanelThreads) {
+                if (k + cta + (int64_t)kZPanelCtas * r >= n) break;
+                double2* row = &s_rows[r * RS];
+                const double2 l = row[jj - 1];
+#pragma unroll 4
+                for (int c = jj + 1; c < kb; ++c) row[c] = zfms(row[c], l, pold[c]);
+            }
+        }
+        if (warp == 0) {
+            const bool got = __all_sync(0xffffffffu, mbar_wait_cluster(&sh.mbar[par], (uint32_t)((jj >> 1) & 1)));
+            if (!got) {
+                if (lane == 0) {
+                    sh.abort = 1;
+                    atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
+                }
+            } else {
+                long long ck = LLONG_MIN;
+                if (lane < kZPanelCtas) ck = sh.msg[par][lane].key;
+                const int wc = zkey_winner(ck, lane);
+                const long long gk = __shfl_sync(0xffffffffu, ck, wc);
+                const unsigned close = __ballot_sync(0xffffffffu, ck != LLONG_MIN && ck >= gk - 64);
+                // an ordinary key (neither zero nor not finite), alone in the
+                // margin, and above the range where TMV_ABS could underflow
+                const double2 z = sh.rowv[par][wc][jj];
                 const long long big = max(__double_as_longlong(z.x) & kZAbsBits, __double_as_longlong(z.y) & kZAbsBits);
-                if (big >= __double_as_longlong(4.0 * DBL_MIN)) {
-                    if (warp == 1) {
-                        const double2 inv1 = tmv_inverse_of(z);
-                        if (lane == 0) {
-                            sh.inv = inv1;
-                            sh.under = 0;
-                            if (cta == 0) P[j] = wr;
-                        }
-                    }
-                    if (tid < kb) {
-                        const double2 v = cluster.map_shared_rank(&sh, wc)->cand_rowv[par][tid];
-                        sh.prow[tid] = v;
-                        if (lj >= 0) s_rows[lj * RS + tid] = v;
-                        if (wr != j && (int)((wr - k) % kZPanelCtas) == cta)
-                            s_rows[(int)((wr - k) / kZPanelCtas) * RS + tid] =
-                                cluster.map_shared_rank(&sh.diag_rowv[par][0], owner_j)[tid];
-                    }
-                    __syncthreads();
-                    zpanel_update<KB>(n, k, kb, jj, rpc, cta, r0, s_rows, sh.prow, sh.inv, false);
-                    continue;
+                const bool alone = gk > kZKeyZero && gk < kZKeyNaNFirst && close == 1u << wc &&
+                                   sh.msg[par][wc].near == 1 && big >= __double_as_longlong(4.0 * DBL_MIN);
+                if (lane == 0) {
+                    sh.from = alone ? wc : -1;
+                    sh.piv = sh.msg[par][wc].row;
                 }
             }
         }
-        // stage 2: TMV_ABS (and TMV_InverseOf) of the rows within 64 key units
-        // (256 ulps of |z|^2) of the largest
-        const long long thr = mk <= LLONG_MIN + 64 ? LLONG_MIN + 1 : mk - 64;
-        long long ba = -2;
-        int br = INT_MAX;
-        double braw = 0.0;
-        double2 binv = make_double2(0.0, 0.0);
-        for (int r = r0 + tid; r < rpc && mk != LLONG_MIN; r += kZPanelThreads) {
+        __syncthreads();
+        if (sh.abort) break;
+        int from = sh.from;
+        if (from >= 0) {
+            if (warp == 1) {
+                const double2 inv1 = tmv_inverse_of(sh.rowv[par][from][jj]);
+                if (lane == 0) {
+                    sh.inv = inv1;
+                    sh.under = 0;
+                }
+            }
+            if (tid < kb) {
+                // the pivot row with what it owes, and row j into its place
+                double2 v = sh.rowv[par][from][tid];
+                if (jj > 0 && tid > jj) v = zfms(v, sh.rowv[par][from][jj - 1], pold[tid]);
+                pnew[tid] = v;
+                const long long wr = sh.piv;
+                if (lj >= 0) s_rows[lj * RS + tid] = v;
+                if (wr != j && (int)((wr - k) % kZPanelCtas) == cta) {
+                    double2 d = sh.diagv[par][tid];
+                    if (jj > 0 && tid > jj) d = zfms(d, sh.diagv[par][jj - 1], pold[tid]);
+                    s_rows[(int)((wr - k) / kZPanelCtas) * RS + tid] = d;
+                }
+                if (tid == 0 && cta == 0) P[j] = wr;
+            }
+        } else {
+            // stage 2: TMV_ABS (and TMV_InverseOf) of the rows within 64 key
+            // units (256 ulps of |z|^2) of the CTA's largest
+            const long long thr = mk <= LLONG_MIN + 64 ? LLONG_MIN + 1 : mk - 64;
+            long long ba = -2;
+            int br = INT_MAX;
+            double braw = 0.0;
+            double2 binv = make_double2(0.0, 0.0);
+            for (int r = r0 + tid; r < rpc && mk != LLONG_MIN; r += kZPanelThreads) {
+                const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
+                if (i >= n) break;
+                const double2 z = s_rows[r * RS + jj];
+                const long long key = r == r0 + tid ? key0 : zproxy_key(z, i == j);
+                if (key < thr) continue;
+                const double raw = tmv_abs(z);
+                const long long a = zabs_key(raw, i == j);
+                if (a > ba || (a == ba && r < br)) {
+                    ba = a;
+                    br = r;
+                    braw = raw;
+                    binv = tmv_inverse_of(z);
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const long long oa = __shfl_xor_sync(0xffffffffu, ba, o);
+                const int orow = __shfl_xor_sync(0xffffffffu, br, o);
+                if (oa > ba || (oa == ba && orow < br)) { ba = oa; br = orow; }
+            }
+            if (lane == 0) { sh.wkey[warp] = ba; sh.wrow[warp] = br; }
+            __syncthreads();
+            ba = sh.wkey[0];
+            br = sh.wrow[0];
+#pragma unroll
+            for (int w = 1; w < kZPanelThreads / 32; ++w)
+                if (sh.wkey[w] > ba || (sh.wkey[w] == ba && sh.wrow[w] < br)) { ba = sh.wkey[w]; br = sh.wrow[w]; }
+            // stage the candidate (its owner thread writes its TMV_ABS and
+            // inverse) and, where owned, row j
+            if (tid < kb) {
+                if (br != INT_MAX) sh.cand_rowv[tid] = s_rows[br * RS + tid];
+                if (lj >= 0) sh.diag_rowv[tid] = s_rows[lj * RS + tid];
+            }
+            if (br != INT_MAX && (br - r0) % kZPanelThreads == tid && br >= r0) {
+                sh.cand_abs = braw;
+                sh.cand_inv = binv;
+            }
+            if (tid == 0) {
+                sh.cand_key = ba;
+                sh.cand_row = br == INT_MAX ? LLONG_MAX : k + cta + (long long)kZPanelCtas * br;
+            }
+            cluster.sync();
+            // the winner over the cluster: lanes 0..15 of every warp read one CTA each
+            long long wa = -3, wr = LLONG_MAX;
+            int wc = 0;
+            if (lane < kZPanelCtas) {
+                ZPanelShared<KB>* o = cluster.map_shared_rank(&sh, lane);
+                wa = o->cand_key;
+                wr = o->cand_row;
+                wc = lane;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const long long oa = __shfl_xor_sync(0xffffffffu, wa, o);
+                const long long orow = __shfl_xor_sync(0xffffffffu, wr, o);
+                const int oc = __shfl_xor_sync(0xffffffffu, wc, o);
+                if (oa > wa || (oa == wa && orow < wr)) { wa = oa; wr = orow; wc = oc; }
+            }
+            // U's row j: the pivot row (or row j with its column zeroed)
+            if (tid < kb) {
+                ZPanelShared<KB>* w = cluster.map_shared_rank(&sh, wc);
+                // the pivot's own modulus (a NaN stays NaN: no underflow)
+                const long long rb = __double_as_longlong(w->cand_abs) & kZAbsBits;
+                const bool under = rb < __double_as_longlong(DBL_MIN);
+                const int64_t p = under ? j : (int64_t)wr;
+                double2 v;
+                if (under) {
+                    v = cluster.map_shared_rank(&sh.diag_rowv[0], owner_j)[tid];
+                    if (tid == jj) v = make_double2(0.0, 0.0);
+                } else {
+                    v = w->cand_rowv[tid];
+                }
+                pnew[tid] = v;
+                if (lj >= 0) s_rows[lj * RS + tid] = v;
+                if (p != j && (int)((p - k) % kZPanelCtas) == cta)
+                    s_rows[(int)((p - k) / kZPanelCtas) * RS + tid] =
+                        cluster.map_shared_rank(&sh.diag_rowv[0], owner_j)[tid];
+                if (tid == 0) {
+                    sh.under = under ? 1 : 0;
+                    sh.inv = under ? make_double2(0.0, 0.0) : w->cand_inv;
+                    if (cta == 0) P[j] = p;
+                }
+            }
+            cluster.sync();  // the staged rows are read
+        }
+        __syncthreads();
+        // scale this CTA's rows below j and update the next column
+        const double2 inv = sh.inv;
+        const bool und = sh.under != 0;
+        for (int r = r0 + tid; r < rpc; r += kZPanelThreads) {
             const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
             if (i >= n) break;
-            const double2 z = s_rows[r * RS + jj];
-            const long long key = r == r0 + tid ? key0 : zproxy_key(z, i == j);
-            if (key < thr) continue;
-            const double raw = tmv_abs(z);
-            const long long a = zabs_key(raw, i == j);
-            if (a > ba || (a == ba && r < br)) {
-                ba = a;
-                br = r;
-                braw = raw;
-                binv = tmv_inverse_of(z);
-            }
+            if (i == j) continue;
+            double2* row = &s_rows[r * RS];
+            const double2 l = und ? make_double2(0.0, 0.0) : zmul(row[jj], inv);
+            row[jj] = l;
+            if (jj + 1 < kb) row[jj + 1] = zfms(row[jj + 1], l, pnew[jj + 1]);
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const long long oa = __shfl_xor_sync(0xffffffffu, ba, o);
-            const int orow = __shfl_xor_sync(0xffffffffu, br, o);
-            if (oa > ba || (oa == ba && orow < br)) { ba = oa; br = orow; }
-        }
-        if (lane == 0) { sh.wkey[warp] = ba; sh.wrow[warp] = br; }
-        __syncthreads();
-        ba = sh.wkey[0];
-        br = sh.wrow[0];
-#pragma unroll
-        for (int w = 1; w < kZPanelThreads / 32; ++w)
-            if (sh.wkey[w] > ba || (sh.wkey[w] == ba && sh.wrow[w] < br)) { ba = sh.wkey[w]; br = sh.wrow[w]; }
-        // stage the candidate (its owner thread writes its TMV_ABS and
-        // inverse); row j is staged already
-        if (tid < kb && br != INT_MAX) sh.cand_rowv[par][tid] = s_rows[br * RS + tid];
-        if (br != INT_MAX && (br - r0) % kZPanelThreads == tid && br >= r0) {
-            sh.cand_abs[par] = braw;
-            sh.cand_inv[par] = binv;
-        }
-        if (tid == 0) {
-            sh.cand_key[par] = ba;
-            sh.cand_row[par] = br == INT_MAX ? LLONG_MAX : k + cta + (long long)kZPanelCtas * br;
-        }
-        cluster.sync();
-        // the winner over the cluster: lanes 0..15 of every warp read one CTA each
-        long long wa = -3, wr = LLONG_MAX;
-        int wc = 0;
-        if (lane < kZPanelCtas) {
-            ZPanelShared<KB>* o = cluster.map_shared_rank(&sh, lane);
-            wa = o->cand_key[par];
-            wr = o->cand_row[par];
-            wc = lane;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const long long oa = __shfl_xor_sync(0xffffffffu, wa, o);
-            const long long orow = __shfl_xor_sync(0xffffffffu, wr, o);
-            const int oc = __shfl_xor_sync(0xffffffffu, wc, o);
-            if (oa > wa || (oa == wa && orow < wr)) { wa = oa; wr = orow; wc = oc; }
-        }
-        // U's row j: the pivot row (or row j with its column zeroed)
-        if (tid < kb) {
-            ZPanelShared<KB>* w = cluster.map_shared_rank(&sh, wc);
-            // the pivot's own modulus (a NaN stays NaN: no underflow)
-            const long long rb = __double_as_longlong(w->cand_abs[par]) & kZAbsBits;
-            const bool under = rb < __double_as_longlong(DBL_MIN);
-            const int64_t p = under ? j : (int64_t)wr;
-            double2 v;
-            if (under) {
-                v = cluster.map_shared_rank(&sh.diag_rowv[par][0], owner_j)[tid];
-                if (tid == jj) v = make_double2(0.0, 0.0);
-            } else {
-                v = w->cand_rowv[par][tid];
-            }
-            sh.prow[tid] = v;
-            if (lj >= 0) s_rows[lj * RS + tid] = v;
-            if (p != j && (int)((p - k) % kZPanelCtas) == cta)
-                s_rows[(int)((p - k) / kZPanelCtas) * RS + tid] =
-                    cluster.map_shared_rank(&sh.diag_rowv[par][0], owner_j)[tid];
-            if (tid == 0) {
-                sh.under = under ? 1 : 0;
-                sh.inv = under ? make_double2(0.0, 0.0) : w->cand_inv[par];
-                if (cta == 0) P[j] = p;
-            }
-        }
-        __syncthreads();
-        zpanel_update<KB>(n, k, kb, jj, rpc, cta, r0, s_rows, sh.prow, sh.inv, sh.under != 0);
         // (the next column reads only this thread's rows until its first
-        // __syncthreads; sh.prow is rewritten only after the next cluster.sync)
+        // __syncthreads)
     }
     __syncthreads();
     for (int t = tid; t < rpc * kb; t += kZPanelThreads) {
@@ -539,7 +606,7 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
         if (i < n) A[i + (k + c) * lda] = s_rows[r * RS + c];
     }
-    cluster.sync();  // no CTA leaves while another may still read its shared memory
+    cluster.sync();  // no CTA leaves while another may still write or read its shared memory
 }
 
 // The panel's interchanges P[k..k+kb) (kb <= 32) applied in order to the
@@ -796,7 +863,7 @@ static tmvg_status zlu_factor_blocked(Context* c, int64_t n, double2* A, int64_t
         const int rpc = (int)ceil_div(n - k, kZPanelCtas);
         cfg.dynamicSmemBytes = (size_t)rpc * (KB + 1) * sizeof(double2);
         ++c->launches;
-        return check_cuda(c, cudaLaunchKernelEx(&cfg, zlu_panel_smem_kernel<KB>, n, A, lda, k, kb, P, rpc),
+        return check_cuda(c, cudaLaunchKernelEx(&cfg, zlu_panel_smem_kernel<KB>, n, A, lda, k, kb, P, rpc, c->dflags),
                           "lu_z: panel launch");
     };
     auto swap = [&](int64_t c0, int64_t c1, int64_t k, int kb) {
