@@ -345,6 +345,10 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
     constexpr int RS = KB + 1;
     const int cta = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // warp 0 holds no rows: it decides (and takes the inverse and the pivot
+    // row) while the others pay what the rows owe
+    constexpr int RT = kZPanelThreads - 32;
+    const int first = warp == 0 ? INT_MAX / 2 : tid - 32;
     if (tid == 0) {
         mbar_init(&sh.mbar[0], 1u);
         mbar_init(&sh.mbar[1], 1u);
@@ -371,11 +375,11 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         // stage 1: largest proxy key (the first row's key kept)
         long long bk = LLONG_MIN, key0 = LLONG_MIN;
         int bp = INT_MAX;
-        for (int r = r0 + tid; r < rpc; r += kZPanelThreads) {
+        for (int r = r0 + first; r < rpc; r += RT) {
             const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
             if (i >= n) break;
             const long long key = zproxy_key(s_rows[r * RS + jj], i == j);
-            if (r == r0 + tid) key0 = key;
+            if (r == r0 + first) key0 = key;
             if (key > bk) {
                 bk = key;
                 bp = r;
@@ -399,13 +403,13 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         }
         // how many of its rows lie within the margin
         int near = 0;
-        for (int r = r0 + tid; r < rpc; r += kZPanelThreads) {
+        for (int r = r0 + first; r < rpc; r += RT) {
             const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
             if (i >= n) break;
-            const long long key = r == r0 + tid ? key0 : zproxy_key(s_rows[r * RS + jj], i == j);
+            const long long key = r == r0 + first ? key0 : zproxy_key(s_rows[r * RS + jj], i == j);
             near += mk != LLONG_MIN && key >= mk - 64;
         }
-        const int several = rpc > kZPanelThreads ? __syncthreads_or(near > 1) : 0;
+        const int several = rpc > RT ? __syncthreads_or(near > 1) : 0;
         near = __syncthreads_count(near > 0) + (several ? 1 : 0);
         if (warp == 0) {
             // the rows as they stand, and the message into every CTA
@@ -430,9 +434,9 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
             }
         }
         // the shadow: what step j - 1 still owes (rows below j - 1, columns
-        // beyond j); every warp, warp 0 after it has sent
+        // beyond j)
         if (jj > 0) {
-            for (int r = r0 + tid; r < rpc; r += kZPanelThreads) {
+            for (int r = r0 + first; r < rpc; r += RT) {
                 if (k + cta + (int64_t)kZPanelCtas * r >= n) break;
                 double2* row = &s_rows[r * RS];
                 const double2 l = row[jj - 1];
@@ -459,36 +463,39 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
                 const long long big = max(__double_as_longlong(z.x) & kZAbsBits, __double_as_longlong(z.y) & kZAbsBits);
                 const bool alone = gk > kZKeyZero && gk < kZKeyNaNFirst && close == 1u << wc &&
                                    sh.msg[par][wc].near == 1 && big >= __double_as_longlong(4.0 * DBL_MIN);
+                const long long wr = sh.msg[par][wc].row;
                 if (lane == 0) {
                     sh.from = alone ? wc : -1;
-                    sh.piv = sh.msg[par][wc].row;
+                    sh.piv = wr;
+                }
+                if (alone) {
+                    // the inverse, and the pivot row with what it owes
+                    const double2 inv1 = tmv_inverse_of(z);
+                    if (lane == 0) {
+                        sh.inv = inv1;
+                        sh.under = 0;
+                        if (cta == 0) P[j] = wr;
+                    }
+                    if (lane < kb) {
+                        double2 v = sh.rowv[par][wc][lane];
+                        if (jj > 0 && lane > jj) v = zfms(v, sh.rowv[par][wc][jj - 1], pold[lane]);
+                        pnew[lane] = v;
+                    }
                 }
             }
         }
         __syncthreads();
         if (sh.abort) break;
-        int from = sh.from;
-        if (from >= 0) {
-            if (warp == 1) {
-                const double2 inv1 = tmv_inverse_of(sh.rowv[par][from][jj]);
-                if (lane == 0) {
-                    sh.inv = inv1;
-                    sh.under = 0;
-                }
-            }
+        if (sh.from >= 0) {
+            // the pivot row and row j into their places
             if (tid < kb) {
-                // the pivot row with what it owes, and row j into its place
-                double2 v = sh.rowv[par][from][tid];
-                if (jj > 0 && tid > jj) v = zfms(v, sh.rowv[par][from][jj - 1], pold[tid]);
-                pnew[tid] = v;
                 const long long wr = sh.piv;
-                if (lj >= 0) s_rows[lj * RS + tid] = v;
+                if (lj >= 0) s_rows[lj * RS + tid] = pnew[tid];
                 if (wr != j && (int)((wr - k) % kZPanelCtas) == cta) {
                     double2 d = sh.diagv[par][tid];
                     if (jj > 0 && tid > jj) d = zfms(d, sh.diagv[par][jj - 1], pold[tid]);
                     s_rows[(int)((wr - k) / kZPanelCtas) * RS + tid] = d;
                 }
-                if (tid == 0 && cta == 0) P[j] = wr;
             }
         } else {
             // stage 2: TMV_ABS (and TMV_InverseOf) of the rows within 64 key
@@ -498,11 +505,11 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
             int br = INT_MAX;
             double braw = 0.0;
             double2 binv = make_double2(0.0, 0.0);
-            for (int r = r0 + tid; r < rpc && mk != LLONG_MIN; r += kZPanelThreads) {
+            for (int r = r0 + first; r < rpc && mk != LLONG_MIN; r += RT) {
                 const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
                 if (i >= n) break;
                 const double2 z = s_rows[r * RS + jj];
-                const long long key = r == r0 + tid ? key0 : zproxy_key(z, i == j);
+                const long long key = r == r0 + first ? key0 : zproxy_key(z, i == j);
                 if (key < thr) continue;
                 const double raw = tmv_abs(z);
                 const long long a = zabs_key(raw, i == j);
@@ -532,7 +539,7 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
                 if (br != INT_MAX) sh.cand_rowv[tid] = s_rows[br * RS + tid];
                 if (lj >= 0) sh.diag_rowv[tid] = s_rows[lj * RS + tid];
             }
-            if (br != INT_MAX && (br - r0) % kZPanelThreads == tid && br >= r0) {
+            if (br != INT_MAX && br >= r0 && (br - r0) % RT == first) {
                 sh.cand_abs = braw;
                 sh.cand_inv = binv;
             }
@@ -588,7 +595,7 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         // scale this CTA's rows below j and update the next column
         const double2 inv = sh.inv;
         const bool und = sh.under != 0;
-        for (int r = r0 + tid; r < rpc; r += kZPanelThreads) {
+        for (int r = r0 + first; r < rpc; r += RT) {
             const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
             if (i >= n) break;
             if (i == j) continue;
