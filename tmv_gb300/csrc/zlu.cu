@@ -16,7 +16,7 @@
 // them; the blocked trailing products and solves' off-diagonal products use
 // fused multiply-adds (values to rounding).
 //
-// Small matrices (n < 128) factor one column per step (pivot search in one
+// Small matrices (n < 32) factor one column per step (pivot search in one
 // CTA, row interchange, scaling, rank-1 update over the grid) and solve one
 // CTA per right-hand side; larger ones factor by panels with look-ahead
 // (zlu_factor_blocked) and solve by 64-row blocks (zlu_ldiveq_blocked).  The
@@ -192,7 +192,7 @@ zlu_update_kernel(int64_t n, double2* A, int64_t lda, int64_t k)
 // ---------------------------------------------------------------------------
 constexpr int kZPanelCtas = 16;
 constexpr int kZPanelThreads = 512;
-constexpr int64_t kZBlockedMin = 128;
+constexpr int64_t kZBlockedMin = 32;
 constexpr size_t kZPanelSmemMax = 200 * 1024;
 constexpr long long kZKeyNaNFirst = 0x7fffffffffffffffLL;  // NaN/inf as row j
 constexpr long long kZKeyNaN = -0x7fffffffffffffffLL;      // NaN/inf elsewhere
