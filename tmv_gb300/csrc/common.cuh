@@ -92,6 +92,8 @@ struct Context {
     size_t work3_bytes = 0;
     // Stream-ordered scratch of the sliced products (created on first use).
     cudaMemPool_t pool = nullptr;
+    // Off for callers that may not allocate: products stay on the FP64 pipe.
+    bool may_pool = true;
     // Device copies of the host entry points' operands (grow-only).
     void* io = nullptr;
     size_t io_bytes = 0;

@@ -788,6 +788,7 @@ bool sliced_wanted(Context* c, int64_t M, int64_t N, int64_t K)
 {
     if (M < 64 || N < 48 || K < 24 || M > INT_MAX / 2 || N > INT_MAX / 2) return false;
     if ((double)M * (double)N * (double)K < 1.2e7) return false;
+    if (!c->may_pool) return false;
     if (!sl_encode_fn()) return false;
     // a captured stream keeps the FP64 pipe: its graph would hold scratch of
     // the pool

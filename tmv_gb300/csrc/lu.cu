@@ -2926,8 +2926,10 @@ extern "C" tmvg_status tmvg_lu_decompose_f64_noalloc(int64_t n, double* A, int64
     unsigned char* s = noalloc_scratch(&st);
     if (!s) return st;
 
-    // A context on the stack: no workspace, flags and barrier in the scratch.
+    // A context on the stack: no workspace, flags and barrier in the scratch,
+    // no scratch pool.
     Context c;
+    c.may_pool = false;
     c.device = dev;
     c.num_sms = std::min(sms, kNoAllocMaxCtas);
     c.stream = static_cast<cudaStream_t>(stream);
