@@ -434,37 +434,30 @@ __device__ __forceinline__ void reg_key_reduce(unsigned long long& key, int& idx
     }
 }
 
-// The lane that wins the same order over the warp (the lowest of the lanes
-// that tie in key and index); key and idx become the winner's.  FP64: one
-// redux.sync and a ballot decide unless keys tie in their upper 32 bits (three
-// redux.sync took 400 clocks on the chain of every column).
+// The lane that wins the same order over the candidates (`cand`) of the warp,
+// the lowest of the lanes that tie in key and index; -1 without a candidate.
+// One redux.sync and a ballot decide unless keys tie (FP64: in their upper 32
+// bits): every redux.sync costs about 100 clocks on the chain of every column,
+// and the winner itself stores what the others read.
 template <typename T>
-__device__ __forceinline__ int reg_key_winner(unsigned long long& key, int& idx)
+__device__ __forceinline__ int reg_key_winner(unsigned long long key, int idx, bool cand)
 {
-    if constexpr (sizeof(T) == 4) {
-        const unsigned k0 = (unsigned)key;
-        const int i0 = idx;
-        reg_key_reduce<T>(key, idx);
-        return __ffs(__ballot_sync(0xffffffffu, k0 == (unsigned)key && i0 == idx)) - 1;
-    } else {
-        const unsigned hi = (unsigned)(key >> 32);
-        const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-        bool in = hi == mhi;
-        unsigned m = __ballot_sync(0xffffffffu, in);
-        if (m & (m - 1)) {
+    const unsigned hi = sizeof(T) == 4 ? (unsigned)key : (unsigned)(key >> 32);
+    const unsigned mhi = __reduce_max_sync(0xffffffffu, cand ? hi : 0u);
+    bool in = cand && hi == mhi;
+    unsigned m = __ballot_sync(0xffffffffu, in);
+    if (m & (m - 1)) {
+        if constexpr (sizeof(T) == 8) {
             const unsigned lo = in ? (unsigned)key : 0u;
             const unsigned mlo = __reduce_max_sync(0xffffffffu, lo);  // (every lane takes part)
             in = in && lo == mlo;
-            const unsigned i = in ? (unsigned)idx : 0xffffffffu;
-            const unsigned mi = __reduce_min_sync(0xffffffffu, i);
-            in = in && i == mi;
-            m = __ballot_sync(0xffffffffu, in);
         }
-        const int w = __ffs(m) - 1;
-        key = ((unsigned long long)mhi << 32) | __shfl_sync(0xffffffffu, (unsigned)key, w);
-        idx = __shfl_sync(0xffffffffu, idx, w);
-        return w;
+        const unsigned i = in ? (unsigned)idx : 0xffffffffu;
+        const unsigned mi = __reduce_min_sync(0xffffffffu, i);
+        in = in && i == mi;
+        m = __ballot_sync(0xffffffffu, in);
     }
+    return __ffs(m) - 1;
 }
 
 // 16-byte vectors of a row held in registers (4 floats or 2 doubles).
@@ -847,20 +840,20 @@ constexpr int kLeafWarps = kLeafThreads / 32;
 // applies them in one).
 template <typename T>
 struct LeafMsg;
+struct alignas(16) LeafHead {
+    unsigned long long key;
+    int pos;  // INT_MAX: no candidate
+    int loc;  // cta << 16 | thread
+};
 template <>
 struct LeafMsg<float> {
-    unsigned long long key;
-    int pos;
-    int loc;  // cta << 16 | thread
+    LeafHead head;
     float leaf[kLeaf];
 };
 template <>
 struct LeafMsg<double> {
-    unsigned long long key;
-    int pos;
-    int loc;
-    double leaf[kLeaf];
-    double owed, pad;
+    LeafHead head;
+    double leaf[kLeaf + 2];  // [kLeaf]: the multiplier owed; a pad
 };
 
 template <typename T, int NB>
@@ -966,19 +959,17 @@ __device__ __forceinline__ void leaf_send_row(const T (&x)[NB], int rot, int pw,
 }
 
 // The winner's leaf part into s_urow[u] (warp 0).  FP64: positions 1..7-u
-// still owe step u-1's update, one per lane; and the pivot's reciprocal.
+// still owe step u-1's update, one per lane.
 template <typename T>
-__device__ __forceinline__ void leaf_pivot_row(const T* sent, T (*s_urow)[kLeaf], int u, bool owe_u, int lane, T* rcp)
+__device__ __forceinline__ void leaf_pivot_row(const T* sent, T (*s_urow)[kLeaf], int u, bool owe_u, int lane)
 {
     if constexpr (sizeof(T) == 8) {
-        const T r = recip_rn(sent[0]);
         if (lane < kLeaf) {
             T v = sent[lane];
             if (owe_u && lane >= 1 && lane <= kLeaf - 1 - u)
                 v = fma(-sent[kLeaf], s_urow[u - 1][lane + 1 < kLeaf ? lane + 1 : lane], v);
             s_urow[u][lane] = v;
         }
-        if (lane == 0) *rcp = r;
     } else {
         using V = Vec16<T>;
         if (lane < kLeaf / V::E)
@@ -1000,23 +991,18 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
     static_assert(sizeof(LeafMsg<T>) % 16 == 0, "message in 16-byte pieces");
     constexpr int kLast = kLeaf - 1;
     constexpr bool kRaw = sizeof(T) == 8;  // candidates travel without their owed update
-    constexpr int kSent = (int)((sizeof(LeafMsg<T>) - 16) / sizeof(T));
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
 
-    __shared__ unsigned long long s_key[kLeafWarps];
-    __shared__ int s_idx[kLeafWarps];
-    __shared__ int s_loc[kLeafWarps];
-    __shared__ __align__(16) T warp_leaf[kLeafWarps][kSent];     // each warp's candidate's leaf part
+    __shared__ __align__(16) LeafMsg<T> wmsg[kLeafWarps];        // each warp's candidate
     __shared__ __align__(16) LeafMsg<T> msg[2][kClusterCtas];   // messages, by column parity
+    __shared__ LeafHead s_win;                                   // the pivot
+    __shared__ T s_rcp[kLeafWarps];  // 1 / candidate, per CTA (one CTA: per warp)
     __shared__ __align__(16) T s_urow[kLeaf][kLeaf];             // the leaf's pivot rows, leaf part
     __shared__ __align__(16) T s_rem[2][kLeaf][NB];              // pivot rows, then U (by leaf parity)
     __shared__ __align__(16) T s_stage[kLeaf][NB];               // this CTA's pivot rows, staged
     __shared__ __align__(8) uint64_t mbar[2];
     __shared__ __align__(8) uint64_t mbar_leaf;
-    __shared__ unsigned long long s_wk;
-    __shared__ T s_rcp;  // FP64: the pivot's reciprocal, taken once (a chain of DFMAs)
-    __shared__ int s_wi, s_wloc;
     __shared__ unsigned char s_mode[kPanelMax];
     __shared__ int s_piv[kPanelMax];
     __shared__ int s_npairs;  // row pairs written so far (used in CTA 0)
@@ -1049,6 +1035,13 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
     int pos = r0 + tid;  // this row's current position
     bool act = have;     // still a candidate (not yet a pivot row)
     const int loc = (cta << 16) | tid;
+    const LeafHead none{0ull, INT_MAX, -1};
+    static_assert(kClusterCtas <= 32 && kLeafWarps >= kClusterCtas, "a candidate per lane, a reciprocal per CTA");
+    // (warp 0's lane d sends to CTA d)
+    const uint32_t to_msg = cluster_addr(&msg[0][cta], lane < G ? lane : 0);
+    const uint32_t to_bar = cluster_addr(&mbar[0], lane < G ? lane : 0);
+    const int rcp_warp = nwarp > 1 ? 1 : 0;
+    if (G > 1 && tid == 0) mbar_expect_tx(&mbar[0], (uint32_t)(G * sizeof(LeafMsg<T>)));
     cluster.sync();  // every CTA's mbarriers are initialised before any message
 
     bool prev_uf = false;
@@ -1076,21 +1069,16 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             const int par = j & 1;
             const bool r2 = s_mode[j] && !prev_uf;
             // 1. this warp's candidate; the winner's leaf part with the owed update applied
-            unsigned long long bk = act ? reg_pivot_key(x[0], pos == j, r2) : 0ull;
-            int bi = act ? pos : INT_MAX;
-            bool win;
-            if constexpr (kRaw) {
-                win = lane == reg_key_winner<T>(bk, bi);
-            } else {
-                reg_key_reduce<T>(bk, bi);
-                win = act && pos == bi;
-            }
-            if (win) {
+            const unsigned long long key = act ? reg_pivot_key(x[0], pos == j, r2) : 0ull;
+            const int wl = reg_key_winner<T>(key, pos, act);
+            if (lane == wl) {
+                LeafMsg<T>& wm = wmsg[warp];
+                wm.head = LeafHead{key, pos, loc};
                 if constexpr (kRaw) {
 #pragma unroll
                     for (int q = 0; q < kLeaf / V::E; ++q)
-                        reinterpret_cast<typename V::type*>(warp_leaf[warp])[q] = V::make(&x[q * V::E]);
-                    warp_leaf[warp][kLeaf] = lprev;
+                        reinterpret_cast<typename V::type*>(wm.leaf)[q] = V::make(&x[q * V::E]);
+                    wm.leaf[kLeaf] = lprev;  // (owed)
                 } else {
                     // (in position order; positions 1..7-u owe step u-1's update,
                     // whose pivot row s_urow[u-1] is in step u-1's position order)
@@ -1100,43 +1088,24 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
                         lp[q] = (owe && q >= 1 && q <= kLast - u) ? fma(-lprev, s_urow[u - 1][q + 1 < kLeaf ? q + 1 : q], x[q]) : x[q];
 #pragma unroll
                     for (int q = 0; q < kLeaf / V::E; ++q)
-                        reinterpret_cast<typename V::type*>(warp_leaf[warp])[q] = V::make(&lp[q * V::E]);
+                        reinterpret_cast<typename V::type*>(wm.leaf)[q] = V::make(&lp[q * V::E]);
                 }
-                s_loc[warp] = loc;
             }
-            if (lane == 0) {
-                s_key[warp] = bk;
-                s_idx[warp] = bi;
-            }
+            if (wl < 0 && lane == 0) wmsg[warp].head = none;
             __syncthreads();
             if (warp == 0) {
                 // 2. this CTA's candidate; with a cluster, one message into every CTA
-                // (s_idx INT_MAX: a warp without candidates)
-                bk = lane < nwarp ? s_key[lane] : 0ull;
-                bi = lane < nwarp ? s_idx[lane] : INT_MAX;
-                const int wn = reg_key_winner<T>(bk, bi);
-                const int ww = bi != INT_MAX ? wn : -1;
+                const LeafHead h = lane < nwarp ? wmsg[lane].head : none;
+                const int ww = reg_key_winner<T>(h.key, h.pos, h.pos != INT_MAX);
                 if (G == 1) {
-                    if (lane == 0) {
-                        s_wk = bk;
-                        s_wi = bi;
-                        s_wloc = ww >= 0 ? s_loc[ww] : -1;
-                    }
-                    if (ww >= 0) leaf_pivot_row<T>(warp_leaf[ww], s_urow, u, owe_u, lane, &s_rcp);
-                } else {
-                    if (lane == 0) mbar_expect_tx(&mbar[par], (uint32_t)(G * sizeof(LeafMsg<T>)));
-                    if (lane < G) {
-                        const uint32_t dst = cluster_addr(&msg[par][cta], lane);
-                        const uint32_t bar = cluster_addr(&mbar[par], lane);
-                        const int wl = ww >= 0 ? s_loc[ww] : -1;
-                        st_async16(dst, make_uint4((unsigned)bk, (unsigned)(bk >> 32), (unsigned)bi, (unsigned)wl), bar);
+                    if (lane == max(ww, 0)) s_win = h;  // (no candidate: lane 0's empty one)
+                    if (ww >= 0) leaf_pivot_row<T>(wmsg[ww].leaf, s_urow, u, owe_u, lane);
+                } else if (lane < G) {
+                    const uint32_t dst = to_msg + (uint32_t)(par * sizeof(msg[0]));
+                    const uint32_t bar = to_bar + (uint32_t)(par * sizeof(mbar[0]));
+                    const uint4* from = reinterpret_cast<const uint4*>(&wmsg[max(ww, 0)]);
 #pragma unroll
-                        for (int q = 1; q < kMsgVecs; ++q) {
-                            const uint4 v = ww >= 0 ? reinterpret_cast<const uint4*>(warp_leaf[ww])[q - 1]
-                                                    : make_uint4(0u, 0u, 0u, 0u);
-                            st_async16(dst + 16 * q, v, bar);
-                        }
-                    }
+                    for (int q = 0; q < kMsgVecs; ++q) st_async16(dst + 16 * q, from[q], bar);
                 }
             }
             // 3. the shadow: work this row owes, while the messages travel
@@ -1146,6 +1115,9 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
                     if (q <= kLast - u) x[q] = fma(-lprev, s_urow[u - 1][q + 1 < kLeaf ? q + 1 : q], x[q]);
             }
             owe = false;
+            // (the next column's messages are counted from here)
+            if (G > 1 && tid == 0 && j + 1 < nb)
+                mbar_expect_tx(&mbar[par ^ 1], (uint32_t)(G * sizeof(LeafMsg<T>)));
             if (send_step >= 0) {
                 leaf_send_row<T, NB>(x, u, pw, G, s_stage[send_step], s_rem[lpar][send_step], &mbar_leaf);
                 send_step = -1;
@@ -1159,22 +1131,25 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
                         atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
                     }
                 } else {
-                    unsigned long long wk = lane < G ? msg[par][lane].key : 0ull;
-                    int wi = lane < G ? msg[par][lane].pos : INT_MAX;
-                    const int wn = reg_key_winner<T>(wk, wi);
-                    const int wo = wi != INT_MAX ? wn : -1;
-                    if (lane == 0) {
-                        s_wk = wk;
-                        s_wi = wi;
-                        s_wloc = wo >= 0 ? msg[par][wo].loc : -1;
-                    }
-                    if (wo >= 0) leaf_pivot_row<T>(msg[par][wo].leaf, s_urow, u, owe_u, lane, &s_rcp);
+                    const LeafHead h = lane < G ? msg[par][lane].head : none;
+                    const int wo = reg_key_winner<T>(h.key, h.pos, h.pos != INT_MAX);
+                    if (lane == max(wo, 0)) s_win = h;
+                    if (wo >= 0) leaf_pivot_row<T>(msg[par][wo].leaf, s_urow, u, owe_u, lane);
+                }
+            }
+            if (warp == rcp_warp) {
+                // every candidate's reciprocal, beside warp 0's decision
+                const bool got = G == 1 || __all_sync(0xffffffffu, mbar_wait(&mbar[par], (uint32_t)((j >> 1) & 1)));
+                if (got && lane < (G > 1 ? G : nwarp)) {
+                    const LeafMsg<T>& cm = G > 1 ? msg[par][lane] : wmsg[lane];
+                    s_rcp[lane] = recip_rn(cm.head.pos != INT_MAX ? cm.leaf[0] : T(1));
                 }
             }
             __syncthreads();
             if (s_abort) break;
             // 5. the decision: bookkeeping, the column's scaling and the next column
-            const bool uf = reg_key_underflows<T>(s_wk);
+            const LeafHead piv = s_win;
+            const bool uf = reg_key_underflows<T>(piv.key);
             bool own;
             owe_u = !uf && u + 2 < kLeaf;
             if (uf) {
@@ -1184,11 +1159,10 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
                 ufmask |= 1u << u;
                 prev_uf = true;
             } else {
-                const int wi = s_wi;
-                own = act && loc == s_wloc;
-                if (tid == 0) s_piv[j] = (int)(k + wi);
+                own = act && loc == piv.loc;
+                if (tid == 0) s_piv[j] = (int)(k + piv.pos);
                 prev_uf = false;
-                if (act && !own && pos == j) pos = wi;  // the interchange
+                if (act && !own && pos == j) pos = piv.pos;  // the interchange
             }
             if (own) {
                 act = false;
@@ -1198,7 +1172,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             }
             if (!uf && act) {
                 // TMV scales the column by the reciprocal of the pivot
-                const T l = x[0] * (kRaw ? s_rcp : recip_rn(s_urow[u][0]));
+                const T l = x[0] * s_rcp[G > 1 ? piv.loc >> 16 : piv.loc >> 5];
                 x[0] = l;
                 if (u < kLast) x[1] = fma(-l, s_urow[u][1], x[1]);
                 if (u + 2 < kLeaf) {
