@@ -833,27 +833,22 @@ constexpr int kLeaf = 8;
 constexpr int kLeafThreads = 512;
 constexpr int kLeafWarps = kLeafThreads / 32;
 
-// What a candidate row sends.  FP32: its leaf part with the owed update
-// applied.  FP64: its leaf part as it stands and the multiplier it owes (a
-// DFMA takes its sub-partition 64 clocks whatever the lanes, so the seven of
-// the owed update would sit on the chain in every warp; the receiver's warp 0
-// applies them in one).
-template <typename T>
-struct LeafMsg;
+// What a candidate row sends: its leaf part as it stands and the multiplier
+// it owes; the receivers' warp 0 applies the owed update, one entry per lane.
+// (Applied by the candidate before it is stored, the update stood on the
+// chain in every warp: FP32 255 clocks a column for the branch, and a DFMA
+// takes its sub-partition 64 clocks whatever the lanes.)
 struct alignas(16) LeafHead {
     unsigned long long key;
     int pos;  // INT_MAX: no candidate
     int loc;  // cta << 16 | thread
 };
-template <>
-struct LeafMsg<float> {
+template <typename T>
+struct LeafMsg {
     LeafHead head;
-    float leaf[kLeaf];
-};
-template <>
-struct LeafMsg<double> {
-    LeafHead head;
-    double leaf[kLeaf + 2];  // [kLeaf]: the multiplier owed; a pad
+    T leaf[kLeaf];
+    T owed;
+    T pad[16 / sizeof(T) - 1];
 };
 
 template <typename T, int NB>
@@ -958,22 +953,16 @@ __device__ __forceinline__ void leaf_send_row(const T (&x)[NB], int rot, int pw,
         bulk_s2cluster(cluster_addr(dst_row, d), stage, (uint32_t)(pw * sizeof(T)), cluster_addr(bar, d));
 }
 
-// The winner's leaf part into s_urow[u] (warp 0).  FP64: positions 1..7-u
-// still owe step u-1's update, one per lane.
+// The winner's leaf part into s_urow[u] (warp 0); positions 1..7-u still owe
+// step u-1's update, one per lane.
 template <typename T>
-__device__ __forceinline__ void leaf_pivot_row(const T* sent, T (*s_urow)[kLeaf], int u, bool owe_u, int lane)
+__device__ __forceinline__ void leaf_pivot_row(const LeafMsg<T>& w, T (*s_urow)[kLeaf], int u, bool owe_u, int lane)
 {
-    if constexpr (sizeof(T) == 8) {
-        if (lane < kLeaf) {
-            T v = sent[lane];
-            if (owe_u && lane >= 1 && lane <= kLeaf - 1 - u)
-                v = fma(-sent[kLeaf], s_urow[u - 1][lane + 1 < kLeaf ? lane + 1 : lane], v);
-            s_urow[u][lane] = v;
-        }
-    } else {
-        using V = Vec16<T>;
-        if (lane < kLeaf / V::E)
-            reinterpret_cast<typename V::type*>(s_urow[u])[lane] = reinterpret_cast<const typename V::type*>(sent)[lane];
+    if (lane < kLeaf) {
+        T v = w.leaf[lane];
+        if (owe_u && lane >= 1 && lane <= kLeaf - 1 - u)
+            v = fma(-w.owed, s_urow[u - 1][lane + 1 < kLeaf ? lane + 1 : lane], v);
+        s_urow[u][lane] = v;
     }
 }
 
@@ -990,7 +979,6 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
     constexpr int kMsgVecs = (int)(sizeof(LeafMsg<T>) / 16);
     static_assert(sizeof(LeafMsg<T>) % 16 == 0, "message in 16-byte pieces");
     constexpr int kLast = kLeaf - 1;
-    constexpr bool kRaw = sizeof(T) == 8;  // candidates travel without their owed update
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
 
@@ -1068,28 +1056,16 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             const int j = jb + u;
             const int par = j & 1;
             const bool r2 = s_mode[j] && !prev_uf;
-            // 1. this warp's candidate; the winner's leaf part with the owed update applied
+            // 1. this warp's candidate
             const unsigned long long key = act ? reg_pivot_key(x[0], pos == j, r2) : 0ull;
             const int wl = reg_key_winner<T>(key, pos, act);
             if (lane == wl) {
                 LeafMsg<T>& wm = wmsg[warp];
                 wm.head = LeafHead{key, pos, loc};
-                if constexpr (kRaw) {
 #pragma unroll
-                    for (int q = 0; q < kLeaf / V::E; ++q)
-                        reinterpret_cast<typename V::type*>(wm.leaf)[q] = V::make(&x[q * V::E]);
-                    wm.leaf[kLeaf] = lprev;  // (owed)
-                } else {
-                    // (in position order; positions 1..7-u owe step u-1's update,
-                    // whose pivot row s_urow[u-1] is in step u-1's position order)
-                    T lp[kLeaf];
-#pragma unroll
-                    for (int q = 0; q < kLeaf; ++q)
-                        lp[q] = (owe && q >= 1 && q <= kLast - u) ? fma(-lprev, s_urow[u - 1][q + 1 < kLeaf ? q + 1 : q], x[q]) : x[q];
-#pragma unroll
-                    for (int q = 0; q < kLeaf / V::E; ++q)
-                        reinterpret_cast<typename V::type*>(wm.leaf)[q] = V::make(&lp[q * V::E]);
-                }
+                for (int q = 0; q < kLeaf / V::E; ++q)
+                    reinterpret_cast<typename V::type*>(wm.leaf)[q] = V::make(&x[q * V::E]);
+                wm.owed = lprev;
             }
             if (wl < 0 && lane == 0) wmsg[warp].head = none;
             __syncthreads();
@@ -1099,7 +1075,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
                 const int ww = reg_key_winner<T>(h.key, h.pos, h.pos != INT_MAX);
                 if (G == 1) {
                     if (lane == max(ww, 0)) s_win = h;  // (no candidate: lane 0's empty one)
-                    if (ww >= 0) leaf_pivot_row<T>(wmsg[ww].leaf, s_urow, u, owe_u, lane);
+                    if (ww >= 0) leaf_pivot_row<T>(wmsg[ww], s_urow, u, owe_u, lane);
                 } else if (lane < G) {
                     const uint32_t dst = to_msg + (uint32_t)(par * sizeof(msg[0]));
                     const uint32_t bar = to_bar + (uint32_t)(par * sizeof(mbar[0]));
@@ -1134,7 +1110,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
                     const LeafHead h = lane < G ? msg[par][lane].head : none;
                     const int wo = reg_key_winner<T>(h.key, h.pos, h.pos != INT_MAX);
                     if (lane == max(wo, 0)) s_win = h;
-                    if (wo >= 0) leaf_pivot_row<T>(msg[par][wo].leaf, s_urow, u, owe_u, lane);
+                    if (wo >= 0) leaf_pivot_row<T>(msg[par][wo], s_urow, u, owe_u, lane);
                 }
             }
             if (warp == rcp_warp) {
