@@ -250,6 +250,234 @@ tf32x3_update_kernel(const __grid_constant__ CUtensorMap mAhi, const __grid_cons
 }
 
 
+// ---------------------------------------------------------------------
+// Streamed form of the update for K <= 64 and at least 128 columns: a
+// persistent CTA sweeps a run of 128 x 128 tiles down C's columns with every
+// stage in flight at once.  Bound by moving C (read and written once) through
+// HBM; a CTA per tile went through load, products, epilogue and store one
+// after the other with one CTA per SM: 163 us for 8128 x 8128 x 64, 3.2 TB/s.
+//
+// The column's B (hi, lo) stays in shared memory over the run, A (hi, lo)
+// comes in 32-deep chunks through two stages, C in slices of 32 columns, and
+// two accumulators of 128 TMEM columns let the products of one tile run beside
+// the epilogue of another.  224 KB of shared memory; warp 0 loads A and B, warp
+// 1 issues the products, warp 2 loads C, warps 4..11 update and store it: a
+// warpgroup per half of the tile's columns, each with three slice buffers of
+// its own (the next slices are on their way while one is updated and one
+// stored).  Buffers shared by the two warpgroups would not do: a barrier tells
+// two phases apart, and a warpgroup that skips a phase the other waits for may
+// take an older one for its own.
+// ---------------------------------------------------------------------
+constexpr int kStThreads = 384;
+constexpr int kStN = 128;                        // tile columns
+constexpr int kStHalf = kStN / 2;                // a warpgroup's columns
+constexpr int kStSlice = 32;                     // columns of a C buffer
+constexpr int kStCBufs = 3;                      // per warpgroup
+constexpr int kStOp = kTcM * 128;                // bytes of one operand chunk (128 rows x 32)
+constexpr int kStCBytes = kTcM * kStSlice * 4;
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+template <int KCH>
+__global__ void __launch_bounds__(kStThreads, 1)
+tf32x3_stream_kernel(const __grid_constant__ CUtensorMap mAhi, const __grid_constant__ CUtensorMap mAlo,
+                     const __grid_constant__ CUtensorMap mBhi, const __grid_constant__ CUtensorMap mBlo,
+                     const __grid_constant__ CUtensorMap mC, int M, int N, int* err)
+{
+    extern __shared__ uint8_t st_smem_raw[];
+    uint8_t* Bs = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(st_smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));  // [KCH][hi, lo]
+    uint8_t* As = Bs + KCH * 2 * kStOp;                                       // [2][hi, lo]
+    uint8_t* Cs = As + 2 * 2 * kStOp;                                         // [2][kStCBufs][32][128]
+    __shared__ __align__(8) uint64_t full[2], empty[2], bfull, bempty, tfull[2], tempty[2], cfull[2][kStCBufs],
+        cempty[2][kStCBufs];
+    __shared__ uint32_t s_tmem;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
+                     "r"((uint32_t)(2 * kStN))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int q = 0; q < 2; ++q) {
+            mbar_init(&full[q], 1);
+            mbar_init(&empty[q], 1);
+            mbar_init(&tfull[q], 1);
+            mbar_init(&tempty[q], 8);
+        }
+        mbar_init(&bfull, 1);
+        mbar_init(&bempty, 1);
+        for (int h = 0; h < 2; ++h)
+            for (int q = 0; q < kStCBufs; ++q) {
+                mbar_init(&cfull[h][q], 1);
+                mbar_init(&cempty[h][q], 1);
+            }
+        mbar_fence_init();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_tmem;
+    // this CTA's run of tiles, down the columns
+    const int mt = (M + kTcM - 1) / kTcM, nt = (N + kStN - 1) / kStN;
+    const int64_t tiles = (int64_t)mt * nt;
+    const int64_t t0 = tiles * blockIdx.x / gridDim.x;
+    const int mine = (int)(tiles * (blockIdx.x + 1) / gridDim.x - t0);
+    const int c0 = (int)(t0 / mt), r0 = (int)(t0 % mt);
+    // warpgroup h's slices of tile column `tc` that lie in C
+    auto slices = [&](int tc, int h) {
+        return min(kStHalf / kStSlice, max(0, (N - tc * kStN - h * kStHalf + kStSlice - 1) / kStSlice));
+    };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t it = 0, cols = 0;
+            bool ok = true;
+            for (int i = 0, tr = r0, tc = c0; i < mine && ok; ++i, ++tr) {
+                if (tr == mt) tr = 0, ++tc;
+                if (i == 0 || tr == 0) {
+                    if (cols > 0) ok = mbar_wait(&bempty, (cols - 1) & 1);
+                    if (!ok) break;
+                    mbar_expect_tx(&bfull, (uint32_t)(KCH * 2 * kStOp));
+#pragma unroll
+                    for (int kc = 0; kc < KCH; ++kc) {
+                        tma_load_2d(Bs + (2 * kc) * kStOp, &mBhi, &bfull, kc * kKChunk, tc * kStN);
+                        tma_load_2d(Bs + (2 * kc + 1) * kStOp, &mBlo, &bfull, kc * kKChunk, tc * kStN);
+                    }
+                    ++cols;
+                }
+                for (int kc = 0; kc < KCH; ++kc, ++it) {
+                    const uint32_t s = it & 1;
+                    if (it >= 2 && !mbar_wait(&empty[s], ((it >> 1) - 1) & 1)) {
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(&full[s], (uint32_t)(2 * kStOp));
+                    tma_load_2d(As + (2 * s) * kStOp, &mAhi, &full[s], kc * kKChunk, tr * kTcM);
+                    tma_load_2d(As + (2 * s + 1) * kStOp, &mAlo, &full[s], kc * kKChunk, tr * kTcM);
+                }
+            }
+            if (!ok) atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
+            // the last loads must have landed before the CTA leaves
+            if (cols > 0) mbar_wait(&bfull, (cols - 1) & 1);
+            for (uint32_t q = it > 2 ? it - 2 : 0; q < it; ++q) mbar_wait(&full[q & 1], (q >> 1) & 1);
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = tf32_idesc<kStN>();
+            uint32_t it = 0, cols = 0;
+            bool ok = true;
+            for (int i = 0, tr = r0; i < mine && ok; ++i, ++tr) {
+                if (tr == mt) tr = 0;
+                if (i == 0 || tr == 0) ok = mbar_wait(&bfull, cols++ & 1);
+                const uint32_t acc = tmem + (uint32_t)((i & 1) * kStN);
+                if (ok && i >= 2) ok = mbar_wait(&tempty[i & 1], ((i >> 1) - 1) & 1);
+                for (int kc = 0; kc < KCH && ok; ++kc, ++it) {
+                    const uint32_t s = it & 1;
+                    ok = mbar_wait(&full[s], (it >> 1) & 1);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t ahi = sw128_desc(As + (2 * s) * kStOp), alo = sw128_desc(As + (2 * s + 1) * kStOp);
+                    const uint64_t bhi = sw128_desc(Bs + (2 * kc) * kStOp), blo = sw128_desc(Bs + (2 * kc + 1) * kStOp);
+#pragma unroll
+                    for (int kk = 0; kk < kKChunk / 8; ++kk) {
+                        const uint64_t off = (uint64_t)(kk * 32) >> 4;  // 8 TF32 = 32 bytes
+                        umma_tf32(acc, alo + off, bhi + off, idesc, (kc > 0 || kk > 0) ? 1u : 0u);
+                        umma_tf32(acc, ahi + off, blo + off, idesc, 1);
+                        umma_tf32(acc, ahi + off, bhi + off, idesc, 1);
+                    }
+                    umma_commit(&empty[s]);
+                }
+                if (!ok) break;
+                if (tr + 1 == mt && i + 1 < mine) umma_commit(&bempty);
+                umma_commit(&tfull[i & 1]);
+            }
+            if (!ok) atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
+            // every product must be done before the tensor memory goes back
+            else if (mine > 0) mbar_wait(&tfull[(mine - 1) & 1], ((mine - 1) >> 1) & 1);
+        }
+    } else if (warp == 2) {
+        if (lane == 0) {
+            uint32_t it[2] = {0, 0};
+            bool ok = true;
+            for (int i = 0, tr = r0, tc = c0; i < mine && ok; ++i, ++tr) {
+                if (tr == mt) tr = 0, ++tc;
+                for (int e = 0; e < 2 * (kStHalf / kStSlice) && ok; ++e) {
+                    const int h = e & 1, sl = e >> 1;
+                    if (sl >= slices(tc, h)) continue;
+                    const uint32_t s = it[h] % kStCBufs;
+                    if (it[h] >= kStCBufs) ok = mbar_wait(&cempty[h][s], (it[h] / kStCBufs - 1) & 1);
+                    if (!ok) break;
+                    mbar_expect_tx(&cfull[h][s], (uint32_t)kStCBytes);
+                    tma_load_2d(Cs + (h * kStCBufs + s) * kStCBytes, &mC, &cfull[h][s], tr * kTcM,
+                                tc * kStN + h * kStHalf + sl * kStSlice);
+                    ++it[h];
+                }
+            }
+            if (!ok) atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
+            for (int h = 0; h < 2; ++h)
+                for (uint32_t q = it[h] > kStCBufs ? it[h] - kStCBufs : 0; q < it[h]; ++q)
+                    mbar_wait(&cfull[h][q % kStCBufs], (q / kStCBufs) & 1);
+        }
+    } else if (warp >= 4) {
+        const int h = (warp - 4) >> 2;          // this warpgroup's half
+        const int rl = (warp & 3) * 32 + lane;  // row within the tile = TMEM lane
+        const uint32_t tl = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(h * kStHalf);
+        uint32_t it = 0;
+        bool ok = true;
+        for (int i = 0, tr = r0, tc = c0; i < mine; ++i, ++tr) {
+            if (tr == mt) tr = 0, ++tc;
+            const int ns = slices(tc, h);
+            // (after a wait that ran out a warp goes on to meet its warpgroup's
+            // barriers, without waiting for data again)
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&tfull[i & 1], (i >> 1) & 1));
+            tc_fence_after();
+            for (int sl = 0; sl < ns; ++sl, ++it) {
+                const uint32_t s = it % kStCBufs;
+                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&cfull[h][s], (it / kStCBufs) & 1));
+                float* Ch = reinterpret_cast<float*>(Cs + (h * kStCBufs + s) * kStCBytes);
+                __syncwarp();
+                if (ok) {
+#pragma unroll
+                    for (int cb = 0; cb < kStSlice; cb += 16) {
+                        uint32_t v[16];
+                        tmem_ld16(tl + (uint32_t)((i & 1) * kStN + sl * kStSlice + cb), v);
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) Ch[(cb + e) * kTcM + rl] -= __uint_as_float(v[e]);
+                    }
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + h) : "memory");
+                if (ok && (warp & 3) == 0 && lane == 0) {
+                    tma_store_2d(&mC, Ch, tr * kTcM, tc * kStN + h * kStHalf + sl * kStSlice);
+                    tma_store_wait_read();  // the buffer is read out before it is loaded again
+                    mbar_arrive(&cempty[h][s]);
+                }
+                __syncwarp();
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (ok && lane == 0) mbar_arrive(&tempty[i & 1]);
+            __syncwarp();
+        }
+        if (!ok && lane == 0) atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * kStN))
+                     : "memory");
+    }
+}
+
+
 // A (m x K, column-major, lda) -> hi/lo row-major m x K (K contiguous), via
 // 32 x 32 shared-memory tiles so both sides stay coalesced.
 __global__ void split_transpose_kernel(int64_t m, int K, const float* __restrict__ A, int64_t lda,
@@ -332,22 +560,38 @@ static tmvg_status launch_update(Context* c, const CUtensorMap* maps, bool tmac,
 {
     constexpr size_t ops = (size_t)KCH * (2 * kTcM * 128 + 2 * BN * 128);
     dim3 grid((unsigned)ceil_div(m, kTcM), (unsigned)ceil_div(n, BN));
-    if (tmac) {
+    if constexpr (BN < kStN) if (tmac) {
         constexpr size_t smem = ops + (size_t)BN * kTcM * 4 + 1024;
         static_assert(smem <= 232448, "shared memory of one CTA");
         cudaFuncSetAttribute(tf32x3_update_kernel<BN, KCH, true>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         tf32x3_update_kernel<BN, KCH, true><<<grid, kTcThreads, smem, c->stream>>>(
             maps[0], maps[1], maps[2], maps[3], maps[4], C, ldc, (int)m, (int)n, c->dflags);
-    } else {
-        constexpr size_t smem = ops + 1024;
-        cudaFuncSetAttribute(tf32x3_update_kernel<BN, KCH, false>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        tf32x3_update_kernel<BN, KCH, false><<<grid, kTcThreads, smem, c->stream>>>(
-            maps[0], maps[1], maps[2], maps[3], maps[0], C, ldc, (int)m, (int)n, c->dflags);
+        ++c->launches;
+        return check_cuda(c, cudaGetLastError(), "tf32x3 update launch");
     }
+    constexpr size_t smem = ops + 1024;
+    cudaFuncSetAttribute(tf32x3_update_kernel<BN, KCH, false>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    tf32x3_update_kernel<BN, KCH, false><<<grid, kTcThreads, smem, c->stream>>>(
+        maps[0], maps[1], maps[2], maps[3], maps[0], C, ldc, (int)m, (int)n, c->dflags);
     ++c->launches;
     return check_cuda(c, cudaGetLastError(), "tf32x3 update launch");
+}
+
+// The streamed form (K = 32 KCH, n >= 128, C reachable by TMA).
+template <int KCH>
+static tmvg_status launch_stream(Context* c, const CUtensorMap* maps, int64_t m, int64_t n, int max_ctas)
+{
+    constexpr size_t smem = (size_t)(KCH * 2 + 4) * kStOp + 2 * kStCBufs * kStCBytes + 1024;
+    static_assert(smem <= 232448 - 512, "shared memory of one CTA");
+    const int64_t tiles = ceil_div(m, kTcM) * ceil_div(n, kStN);
+    const int64_t cap = max_ctas > 0 ? max_ctas : c->num_sms;
+    cudaFuncSetAttribute(tf32x3_stream_kernel<KCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    tf32x3_stream_kernel<KCH><<<(unsigned)std::min(tiles, cap), kStThreads, smem, c->stream>>>(
+        maps[0], maps[1], maps[2], maps[3], maps[4], (int)m, (int)n, c->dflags);
+    ++c->launches;
+    return check_cuda(c, cudaGetLastError(), "tf32x3 stream launch");
 }
 
 // C (m x n, column-major, ldc) as a tensor of 128 x BN tiles, rows innermost.
@@ -413,7 +657,7 @@ tmvg_status gemm_f32_tf32x3_update(Context* c, int64_t m, int64_t n, int64_t K, 
 }
 
 tmvg_status tf32x3_apply(Context* c, int64_t m, int64_t n, int64_t K, const Tf32x3Buffers& b, float* C,
-                         int64_t ldc)
+                         int64_t ldc, int max_ctas)
 {
     if (m <= 0 || n <= 0 || K <= 0) return TMVG_OK;
     if (!tf32x3_supported(K)) return set_error(c, TMVG_UNSUPPORTED, "tf32x3: K must be 32, 64, 96 or 128");
@@ -427,8 +671,10 @@ tmvg_status tf32x3_apply(Context* c, int64_t m, int64_t n, int64_t K, const Tf32
         return set_error(c, TMVG_CUDA_ERROR, "tf32x3: tensor map encoding failed");
     // the C tile by TMA when C's base and column stride are 16-byte aligned
     const bool tmac = (reinterpret_cast<uintptr_t>(C) & 15) == 0 && ldc % 4 == 0 &&
-                      make_c_map(&maps[4], C, m, n, ldc, BN);
+                      make_c_map(&maps[4], C, m, n, ldc, wide ? kStSlice : BN);
     const int kch = (int)(K / kKChunk);
+    if (wide && tmac)
+        return kch == 1 ? launch_stream<1>(c, maps, m, n, max_ctas) : launch_stream<2>(c, maps, m, n, max_ctas);
     if (wide) {
         if (kch == 1) return launch_update<128, 1>(c, maps, tmac, C, ldc, m, n);
         return launch_update<128, 2>(c, maps, tmac, C, ldc, m, n);

@@ -33,7 +33,7 @@ tmvg_status tf32x3_split_b(Context* c, int64_t n, int64_t K, const float* B, int
                            const Tf32x3Buffers& b);
 // C (m x n, column-major, ldc) -= A B from the split copies in b.
 tmvg_status tf32x3_apply(Context* c, int64_t m, int64_t n, int64_t K, const Tf32x3Buffers& b, float* C,
-                         int64_t ldc);
+                         int64_t ldc, int max_ctas = 0);
 
 // C (m x n, column-major, ldc) -= A (m x K, column-major, lda) * B (K x n,
 // column-major, ldb), FP32 data, 3xTF32 products accumulated in FP32.

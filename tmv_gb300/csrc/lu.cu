@@ -2120,7 +2120,10 @@ static tmvg_status update_columns(Context* c, int64_t n, T* A, int64_t lda, int6
     }
     if constexpr (std::is_same<T, float>::value) {
         // FP32 factor: 3xTF32 on the tensor cores keeps FP32 accuracy
-        if (tc) return tf32x3_apply(c, rest, nc, nb, bc, A + (k + nb) + c0 * lda, lda);
+        // (persistent, like the sliced product below: the next panel's cluster keeps its SMs)
+        if (tc)
+            return tf32x3_apply(c, rest, nc, nb, bc, A + (k + nb) + c0 * lda, lda,
+                                std::max(1, c->num_sms - kClusterCtas));
     } else {
         // the sliced product is persistent, one CTA per SM: it leaves the next
         // panel's cluster its SMs, or that cluster's share of the tiles would
