@@ -47,21 +47,26 @@ template <typename T>
 constexpr int panel_width() { return sizeof(T) == 8 ? 64 : 128; }
 
 // ---------------------------------------------------------------------
-// Columns that TMV factors as the second column of a two-column leaf of its
-// recursion (split N1 = R/2, rounded down to a multiple of 64 above 64,
-// src/TMV_LUDecompose.cpp:241-245).  Their pivot scan starts from max = 0,
-// which only matters for NaN input.
+// Whether TMV factors column j of R as the second column of a two-column leaf
+// of its recursion (split N1 = R/2, rounded down to a multiple of 64 above 64,
+// src/TMV_LUDecompose.cpp:241-245).  Its pivot scan starts from max = 0, which
+// only matters for NaN input.  The panel kernels follow the recursion
+// themselves while their columns are loaded; a table made on the host cost
+// every factorisation an upload and a wait for it.
 // ---------------------------------------------------------------------
-static void leaf_modes(int64_t off, int64_t R, std::vector<unsigned char>& modes)
+__device__ __forceinline__ bool second_of_pair(int64_t R, int64_t j)
 {
-    if (R > 2) {
+    while (R > 2) {
         int64_t N1 = R / 2;
         if (N1 > 64) N1 = (N1 / 64) * 64;
-        leaf_modes(off, N1, modes);
-        leaf_modes(off + N1, R - N1, modes);
-    } else if (R == 2) {
-        modes[off + 1] = 1;
+        if (j < N1) {
+            R = N1;
+        } else {
+            j -= N1;
+            R -= N1;
+        }
     }
+    return R == 2 && j == 1;
 }
 
 // ---------------------------------------------------------------------
@@ -70,7 +75,7 @@ static void leaf_modes(int64_t off, int64_t R, std::vector<unsigned char>& modes
 template <typename T>
 __global__ void __launch_bounds__(kPanelThreads)
 lu_panel_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int nb,
-                int64_t* __restrict__ P, const unsigned char* __restrict__ modes,
+                int64_t* __restrict__ P,
                 int rows_per_cta, double* cand_key, long long* cand_idx,
                 T* cand_rows, T* diag_row, unsigned* bar, int* err, int* pairs)
 {
@@ -82,6 +87,7 @@ lu_panel_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int nb,
     __shared__ double w_key;
     __shared__ long long w_idx;
     __shared__ T urow[kPanelMax];
+    __shared__ unsigned char s_mode[kPanelMax];
     __shared__ int s_piv[kPanelMax];
 
     const int G = gridDim.x;
@@ -95,12 +101,13 @@ lu_panel_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int nb,
         const int r = t % nr, cc = t / nr;
         rows[r * ldp + cc] = A[(k + r0 + r) + (k + cc) * lda];
     }
+    for (int j = tid; j < nb; j += kPanelThreads) s_mode[j] = second_of_pair(n, k + j);
     __syncthreads();
 
     bool prev_uf = false;
     for (int jj = 0; jj < nb; ++jj) {
         const int par = jj & 1;
-        const bool r2 = modes[jj] && !prev_uf;
+        const bool r2 = s_mode[jj] && !prev_uf;
 
         // 1. this CTA's best candidate among panel rows >= jj
         double bk = -INFINITY;
@@ -217,7 +224,7 @@ constexpr int kClusterCtas = 16;
 template <typename T>
 __global__ void __launch_bounds__(kPanelThreads)
 lu_panel_cluster_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int nb,
-                        int64_t* __restrict__ P, const unsigned char* __restrict__ modes,
+                        int64_t* __restrict__ P,
                         int rows_per_cta, int* pairs)
 {
     namespace cg = cooperative_groups;
@@ -235,6 +242,7 @@ lu_panel_cluster_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, in
     __shared__ T cand_row[2][kPanelMax];
     __shared__ T diag_row[2][kPanelMax];
     __shared__ T urow[kPanelMax];
+    __shared__ unsigned char s_mode[kPanelMax];
     __shared__ int s_piv[kPanelMax];
 
     const int G = (int)cluster.num_blocks();
@@ -248,12 +256,13 @@ lu_panel_cluster_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, in
         const int r = t % nr, cc = t / nr;
         rows[r * ldp + cc] = A[(k + r0 + r) + (k + cc) * lda];
     }
+    for (int j = tid; j < nb; j += kPanelThreads) s_mode[j] = second_of_pair(n, k + j);
     __syncthreads();
 
     bool prev_uf = false;
     for (int jj = 0; jj < nb; ++jj) {
         const int par = jj & 1;
-        const bool r2 = modes[jj] && !prev_uf;
+        const bool r2 = s_mode[jj] && !prev_uf;
         const int owner_j = jj / rows_per_cta;
         // each thread scans (and later updates) the rows tid, tid + 256, ...
         double bk = -INFINITY;
@@ -573,7 +582,7 @@ __device__ __forceinline__ void reg2_update(T (&x)[NB], T lx, bool ux, T (&y)[NB
 template <typename T, int NB>
 __global__ void __launch_bounds__(kReg2Threads, 1)
 lu_panel_cluster_reg2_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int nb,
-                             int64_t* __restrict__ P, const unsigned char* __restrict__ modes,
+                             int64_t* __restrict__ P,
                              int rows_per_cta, int* pairs, int* err, float* __restrict__ ahi,
                              float* __restrict__ alo, const T* __restrict__ Sp, int64_t lds)
 {
@@ -617,7 +626,7 @@ lu_panel_cluster_reg2_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t 
         s_abort = 0;
         mbar_fence_init();
     }
-    for (int j = tid; j < nb; j += kReg2Threads) s_mode[j] = modes[j];
+    for (int j = tid; j < nb; j += kReg2Threads) s_mode[j] = second_of_pair(n, k + j);
     const T* Xp = Sp ? Sp : Ap;
     const int64_t ldx = Sp ? lds : lda;
     T x[NB], y[NB];
@@ -969,7 +978,7 @@ __device__ __forceinline__ void leaf_pivot_row(const LeafMsg<T>& w, T (*s_urow)[
 template <typename T, int NB>
 __global__ void __launch_bounds__(kLeafThreads, 1)
 lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int nb,
-                     int64_t* __restrict__ P, const unsigned char* __restrict__ modes,
+                     int64_t* __restrict__ P,
                      int rows_per_cta, int* pairs, int* err, float* __restrict__ ahi,
                      float* __restrict__ alo, const T* __restrict__ Sp, int64_t lds)
 {
@@ -1014,12 +1023,12 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
         s_npairs = 0;
         mbar_fence_init();
     }
-    for (int j = tid; j < nb; j += nthr) s_mode[j] = modes[j];
     const T* Xp = Sp ? Sp : Ap;
     const int64_t ldx = Sp ? lds : lda;
     T x[NB];
 #pragma unroll
     for (int c = 0; c < NB; ++c) x[c] = (have && c < nb) ? Xp[r0 + tid + c * ldx] : T(0);
+    for (int j = tid; j < nb; j += nthr) s_mode[j] = second_of_pair(n, k + j);  // (while the row is loaded)
     int pos = r0 + tid;  // this row's current position
     bool act = have;     // still a candidate (not yet a pivot row)
     const int loc = (cta << 16) | tid;
@@ -2205,7 +2214,7 @@ static int cluster_panel_width(int64_t n)
 
 template <typename T>
 static tmvg_status launch_panel_cluster(Context* c, cudaStream_t s, T* A, int64_t lda, int64_t n, int64_t k,
-                                        int nb, int64_t* P, const unsigned char* modes, int* pairs)
+                                        int nb, int64_t* P, int* pairs)
 {
     const int64_t m = n - k;
     const int rpc = (int)ceil_div(m, kClusterCtas);
@@ -2224,7 +2233,7 @@ static tmvg_status launch_panel_cluster(Context* c, cudaStream_t s, T* A, int64_
     ++c->launches;
     return check_cuda(c,
                       cudaLaunchKernelEx(&cfg, lu_panel_cluster_kernel<T>, A, lda, n, k, nb, P,
-                                         modes, rpc, pairs),
+                                         rpc, pairs),
                       "lu: cluster panel launch");
 }
 
@@ -2265,7 +2274,7 @@ static bool reg_panel_ok(Context* c)
 
 template <typename T>
 static tmvg_status launch_panel_cluster_reg(Context* c, cudaStream_t s, T* A, int64_t lda, int64_t n,
-                                            int64_t k, int nb, int64_t* P, const unsigned char* modes,
+                                            int64_t k, int nb, int64_t* P,
                                             int* pairs, float* ahi, float* alo, const T* Sp = nullptr,
                                             int64_t lds = 0)
 {
@@ -2305,12 +2314,12 @@ static tmvg_status launch_panel_cluster_reg(Context* c, cudaStream_t s, T* A, in
     if (c->panel_reg2)
         return check_cuda(c,
                           cudaLaunchKernelEx(&cfg, lu_panel_cluster_reg2_kernel<T, RegPanel<T>::NB>, A,
-                                             lda, n, k, nb, P, modes, rpc, pairs, c->dflags, ahi, alo, Sp,
+                                             lda, n, k, nb, P, rpc, pairs, c->dflags, ahi, alo, Sp,
                                              lds),
                           "lu: register panel launch");
     return check_cuda(c,
                       cudaLaunchKernelEx(&cfg, lu_panel_leaf_kernel<T, RegPanel<T>::NB>, A, lda, n, k,
-                                         nb, P, modes, rpc, pairs, c->dflags, ahi, alo, Sp, lds),
+                                         nb, P, rpc, pairs, c->dflags, ahi, alo, Sp, lds),
                       "lu: leaf register panel launch");
 }
 
@@ -2331,13 +2340,12 @@ tmvg_status lu_factor(Context* c, int64_t n, T* A, int64_t lda, int64_t* P)
     if (smem_full > 200 * 1024)
         return set_error(c, TMVG_UNSUPPORTED, "lu: matrix too tall for the shared-memory panel");
 
-    // Workspace: modes (n bytes), candidate keys/indices/rows, diag rows.
+    // Workspace: candidate keys/indices/rows, diag rows, row pairs.
     const size_t off_key = 0;
     const size_t off_idx = off_key + sizeof(double) * 2 * G_full;
     const size_t off_rows = (off_idx + sizeof(long long) * 2 * G_full + 255) & ~size_t(255);
     const size_t off_diag = off_rows + sizeof(T) * 2 * G_full * kPanelMax;
-    const size_t off_modes = (off_diag + sizeof(T) * 2 * kPanelMax + 255) & ~size_t(255);
-    const size_t off_pairs = (off_modes + (size_t)n + 255) & ~size_t(255);
+    const size_t off_pairs = (off_diag + sizeof(T) * 2 * kPanelMax + 255) & ~size_t(255);
     // two pair lists: with look-ahead, step s+1's panel writes its list while
     // step s's interchanges still read theirs
     const size_t pairs_len = 1 + 2 * (size_t)kMaxPairs;
@@ -2348,20 +2356,7 @@ tmvg_status lu_factor(Context* c, int64_t n, T* A, int64_t lda, int64_t* P)
     long long* cand_idx = (long long*)(ws + off_idx);
     T* cand_rows = (T*)(ws + off_rows);
     T* diag_row = (T*)(ws + off_diag);
-    unsigned char* modes = ws + off_modes;
     int* pairs = (int*)(ws + off_pairs);
-    {
-        std::vector<unsigned char> hm((size_t)n, 0);
-        leaf_modes(0, n, hm);
-        tmvg_status st = check_cuda(
-            c, cudaMemcpyAsync(modes, hm.data(), (size_t)n, cudaMemcpyHostToDevice, c->stream),
-            "lu: modes upload");
-        if (st) return st;
-        // the host vector must outlive the copy
-        st = check_cuda(c, cudaStreamSynchronize(c->stream), "lu: modes sync");
-        if (st) return st;
-    }
-
     static bool attr_set[2] = {false, false};
     const int ai = sizeof(T) == 8 ? 0 : 1;
     if (!attr_set[ai]) {
@@ -2424,10 +2419,10 @@ tmvg_status lu_factor(Context* c, int64_t n, T* A, int64_t lda, int64_t* P)
             int* pp = pairs_of(step);
             tmvg_status s2 =
                 reg ? (from_scratch
-                           ? launch_panel_cluster_reg<T>(c, side, A, lda, n, kk, w, P, modes + kk, pp, ahi, alo,
+                           ? launch_panel_cluster_reg<T>(c, side, A, lda, n, kk, w, P, pp, ahi, alo,
                                                          Sbuf[(step - 1) & 1] + nbmax, n)
-                           : launch_panel_cluster_reg<T>(c, side, A, lda, n, kk, w, P, modes + kk, pp, ahi, alo))
-                    : launch_panel_cluster<T>(c, side, A, lda, n, kk, w, P, modes + kk, pp);
+                           : launch_panel_cluster_reg<T>(c, side, A, lda, n, kk, w, P, pp, ahi, alo))
+                    : launch_panel_cluster<T>(c, side, A, lda, n, kk, w, P, pp);
             if (!s2 && c->serialize_lookahead) s2 = check_cuda(c, cudaStreamSynchronize(side), "lu: serialize");
             return s2;
         };
@@ -2519,12 +2514,11 @@ tmvg_status lu_factor(Context* c, int64_t n, T* A, int64_t lda, int64_t* P)
         if (st) return st;
         T* Ap = A;
         int64_t* Pp = P;
-        const unsigned char* mp = modes + k;
         int64_t ldav = lda, nv = n, kv = k;
         int nbv = nb, rpc = rows_per_cta;
         unsigned* bar = c->dbar;
         int* err = c->dflags;
-        void* args[] = {&Ap, &ldav, &nv, &kv, &nbv, &Pp, &mp, &rpc, &cand_key, &cand_idx,
+        void* args[] = {&Ap, &ldav, &nv, &kv, &nbv, &Pp, &rpc, &cand_key, &cand_idx,
                         &cand_rows, &diag_row, &bar, &err, &pairs};
         {
             ScopedTimer timer(c, kClsPanel, 2.0 * sizeof(T) * m * nb, panel_flops(m, nb));
@@ -2803,7 +2797,7 @@ template tmvg_status copy_matrix<float>(Context*, int64_t, int64_t, const float*
 // simplest schedule: the cooperative grid-barrier panel (lu_panel_kernel)
 // with no look-ahead, and every scratch word taken from the file-scope array
 // below, which each GPU that loads this library holds until the process
-// exits (kNoAllocBytes = 353,540 bytes, about 345 KiB).  It needs no
+// exits (kNoAllocBytes = 337,156 bytes, about 329 KiB).  It needs no
 // tmvg_handle (creating one allocates).  Limits: n <= kNoAllocMaxN = 16384
 // (larger n returns TMVG_UNSUPPORTED before any device work); at most
 // kNoAllocMaxCtas = 160 panel CTAs are used, and a panel CTA's rows must fit
@@ -2820,8 +2814,7 @@ constexpr size_t kNaOffKey = 256;  // double[2 * kNoAllocMaxCtas]
 constexpr size_t kNaOffIdx = kNaOffKey + sizeof(double) * 2 * kNoAllocMaxCtas;
 constexpr size_t kNaOffRows = kNaOffIdx + sizeof(long long) * 2 * kNoAllocMaxCtas;
 constexpr size_t kNaOffDiag = kNaOffRows + sizeof(double) * 2 * kNoAllocMaxCtas * kPanelMax;
-constexpr size_t kNaOffModes = kNaOffDiag + sizeof(double) * 2 * kPanelMax;
-constexpr size_t kNaOffPairs = kNaOffModes + kNoAllocMaxN;  // int[1 + 2*kMaxPairs]
+constexpr size_t kNaOffPairs = kNaOffDiag + sizeof(double) * 2 * kPanelMax;  // int[1 + 2*kMaxPairs]
 constexpr size_t kNoAllocBytes = kNaOffPairs + sizeof(int) * (1 + 2 * kMaxPairs);
 constexpr size_t kNoAllocSmemMax = 200 * 1024;
 }  // namespace
@@ -2892,21 +2885,11 @@ extern "C" tmvg_status tmvg_lu_decompose_f64_noalloc(int64_t n, double* A, int64
     long long* cand_idx = reinterpret_cast<long long*>(s + kNaOffIdx);
     double* cand_rows = reinterpret_cast<double*>(s + kNaOffRows);
     double* diag_row = reinterpret_cast<double*>(s + kNaOffDiag);
-    unsigned char* modes = s + kNaOffModes;
     int* pairs = reinterpret_cast<int*>(s + kNaOffPairs);
 
     // The array keeps the last call's contents: clear the error words.
     st = check_cuda(&c, cudaMemsetAsync(s, 0, 256, c.stream), "noalloc: clear");
     if (st) return st;
-    {
-        std::vector<unsigned char> hm((size_t)n, 0);
-        leaf_modes(0, n, hm);
-        st = check_cuda(&c, cudaMemcpyAsync(modes, hm.data(), (size_t)n, cudaMemcpyHostToDevice, c.stream),
-                        "noalloc: modes");
-        if (st) return st;
-        st = check_cuda(&c, cudaStreamSynchronize(c.stream), "noalloc: modes sync");
-        if (st) return st;
-    }
     for (int64_t k = 0; k < n; k += nbmax) {
         const int nb = (int)std::min<int64_t>(nbmax, n - k);
         const int64_t m = n - k;
@@ -2917,12 +2900,11 @@ extern "C" tmvg_status tmvg_lu_decompose_f64_noalloc(int64_t n, double* A, int64
         if (st) return st;
         double* Ap = A;
         int64_t* Pp = P;
-        const unsigned char* mp = modes + k;
         int64_t ldav = lda, nv = n, kv = k;
         int nbv = nb, rpc = rows_per_cta;
         unsigned* bar = c.dbar;
         int* err = c.dflags;
-        void* args[] = {&Ap, &ldav, &nv, &kv, &nbv, &Pp, &mp, &rpc, &cand_key, &cand_idx,
+        void* args[] = {&Ap, &ldav, &nv, &kv, &nbv, &Pp, &rpc, &cand_key, &cand_idx,
                         &cand_rows, &diag_row, &bar, &err, &pairs};
         st = check_cuda(&c,
                         cudaLaunchCooperativeKernel((const void*)lu_panel_kernel<double>, dim3(G),
