@@ -975,6 +975,44 @@ __device__ __forceinline__ void leaf_pivot_row(const LeafMsg<T>& w, T (*s_urow)[
     }
 }
 
+// The leaf's U12 in place: rows t of Ur, columns [kLeaf, pw), lane (t, c) of a
+// warp for entry (t, column c of four), two groups of four columns at a time.
+// Row q's values go to the rows below by shuffle, so the chain is 7 fused
+// multiply-adds; a column per thread was a chain of 28, and a DFMA takes its
+// sub-partition 64 clocks whatever the lanes.
+template <typename T, int NB>
+__device__ __forceinline__ void leaf_u12(T (*Ur)[NB], unsigned ufmask, int pw, int warp, int nwarp, int lane)
+{
+    using V = Vec16<T>;
+    const int t = lane >> 2, c = lane & 3;
+    if (kLeaf + 4 * warp >= pw) return;
+    // (a lane's multipliers in vectors: the rows share their banks)
+    T l[kLeaf];
+#pragma unroll
+    for (int v = 0; v < kLeaf / V::E; ++v) {
+        const typename V::type lv = reinterpret_cast<const typename V::type*>(Ur[t])[v];
+#pragma unroll
+        for (int e = 0; e < V::E; ++e) l[v * V::E + e] = V::get(lv, e);
+    }
+    for (int p0 = kLeaf + 4 * warp; p0 < pw; p0 += 8 * nwarp) {  // (the same in every lane)
+        const int pa = p0 + c, pb = p0 + 4 * nwarp + c;
+        const bool two = p0 + 4 * nwarp < pw;
+        T ua = pa < pw ? Ur[t][pa] : T(0), ub = pb < pw ? Ur[t][pb] : T(0);
+#pragma unroll
+        for (int q = 0; q < kLeaf - 1; ++q) {
+            const bool on = t > q && !((ufmask >> q) & 1u);
+            const T qa = __shfl_sync(0xffffffffu, ua, 4 * q + c);
+            if (on) ua = fma(-l[q], qa, ua);
+            if (two) {
+                const T qb = __shfl_sync(0xffffffffu, ub, 4 * q + c);
+                if (on) ub = fma(-l[q], qb, ub);
+            }
+        }
+        if (pa < pw) Ur[t][pa] = ua;
+        if (pb < pw) Ur[t][pb] = ub;
+    }
+}
+
 template <typename T, int NB>
 __global__ void __launch_bounds__(kLeafThreads, 1)
 lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int nb,
@@ -1033,11 +1071,12 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
     bool act = have;     // still a candidate (not yet a pivot row)
     const int loc = (cta << 16) | tid;
     const LeafHead none{0ull, INT_MAX, -1};
-    static_assert(kClusterCtas <= 32 && kLeafWarps >= kClusterCtas, "a candidate per lane, a reciprocal per CTA");
-    // (warp 0's lane d sends to CTA d)
-    const uint32_t to_msg = cluster_addr(&msg[0][cta], lane < G ? lane : 0);
-    const uint32_t to_bar = cluster_addr(&mbar[0], lane < G ? lane : 0);
-    const int rcp_warp = nwarp > 1 ? 1 : 0;
+    static_assert(kClusterCtas == 16 && kLeafWarps >= kClusterCtas, "a candidate per lane, a reciprocal per CTA");
+    // (warp 0's lanes d and d + 16 send to CTA d)
+    const int dest = lane & (kClusterCtas - 1);
+    const uint32_t to_msg = cluster_addr(&msg[0][cta], dest < G ? dest : 0);
+    const uint32_t to_bar = cluster_addr(&mbar[0], dest < G ? dest : 0);
+    constexpr int kRcpWarp = 1;  // (every block has two warps)
     if (G > 1 && tid == 0) mbar_expect_tx(&mbar[0], (uint32_t)(G * sizeof(LeafMsg<T>)));
     cluster.sync();  // every CTA's mbarriers are initialised before any message
 
@@ -1085,12 +1124,15 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
                 if (G == 1) {
                     if (lane == max(ww, 0)) s_win = h;  // (no candidate: lane 0's empty one)
                     if (ww >= 0) leaf_pivot_row<T>(wmsg[ww], s_urow, u, owe_u, lane);
-                } else if (lane < G) {
+                } else if (dest < G) {
                     const uint32_t dst = to_msg + (uint32_t)(par * sizeof(msg[0]));
                     const uint32_t bar = to_bar + (uint32_t)(par * sizeof(mbar[0]));
                     const uint4* from = reinterpret_cast<const uint4*>(&wmsg[max(ww, 0)]);
 #pragma unroll
-                    for (int q = 0; q < kMsgVecs; ++q) st_async16(dst + 16 * q, from[q], bar);
+                    for (int q = 0; q < kMsgVecs; q += 2) {
+                        const int v = q + (lane >> 4);
+                        if (v < kMsgVecs) st_async16(dst + 16 * v, from[v], bar);
+                    }
                 }
             }
             // 3. the shadow: work this row owes, while the messages travel
@@ -1122,7 +1164,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
                     if (wo >= 0) leaf_pivot_row<T>(msg[par][wo], s_urow, u, owe_u, lane);
                 }
             }
-            if (warp == rcp_warp) {
+            if (warp == kRcpWarp) {
                 // every candidate's reciprocal, beside warp 0's decision
                 const bool got = G == 1 || __all_sync(0xffffffffu, mbar_wait(&mbar[par], (uint32_t)((j >> 1) & 1)));
                 if (got && lane < (G > 1 ? G : nwarp)) {
@@ -1187,19 +1229,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             __syncthreads();
             if (s_abort) break;
             T(*Ur)[NB] = s_rem[lpar];
-            for (int p = kLeaf + tid; p < pw; p += nthr) {
-                T uc[kLeaf];
-#pragma unroll
-                for (int t = 0; t < kLeaf; ++t) uc[t] = Ur[t][p];
-#pragma unroll
-                for (int t = 1; t < kLeaf; ++t) {
-#pragma unroll
-                    for (int q = 0; q < t; ++q)
-                        if (!((ufmask >> q) & 1u)) uc[t] = fma(-Ur[t][q], uc[q], uc[t]);
-                }
-#pragma unroll
-                for (int t = 0; t < kLeaf; ++t) Ur[t][p] = uc[t];
-            }
+            leaf_u12<T, NB>(Ur, ufmask, pw, warp, nwarp, lane);
             __syncthreads();
             if (act) leaf_rank8<T, NB, 0, 0, NB>(x, &Ur[0][0], ufmask, pw);
             else if (dstep >= 0) leaf_take_u<T, NB>(x, Ur[dstep], pw);
@@ -2303,9 +2333,10 @@ static tmvg_status launch_panel_cluster_reg(Context* c, cudaStream_t s, T* A, in
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(G);
-    // the leaf panel launches no warps without rows (at least two: warp 0 also
-    // decides)
-    cfg.blockDim = dim3(c->panel_reg2 ? kReg2Threads : std::max(64, (int)ceil_div(rpc, 32) * 32));
+    // the leaf panel launches no warps without rows, but at least one per
+    // sub-partition: warp 0 decides, warp 1 takes the reciprocals, and all
+    // share the leaf's U12
+    cfg.blockDim = dim3(c->panel_reg2 ? kReg2Threads : std::max(128, (int)ceil_div(rpc, 32) * 32));
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
     cfg.attrs = attr;
