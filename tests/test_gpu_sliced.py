@@ -48,9 +48,9 @@ def _sliced(a, b):
     return ta[:, None] + tb[None, :] - k >= np.ceil(1.75 * np.sqrt(k))
 
 
-# tiles are 128 x 64, stages 32 and accumulation chunks 128 in K
+# tiles are 128 x 64 (128 x 32 for short K), stages 32 and accumulation chunks 128 in K
 SIZES = [(128, 64, 1500), (127, 64, 1600), (129, 65, 1537), (300, 200, 255), (640, 257, 129), (257, 700, 97),
-         (1000, 500, 32), (70, 2800, 64), (64, 3000, 160), (2500, 50, 128)]
+         (1000, 500, 32), (70, 2800, 64), (64, 3000, 160), (2500, 50, 128), (600, 289, 96), (1300, 97, 127)]
 
 
 @pytest.mark.parametrize("m,n,k", SIZES)

@@ -33,7 +33,9 @@
 // digit i of A with digits 0..7-i of B at once (they lie behind one another
 // in shared memory, and so do their accumulators in the 512 TMEM columns:
 // N = 64 (8 - i), in pieces of up to 256, so that A is read once per 256
-// columns); sixteen warps drain the accumulators after every K = 128.
+// columns); sixteen warps drain the accumulators after every K = 128.  Short K
+// takes tiles of 128 x 32: two sets of accumulators fit, and one tile is
+// multiplied while another is drained.
 // All waits are bounded; on a timeout the kernel records kDevTimeout.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -48,14 +50,11 @@
 namespace tmvg {
 
 constexpr int kSlices = 8;
-constexpr int kSlM = 128, kSlN = 64;    // tile of C
+constexpr int kSlM = 128, kSlN = 64;    // tile of C (short K: 128 x 32)
 constexpr int kSlK = 32;                // K per stage: 64 bytes of BF16
 constexpr int kSlChunk = 4;             // stages per accumulation chunk (K = 128)
 constexpr int kSlStages = 2;
 constexpr int kSlABytes = kSlices * kSlM * kSlK * 2;
-constexpr int kSlBBytes = kSlices * kSlN * kSlK * 2;
-constexpr int kSlStageBytes = kSlABytes + kSlBBytes;
-constexpr size_t kSlSmem = (size_t)kSlStages * kSlStageBytes + 1024;
 constexpr int kSlEpiWarps = 16;  // 4 per scheduler: the epilogue is bound by latencies
 constexpr int kSlThreads = 32 * (kSlEpiWarps + 2);
 static_assert(kSlM / 16 * kSlN == 32 * kSlEpiWarps, "a prefetch per epilogue thread");
@@ -325,6 +324,19 @@ __device__ __forceinline__ void sl_combine(const uint32_t (&a)[kSlices], long lo
     q = (long long)i3 * 16777216 + ((long long)i4 * 65536 + ((long long)i5 * 256 + (long long)i6 * 4));
 }
 
+// A chunk's eight accumulators of one element into its 96-bit sum: q + (p << 32).
+__device__ __forceinline__ void sl_add(const uint32_t (&a)[kSlices], uint32_t& t0, uint32_t& t1, uint32_t& t2)
+{
+    long long p, q;
+    sl_combine(a, p, q);
+    const uint32_t q0 = (uint32_t)q, q1 = (uint32_t)((unsigned long long)q >> 32);
+    const uint32_t p0 = (uint32_t)p, p1 = (uint32_t)((unsigned long long)p >> 32);
+    asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
+        : "+r"(t0), "+r"(t1), "+r"(t2)
+        : "r"(q0), "r"(q1), "r"((uint32_t)((int)q1 >> 31)));
+    asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, %3;" : "+r"(t1), "+r"(t2) : "r"(p0), "r"(p1));
+}
+
 // The 96-bit integer (w2:w1:w0) 2^(e - 62) rounded to FP64 (nearest; a tie
 // goes away from zero), on the integer pipe and without branches.
 __device__ __forceinline__ double sl_to_double(uint32_t w0, uint32_t w1, uint32_t w2, int e)
@@ -384,13 +396,14 @@ __device__ __forceinline__ void sl_tile(const SlicedArgs& g, int64_t t, int64_t&
 }
 
 // First look at a tile: 1 good, 0 undecided, -1 for the FP64 pipe.
+template <int TN>
 __device__ __forceinline__ int sl_look(const SlicedArgs& g, int64_t mi, int64_t ni)
 {
     int a = INT_MAX / 4, b = INT_MAX / 4;
     const int64_t a1 = min((g.M - 1) / g.ga, (mi * kSlM + kSlM - 1) / g.ga);
-    const int64_t b1 = min((g.N - 1) / g.gb, (ni * kSlN + kSlN - 1) / g.gb);
+    const int64_t b1 = min((g.N - 1) / g.gb, (ni * TN + TN - 1) / g.gb);
     for (int64_t i = mi * kSlM / g.ga; i <= a1; ++i) a = min(a, __ldg(&g.fa[i]));
-    for (int64_t i = ni * kSlN / g.gb; i <= b1; ++i) b = min(b, __ldg(&g.fb[i]));
+    for (int64_t i = ni * TN / g.gb; i <= b1; ++i) b = min(b, __ldg(&g.fb[i]));
     if (a < 0 || b < 0) return -1;
     return (int64_t)a + b - g.K >= g.need ? 1 : 0;
 }
@@ -398,12 +411,13 @@ __device__ __forceinline__ int sl_look(const SlicedArgs& g, int64_t mi, int64_t 
 // Second look (the whole CTA): the sum of |leading digit of a| |leading digit
 // of b| over K reaches need_sum for every element, or the element's row or
 // column is zero.
+template <int TN>
 __device__ __noinline__ bool sl_look_again(const SlicedArgs& g, int64_t mi, int64_t ni)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool work = warp < kSlEpiWarps;
+    const bool work = warp < kSlEpiWarps / (kSlN / TN);
     const int64_t r = mi * kSlM + (warp & 3) * 32 + lane;
-    const int64_t c0 = ni * kSlN + (int64_t)(warp >> 2) * kSlCols;
+    const int64_t c0 = ni * TN + (int64_t)(warp >> 2) * kSlCols;
     const int nc = work ? (int)max((int64_t)0, min((int64_t)kSlCols, g.N - c0)) : 0;
     bool pass = !work || r >= g.M || __ldg(&g.ea[r]) == kZeroExp;
     unsigned todo = pass ? 0u : (1u << nc) - 1u;
@@ -434,14 +448,24 @@ __device__ __noinline__ bool sl_look_again(const SlicedArgs& g, int64_t mi, int6
     return false;
 }
 
+template <int TN>
+__host__ __device__ constexpr int sl_stage_bytes() { return kSlABytes + kSlices * TN * kSlK * 2; }
+
+template <int TN>
 __global__ void __launch_bounds__(kSlThreads, 1)
 sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB,
                    const __grid_constant__ SlicedArgs g, int* err)
 {
+    // TN = 64: the accumulators of a tile take all 512 TMEM columns, and all
+    // sixteen epilogue warps drain them.  TN = 32: two tiles' accumulators, and
+    // eight warps for each, so that one tile is multiplied while the other is
+    // drained, rounded and stored.
+    constexpr int GR = kSlN / TN, GW = kSlEpiWarps / GR;
+    constexpr int kStageBytes = sl_stage_bytes<TN>();
     extern __shared__ uint8_t sl_smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(sl_smem_raw) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
-    __shared__ __align__(8) uint64_t full[kSlStages], empty[kSlStages], acc_full, acc_empty;
+    __shared__ __align__(8) uint64_t full[kSlStages], empty[kSlStages], acc_full[GR], acc_empty[GR];
     __shared__ uint32_t s_tmem;
     __shared__ uint32_t s_ok[kMaxTilesPerCta / 32];
     __shared__ int s_open;
@@ -459,8 +483,10 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
             mbar_init(&empty[s], 1);
         }
         s_open = 0;
-        mbar_init(&acc_full, 1);
-        mbar_init(&acc_empty, kSlEpiWarps);
+        for (int s = 0; s < GR; ++s) {
+            mbar_init(&acc_full[s], 1);
+            mbar_init(&acc_empty[s], GW);
+        }
         mbar_fence_init();
     }
     sl_fence_before();
@@ -477,7 +503,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
         int look = 1;
         if (i0 + lane < mine) {
             sl_tile(g, blockIdx.x + (int64_t)(i0 + lane) * gridDim.x, mi, ni);
-            look = sl_look(g, mi, ni);
+            look = sl_look<TN>(g, mi, ni);
         }
         const unsigned good = __ballot_sync(0xffffffffu, look == 1), open = __ballot_sync(0xffffffffu, look == 0);
         if (lane == 0) {
@@ -491,7 +517,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
             if ((s_ok[i >> 5] >> (i & 31)) & 1u) continue;
             int64_t mi, ni;
             sl_tile(g, blockIdx.x + (int64_t)i * gridDim.x, mi, ni);
-            const bool again = sl_look(g, mi, ni) == 0 && sl_look_again(g, mi, ni);
+            const bool again = sl_look<TN>(g, mi, ni) == 0 && sl_look_again<TN>(g, mi, ni);
             __syncthreads();  // every thread has read the word
             if (again && tid == 0) s_ok[i >> 5] |= 1u << (i & 31);
             __syncthreads();
@@ -514,10 +540,10 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
                         ok = false;
                         break;
                     }
-                    uint8_t* st = base + slot * kSlStageBytes;
-                    mbar_expect_tx(&full[slot], (uint32_t)kSlStageBytes);
+                    uint8_t* st = base + slot * kStageBytes;
+                    mbar_expect_tx(&full[slot], (uint32_t)kStageBytes);
                     sl_tma_3d(st, &mA, &full[slot], s * kSlK, (int)(mi * kSlM));
-                    sl_tma_3d(st + kSlABytes, &mB, &full[slot], s * kSlK, (int)(ni * kSlN));
+                    sl_tma_3d(st + kSlABytes, &mB, &full[slot], s * kSlK, (int)(ni * TN));
                 }
             }
             if (!ok) atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
@@ -528,57 +554,60 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
     } else if (warp == kSlEpiWarps + 1) {
         // products
         if (lane == 0) {
-            uint32_t it = 0, ch = 0;
+            uint32_t it = 0, ch[GR] = {};
             bool ok = true;
             for (int i = 0; i < mine && ok; ++i) {
                 if (!sliced(i)) continue;
-                int64_t mi, ni;
-                sl_tile(g, blockIdx.x + (int64_t)i * gridDim.x, mi, ni);
+                const int gr = i % GR;
+                const uint32_t acc0 = tmem + (uint32_t)(gr * kSlices * TN);
                 for (int s = 0; s < nst && ok; ++s, ++it) {
                     const bool first = s % kSlChunk == 0;
-                    if (first && ch > 0) ok = mbar_wait(&acc_empty, (ch - 1) & 1);
+                    if (first && ch[gr] > 0) ok = mbar_wait(&acc_empty[gr], (ch[gr] - 1) & 1);
                     const uint32_t slot = it % kSlStages;
                     ok = ok && mbar_wait(&full[slot], (it / kSlStages) & 1);
                     if (!ok) break;
                     sl_fence_after();
-                    const uint32_t a0 = smem_u32(base + slot * kSlStageBytes), b0 = a0 + kSlABytes;
+                    const uint32_t a0 = smem_u32(base + slot * kStageBytes), b0 = a0 + kSlABytes;
 #pragma unroll
                     for (int kk = 0; kk < kSlK / 16; ++kk) {
                         const uint64_t bd = sw64_desc(b0 + kk * 32);
 #pragma unroll
                         for (int d = 0; d < kSlices; ++d) {
                             const uint64_t ad = sw64_desc(a0 + d * (kSlM * kSlK * 2) + kk * 32);
-                            const int cols = kSlN * (kSlices - d);
+                            const int cols = TN * (kSlices - d);
                             const uint32_t acc = (first && kk == 0 && d == 0) ? 0u : 1u;
                             const int n0 = cols < 256 ? cols : 256;
-                            sl_umma(tmem + kSlN * d, ad, bd, bf16_idesc(n0), acc);
+                            sl_umma(acc0 + TN * d, ad, bd, bf16_idesc(n0), acc);
                             if (cols > 256)
-                                sl_umma(tmem + kSlN * d + 256, ad, bd + ((256 * kSlK * 2) >> 4),
+                                sl_umma(acc0 + TN * d + 256, ad, bd + ((256 * kSlK * 2) >> 4),
                                         bf16_idesc(cols - 256), acc);
                         }
                     }
                     sl_commit(&empty[slot]);
                     if (s % kSlChunk == kSlChunk - 1 || s == nst - 1) {
-                        sl_commit(&acc_full);
-                        ++ch;
+                        sl_commit(&acc_full[gr]);
+                        ++ch[gr];
                     }
                 }
             }
             if (!ok) atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
             // every product must be done before the tensor memory goes back
-            else if (ch > 0) mbar_wait(&acc_full, (ch - 1) & 1);
+            else
+                for (int s = 0; s < GR; ++s)
+                    if (ch[s] > 0) mbar_wait(&acc_full[s], (ch[s] - 1) & 1);
         }
     } else {
-        // sixteen warps: warp w drains lanes 32 (w % 4).. (rows of the tile) and
-        // columns 16 (w / 4).. of every accumulator
-        const int rl = (warp & 3) * 32 + lane, ch0 = (warp >> 2) * kSlCols;
-        const uint32_t tb = tmem + ((uint32_t)((warp & 3) * 32) << 16) + ch0;
+        // the warps of a tile: warp w of them drains lanes 32 (w % 4).. (rows of
+        // the tile) and columns 16 (w / 4).. of every accumulator
+        const int gr = warp / GW, tg = tid - gr * GW * 32;
+        const int rl = (warp & 3) * 32 + lane, ch0 = (tg >> 7) * kSlCols;
+        const uint32_t tb = tmem + ((uint32_t)((warp & 3) * 32) << 16) + ch0 + gr * kSlices * TN;
         uint32_t ch = 0;
         bool ok = true;
-        for (int i = 0; i < mine && ok; ++i) {
+        for (int i = gr; i < mine && ok; i += GR) {
             int64_t mi, ni;
             sl_tile(g, blockIdx.x + (int64_t)i * gridDim.x, mi, ni);
-            const int64_t r = mi * kSlM + rl, col0 = ni * kSlN + ch0;
+            const int64_t r = mi * kSlM + rl, col0 = ni * TN + ch0;
             const bool in = r < g.M;
             const int nc = (int)max((int64_t)0, min((int64_t)kSlCols, g.N - col0));
             double* Cp = g.C + r + col0 * g.ldc;
@@ -609,80 +638,112 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
             // their way while the products run
             const int ea = in ? __ldg(&g.ea[r]) : 0;
             const int ebl = lane < nc ? __ldg(&g.eb[col0 + lane]) : 0;
-            constexpr int CB = 8;
-            double cold[CB];
             const bool add = g.add != 0;
-#pragma unroll
-            for (int q = 0; q < CB; ++q) cold[q] = (add && in && q < nc) ? Cp[q * g.ldc] : 0.0;
-            if (add && i + 1 < mine) {
+            if (add && i + GR < mine) {
                 // the next tile of C into L2: a line of 16 rows per thread
                 int64_t mx, nx;
-                sl_tile(g, blockIdx.x + (int64_t)(i + 1) * gridDim.x, mx, nx);
-                const int64_t rx = mx * kSlM + 16 * (tid & 7), cx = nx * kSlN + (tid >> 3);
+                sl_tile(g, blockIdx.x + (int64_t)(i + GR) * gridDim.x, mx, nx);
+                const int64_t rx = mx * kSlM + 16 * (tg & 7), cx = nx * TN + (tg >> 3);
                 if (rx < g.M && cx < g.N)
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(g.C + rx + cx * g.ldc));
             }
-            uint32_t t0[kSlCols], t1[kSlCols], t2[kSlCols];
+            // one element rounded and into C (alpha +-1 by the sign bit)
+            const auto store = [&](int j, uint32_t w0, uint32_t w1, uint32_t w2, double cold) {
+                double v = sl_to_double(w0, w1, w2, ea + __shfl_sync(0xffffffffu, ebl, j));
+                if (g.unit != 0) {
+                    v = __hiloint2double(__double2hiint(v) ^ (g.unit & (int)0x80000000u), __double2loint(v));
+                    if (add) v = cold + v;
+                } else {
+                    v = add ? fma(g.alpha, v, cold) : g.alpha * v;
+                }
+                if (in && j < nc) Cp[j * g.ldc] = v;
+            };
+            const auto load_c = [&](auto& cold, int j) {
 #pragma unroll
-            for (int j = 0; j < kSlCols; ++j) t0[j] = t1[j] = t2[j] = 0u;
-            for (int s = 0; s < nst; s += kSlChunk, ++ch) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&acc_full, ch & 1));
+                for (int e = 0; e < (int)(sizeof(cold) / sizeof(double)); ++e) cold[e] = (add && in && j + e < nc) ? Cp[(j + e) * g.ldc] : 0.0;
+            };
+            if constexpr (GR > 1) {
+                // a single chunk: four columns at a time from the accumulators
+                // into C, the next four on their way
+                uint32_t v[2][kSlices][4];
+                double cold[2][4];
+                load_c(cold[0], 0);
+                ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[gr], ch & 1));
+                ++ch;
                 if (!ok) break;
                 sl_fence_after();
+                __syncwarp();
+#pragma unroll
+                for (int d = 0; d < kSlices; ++d) sl_ld4(tb + d * TN, v[0][d]);
 #pragma unroll
                 for (int j = 0; j < kSlCols; j += 4) {
-                    uint32_t v[kSlices][4];
+                    const int cur = (j >> 2) & 1;
                     __syncwarp();
-#pragma unroll
-                    for (int d = 0; d < kSlices; ++d) sl_ld4(tb + d * kSlN + j, v[d]);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (j + 4 == kSlCols) {
+                    if (j + 4 < kSlCols) {
+#pragma unroll
+                        for (int d = 0; d < kSlices; ++d) sl_ld4(tb + d * TN + j + 4, v[cur ^ 1][d]);
+                        load_c(cold[cur ^ 1], j + 4);
+                    } else {
                         // drained: the next products may start
                         sl_fence_before();
                         __syncwarp();
-                        if (lane == 0) sl_arrive(&acc_empty);
+                        if (lane == 0) sl_arrive(&acc_empty[gr]);
                     }
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         uint32_t a[kSlices];
 #pragma unroll
-                        for (int d = 0; d < kSlices; ++d) a[d] = v[d][e];
-                        long long p, q;
-                        sl_combine(a, p, q);
-                        // q + (p << 32) into the 96-bit sum
-                        const uint32_t q0 = (uint32_t)q, q1 = (uint32_t)((unsigned long long)q >> 32);
-                        const uint32_t p0 = (uint32_t)p, p1 = (uint32_t)((unsigned long long)p >> 32);
-                        asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
-                            : "+r"(t0[j + e]), "+r"(t1[j + e]), "+r"(t2[j + e])
-                            : "r"(q0), "r"(q1), "r"((uint32_t)((int)q1 >> 31)));
-                        asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, %3;"
-                            : "+r"(t1[j + e]), "+r"(t2[j + e])
-                            : "r"(p0), "r"(p1));
+                        for (int d = 0; d < kSlices; ++d) a[d] = v[cur][d][e];
+                        uint32_t t0 = 0u, t1 = 0u, t2 = 0u;
+                        sl_add(a, t0, t1, t2);
+                        store(j + e, t0, t1, t2, cold[cur][e]);
                     }
                 }
-            }
-            if (!ok) break;
-            // rounded and into C, the next columns of C loaded ahead
+            } else {
+                constexpr int CB = 8;
+                double cold[CB];
+                load_c(cold, 0);
+                uint32_t t0[kSlCols], t1[kSlCols], t2[kSlCols];
 #pragma unroll
-            for (int j0 = 0; j0 < kSlCols; j0 += CB) {
-                double next[CB];
-                if (j0 + CB < kSlCols) {
+                for (int j = 0; j < kSlCols; ++j) t0[j] = t1[j] = t2[j] = 0u;
+                for (int s = 0; s < nst; s += kSlChunk, ++ch) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[gr], ch & 1));
+                    if (!ok) break;
+                    sl_fence_after();
 #pragma unroll
-                    for (int q = 0; q < CB; ++q)
-                        next[q] = (add && in && j0 + CB + q < nc) ? Cp[(j0 + CB + q) * g.ldc] : 0.0;
+                    for (int j = 0; j < kSlCols; j += 4) {
+                        uint32_t v[kSlices][4];
+                        __syncwarp();
+#pragma unroll
+                        for (int d = 0; d < kSlices; ++d) sl_ld4(tb + d * TN + j, v[d]);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        if (j + 4 == kSlCols) {
+                            // drained: the next products may start
+                            sl_fence_before();
+                            __syncwarp();
+                            if (lane == 0) sl_arrive(&acc_empty[gr]);
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            uint32_t a[kSlices];
+#pragma unroll
+                            for (int d = 0; d < kSlices; ++d) a[d] = v[d][e];
+                            sl_add(a, t0[j + e], t1[j + e], t2[j + e]);
+                        }
+                    }
                 }
+                if (!ok) break;
+                // rounded and into C, the next columns of C loaded ahead
 #pragma unroll
-                for (int q = 0; q < CB; ++q) {
-                    const int j = j0 + q;
-                    const double v = sl_to_double(t0[j], t1[j], t2[j], ea + __shfl_sync(0xffffffffu, ebl, j));
-                    double o;
-                    // (a comparison of doubles would take the FP64 pipe)
-                    if (!add) o = g.unit == 1 ? v : g.alpha * v;
-                    else o = g.unit == 1 ? cold[q] + v : g.unit == -1 ? cold[q] - v : fma(g.alpha, v, cold[q]);
-                    if (in && j < nc) Cp[j * g.ldc] = o;
+                for (int j0 = 0; j0 < kSlCols; j0 += CB) {
+                    double next[CB];
+                    if (j0 + CB < kSlCols) load_c(next, j0 + CB);
+#pragma unroll
+                    for (int q = 0; q < CB; ++q) store(j0 + q, t0[j0 + q], t1[j0 + q], t2[j0 + q], cold[q]);
+#pragma unroll
+                    for (int q = 0; q < CB; ++q) cold[q] = next[q];
                 }
-#pragma unroll
-                for (int q = 0; q < CB; ++q) cold[q] = next[q];
             }
             __syncwarp();
         }
@@ -730,7 +791,17 @@ tmvg_status sliced_apply(Context* c, int64_t M, int64_t N, int64_t K, double alp
 {
     if (M <= 0 || N <= 0 || K <= 0) return TMVG_OK;
     CUtensorMap mA, mB;
-    if (!sl_map(&mA, sa, kSlM) || !sl_map(&mB, sb, kSlN))
+    // a single chunk takes tiles of 32 columns, whose epilogues overlap (alpha
+    // A B + C, normal data, 64 against 32 columns: 4096 x 4096 x 32 139 -> 123
+    // us, 8192 x 8192 x 32 496 -> 435, 2048 x 2048 x 64 52 -> 43.5, 700 x 700 x 32
+    // 31 -> 19), except a full one over many tiles, where reading A's digits
+    // twice as often costs more (4096 x 4096 x 128: 156 -> 167; 2048 x 2048 x 128:
+    // 56 -> 54)
+    const int64_t cap = max_ctas > 0 ? max_ctas : c->num_sms;
+    const bool narrow = K <= (kSlChunk - 1) * kSlK ||
+                        (K <= kSlChunk * kSlK && ceil_div(M, (int64_t)kSlM) * ceil_div(N, (int64_t)kSlN) <= 4 * cap);
+    const int tn = narrow ? 32 : kSlN;
+    if (!sl_map(&mA, sa, kSlM) || !sl_map(&mB, sb, tn))
         return set_error(c, TMVG_CUDA_ERROR, "sliced product: tensor map encoding failed");
     SlicedArgs g;
     g.M = M, g.N = N, g.K = K, g.alpha = alpha, g.add = beta != 0.0, g.unit = alpha == 1.0 ? 1 : alpha == -1.0 ? -1 : 0;
@@ -744,14 +815,14 @@ tmvg_status sliced_apply(Context* c, int64_t M, int64_t N, int64_t K, double alp
     g.need_sum = (float)(112.0 * std::sqrt((double)K));
     g.da = sa.digits, g.db = sb.digits, g.Kp = sa.Kp;
     g.C = C, g.ldc = ldc;
-    g.mt = ceil_div(M, (int64_t)kSlM), g.nt = ceil_div(N, (int64_t)kSlN);
-    const int64_t cap = max_ctas > 0 ? max_ctas : c->num_sms;
+    g.mt = ceil_div(M, (int64_t)kSlM), g.nt = ceil_div(N, (int64_t)tn);
     const unsigned grid = (unsigned)std::min<int64_t>(g.mt * g.nt, cap);
+    auto kern = tn == 32 ? sliced_gemm_kernel<32> : sliced_gemm_kernel<kSlN>;
+    const size_t smem = (size_t)kSlStages * (tn == 32 ? sl_stage_bytes<32>() : sl_stage_bytes<kSlN>()) + 1024;
     tmvg_status st = check_cuda(
-        c, cudaFuncSetAttribute(sliced_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlSmem),
-        "sliced product");
+        c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "sliced product");
     if (st) return st;
-    sliced_gemm_kernel<<<grid, kSlThreads, kSlSmem, c->stream>>>(mA, mB, g, c->dflags);
+    kern<<<grid, kSlThreads, smem, c->stream>>>(mA, mB, g, c->dflags);
     ++c->launches;
     return check_cuda(c, cudaGetLastError(), "sliced product launch");
 }
@@ -810,7 +881,7 @@ tmvg_status sliced_gemm(Context* c, int64_t M, int64_t N, int64_t K, double alph
     const int64_t cap = std::max<int64_t>(kSlM, (((int64_t)1 << 28) / (2 * kSlices * (kb + kSlK))) / kSlM * kSlM);
     const int64_t mb = std::min(M, cap);
     const int64_t nb = std::min(std::min(N, cap), std::max<int64_t>(1, kMaxTilesPerCta / ceil_div(mb, (int64_t)kSlM)) *
-                                                      kSlN * (max_ctas > 0 ? max_ctas : c->num_sms));
+                                                      32 * (max_ctas > 0 ? max_ctas : c->num_sms));
     const size_t ba = (sliced_bytes(mb, kb) + 255) & ~size_t(255);
     unsigned char* ws = (unsigned char*)scratch_alloc(c, ba + sliced_bytes(nb, kb), c->stream);
     if (!ws) return TMVG_UNSUPPORTED;
