@@ -176,7 +176,7 @@ class Handle:
             pass
 
     def set_stream(self, stream_ptr: int) -> None:
-        self.check(self.lib.tmvg_set_stream(self.h, vp(stream_ptr)))
+        self.check(self.lib.tmvg_set_stream(self.h, stream_ptr))
 
     def check(self, st: int, what: str = "") -> None:
         if st == 0:

@@ -21,12 +21,17 @@ def handle(device: int | None = None) -> _lib.Handle:
     """The per-device context, bound to torch's current stream."""
     if device is None:
         device = torch.cuda.current_device()
-    with _lock:
-        h = _handles.get(device)
-        if h is None:
-            h = _lib.Handle(device)
-            _handles[device] = h
-    h.set_stream(torch.cuda.current_stream(device).cuda_stream)
+    h = _handles.get(device)
+    if h is None:
+        with _lock:
+            h = _handles.get(device)
+            if h is None:
+                torch.cuda.current_stream(device)  # torch's own initialisation
+                h = _lib.Handle(device)
+                _handles[device] = h
+    # (the stream as a number: the Stream object of current_stream() took longer
+    # to make than a small product to launch)
+    h.set_stream(torch._C._cuda_getCurrentRawStream(device))
     return h
 
 
@@ -62,12 +67,14 @@ def multmm(add: bool, alpha: float, A: torch.Tensor, B: torch.Tensor, C_: torch.
     _check_f64_cuda(A, B, C_)
     m, k = A.shape
     k2, n = B.shape
-    if k2 != k or tuple(C_.shape) != (m, n):
+    if k2 != k or C_.shape != (m, n):
         raise ValueError("multmm: shape mismatch")
+    sai, saj = A.stride()
+    sbi, sbj = B.stride()
+    sci, scj = C_.stride()
     h = handle(C_.device.index)
-    h.check(h.call("tmvg_multmm_f64", int(bool(add)), float(alpha), m, n, k,
-                   _ptr(A), A.stride(0), A.stride(1), _ptr(B), B.stride(0), B.stride(1),
-                   _ptr(C_), C_.stride(0), C_.stride(1)), "multmm")
+    h.check(h.call("tmvg_multmm_f64", 1 if add else 0, float(alpha), m, n, k, A.data_ptr(), sai, saj,
+                   B.data_ptr(), sbi, sbj, C_.data_ptr(), sci, scj), "multmm")
 
 
 def lu_decompose(A: torch.Tensor, P: torch.Tensor | None = None) -> torch.Tensor:

@@ -149,7 +149,7 @@ class Matrix:
     def __mul__(self, other):
         if isinstance(other, (int, float)):
             return Matrix(self.t * float(other))
-        if (isinstance(other, torch.Tensor) or isinstance(other, np.ndarray)) and other.ndim == 1:
+        if isinstance(other, (torch.Tensor, np.ndarray)) and other.ndim == 1:
             # y = A x (MultMV<false>, src/TMV_MultMV.cpp:1134)
             x = torch.as_tensor(other, dtype=torch.float64, device=self.t.device)
             y = torch.empty(self.colsize(), dtype=torch.float64, device=self.t.device)
@@ -157,12 +157,13 @@ class Matrix:
             return y
         if not isinstance(other, Matrix):
             other = Matrix(other)
-        m, k = self.shape
-        k2, n = other.shape
+        a, b = self.t, other.t
+        m, k = a.shape
+        k2, n = b.shape
         if k != k2:
             raise ValueError("size mismatch in product")
-        out = torch.empty((n, m), dtype=torch.float64, device=self.t.device).t()
-        linalg.multmm(False, 1.0, self.t, other.t, out)
+        out = torch.empty_strided((m, n), (1, max(m, 1)), dtype=torch.float64, device=a.device)
+        linalg.multmm(False, 1.0, a, b, out)
         return Matrix._wrap(out)
 
     __matmul__ = __mul__
