@@ -642,33 +642,32 @@ ztri_inv64_kernel(int64_t n, const double* __restrict__ z, int64_t tsi, int64_t 
         });
 }
 
-tmvg_status ztrsm_sync_free(Context* c, int64_t n, const double* z, int64_t ld, bool upper, int64_t nrhs, double* X,
-                            const double2* recip)
+tmvg_status ztrsm_sync_free(Context* c, int64_t n, const double* z, int64_t tsi, int64_t tsj, bool upper, bool unit,
+                            int64_t nrhs, double* X, const double2* recip)
 {
     const int64_t N = 2 * n, nblk = ceil_div(N, kTrsvBlock);
     double* dinv = nullptr;
     int* dsing = nullptr;
     tmvg_status st = inverse_blocks_buffer(c, nblk, &dinv, &dsing);
     if (st) return st;
-    const double* tri = z;
-    int64_t si = 1, sj = ld, bsi = 1, rstep = 1;
+    int64_t bsi = 1, rstep = 1;
     double sgn = 1.0;
     if (upper) {
-        tri = z + 2 * (n - 1) * (1 + ld);
-        si = -1;
-        sj = -ld;
+        z += 2 * (n - 1) * (tsi + tsj);
+        tsi = -tsi;
+        tsj = -tsj;
         X += N - 1;
         bsi = -1;
         recip += n - 1;
         rstep = -1;
         sgn = -1.0;
     }
-    ztri_inv64_kernel<<<(unsigned)nblk * kInvCtas, kInvThreads, 0, c->stream>>>(N, tri, si, sj, sgn, !upper, recip, rstep,
+    ztri_inv64_kernel<<<(unsigned)nblk * kInvCtas, kInvThreads, 0, c->stream>>>(N, z, tsi, tsj, sgn, unit, recip, rstep,
                                                                              dinv, dsing);
     ++c->launches;
     st = check_cuda(c, cudaGetLastError(), "trsv inverse blocks");
     if (st) return st;
-    return launch_trsm<double, true>(c, N, tri, si, sj, sgn, !upper, nrhs, X, bsi, N, true, dinv, dsing, true);
+    return launch_trsm<double, true>(c, N, z, tsi, tsj, sgn, unit, nrhs, X, bsi, N, true, dinv, dsing, true);
 }
 
 // ---------------------------------------------------------------------

@@ -16,12 +16,12 @@ tmvg_status trsm_sync_free(Context* c, int64_t n, const T* tri, int64_t tsi, int
                            bool upper, bool unit, int64_t nrhs, T* B, int64_t bsi, int64_t bsj,
                            bool skip_zero);
 
-// X := T^-1 X for the unit lower or the upper triangle of a packed complex LU
-// factor (z column-major, ld in complex entries; recip: 1 / U(j,j), 0 where that
-// is zero), X n x nrhs contiguous.  Records kDevRetry in the device error word
-// where the result is not finite or a U(j,j) is zero.
-tmvg_status ztrsm_sync_free(Context* c, int64_t n, const double* z, int64_t ld, bool upper, int64_t nrhs, double* X,
-                            const double2* recip);
+// X := T^-1 X for the lower or upper triangle T(i, j) = z[i tsi + j tsj] of
+// complex entries (unit diagonal not read when unit; recip: 1 / T(j,j), 0 where
+// that is zero), X n x nrhs contiguous.  Records kDevRetry in the device error
+// word where the result is not finite or a T(j,j) is zero.
+tmvg_status ztrsm_sync_free(Context* c, int64_t n, const double* z, int64_t tsi, int64_t tsj, bool upper, bool unit,
+                            int64_t nrhs, double* X, const double2* recip);
 
 // For the inverse: the inverted 64-row diagonal blocks of a packed LU factor
 // (row-major 64 x 64 each, in the context's buffer), and Y := D^-1 Y with one
