@@ -445,22 +445,27 @@ __device__ __forceinline__ void reg_key_reduce(unsigned long long& key, int& idx
 
 // The lane that wins the same order over the candidates (`cand`) of the warp,
 // the lowest of the lanes that tie in key and index; -1 without a candidate.
-// One redux.sync and a ballot decide unless keys tie (FP64: in their upper 32
-// bits): every redux.sync costs about 100 clocks on the chain of every column,
-// and the winner itself stores what the others read.
+// FP64: one redux.sync and a ballot decide unless keys tie in their upper 32
+// bits (three redux.sync took 400 clocks on the chain of every column), and the
+// winner itself stores what the others read.  FP32 keeps its two redux.sync: the
+// branch for ties costs more (mixed solve, n = 8192: 18.1 against 17.6 ms with
+// the two other FP32 choices below).
 template <typename T>
 __device__ __forceinline__ int reg_key_winner(unsigned long long key, int idx, bool cand)
 {
-    const unsigned hi = sizeof(T) == 4 ? (unsigned)key : (unsigned)(key >> 32);
+    if constexpr (sizeof(T) == 4) {
+        int first = cand ? idx : INT_MAX;
+        reg_key_reduce<T>(key, first);
+        return __ffs(__ballot_sync(0xffffffffu, cand && idx == first)) - 1;
+    }
+    const unsigned hi = (unsigned)(key >> 32);
     const unsigned mhi = __reduce_max_sync(0xffffffffu, cand ? hi : 0u);
     bool in = cand && hi == mhi;
     unsigned m = __ballot_sync(0xffffffffu, in);
     if (m & (m - 1)) {
-        if constexpr (sizeof(T) == 8) {
-            const unsigned lo = in ? (unsigned)key : 0u;
-            const unsigned mlo = __reduce_max_sync(0xffffffffu, lo);  // (every lane takes part)
-            in = in && lo == mlo;
-        }
+        const unsigned lo = in ? (unsigned)key : 0u;
+        const unsigned mlo = __reduce_max_sync(0xffffffffu, lo);  // (every lane takes part)
+        in = in && lo == mlo;
         const unsigned i = in ? (unsigned)idx : 0xffffffffu;
         const unsigned mi = __reduce_min_sync(0xffffffffu, i);
         in = in && i == mi;
@@ -975,14 +980,32 @@ __device__ __forceinline__ void leaf_pivot_row(const LeafMsg<T>& w, T (*s_urow)[
     }
 }
 
-// The leaf's U12 in place: rows t of Ur, columns [kLeaf, pw), lane (t, c) of a
-// warp for entry (t, column c of four), two groups of four columns at a time.
-// Row q's values go to the rows below by shuffle, so the chain is 7 fused
+// The leaf's U12 in place: rows t of Ur, columns [kLeaf, pw).  FP64: lane (t, c)
+// of a warp for entry (t, column c of four), two groups of four columns at a
+// time.  Row q's values go to the rows below by shuffle, so the chain is 7 fused
 // multiply-adds; a column per thread was a chain of 28, and a DFMA takes its
-// sub-partition 64 clocks whatever the lanes.
+// sub-partition 64 clocks whatever the lanes.  FP32: a column per thread (the
+// shuffles and the rows' shared banks cost more than the short chain gains).
 template <typename T, int NB>
-__device__ __forceinline__ void leaf_u12(T (*Ur)[NB], unsigned ufmask, int pw, int warp, int nwarp, int lane)
+__device__ __forceinline__ void leaf_u12(T (*Ur)[NB], unsigned ufmask, int pw, int tid, int nthr)
 {
+    if constexpr (sizeof(T) == 4) {
+        for (int p = kLeaf + tid; p < pw; p += nthr) {
+            T uc[kLeaf];
+#pragma unroll
+            for (int t = 0; t < kLeaf; ++t) uc[t] = Ur[t][p];
+#pragma unroll
+            for (int t = 1; t < kLeaf; ++t) {
+#pragma unroll
+                for (int q = 0; q < t; ++q)
+                    if (!((ufmask >> q) & 1u)) uc[t] = fma(-Ur[t][q], uc[q], uc[t]);
+            }
+#pragma unroll
+            for (int t = 0; t < kLeaf; ++t) Ur[t][p] = uc[t];
+        }
+        return;
+    }
+    const int warp = tid >> 5, nwarp = nthr >> 5, lane = tid & 31;
     using V = Vec16<T>;
     const int t = lane >> 2, c = lane & 3;
     if (kLeaf + 4 * warp >= pw) return;
@@ -1076,7 +1099,8 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
     const int dest = lane & (kClusterCtas - 1);
     const uint32_t to_msg = cluster_addr(&msg[0][cta], dest < G ? dest : 0);
     const uint32_t to_bar = cluster_addr(&mbar[0], dest < G ? dest : 0);
-    constexpr int kRcpWarp = 1;  // (every block has two warps)
+    constexpr int kRcpWarp = 1;  // (every block has several warps)
+    constexpr bool kLongRcp = sizeof(T) == 8;  // 400 clocks; FP32's is cheaper in every thread
     if (G > 1 && tid == 0) mbar_expect_tx(&mbar[0], (uint32_t)(G * sizeof(LeafMsg<T>)));
     cluster.sync();  // every CTA's mbarriers are initialised before any message
 
@@ -1164,7 +1188,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
                     if (wo >= 0) leaf_pivot_row<T>(msg[par][wo], s_urow, u, owe_u, lane);
                 }
             }
-            if (warp == kRcpWarp) {
+            if (kLongRcp && warp == kRcpWarp) {
                 // every candidate's reciprocal, beside warp 0's decision
                 const bool got = G == 1 || __all_sync(0xffffffffu, mbar_wait(&mbar[par], (uint32_t)((j >> 1) & 1)));
                 if (got && lane < (G > 1 ? G : nwarp)) {
@@ -1199,7 +1223,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             }
             if (!uf && act) {
                 // TMV scales the column by the reciprocal of the pivot
-                const T l = x[0] * s_rcp[G > 1 ? piv.loc >> 16 : piv.loc >> 5];
+                const T l = x[0] * (kLongRcp ? s_rcp[G > 1 ? piv.loc >> 16 : piv.loc >> 5] : recip_rn(s_urow[u][0]));
                 x[0] = l;
                 if (u < kLast) x[1] = fma(-l, s_urow[u][1], x[1]);
                 if (u + 2 < kLeaf) {
@@ -1229,7 +1253,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             __syncthreads();
             if (s_abort) break;
             T(*Ur)[NB] = s_rem[lpar];
-            leaf_u12<T, NB>(Ur, ufmask, pw, warp, nwarp, lane);
+            leaf_u12<T, NB>(Ur, ufmask, pw, tid, nthr);
             __syncthreads();
             if (act) leaf_rank8<T, NB, 0, 0, NB>(x, &Ur[0][0], ufmask, pw);
             else if (dstep >= 0) leaf_take_u<T, NB>(x, Ur[dstep], pw);
