@@ -209,6 +209,16 @@ def fp64_roofline(achieved_tflops: float) -> dict:
             "peak_source": FP64_PEAK.get("source", "not measured")}
 
 
+def sliced_roofline(achieved_tflops: float) -> dict:
+    """FP64 products on the tensor cores: 36 BF16 products of 8-bit digits per
+    multiplication, so 1/36 of the measured cuBLAS bf16 rate."""
+    pk = peaks()
+    peak = float(pk["bf16_tflops"]) / 36.0
+    return {"bound": "bf16 tensor cores / 36", "achieved": round(achieved_tflops, 4), "peak": round(peak, 3),
+            "unit": "TFLOP/s", "frac": round(achieved_tflops / peak, 4),
+            "peak_source": f"{pk['_source']} cuBLAS bf16 (bf16_tflops) over 36 digit products"}
+
+
 def run_gpu(args) -> dict:
     import torch
 
@@ -564,7 +574,8 @@ def batched_bench(dev, args, with_cpu: bool) -> dict:
 # byte of each kernel class, from one ncu capture of the class's main kernel
 # on the n = 8192 workload (commands and figures in profiles/):
 #   panel: lu_panel_leaf_kernel, k = 320: 2.08 MB / 4.03 MB
-#   trailing_update: tf32x3_update_kernel, k = 256: 432.1 MB / 495.7 MB
+#   trailing_update: the 3xTF32 update, k = 256: 432.1 MB / 495.7 MB (tf32x3_update_kernel;
+#   the streamed form reads and writes the same tiles)
 #   tri_solve: trsv_pub_async_kernel: 140.4 MB / 138.5 MB
 # The traffic of a span is its algorithmic bytes times the ratio.
 NCU_TRAFFIC_PER_ALG_BYTE: dict = {"panel": 0.516, "trailing_update": 0.872, "tri_solve": 1.014}
@@ -572,8 +583,8 @@ NCU_TRAFFIC_PER_ALG_BYTE: dict = {"panel": 0.516, "trailing_update": 0.872, "tri
 KERNEL_NAMES = {
     "panel": "lu_panel_leaf_kernel (16-CTA cluster, 512 threads, one register-resident FP32 panel row "
              "per thread, 8-column leaves)",
-    "trailing_update": "U12 solve + A22 -= L21 U12 (FP32: u12_reg_kernel + tf32x3_update_kernel "
-                       "on tcgen05; FP64: u12_reg_kernel + gemm_simt_kernel<double>)",
+    "trailing_update": "U12 solve + A22 -= L21 U12 (FP32: u12_reg_kernel + tf32x3_stream_kernel "
+                       "on tcgen05; FP64: u12_f64_kernel + sliced_gemm_kernel on tcgen05)",
     "tri_solve": "trsv_pub_async_kernel (FP32 inverse-block triangular solve, tiles staged in "
                  "shared memory by cp.async, link blocks, helper CTAs for long block rows)",
     "residual": "residual_partial_kernel + residual_final_kernel (FP64 b - A x)",
@@ -608,7 +619,8 @@ def dominant_roofline(kernels: dict, mixed: bool) -> dict | None:
     The FP32 factorisation's classes and the FP64 residual are bounded by
     HBM bandwidth (arithmetic intensity below the ridge; the panel is in
     practice latency-bound and its fraction shows it).  The FP64 trailing
-    update is bounded by the FP64 DFMA rate."""
+    update is set against the FP64 DFMA rate, which its tensor-core products
+    exceed (a fraction above 1)."""
     if not kernels:
         return None
     cls = max(kernels, key=lambda k: kernels[k]["ms_per_step"])
@@ -720,8 +732,8 @@ def other_workloads(dev, with_cpu: bool) -> dict:
     ms = ev_time(lambda: linalg.multmm(False, 1.0, A, Bm, C))
     tf = 2.0 * m ** 3 / (ms * 1e-3) / 1e12
     out["fp64_gemm_1024"] = {"value": round(tf, 4), "unit": "TFLOP/s", "ms": round(ms, 4),
-                             "roofline": fp64_roofline(tf),
-                             "kernel": "gemm_simt_kernel<double> (MultMM, column-major operands)",
+                             "roofline": sliced_roofline(tf),
+                             "kernel": "sliced_split_kernel + sliced_gemm_kernel (MultMM, column-major operands)",
                              "flush": "256 MiB written between runs"}
     if with_cpu:
         orc, kind, what = cpu_reference()
@@ -743,7 +755,7 @@ def other_workloads(dev, with_cpu: bool) -> dict:
     fl = lu_solve_flops(n, 8)
     tf = fl / (ms * 1e-3) / 1e12
     out["fp64_lu_solve_4096"] = {"value": round(tf, 4), "unit": "TFLOP/s", "ms": round(ms, 3),
-                                 "roofline": fp64_roofline(tf),
+                                 "roofline": sliced_roofline(tf),
                                  "workload": "X = B/A, n = 4096, 8 right-hand sides, A ~ N(0,1) + 4 sqrt(n) I"}
     n = 2048
     A5 = torch.randn((n, n), dtype=torch.float64, device=dev, generator=g)
@@ -758,7 +770,7 @@ def other_workloads(dev, with_cpu: bool) -> dict:
         "forward_ms": round(fwd_ms, 3), "backward_ms": round(bwd_ms, 3),
         "forward_tflops": round(lu_solve_flops(n, 64) / (fwd_ms * 1e-3) / 1e12, 4),
         "backward_tflops": round(4.0 * n * n * 64 / (bwd_ms * 1e-3) / 1e12, 4),
-        "forward_roofline": fp64_roofline(lu_solve_flops(n, 64) / (fwd_ms * 1e-3) / 1e12),
+        "forward_roofline": sliced_roofline(lu_solve_flops(n, 64) / (fwd_ms * 1e-3) / 1e12),
         "backward_roofline": fp64_roofline(4.0 * n * n * 64 / (bwd_ms * 1e-3) / 1e12),
         "workload": "X = A^-1 B (n = 2048, 64 right-hand sides), backward gB = A^-T G and gA = -gB X^T "
                     "from the stored factors"}
@@ -816,7 +828,7 @@ def complex_workload(dev, with_cpu: bool) -> dict:
     tf = zfl / (ms * 1e-3) / 1e12
     res = (Az @ Xz - Bz).abs().max().item() / (Az.abs().sum(dim=1).max().item() * Xz.abs().max().item())
     out = {
-        "value": round(tf, 4), "unit": "TFLOP/s", "ms": round(ms, 3), "roofline": fp64_roofline(tf),
+        "value": round(tf, 4), "unit": "TFLOP/s", "ms": round(ms, 3), "roofline": sliced_roofline(tf),
         "normwise_backward_error": res,
         "workload": "complex<double> X = B/A, n = 4096, 8 right-hand sides, A ~ CN(0,1) + 4 sqrt(n) I; "
                     "flops 8n^3/3 + 8 n^2 nrhs (timed region includes the two device copies of A and B)"}

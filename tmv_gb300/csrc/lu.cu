@@ -2148,13 +2148,13 @@ static tmvg_status update_columns(Context* c, int64_t n, T* A, int64_t lda, int6
                 nb, (const double*)L11, lda, (double*)A12, nc);
         } else if (nc <= NB) {
             const unsigned grid = (unsigned)ceil_div(nc, kU12NarrowCols);
-            if (tc)
-                u12_reg_kernel<T, NB, true, kU12NarrowCols><<<grid, kU12RegBlock, 0, c->stream>>>(
+            if (std::is_same<T, float>::value && tc)
+                u12_reg_kernel<T, NB, std::is_same<T, float>::value, kU12NarrowCols><<<grid, kU12RegBlock, 0, c->stream>>>(
                     nb, L11, lda, A12, nc, bc.Bhi, bc.Blo, sp, k);
             else
                 u12_reg_kernel<T, NB, false, kU12NarrowCols><<<grid, kU12RegBlock, 0, c->stream>>>(
                     nb, L11, lda, A12, nc, nullptr, nullptr, sp, k);
-        } else {
+        } else if constexpr (std::is_same<T, float>::value) {  // (FP64: the first kernel)
             const unsigned grid = (unsigned)ceil_div(nc, kU12RegThreads);
             if (tc)
                 u12_reg_kernel<T, NB, true, kU12RegThreads><<<grid, kU12RegBlock, 0, c->stream>>>(

@@ -333,7 +333,9 @@ __device__ __forceinline__ double2 zfms(double2 a, double2 l, double2 u)
 // with column j, so when every message of j + 1 is in, j's buffers are free.
 // Waits are bounded; a CTA that gives up records kDevTimeout and the others
 // time out in turn.  Per column at m = 2048 (clocks): 17500 with cluster
-// barriers, remote reads by every warp and the whole update on the chain.
+// barriers, remote reads by every warp and the whole update on the chain; factor
+// and solve at n = 2048 took 16.4 ms with the messages, 14.0 ms once the warp that
+// decides held no rows.
 template <int KB>
 __global__ void __launch_bounds__(kZPanelThreads)
 zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k, int kb, int64_t* __restrict__ P,
