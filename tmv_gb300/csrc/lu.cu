@@ -1706,23 +1706,26 @@ u12_f64_kernel(int nb, const double* __restrict__ L, int64_t lda, double* __rest
 
 // The next panel's columns [c0, c0+nc) with step k (the "narrow" update), out
 // of place like narrow_update_f32_kernel: row interchanges by gather, U12, and
-// the rank-32 update of kNarrow64Rows rows per CTA, into the scratch panel S.
+// the rank-32 update of R rows per CTA, into the scratch panel S.
 // A cluster of 8 CTAs solves U12 together (4 columns each, a warp per column,
 // a lane per row: 31 steps of one DFMA and a shuffle, 1.5 us) and shares it
 // through DSMEM.  Bound: rest * 32 * 32 DFMAs on the FP64 pipe (7 us at
-// rest = 4096, less a launch).
-constexpr int kNarrow64Rows = 16;
+// rest = 4096, less a launch).  R is the fewest rows (4, 8, 16) whose CTAs find an
+// SM each: a CTA's product takes R / 4 us (n = 200: the solve 670 -> 642 us with
+// 4 instead of 16, n = 2048 with all three 7.86 -> 7.76 ms).
 constexpr int kNarrow64Threads = 256;
 constexpr int kNarrow64Ctas = 8;
 
+template <int R>
 __global__ void __cluster_dims__(kNarrow64Ctas, 1, 1) __launch_bounds__(kNarrow64Threads)
 narrow_update_f64_kernel(const double* __restrict__ A, int64_t lda, int64_t n, int64_t k, int64_t c0, int nc,
                          const int* __restrict__ pairs, double* __restrict__ S, int64_t lds)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
-    constexpr int NB = RegPanel<double>::NB, R = kNarrow64Rows;
-    static_assert(NB == 32 && NB == kNarrow64Ctas * 4 && kNarrow64Threads == 16 * R, "shape");
+    constexpr int NB = RegPanel<double>::NB;
+    constexpr int E = R == 16 ? 2 : 1;  // columns per thread
+    static_assert(NB == 32 && NB == kNarrow64Ctas * 4 && R * NB <= kNarrow64Threads * E, "shape");
     __shared__ __align__(16) double UT[NB][NB];  // UT[t][c] = U12(t, c)
     __shared__ double Ls[R][NB + 1];
     __shared__ int s_dst[2 * NB], s_src[2 * NB], map_blk[NB], map_row[R];
@@ -1755,10 +1758,12 @@ narrow_update_f64_kernel(const double* __restrict__ A, int64_t lda, int64_t n, i
         else if (d >= r0 && d < r0 + rows) map_row[d - r0] = s_src[tid];
     }
     __syncthreads();
-    const int rr = tid % R, cc = 2 * (tid / R);
-    double old[2], acc[2] = {0.0, 0.0};
+    const int rr = tid % R, cc = E * (tid / R);
+    double old[E], acc[E];
 #pragma unroll
-    for (int e = 0; e < 2; ++e)
+    for (int e = 0; e < E; ++e) acc[e] = 0.0;
+#pragma unroll
+    for (int e = 0; e < E; ++e)
         old[e] = (rr < rows && cc + e < nc) ? A[map_row[rr] + (c0 + cc + e) * lda] : 0.0;
     if (warp < 4) {
         const int c = 4 * rank + warp;
@@ -1775,15 +1780,20 @@ narrow_update_f64_kernel(const double* __restrict__ A, int64_t lda, int64_t n, i
     if (blockIdx.x == 0) {
         for (int t = tid; t < NB * nc; t += kNarrow64Threads) S[t % NB + (int64_t)(t / NB) * lds] = UT[t % NB][t / NB];
     }
+    if (cc >= NB) return;
 #pragma unroll 8
     for (int t = 0; t < NB; ++t) {
         const double lv = Ls[rr][t];
-        const double2 u = *reinterpret_cast<const double2*>(&UT[t][cc]);
-        acc[0] = fma(lv, u.x, acc[0]);
-        acc[1] = fma(lv, u.y, acc[1]);
+        if constexpr (E == 2) {
+            const double2 u = *reinterpret_cast<const double2*>(&UT[t][cc]);
+            acc[0] = fma(lv, u.x, acc[0]);
+            acc[1] = fma(lv, u.y, acc[1]);
+        } else {
+            acc[0] = fma(lv, UT[t][cc], acc[0]);
+        }
     }
 #pragma unroll
-    for (int e = 0; e < 2; ++e)
+    for (int e = 0; e < E; ++e)
         if (rr < rows && cc + e < nc) S[(r0 + rr - k) + (cc + e) * lds] = old[e] - acc[e];
 }
 
@@ -1794,9 +1804,10 @@ static tmvg_status narrow_update_f64(Context* c, const double* A, int64_t lda, i
     const int64_t rest = n - k - NB;
     const double fr = (double)rest, fc = (double)nc;
     ScopedTimer timer(c, kClsTrailingUpdate, sizeof(double) * (2.0 * fr * fc + fr * NB + NB * fc), 2.0 * fr * fc * NB);
-    const unsigned clusters = (unsigned)std::max<int64_t>(1, ceil_div(rest, kNarrow64Rows * kNarrow64Ctas));
-    narrow_update_f64_kernel<<<clusters * kNarrow64Ctas, kNarrow64Threads, 0, c->stream>>>(A, lda, n, k, c0, nc, pairs,
-                                                                                         S, lds);
+    const int R = rest <= 4 * c->num_sms ? 4 : rest <= 8 * c->num_sms ? 8 : 16;
+    auto kern = R == 4 ? narrow_update_f64_kernel<4> : R == 8 ? narrow_update_f64_kernel<8> : narrow_update_f64_kernel<16>;
+    const unsigned clusters = (unsigned)std::max<int64_t>(1, ceil_div(rest, R * kNarrow64Ctas));
+    kern<<<clusters * kNarrow64Ctas, kNarrow64Threads, 0, c->stream>>>(A, lda, n, k, c0, nc, pairs, S, lds);
     ++c->launches;
     return check_cuda(c, cudaGetLastError(), "lu: narrow update launch");
 }
