@@ -693,30 +693,33 @@ zlu_trsm_kernel(int64_t c1, double2* A, int64_t lda, int64_t k, int64_t c0)
     if (lane < KB) a[lane] = x;
 }
 
-// A22 -= L21 U12 (K = KB): 64 x 64 complex tiles, each of the 256 threads a
-// 4 x 4 block, complex products on the DFMA pipe.
+// A22 -= L21 U12 (K = KB): 16 RT x 16 RT complex tiles, each of the 256 threads
+// RT x RT entries, complex products on the DFMA pipe.  A 64 x 64 tile is 143 us on
+// an SM whatever the matrix, for the last steps as long as a panel: RT = 4 only
+// where every SM gets one, else RT = 1 (LU, n = 2048: 12.71 -> 12.62 ms).
 constexpr int kZgBM = 64, kZgBN = 64, kZgBK = 8;
-template <int KB>
+template <int KB, int RT>
 __global__ void __launch_bounds__(256)
 zlu_gemm_kernel(int64_t n, double2* A, int64_t lda, int64_t k, int64_t cbeg, int64_t cend)
 {
-    __shared__ double2 s_a[kZgBK][kZgBM];
-    __shared__ double2 s_b[kZgBK][kZgBN + 1];
+    constexpr int BT = 16 * RT;
+    __shared__ double2 s_a[kZgBK][BT];
+    __shared__ double2 s_b[kZgBK][BT + 1];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int64_t r0 = k + KB + (int64_t)blockIdx.x * kZgBM;  // rows of A22
-    const int64_t c0 = cbeg + (int64_t)blockIdx.y * kZgBN;    // columns [cbeg, cend) of A22
-    double2 acc[4][4];
+    const int64_t r0 = k + KB + (int64_t)blockIdx.x * BT;  // rows of A22
+    const int64_t c0 = cbeg + (int64_t)blockIdx.y * BT;    // columns [cbeg, cend) of A22
+    double2 acc[RT][RT];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < RT; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = make_double2(0.0, 0.0);
+        for (int b = 0; b < RT; ++b) acc[a][b] = make_double2(0.0, 0.0);
     for (int kk = 0; kk < KB; kk += kZgBK) {
-        for (int t = tid; t < kZgBK * kZgBM; t += 256) {
-            const int r = t % kZgBM, q = t / kZgBM;
+        for (int t = tid; t < kZgBK * BT; t += 256) {
+            const int r = t % BT, q = t / BT;
             const int64_t gi = r0 + r;
             s_a[q][r] = gi < n ? A[gi + (k + kk + q) * lda] : make_double2(0.0, 0.0);
         }
-        for (int t = tid; t < kZgBK * kZgBN; t += 256) {
+        for (int t = tid; t < kZgBK * BT; t += 256) {
             const int q = t % kZgBK, cc = t / kZgBK;
             const int64_t gj = c0 + cc;
             s_b[q][cc] = gj < cend ? A[(k + kk + q) + gj * lda] : make_double2(0.0, 0.0);
@@ -724,15 +727,15 @@ zlu_gemm_kernel(int64_t n, double2* A, int64_t lda, int64_t k, int64_t cbeg, int
         __syncthreads();
 #pragma unroll
         for (int q = 0; q < kZgBK; ++q) {
-            double2 av[4], bv[4];
+            double2 av[RT], bv[RT];
 #pragma unroll
-            for (int a = 0; a < 4; ++a) av[a] = s_a[q][tx + 16 * a];
+            for (int a = 0; a < RT; ++a) av[a] = s_a[q][tx + 16 * a];
 #pragma unroll
-            for (int b = 0; b < 4; ++b) bv[b] = s_b[q][ty + 16 * b];
+            for (int b = 0; b < RT; ++b) bv[b] = s_b[q][ty + 16 * b];
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+            for (int a = 0; a < RT; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) {
+                for (int b = 0; b < RT; ++b) {
                     acc[a][b].x = fma(av[a].x, bv[b].x, acc[a][b].x);
                     acc[a][b].x = fma(-av[a].y, bv[b].y, acc[a][b].x);
                     acc[a][b].y = fma(av[a].x, bv[b].y, acc[a][b].y);
@@ -742,11 +745,11 @@ zlu_gemm_kernel(int64_t n, double2* A, int64_t lda, int64_t k, int64_t cbeg, int
         __syncthreads();
     }
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
+    for (int b = 0; b < RT; ++b) {
         const int64_t gj = c0 + ty + 16 * b;
         if (gj >= cend) continue;
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
+        for (int a = 0; a < RT; ++a) {
             const int64_t gi = r0 + tx + 16 * a;
             if (gi < n) {
                 double2* p = &A[gi + gj * lda];
@@ -903,8 +906,12 @@ static tmvg_status zlu_factor_blocked(Context* c, int64_t n, double2* A, int64_t
                 (double*)(A + (k + KB) + c0 * lda), 2 * lda, std::max(1, c->num_sms - kZPanelCtas), true);
             if (s2 != TMVG_UNSUPPORTED) return s2;
         }
-        const dim3 grid((unsigned)ceil_div(m, kZgBM), (unsigned)ceil_div(nc, kZgBN));
-        zlu_gemm_kernel<KB><<<grid, 256, 0, c->stream>>>(n, A, lda, k, c0, c1);
+        if (ceil_div(m, (int64_t)64) * ceil_div(nc, (int64_t)64) < c->num_sms)
+            zlu_gemm_kernel<KB, 1><<<dim3((unsigned)ceil_div(m, 16), (unsigned)ceil_div(nc, 16)), 256, 0, c->stream>>>(
+                n, A, lda, k, c0, c1);
+        else
+            zlu_gemm_kernel<KB, 4><<<dim3((unsigned)ceil_div(m, 64), (unsigned)ceil_div(nc, 64)), 256, 0, c->stream>>>(
+                n, A, lda, k, c0, c1);
         ++c->launches;
         return TMVG_OK;
     };
