@@ -404,6 +404,12 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
                 mr = wr;
             }
         }
+        // the rows as they stand, before the others pay what theirs owe (below
+        // the next barrier)
+        if (warp == 0 && lane < kb) {
+            sh.stage[par][0][lane] = mr != INT_MAX ? s_rows[mr * RS + lane] : make_double2(0.0, 0.0);
+            if (lj >= 0) sh.stage[par][1][lane] = s_rows[lj * RS + lane];
+        }
         // how many of its rows lie within the margin
         int near = 0;
         for (int r = r0 + first; r < rpc; r += RT) {
@@ -415,11 +421,7 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         const int several = rpc > RT ? __syncthreads_or(near > 1) : 0;
         near = __syncthreads_count(near > 0) + (several ? 1 : 0);
         if (warp == 0) {
-            // the rows as they stand, and the message into every CTA
-            if (lane < kb) {
-                sh.stage[par][0][lane] = mr != INT_MAX ? s_rows[mr * RS + lane] : make_double2(0.0, 0.0);
-                if (lj >= 0) sh.stage[par][1][lane] = s_rows[lj * RS + lane];
-            }
+            // the message into every CTA
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0)
