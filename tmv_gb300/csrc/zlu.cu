@@ -335,7 +335,7 @@ __device__ __forceinline__ double2 zfms(double2 a, double2 l, double2 u)
 // time out in turn.  Per column at m = 2048 (clocks): 17500 with cluster
 // barriers, remote reads by every warp and the whole update on the chain; factor
 // and solve at n = 2048 took 16.4 ms with the messages, 14.0 ms once the warp that
-// decides held no rows.
+// decides held no rows, 13.6 with several threads paying for a row.
 template <int KB>
 __global__ void __launch_bounds__(kZPanelThreads)
 zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k, int kb, int64_t* __restrict__ P,
@@ -352,6 +352,11 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
     // row) while the others pay what the rows owe
     constexpr int RT = kZPanelThreads - 32;
     const int first = warp == 0 ? INT_MAX / 2 : tid - 32;
+    // threads that pay what a row owes: few rows leave sub-partitions idle, and a
+    // DFMA takes its own 64 clocks whatever the lanes (LU with one thread per row
+    // against this: n = 256 1.47 -> 1.32 ms, 1024 5.98 -> 5.60, 2048 12.58 -> 12.37)
+    int tpr = 1;
+    while (tpr < 8 && 2 * tpr * rpc <= RT) tpr *= 2;
     if (tid == 0) {
         mbar_init(&sh.mbar[0], 1u);
         mbar_init(&sh.mbar[1], 1u);
@@ -441,12 +446,12 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         // the shadow: what step j - 1 still owes (rows below j - 1, columns
         // beyond j)
         if (jj > 0) {
-            for (int r = r0 + first; r < rpc; r += RT) {
+            for (int r = r0 + first / tpr; r < rpc; r += RT / tpr) {
                 if (k + cta + (int64_t)kZPanelCtas * r >= n) break;
                 double2* row = &s_rows[r * RS];
                 const double2 l = row[jj - 1];
 #pragma unroll 4
-                for (int c = jj + 1; c < kb; ++c) row[c] = zfms(row[c], l, pold[c]);
+                for (int c = jj + 1 + first % tpr; c < kb; c += tpr) row[c] = zfms(row[c], l, pold[c]);
             }
         }
         if (warp == 0) {
