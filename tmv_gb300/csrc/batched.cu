@@ -809,6 +809,11 @@ static tmvg_status build_graph(BatchPlan* p)
                                                                   kBatchThreads, p->smem),
                     "batched: occupancy");
     if (st) return st;
+    // A fifth CTA per SM pays where every slot has several systems (n 2..64, 8000
+    // systems: 1710 -> 1442 us).  With few, the last large systems run five to an SM
+    // and the batch waits for them (n 20..256, 800 systems: 7980 -> 9666; 2500:
+    // 10093 -> 10614).
+    if (2 * p->count < 7 * (int64_t)per_sm * c->num_sms) per_sm = std::min(per_sm, 4);
     per_sm = std::max(per_sm, 1);
     p->grid = (int)std::min<int64_t>((int64_t)per_sm * c->num_sms, std::max<int64_t>(p->count, 1));
     // capture: reset the queue, run the persistent kernel
