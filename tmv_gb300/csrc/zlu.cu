@@ -378,16 +378,20 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         const int64_t d0 = j - k - cta;
         const int r0 = d0 <= 0 ? 0 : (int)((d0 + kZPanelCtas - 1) / kZPanelCtas);
         const int lj = cta == owner_j ? jj / kZPanelCtas : -1;
+        // this thread's first row at or below j: rows first, first + RT, ... are
+        // its own in every column (r0 <= KB / 16 <= RT), so that what it writes at
+        // a column's end no other thread reads at the next one's start
+        const int own = first >= r0 ? first : first + RT;
         const double2* pold = sh.prow[par ^ 1];
         double2* pnew = sh.prow[par];
         // stage 1: largest proxy key (the first row's key kept)
         long long bk = LLONG_MIN, key0 = LLONG_MIN;
         int bp = INT_MAX;
-        for (int r = r0 + first; r < rpc; r += RT) {
+        for (int r = own; r < rpc; r += RT) {
             const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
             if (i >= n) break;
             const long long key = zproxy_key(s_rows[r * RS + jj], i == j);
-            if (r == r0 + first) key0 = key;
+            if (r == own) key0 = key;
             if (key > bk) {
                 bk = key;
                 bp = r;
@@ -417,10 +421,10 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         }
         // how many of its rows lie within the margin
         int near = 0;
-        for (int r = r0 + first; r < rpc; r += RT) {
+        for (int r = own; r < rpc; r += RT) {
             const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
             if (i >= n) break;
-            const long long key = r == r0 + first ? key0 : zproxy_key(s_rows[r * RS + jj], i == j);
+            const long long key = r == own ? key0 : zproxy_key(s_rows[r * RS + jj], i == j);
             near += mk != LLONG_MIN && key >= mk - 64;
         }
         const int several = rpc > RT ? __syncthreads_or(near > 1) : 0;
@@ -515,11 +519,11 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
             int br = INT_MAX;
             double braw = 0.0;
             double2 binv = make_double2(0.0, 0.0);
-            for (int r = r0 + first; r < rpc && mk != LLONG_MIN; r += RT) {
+            for (int r = own; r < rpc && mk != LLONG_MIN; r += RT) {
                 const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
                 if (i >= n) break;
                 const double2 z = s_rows[r * RS + jj];
-                const long long key = r == r0 + first ? key0 : zproxy_key(z, i == j);
+                const long long key = r == own ? key0 : zproxy_key(z, i == j);
                 if (key < thr) continue;
                 const double raw = tmv_abs(z);
                 const long long a = zabs_key(raw, i == j);
@@ -549,7 +553,7 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
                 if (br != INT_MAX) sh.cand_rowv[tid] = s_rows[br * RS + tid];
                 if (lj >= 0) sh.diag_rowv[tid] = s_rows[lj * RS + tid];
             }
-            if (br != INT_MAX && br >= r0 && (br - r0) % RT == first) {
+            if (br != INT_MAX && br % RT == first) {
                 sh.cand_abs = braw;
                 sh.cand_inv = binv;
             }
@@ -605,7 +609,7 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         // scale this CTA's rows below j and update the next column
         const double2 inv = sh.inv;
         const bool und = sh.under != 0;
-        for (int r = r0 + first; r < rpc; r += RT) {
+        for (int r = own; r < rpc; r += RT) {
             const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
             if (i >= n) break;
             if (i == j) continue;
@@ -614,8 +618,8 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
             row[jj] = l;
             if (jj + 1 < kb) row[jj + 1] = zfms(row[jj + 1], l, pnew[jj + 1]);
         }
-        // (the next column reads only this thread's rows until its first
-        // __syncthreads)
+        // (until its first __syncthreads the next column reads only rows that
+        // this thread wrote)
     }
     __syncthreads();
     for (int t = tid; t < rpc * kb; t += kZPanelThreads) {
