@@ -1731,6 +1731,9 @@ narrow_update_f64_kernel(const double* __restrict__ A, int64_t lda, int64_t n, i
     __shared__ int s_dst[2 * NB], s_src[2 * NB], map_blk[NB], map_row[R];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rank = (int)cluster.block_rank();
+    // (a CTA's shared memory may be written by its peers once it has started:
+    // waited for where they do, behind the loads)
+    cluster.barrier_arrive();
     const int64_t r0 = k + NB + (int64_t)blockIdx.x * R;
     const int rows = (int)max((int64_t)0, min((int64_t)R, n - r0));
     // loads that need no row map
@@ -1765,14 +1768,18 @@ narrow_update_f64_kernel(const double* __restrict__ A, int64_t lda, int64_t n, i
 #pragma unroll
     for (int e = 0; e < E; ++e)
         old[e] = (rr < rows && cc + e < nc) ? A[map_row[rr] + (c0 + cc + e) * lda] : 0.0;
+    const int c = 4 * rank + warp;
+    double x = 0.0;
     if (warp < 4) {
-        const int c = 4 * rank + warp;
-        double x = c < nc ? A[map_blk[lane] + (c0 + c) * lda] : 0.0;
+        if (c < nc) x = A[map_blk[lane] + (c0 + c) * lda];
 #pragma unroll
         for (int j = 0; j < NB - 1; ++j) {
             const double r = fma(-l[j], __shfl_sync(0xffffffffu, x, j), x);
             if (lane > j) x = r;
         }
+    }
+    cluster.barrier_wait();  // every CTA of the cluster has started
+    if (warp < 4) {
 #pragma unroll
         for (int d = 0; d < kNarrow64Ctas; ++d) *cluster.map_shared_rank(&UT[lane][c], d) = x;
     }
