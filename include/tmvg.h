@@ -104,7 +104,10 @@ tmvg_status tmvg_probe_fp64_rate(tmvg_handle h, double* tflops);
  * solved and their results never published: the first block that waits on
  * one gives up after poll_limit polls, the others stop in turn, and the call
  * returns TMVG_TIMEOUT with the handle still usable (the hook resets itself
- * after that one launch).  Nothing traps or hangs. */
+ * after that one launch).  Of the complex factorisation's panels it shortens the
+ * waits for one another's candidates, and one CTA of the next panel sends none:
+ * the interchanges and factors of that call are then not to be used, and the
+ * timeout is reported as for tmvg_lu_decompose_z64.  Nothing traps or hangs. */
 tmvg_status tmvg_test_set_wait(tmvg_handle h, uint32_t poll_limit, int32_t skip_blocks);
 
 /* ---- MultMM ----------------------------------------------------------
@@ -268,6 +271,8 @@ tmvg_status tmvg_multmv_f64(tmvg_handle h, int add, double alpha, int64_t m,
  * TMV's modulus (TMV_ABS, include/tmv/TMV_Base.h:312-325); a column whose
  * largest modulus is below DBL_MIN is zeroed with P[j] = j; the column is
  * scaled by TMV_InverseOf of the pivot.  Never fails on singular input.
+ * Asynchronous: a bounded device-side wait that ran out is reported, as
+ * TMVG_TIMEOUT, by the next call on the handle that synchronises.
  * Replaces: template void tmv::LU_Decompose(MatrixView<std::complex<double> >,
  *           ptrdiff_t*) (src/TMV_LUDecompose.cpp:514-559).
  * tmvg_lu_ldiveq_z64: B := (P L U)^-1 B, each column with TMV's vector

@@ -126,7 +126,8 @@ struct Context {
     // Failure-path test hooks (tmvg_test_set_wait): the poll limit of the
     // sync-free triangular solve's block-flag waits (0: kSpinLimit), and a
     // number of leading blocks the next such solve never hands out, so their
-    // flags are never published (reset after one launch).
+    // flags are never published (reset after one launch); likewise the complex
+    // panel's waits (0: kTryWaitLimit), whose last CTA then sends nothing.
     unsigned poll_limit = 0;
     int test_skip_blocks = 0;
 };

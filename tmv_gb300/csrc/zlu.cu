@@ -277,6 +277,7 @@ struct ZPanelShared {
     double2 prow[2][KB];       // the pivot row after the interchange: U's row j
     uint64_t mbar[2];
     // the second exchange
+    uint64_t met;              // an arrival per CTA
     long long cand_key;        // this CTA's candidate: zabs_key (-2: none)
     double cand_abs;           // its TMV_ABS (NaN kept)
     long long cand_row;        // its global row (LLONG_MAX: none)
@@ -327,19 +328,23 @@ __device__ __forceinline__ double2 zfms(double2 a, double2 l, double2 u)
 // j) is owed and paid while the next column's messages travel.  A candidate's
 // row is therefore sent as it stands, and the receiver applies what it owes, a
 // column per lane.  The exchange is one message per CTA and destination (the
-// key by st.async, the row by a bulk copy) on the receiver's mbarrier; only the
-// second exchange uses cluster barriers.  Messages are double-buffered by
+// key by st.async, the row by a bulk copy) on the receiver's mbarrier; the
+// second exchange meets twice on another one, before and after the CTAs read one
+// another's candidates.  Messages are double-buffered by
 // column parity: a CTA sends for column j + 1 after all its threads are done
 // with column j, so when every message of j + 1 is in, j's buffers are free.
-// Waits are bounded; a CTA that gives up records kDevTimeout and the others
-// time out in turn.  Per column at m = 2048 (clocks): 17500 with cluster
-// barriers, remote reads by every warp and the whole update on the chain; factor
+// Waits are bounded; a CTA that gives up records kDevTimeout, and the others
+// time out in turn: no wait but the last is a cluster barrier, and a CTA reads
+// its peers only after all have arrived for it, so that every CTA stays until
+// the last barrier and none reads one that has left.  The interchanges that are
+// then missing are written as none, for the kernels that follow.  Per column at
+// m = 2048 (clocks): 17500 with cluster barriers, remote reads by every warp and the whole update on the chain; factor
 // and solve at n = 2048 took 16.4 ms with the messages, 14.0 ms once the warp that
 // decides held no rows, 13.6 with several threads paying for a row.
 template <int KB>
 __global__ void __launch_bounds__(kZPanelThreads)
 zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k, int kb, int64_t* __restrict__ P,
-                      int rpc, int* err)
+                      int rpc, int* err, unsigned poll_limit, int silent)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -360,6 +365,7 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
     if (tid == 0) {
         mbar_init(&sh.mbar[0], 1u);
         mbar_init(&sh.mbar[1], 1u);
+        mbar_init(&sh.met, (uint32_t)kZPanelCtas);
         sh.abort = 0;
         mbar_fence_init();
     }
@@ -370,7 +376,25 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         s_rows[r * RS + c] = i < n ? A[i + (k + c) * lda] : make_double2(0.0, 0.0);
     }
     cluster.sync();  // every CTA's mbarriers are initialised before any message
-    for (int jj = 0; jj < kb; ++jj) {
+    const auto give_up = [&] {
+        sh.abort = 1;
+        atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
+    };
+    // Every CTA's earlier work is done and seen (false: one never arrived).
+    uint32_t met = 0;
+    const auto meet = [&] {
+        __syncthreads();
+        if (warp == 0) {
+            if (lane < kZPanelCtas) mbar_arrive_remote_release(cluster_addr(&sh.met, lane));
+            const bool got = __all_sync(0xffffffffu, mbar_wait_cluster(&sh.met, met, poll_limit));
+            if (!got && lane == 0) give_up();
+        }
+        met ^= 1u;
+        __syncthreads();
+        return sh.abort == 0;
+    };
+    int jj = 0;
+    for (; jj < kb; ++jj) {
         const int par = jj & 1;
         const int64_t j = k + jj;
         const int owner_j = jj % kZPanelCtas;
@@ -436,7 +460,7 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
             if (lane == 0)
                 mbar_expect_tx(&sh.mbar[par], (uint32_t)(kZPanelCtas * (sizeof(ZMsg) + KB * sizeof(double2)) +
                                                          KB * sizeof(double2)));
-            if (lane < kZPanelCtas) {
+            if (lane < kZPanelCtas && cta != silent) {
                 const uint32_t bar = cluster_addr(&sh.mbar[par], lane);
                 const uint32_t dst = cluster_addr(&sh.msg[par][cta], lane);
                 const long long row = mr == INT_MAX ? LLONG_MAX : k + cta + (long long)kZPanelCtas * mr;
@@ -459,12 +483,9 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
             }
         }
         if (warp == 0) {
-            const bool got = __all_sync(0xffffffffu, mbar_wait_cluster(&sh.mbar[par], (uint32_t)((jj >> 1) & 1)));
+            const bool got = __all_sync(0xffffffffu, mbar_wait_cluster(&sh.mbar[par], (uint32_t)((jj >> 1) & 1), poll_limit));
             if (!got) {
-                if (lane == 0) {
-                    sh.abort = 1;
-                    atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
-                }
+                if (lane == 0) give_up();
             } else {
                 long long ck = LLONG_MIN;
                 if (lane < kZPanelCtas) ck = sh.msg[par][lane].key;
@@ -561,7 +582,7 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
                 sh.cand_key = ba;
                 sh.cand_row = br == INT_MAX ? LLONG_MAX : k + cta + (long long)kZPanelCtas * br;
             }
-            cluster.sync();
+            if (!meet()) break;
             // the winner over the cluster: lanes 0..15 of every warp read one CTA each
             long long wa = -3, wr = LLONG_MAX;
             int wc = 0;
@@ -603,7 +624,7 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
                     if (cta == 0) P[j] = p;
                 }
             }
-            cluster.sync();  // the staged rows are read
+            if (!meet()) break;  // the staged rows are read
         }
         __syncthreads();
         // scale this CTA's rows below j and update the next column
@@ -622,6 +643,8 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         // this thread wrote)
     }
     __syncthreads();
+    if (cta == 0)
+        for (int t = jj + tid; t < kb; t += kZPanelThreads) P[k + t] = k + t;  // (given up)
     for (int t = tid; t < rpc * kb; t += kZPanelThreads) {
         const int r = t % rpc, c = t / rpc;
         const int64_t i = k + cta + (int64_t)kZPanelCtas * r;
@@ -887,7 +910,10 @@ static tmvg_status zlu_factor_blocked(Context* c, int64_t n, double2* A, int64_t
         const int rpc = (int)ceil_div(n - k, kZPanelCtas);
         cfg.dynamicSmemBytes = (size_t)rpc * (KB + 1) * sizeof(double2);
         ++c->launches;
-        return check_cuda(c, cudaLaunchKernelEx(&cfg, zlu_panel_smem_kernel<KB>, n, A, lda, k, kb, P, rpc, c->dflags),
+        const int silent = c->test_skip_blocks > 0 ? kZPanelCtas - 1 : -1;
+        c->test_skip_blocks = 0;
+        return check_cuda(c, cudaLaunchKernelEx(&cfg, zlu_panel_smem_kernel<KB>, n, A, lda, k, kb, P, rpc, c->dflags,
+                                                c->poll_limit ? c->poll_limit : kTryWaitLimit, silent),
                           "lu_z: panel launch");
     };
     auto swap = [&](int64_t c0, int64_t c1, int64_t k, int kb) {
