@@ -104,11 +104,17 @@ tmvg_status tmvg_probe_fp64_rate(tmvg_handle h, double* tflops);
  * solved and their results never published: the first block that waits on
  * one gives up after poll_limit polls, the others stop in turn, and the call
  * returns TMVG_TIMEOUT with the handle still usable (the hook resets itself
- * after that one launch).  Of the complex factorisation's panels it shortens the
- * waits for one another's candidates, and one CTA of the next panel sends none:
- * the interchanges and factors of that call are then not to be used, and the
- * timeout is reported as for tmvg_lu_decompose_z64.  Nothing traps or hangs. */
+ * after that one launch).  Nothing traps or hangs. */
 tmvg_status tmvg_test_set_wait(tmvg_handle h, uint32_t poll_limit, int32_t skip_blocks);
+/* The same for waits of one kernel's parts on one another.  TMVG_SILENT_PANEL:
+ * one CTA of the next clustered panel of a factorisation sends no candidate.
+ * The waits give up (real panels after about a second, complex ones after
+ * tmvg_test_set_wait's poll_limit; 0: 2^22 polls, up to 4 us each), the results of
+ * that call are not to be used, and the timeout is reported as that entry
+ * point says.  The hook resets itself after that one launch; TMVG_SILENT_NONE
+ * withdraws it. */
+enum { TMVG_SILENT_NONE = 0, TMVG_SILENT_PANEL = 1 };
+tmvg_status tmvg_test_set_silent(tmvg_handle h, int32_t what);
 
 /* ---- MultMM ----------------------------------------------------------
  * C (+)= alpha * A * B;  A m x k, B k x n, C m x n.  add = 0: C = alpha*A*B,

@@ -35,6 +35,7 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes)
 // Wait for the phase with the given parity to complete; false on timeout.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned limit = kTryWaitLimit)
 {
+#pragma unroll 1
     for (unsigned spins = 0; spins < limit; ++spins) {
         uint32_t done;
         asm volatile(
@@ -71,6 +72,7 @@ __device__ __forceinline__ void st_async16(uint32_t dst, const uint4& v, uint32_
 // CTAs of the cluster); false on timeout.
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, unsigned limit = kTryWaitLimit)
 {
+#pragma unroll 1
     for (unsigned spins = 0; spins < limit; ++spins) {
         uint32_t done;
         asm volatile(

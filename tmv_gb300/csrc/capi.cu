@@ -533,6 +533,15 @@ tmvg_status tmvg_test_set_wait(tmvg_handle h, uint32_t poll_limit, int32_t skip_
     return TMVG_OK;
 }
 
+tmvg_status tmvg_test_set_silent(tmvg_handle h, int32_t what)
+{
+    CTX_OR_BAIL(h);
+    if (what < TMVG_SILENT_NONE || what > TMVG_SILENT_PANEL)
+        return set_error(c, TMVG_BAD_ARG, "test_set_silent: unknown part");
+    c->test_silent = what;
+    return TMVG_OK;
+}
+
 tmvg_status tmvg_probe_fp64_rate(tmvg_handle h, double* tflops)
 {
     CTX_OR_BAIL(h);

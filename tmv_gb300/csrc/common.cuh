@@ -126,10 +126,18 @@ struct Context {
     // Failure-path test hooks (tmvg_test_set_wait): the poll limit of the
     // sync-free triangular solve's block-flag waits (0: kSpinLimit), and a
     // number of leading blocks the next such solve never hands out, so their
-    // flags are never published (reset after one launch); likewise the complex
-    // panel's waits (0: kTryWaitLimit), whose last CTA then sends nothing.
+    // flags are never published (reset after one launch).
     unsigned poll_limit = 0;
     int test_skip_blocks = 0;
+    // tmvg_test_set_silent: the part that stays silent in the next launch that
+    // has it (TMVG_SILENT_*).
+    int test_silent = 0;
+    bool silenced(int what)
+    {
+        const bool hit = test_silent == what;
+        if (hit) test_silent = 0;
+        return hit;
+    }
 };
 
 // The side stream and its events (nullptr-safe to call repeatedly).

@@ -145,7 +145,14 @@ lu_panel_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int nb,
                     __stcg(&diag_row[par * kPanelMax + cc], rows[r * ldp + cc]);
             }
         }
-        if (!grid_barrier(bar, (unsigned)(jj + 1) * (unsigned)G, err)) return;
+        if (!grid_barrier(bar, (unsigned)(jj + 1) * (unsigned)G, err)) {
+            // (given up: no interchanges, for the kernels that follow)
+            if (cta == 0) {
+                for (int t = jj + tid; t < nb; t += kPanelThreads) P[k + t] = k + t;
+                if (tid == 0) pairs[0] = 0;
+            }
+            return;
+        }
 
         // 3. global winner
         if (warp == 0) {
@@ -584,12 +591,18 @@ __device__ __forceinline__ void reg2_update(T (&x)[NB], T lx, bool ux, T (&y)[NB
     }
 }
 
+// Polls of the panels' waits for their cluster's messages: about a second (a
+// poll suspends the thread for up to 4 us).  A constant: as a kernel argument
+// it made the FP64 panels 1 to 2 % slower.
+constexpr unsigned kPanelPolls = 1u << 18;
+
 template <typename T, int NB>
 __global__ void __launch_bounds__(kReg2Threads, 1)
 lu_panel_cluster_reg2_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int nb,
                              int64_t* __restrict__ P,
                              int rows_per_cta, int* pairs, int* err, float* __restrict__ ahi,
-                             float* __restrict__ alo, const T* __restrict__ Sp, int64_t lds)
+                             float* __restrict__ alo, const T* __restrict__ Sp, int64_t lds,
+                             int silent)
 {
     // Sp: the panel's columns come from this scratch panel (row i, column c
     // at Sp[i + c lds]) instead of A
@@ -699,13 +712,13 @@ lu_panel_cluster_reg2_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t 
                         reinterpret_cast<uint4*>(pub_row[par])[lane] =
                             reinterpret_cast<const uint4*>(warp_row[((bi - r0) & (kReg2Threads - 1)) >> 5])[lane];
                     __syncwarp();
-                    if (lane < G) {
+                    if (lane < G && cta != silent) {
                         st_cluster16(cluster_addr(&slot[par][cta], lane),
                                      make_uint4((unsigned)bk, (unsigned)(bk >> 32), (unsigned)bi, 0u));
                         mbar_arrive_remote_release(cluster_addr(&mbar[par], lane));
                     }
                     // 3. wait for every CTA's record (bounded), reduce, pull rows
-                    const bool got = __all_sync(0xffffffffu, mbar_wait_cluster(&mbar[par], (uint32_t)((jj >> 1) & 1)));
+                    const bool got = __all_sync(0xffffffffu, mbar_wait_cluster(&mbar[par], (uint32_t)((jj >> 1) & 1), kPanelPolls));
                     if (!got) {
                         if (lane == 0) {
                             s_abort = 1;
@@ -808,6 +821,10 @@ lu_panel_cluster_reg2_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t 
             for (int j = tid; j < nb; j += kReg2Threads) P[k + j] = s_piv[j];
             if (warp == 0) panel_row_pairs(k, nb, s_piv, pairs);
         }
+    } else if (cta == 0) {
+        // (given up: no interchanges, for the kernels that follow)
+        for (int j = tid; j < nb; j += kReg2Threads) P[k + j] = k + j;
+        if (tid == 0) pairs[0] = 0;
     }
     cluster.sync();  // no CTA leaves while another may still store into it
 }
@@ -1041,7 +1058,7 @@ __global__ void __launch_bounds__(kLeafThreads, 1)
 lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int nb,
                      int64_t* __restrict__ P,
                      int rows_per_cta, int* pairs, int* err, float* __restrict__ ahi,
-                     float* __restrict__ alo, const T* __restrict__ Sp, int64_t lds)
+                     float* __restrict__ alo, const T* __restrict__ Sp, int64_t lds, int silent)
 {
     static_assert(NB % kLeaf == 0 && NB >= 2 * kLeaf, "whole leaves");
     static_assert(NB * sizeof(T) == 256, "a row is 16 vectors of 16 bytes");
@@ -1096,7 +1113,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
     const LeafHead none{0ull, INT_MAX, -1};
     static_assert(kClusterCtas == 16 && kLeafWarps >= kClusterCtas, "a candidate per lane, a reciprocal per CTA");
     // (warp 0's lanes d and d + 16 send to CTA d)
-    const int dest = lane & (kClusterCtas - 1);
+    const int dest = cta == silent ? kClusterCtas : lane & (kClusterCtas - 1);
     const uint32_t to_msg = cluster_addr(&msg[0][cta], dest < G ? dest : 0);
     const uint32_t to_bar = cluster_addr(&mbar[0], dest < G ? dest : 0);
     constexpr int kRcpWarp = 1;  // (every block has several warps)
@@ -1175,7 +1192,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             }
             if (warp == 0 && G > 1) {
                 // 4. every CTA's message (bounded wait), reduced here
-                const bool got = __all_sync(0xffffffffu, mbar_wait(&mbar[par], (uint32_t)((j >> 1) & 1)));
+                const bool got = __all_sync(0xffffffffu, mbar_wait(&mbar[par], (uint32_t)((j >> 1) & 1), kPanelPolls));
                 if (!got) {
                     if (lane == 0) {
                         s_abort = 1;
@@ -1190,7 +1207,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             }
             if (kLongRcp && warp == kRcpWarp) {
                 // every candidate's reciprocal, beside warp 0's decision
-                const bool got = G == 1 || __all_sync(0xffffffffu, mbar_wait(&mbar[par], (uint32_t)((j >> 1) & 1)));
+                const bool got = G == 1 || __all_sync(0xffffffffu, mbar_wait(&mbar[par], (uint32_t)((j >> 1) & 1), kPanelPolls));
                 if (got && lane < (G > 1 ? G : nwarp)) {
                     const LeafMsg<T>& cm = G > 1 ? msg[par][lane] : wmsg[lane];
                     s_rcp[lane] = recip_rn(cm.head.pos != INT_MAX ? cm.leaf[0] : T(1));
@@ -1244,7 +1261,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
                 send_step = -1;
             }
             if (G > 1) {
-                if (!mbar_wait(&mbar_leaf, leaf_uses & 1u)) {
+                if (!mbar_wait(&mbar_leaf, leaf_uses & 1u, kPanelPolls)) {
                     if (tid == 0) atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
                     s_abort = 1;  // every thread of the CTA reaches this
                 }
@@ -1285,9 +1302,12 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
         }
         if (cta == 0)
             for (int j = tid; j < nb; j += nthr) P[k + j] = s_piv[j];
+    } else if (cta == 0) {
+        // (given up: no interchanges, for the kernels that follow)
+        for (int j = tid; j < nb; j += nthr) P[k + j] = k + j;
     }
     cluster.sync();  // no CTA leaves while another may still store into it
-    if (cta == 0 && tid == 0 && !s_abort) pairs[0] = s_npairs;
+    if (cta == 0 && tid == 0) pairs[0] = s_abort ? 0 : s_npairs;
 }
 
 // ---------------------------------------------------------------------
@@ -2384,15 +2404,16 @@ static tmvg_status launch_panel_cluster_reg(Context* c, cudaStream_t s, T* A, in
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     ++c->launches;
+    const int silent = G > 1 && c->silenced(TMVG_SILENT_PANEL) ? G - 1 : -1;
     if (c->panel_reg2)
         return check_cuda(c,
                           cudaLaunchKernelEx(&cfg, lu_panel_cluster_reg2_kernel<T, RegPanel<T>::NB>, A,
                                              lda, n, k, nb, P, rpc, pairs, c->dflags, ahi, alo, Sp,
-                                             lds),
+                                             lds, silent),
                           "lu: register panel launch");
     return check_cuda(c,
                       cudaLaunchKernelEx(&cfg, lu_panel_leaf_kernel<T, RegPanel<T>::NB>, A, lda, n, k,
-                                         nb, P, rpc, pairs, c->dflags, ahi, alo, Sp, lds),
+                                         nb, P, rpc, pairs, c->dflags, ahi, alo, Sp, lds, silent),
                       "lu: leaf register panel launch");
 }
 

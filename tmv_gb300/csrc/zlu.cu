@@ -910,8 +910,7 @@ static tmvg_status zlu_factor_blocked(Context* c, int64_t n, double2* A, int64_t
         const int rpc = (int)ceil_div(n - k, kZPanelCtas);
         cfg.dynamicSmemBytes = (size_t)rpc * (KB + 1) * sizeof(double2);
         ++c->launches;
-        const int silent = c->test_skip_blocks > 0 ? kZPanelCtas - 1 : -1;
-        c->test_skip_blocks = 0;
+        const int silent = c->silenced(TMVG_SILENT_PANEL) ? kZPanelCtas - 1 : -1;
         return check_cuda(c, cudaLaunchKernelEx(&cfg, zlu_panel_smem_kernel<KB>, n, A, lda, k, kb, P, rpc, c->dflags,
                                                 c->poll_limit ? c->poll_limit : kTryWaitLimit, silent),
                           "lu_z: panel launch");
