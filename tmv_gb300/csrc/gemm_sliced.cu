@@ -22,10 +22,11 @@
 // the tile's rows and columns must overlap in 1.75 sqrt(K) places (pigeonhole)
 // the tile is good; otherwise the CTA sums the products of the leading digits'
 // moduli, which ends as soon as every element has passed.  A tile that fails
-// both, or has an entry that is not finite or a vector of extreme scale, takes
-// the FP64 pipe on the unsliced operands, with the FMA chain of
-// gemm_simt_kernel (65 us for K = 32 against 5: the second look keeps tiles of
-// ordinary data, of which one in some thousand fails the first, off it).
+// both, or has an entry that is not finite or a vector of extreme scale, is put
+// on a list and multiplied by a kernel of its own on the FP64 pipe, from the
+// unsliced operands and with the FMA chain of gemm_simt_kernel (the second look
+// keeps tiles of ordinary data, of which one in some thousand fails the first,
+// off that list).
 //
 // Data flow per CTA (persistent over 128 x 64 tiles of C): one thread loads
 // stages of K = 32 (8 digits x (128 + 64) rows x 64 bytes = 96 KB, two
@@ -215,25 +216,26 @@ __device__ __forceinline__ void split_vectors(const SplitSide& s, int64_t grp, i
 }
 
 // Both operands in one launch: groups_a CTAs for A, the rest for B.
+// `listed`: the count of the product's list, cleared here.
 template <int R, bool ZLEFT>
 __global__ void __launch_bounds__(kSplitThreads)
-sliced_split_kernel(SplitSide sa, SplitSide sb, int64_t groups_a, int64_t K)
+sliced_split_kernel(SplitSide sa, SplitSide sb, int64_t groups_a, int64_t K, int* listed)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *listed = 0;
     if ((int64_t)blockIdx.x < groups_a) split_vectors<R, ZLEFT>(sa, blockIdx.x, K);
     else split_vectors<R, false>(sb, blockIdx.x - groups_a, K);
 }
 
-tmvg_status sliced_split(Context* c, int64_t K, Mat<const double> A, const SlicedOperand& sa,
-                         Mat<const double> B, const SlicedOperand& sb, bool zleft)
+static tmvg_status sliced_split(Context* c, int64_t K, Mat<const double> A, const SlicedOperand& sa,
+                                Mat<const double> B, const SlicedOperand& sb, int* listed, bool zleft)
 {
     const int R = sa.rows ? sa.group : sb.group;
     const SplitSide a{A.p, A.si, A.sj, sa.digits, sa.exps, sa.fill, sa.rows, sa.Kp};
     const SplitSide b{B.p, B.sj, B.si, sb.digits, sb.exps, sb.fill, sb.rows, sb.Kp};
     const int64_t ga = ceil_div(sa.rows, (int64_t)R), gb = ceil_div(sb.rows, (int64_t)R);
-    if (ga + gb == 0) return TMVG_OK;
     auto kern = R == 64 ? (zleft ? sliced_split_kernel<64, true> : sliced_split_kernel<64, false>)
                         : (zleft ? sliced_split_kernel<16, true> : sliced_split_kernel<16, false>);
-    kern<<<(unsigned)(ga + gb), kSplitThreads, 0, c->stream>>>(a, b, ga, K);
+    kern<<<(unsigned)(ga + gb), kSplitThreads, 0, c->stream>>>(a, b, ga, K, listed);
     ++c->launches;
     return check_cuda(c, cudaGetLastError(), "sliced split launch");
 }
@@ -370,7 +372,7 @@ struct SlicedArgs {
     double alpha;
     int add;                         // beta
     int unit;                        // alpha: 1 or -1, or 0 for any other value
-    const double *A, *B;             // the operands themselves (FP64 tiles)
+    const double *A, *B;             // the operands themselves (listed tiles)
     int64_t asi, asj, bsi, bsj;
     bool zleft;
     const int *ea, *eb, *fa, *fb;
@@ -382,6 +384,7 @@ struct SlicedArgs {
     double* C;
     int64_t ldc;
     int64_t mt, nt;                  // tiles
+    int* listed;                     // the tiles for the FP64 pipe: their count, then their numbers
 };
 
 // Tile t of the persistent order: columns of 16 tile rows, so that the tiles
@@ -410,40 +413,70 @@ __device__ __forceinline__ int sl_look(const SlicedArgs& g, int64_t mi, int64_t 
 
 // Second look (the whole CTA): the sum of |leading digit of a| |leading digit
 // of b| over K reaches need_sum for every element, or the element's row or
-// column is zero.
+// column is zero.  A warp's 32 x 16 elements as 2 x 2 BF16 tiles of the warp-wide
+// tensor instruction (a tile that fails looks at all of K: by FMAs that took 3 us
+// per 32 places, 640 us of a product of K = 2048).
 template <int TN>
 __device__ __noinline__ bool sl_look_again(const SlicedArgs& g, int64_t mi, int64_t ni)
 {
+    constexpr int64_t kStep = 64;  // places between two votes
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int q = lane >> 2, t = lane & 3;
     const bool work = warp < kSlEpiWarps / (kSlN / TN);
-    const int64_t r = mi * kSlM + (warp & 3) * 32 + lane;
-    const int64_t c0 = ni * TN + (int64_t)(warp >> 2) * kSlCols;
-    const int nc = work ? (int)max((int64_t)0, min((int64_t)kSlCols, g.N - c0)) : 0;
-    bool pass = !work || r >= g.M || __ldg(&g.ea[r]) == kZeroExp;
-    unsigned todo = pass ? 0u : (1u << nc) - 1u;
-    float sum[kSlCols];
+    const int64_t r0 = mi * kSlM + (warp & 3) * 32 + q;                 // rows r0 + 8 (0..3)
+    const int64_t c0 = ni * TN + (int64_t)(warp >> 2) * kSlCols;        // columns
+    // (rows and columns outside read the last one's digits; they do not vote)
+    const uint16_t *pa[4], *pb[2];
 #pragma unroll
-    for (int j = 0; j < kSlCols; ++j) sum[j] = 0.0f;
-    for (int64_t k = 0; k < g.Kp; k += 8) {
-        if (todo) {
-            const uint4 av = *reinterpret_cast<const uint4*>(g.da + r * g.Kp + k);
-            const uint32_t aw[4] = {av.x, av.y, av.z, av.w};
+    for (int u = 0; u < 4; ++u) pa[u] = g.da + min(r0 + 8 * u, g.M - 1) * g.Kp + 2 * t;
 #pragma unroll
-            for (int j = 0; j < kSlCols; ++j) {
-                if (j < nc) {
-                    const uint4 bv = *reinterpret_cast<const uint4*>(g.db + (c0 + j) * g.Kp + k);
-                    const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+    for (int u = 0; u < 2; ++u) pb[u] = g.db + min(c0 + 8 * u + q, g.N - 1) * g.Kp + 2 * t;
+    auto digits = [](const uint16_t* p) { return __ldg(reinterpret_cast<const uint32_t*>(p)) & 0x7fff7fffu; };
+    float sum[2][2][4] = {};
+    // which of sum's elements need no more: bit 8 i + 4 j + e
+    unsigned done = work ? 0u : 0xffffu;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        sum[j] = fmaf(__uint_as_float((aw[q] << 16) & 0x7fffffffu),
-                                      __uint_as_float((bw[q] << 16) & 0x7fffffffu), sum[j]);
-                        sum[j] = fmaf(__uint_as_float(aw[q] & 0x7fff0000u), __uint_as_float(bw[q] & 0x7fff0000u), sum[j]);
-                    }
-                    if (sum[j] >= g.need_sum || __ldg(&g.eb[c0 + j]) == kZeroExp) todo &= ~(1u << j);
-                }
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int64_t r = r0 + 16 * i + 8 * (e >> 1), c = c0 + 8 * j + 2 * t + (e & 1);
+                if (r >= g.M || c >= g.N || __ldg(&g.ea[min(r, g.M - 1)]) == kZeroExp ||
+                    __ldg(&g.eb[min(c, g.N - 1)]) == kZeroExp)
+                    done |= 1u << (8 * i + 4 * j + e);
             }
+    for (int64_t k0 = 0; k0 < g.Kp; k0 += kStep) {
+        if (__any_sync(0xffffffffu, done != 0xffffu)) {
+            for (int64_t k = k0; k < min(k0 + kStep, g.Kp); k += 16) {
+                uint32_t a[2][4], b[2][2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) a[i][e] = digits(pa[2 * i + (e & 1)] + k + 8 * (e >> 1));
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) b[j][e] = digits(pb[j] + k + 8 * e);
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        asm volatile(
+                            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+                            "{%8, %9}, {%0, %1, %2, %3};"
+                            : "+f"(sum[i][j][0]), "+f"(sum[i][j][1]), "+f"(sum[i][j][2]), "+f"(sum[i][j][3])
+                            : "r"(a[i][0]), "r"(a[i][1]), "r"(a[i][2]), "r"(a[i][3]), "r"(b[j][0]), "r"(b[j][1]));
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (sum[i][j][e] >= g.need_sum) done |= 1u << (8 * i + 4 * j + e);
         }
-        if (__syncthreads_and(todo == 0u)) return true;
+        if (__syncthreads_and(done == 0xffffu)) return true;
     }
     return false;
 }
@@ -505,10 +538,10 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
             sl_tile(g, blockIdx.x + (int64_t)(i0 + lane) * gridDim.x, mi, ni);
             look = sl_look<TN>(g, mi, ni);
         }
-        const unsigned good = __ballot_sync(0xffffffffu, look == 1), open = __ballot_sync(0xffffffffu, look == 0);
+        const unsigned good = __ballot_sync(0xffffffffu, look == 1);
         if (lane == 0) {
             s_ok[i0 >> 5] = good;
-            if (open) s_open = 1;
+            if (good != 0xffffffffu) s_open = 1;
         }
     }
     __syncthreads();
@@ -516,10 +549,14 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
         for (int i = 0; i < mine; ++i) {
             if ((s_ok[i >> 5] >> (i & 31)) & 1u) continue;
             int64_t mi, ni;
-            sl_tile(g, blockIdx.x + (int64_t)i * gridDim.x, mi, ni);
+            const int64_t t = blockIdx.x + (int64_t)i * gridDim.x;
+            sl_tile(g, t, mi, ni);
             const bool again = sl_look<TN>(g, mi, ni) == 0 && sl_look_again<TN>(g, mi, ni);
             __syncthreads();  // every thread has read the word
-            if (again && tid == 0) s_ok[i >> 5] |= 1u << (i & 31);
+            if (tid == 0) {
+                if (again) s_ok[i >> 5] |= 1u << (i & 31);
+                else g.listed[1 + atomicAdd(g.listed, 1)] = (int)t;
+            }
             __syncthreads();
         }
     }
@@ -611,29 +648,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
             const bool in = r < g.M;
             const int nc = (int)max((int64_t)0, min((int64_t)kSlCols, g.N - col0));
             double* Cp = g.C + r + col0 * g.ldc;
-            if (!sliced(i)) {
-                // the FP64 pipe: a row and 8 columns of C at a time
-                for (int j0 = 0; in && j0 < nc; j0 += 8) {
-                    double acc[8];
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) acc[q] = 0.0;
-                    for (int64_t k = 0; k < g.K; ++k) {
-                        const double av = g.zleft ? sl_at<true>(g.A, g.asi, g.asj, r, k) : sl_at<false>(g.A, g.asi, g.asj, r, k);
-#pragma unroll
-                        for (int q = 0; q < 8; ++q)
-                            if (j0 + q < nc) acc[q] = fma(av, __ldg(&g.B[k * g.bsi + (col0 + j0 + q) * g.bsj]), acc[q]);
-                    }
-#pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        if (j0 + q < nc) {
-                            const double v = g.alpha * acc[q];
-                            double* cp = Cp + (j0 + q) * g.ldc;
-                            *cp = g.add ? v + *cp : v;
-                        }
-                }
-                __syncwarp();
-                continue;
-            }
+            if (!sliced(i)) continue;
             // this row's scale, and a column's per lane; C's first columns on
             // their way while the products run
             const int ea = in ? __ldg(&g.ea[r]) : 0;
@@ -751,9 +766,91 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
     }
     sl_fence_before();
     __syncthreads();
+    // (at the end: the listed tiles' CTAs would hold the SMs that a smaller grid
+    // leaves to others while they wait)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (warp == kSlEpiWarps) {
         sl_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+
+// ---------------------------------------------------------------------
+// The listed tiles on the FP64 pipe, 8 x 8 entries of C at a time, one per
+// thread, over all of this launch's CTAs: sixteen groups of two warps each.  The
+// same chain of FMAs per entry as gemm_simt_kernel.  Bound: 2 FMAs per SM per
+// clock; a single tile takes 128 groups K x 64 clocks.  In the kernel above, where
+// a CTA multiplied its own, one tile took K x 4096 clocks, and the loader and the
+// multiplier waited for it.  One CTA per SM (by its shared memory), so that a
+// grid smaller than the device leaves the other SMs free.  Launched as a
+// dependent of the kernel above, so that an empty list costs little
+// (0.8 us at 1024 x 1024 x 1024; as a plain launch 4).  1024 x 1024 x 1024 with a NaN in A:
+// 2.1 ms -> 0.33, A lower triangular 2.6 -> 0.33, 300 x 300 x 300 with such an A 0.79 -> 0.08.
+// ---------------------------------------------------------------------
+constexpr int kRestGroups = 16;  // (named barriers 0..15)
+constexpr int kRestB = 8, kRestK = 32;
+constexpr int kRestThreads = kRestGroups * kRestB * kRestB;
+struct RestBlock {
+    double a[kRestK][kRestB + 1], b[kRestK][kRestB + 1];
+};
+constexpr int kRestSmem = 120 * 1024;
+static_assert(kRestGroups * sizeof(RestBlock) <= kRestSmem && kRestSmem > 114 * 1024, "one CTA per SM");
+
+template <int TN, bool Z>
+__global__ void __launch_bounds__(kRestThreads)
+sliced_rest_kernel(const __grid_constant__ SlicedArgs g)
+{
+    constexpr int kSub = (kSlM / kRestB) * (TN / kRestB);  // per tile
+    constexpr int kLoads = kRestK / kRestB;
+    extern __shared__ __align__(16) unsigned char rest_smem[];
+    const int group = threadIdx.x / (kRestB * kRestB), gt = threadIdx.x % (kRestB * kRestB);
+    RestBlock& sh = reinterpret_cast<RestBlock*>(rest_smem)[group];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int64_t items = (int64_t)g.listed[0] * kSub;
+    const int tx = gt % kRestB, ty = gt / kRestB;
+    const bool ak = !Z && g.asj == 1, bk = g.bsi == 1;  // K contiguous
+    auto a_at = [&](int t, int& r, int& k) { r = ak ? t / kRestK : t % kRestB, k = ak ? t % kRestK : t / kRestB; };
+    auto b_at = [&](int t, int& q, int& k) { q = bk ? t / kRestK : t % kRestB, k = bk ? t % kRestK : t / kRestB; };
+    auto sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(group) : "memory"); };
+    for (int64_t it = (int64_t)group * gridDim.x + blockIdx.x; it < items; it += (int64_t)kRestGroups * gridDim.x) {
+        int64_t mi, ni;
+        sl_tile(g, g.listed[1 + it / kSub], mi, ni);
+        const int sub = (int)(it % kSub);
+        const int64_t r0 = mi * kSlM + (sub % (kSlM / kRestB)) * kRestB, c0 = ni * TN + (sub / (kSlM / kRestB)) * kRestB;
+        if (r0 >= g.M || c0 >= g.N) continue;
+        double pa[kLoads], pb[kLoads], acc = 0.0;
+        auto load = [&](int64_t k0) {
+#pragma unroll
+            for (int u = 0; u < kLoads; ++u) {
+                int r, q, k;
+                a_at(gt + u * kRestB * kRestB, r, k);
+                pa[u] = r0 + r < g.M && k0 + k < g.K ? sl_at<Z>(g.A, g.asi, g.asj, r0 + r, k0 + k) : 0.0;
+                b_at(gt + u * kRestB * kRestB, q, k);
+                pb[u] = c0 + q < g.N && k0 + k < g.K ? __ldg(&g.B[(k0 + k) * g.bsi + (c0 + q) * g.bsj]) : 0.0;
+            }
+        };
+        load(0);
+        for (int64_t k0 = 0; k0 < g.K; k0 += kRestK) {
+            sync();  // the group is done with the last block
+#pragma unroll
+            for (int u = 0; u < kLoads; ++u) {
+                int r, q, k;
+                a_at(gt + u * kRestB * kRestB, r, k);
+                sh.a[k][r] = pa[u];
+                b_at(gt + u * kRestB * kRestB, q, k);
+                sh.b[k][q] = pb[u];
+            }
+            sync();
+            if (k0 + kRestK < g.K) load(k0 + kRestK);
+            const int kn = (int)min((int64_t)kRestK, g.K - k0);
+#pragma unroll 8
+            for (int k = 0; k < kn; ++k) acc = fma(sh.a[k][tx], sh.b[k][ty], acc);
+        }
+        if (r0 + tx < g.M && c0 + ty < g.N) {
+            double* cp = g.C + (r0 + tx) + (c0 + ty) * g.ldc;
+            const double v = g.alpha * acc;
+            *cp = g.add ? v + *cp : v;
+        }
     }
 }
 
@@ -785,9 +882,12 @@ static bool sl_map(CUtensorMap* map, const SlicedOperand& s, int box_rows)
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-tmvg_status sliced_apply(Context* c, int64_t M, int64_t N, int64_t K, double alpha, Mat<const double> A,
-                         const SlicedOperand& sa, Mat<const double> B, const SlicedOperand& sb, double beta,
-                         double* C, int64_t ldc, int max_ctas, bool zleft)
+// C (M x N, column-major) = alpha A B + beta C (beta 0 or 1) from the slices; A
+// and B themselves are read only for listed tiles.  `max_ctas` bounds the
+// persistent grid (0: one per SM).
+static tmvg_status sliced_apply(Context* c, int64_t M, int64_t N, int64_t K, double alpha, Mat<const double> A,
+                                const SlicedOperand& sa, Mat<const double> B, const SlicedOperand& sb, double beta,
+                                double* C, int64_t ldc, int* listed, int max_ctas, bool zleft)
 {
     if (M <= 0 || N <= 0 || K <= 0) return TMVG_OK;
     CUtensorMap mA, mB;
@@ -816,6 +916,7 @@ tmvg_status sliced_apply(Context* c, int64_t M, int64_t N, int64_t K, double alp
     g.da = sa.digits, g.db = sb.digits, g.Kp = sa.Kp;
     g.C = C, g.ldc = ldc;
     g.mt = ceil_div(M, (int64_t)kSlM), g.nt = ceil_div(N, (int64_t)tn);
+    g.listed = listed;
     const unsigned grid = (unsigned)std::min<int64_t>(g.mt * g.nt, cap);
     auto kern = tn == 32 ? sliced_gemm_kernel<32> : sliced_gemm_kernel<kSlN>;
     const size_t smem = (size_t)kSlStages * (tn == 32 ? sl_stage_bytes<32>() : sl_stage_bytes<kSlN>()) + 1024;
@@ -824,7 +925,24 @@ tmvg_status sliced_apply(Context* c, int64_t M, int64_t N, int64_t K, double alp
     if (st) return st;
     kern<<<grid, kSlThreads, smem, c->stream>>>(mA, mB, g, c->dflags);
     ++c->launches;
-    return check_cuda(c, cudaGetLastError(), "sliced product launch");
+    if ((st = check_cuda(c, cudaGetLastError(), "sliced product launch"))) return st;
+    auto rest = tn == 32 ? (zleft ? sliced_rest_kernel<32, true> : sliced_rest_kernel<32, false>)
+                         : (zleft ? sliced_rest_kernel<kSlN, true> : sliced_rest_kernel<kSlN, false>);
+    st = check_cuda(c, cudaFuncSetAttribute(rest, cudaFuncAttributeMaxDynamicSharedMemorySize, kRestSmem),
+                    "sliced product");
+    if (st) return st;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3((unsigned)cap);
+    cfg.blockDim = dim3(kRestThreads);
+    cfg.dynamicSmemBytes = kRestSmem;
+    cfg.stream = c->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    ++c->launches;
+    return check_cuda(c, cudaLaunchKernelEx(&cfg, rest, g), "sliced product, listed tiles");
 }
 
 void* scratch_alloc(Context* c, size_t bytes, cudaStream_t s)
@@ -882,9 +1000,12 @@ tmvg_status sliced_gemm(Context* c, int64_t M, int64_t N, int64_t K, double alph
     const int64_t mb = std::min(M, cap);
     const int64_t nb = std::min(std::min(N, cap), std::max<int64_t>(1, kMaxTilesPerCta / ceil_div(mb, (int64_t)kSlM)) *
                                                       32 * (max_ctas > 0 ? max_ctas : c->num_sms));
-    const size_t ba = (sliced_bytes(mb, kb) + 255) & ~size_t(255);
-    unsigned char* ws = (unsigned char*)scratch_alloc(c, ba + sliced_bytes(nb, kb), c->stream);
+    auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
+    const size_t ba = al(sliced_bytes(mb, kb)), bb = al(sliced_bytes(nb, kb));
+    const size_t bl = sizeof(int) * (size_t)(1 + ceil_div(mb, (int64_t)kSlM) * ceil_div(nb, (int64_t)32));
+    unsigned char* ws = (unsigned char*)scratch_alloc(c, ba + bb + bl, c->stream);
     if (!ws) return TMVG_UNSUPPORTED;
+    int* listed = reinterpret_cast<int*>(ws + ba + bb);
     tmvg_status st = TMVG_OK;
     for (int64_t k0 = 0; k0 < K && !st; k0 += kb) {
         const int64_t k = std::min(kb, K - k0);
@@ -899,10 +1020,10 @@ tmvg_status sliced_gemm(Context* c, int64_t M, int64_t N, int64_t K, double alph
                 const SlicedOperand sb = sliced_layout(ws + ba, n, k);
                 SlicedOperand one = sa;
                 if (j0 > 0) one.rows = 0;  // A's block is sliced already
-                st = sliced_split(c, k, a, one, b, sb, zleft);
+                st = sliced_split(c, k, a, one, b, sb, listed, zleft);
                 if (!st)
                     st = sliced_apply(c, m, n, k, alpha, a, sa, b, sb, k0 > 0 ? 1.0 : beta, C + i0 + j0 * ldc, ldc,
-                                      max_ctas, zleft);
+                                      listed, max_ctas, zleft);
             }
         }
     }

@@ -20,29 +20,17 @@ struct SlicedOperand {
 size_t sliced_bytes(int64_t rows, int64_t K);
 SlicedOperand sliced_layout(void* buf, int64_t rows, int64_t K);
 
-// A left operand may be a complex matrix in its real form (zleft): A.p is the
+// Whether a product of this size is faster sliced than on the FP64 pipe.
+bool sliced_wanted(Context* c, int64_t M, int64_t N, int64_t K);
+
+// C (M x N, column-major) = alpha A B + beta C (beta 0 or 1).  `max_ctas` bounds
+// the persistent grids (0: one CTA per SM).  TMVG_UNSUPPORTED (with nothing
+// launched) where the workspace is not to be had.
+// The left operand may be a complex matrix in its real form (zleft): A.p is the
 // complex data, A.si and A.sj its strides in complex elements, and the operand
 // is the 2m x 2k real matrix of 2 x 2 blocks (re, -im; im, re).  With B and C
 // the interleaved parts as they lie in memory (2k x n and 2m x n) the product
 // is the complex one.
-
-// Slices the rows of A (M x K) and the columns of B (K x N) in one launch on
-// c->stream; either may be left out (rows == 0).
-tmvg_status sliced_split(Context* c, int64_t K, Mat<const double> A, const SlicedOperand& sa,
-                         Mat<const double> B, const SlicedOperand& sb, bool zleft = false);
-
-// C (M x N, column-major) = alpha A B + beta C (beta 0 or 1) from the slices;
-// A and B themselves are read only where a tile's range of magnitudes needs
-// the FP64 pipe.  `max_ctas` bounds the persistent grid (0: one per SM).
-tmvg_status sliced_apply(Context* c, int64_t M, int64_t N, int64_t K, double alpha, Mat<const double> A,
-                         const SlicedOperand& sa, Mat<const double> B, const SlicedOperand& sb, double beta,
-                         double* C, int64_t ldc, int max_ctas = 0, bool zleft = false);
-
-// Whether a product of this size is faster sliced than on the FP64 pipe.
-bool sliced_wanted(Context* c, int64_t M, int64_t N, int64_t K);
-
-// The whole product; TMVG_UNSUPPORTED (with nothing launched) where the
-// workspace or the tensor-map encoder is not to be had.
 tmvg_status sliced_gemm(Context* c, int64_t M, int64_t N, int64_t K, double alpha, Mat<const double> A,
                         Mat<const double> B, double beta, double* C, int64_t ldc, int max_ctas = 0,
                         bool zleft = false);
