@@ -82,7 +82,7 @@ tmvg_status tmvg_timing_enable(tmvg_handle h, int on);
 tmvg_status tmvg_timing_read(tmvg_handle h, int kclass, tmvg_kernel_timing* out);
 /* Use this cudaStream_t for all later calls (NULL = legacy default stream). */
 tmvg_status tmvg_set_stream(tmvg_handle h, void* cuda_stream);
-tmvg_status tmvg_synchronize(tmvg_handle h);
+tmvg_status tmvg_synchronize(tmvg_handle h);  /* and reports what asynchronous calls left */
 /* Text of the last error on this handle ("" if none). */
 const char* tmvg_last_error(tmvg_handle h);
 /* Number of kernels this handle has launched since creation. */
@@ -108,12 +108,12 @@ tmvg_status tmvg_probe_fp64_rate(tmvg_handle h, double* tflops);
 tmvg_status tmvg_test_set_wait(tmvg_handle h, uint32_t poll_limit, int32_t skip_blocks);
 /* The same for waits of one kernel's parts on one another.  TMVG_SILENT_PANEL:
  * one CTA of the next clustered panel of a factorisation sends no candidate.
- * The waits give up (real panels after about a second, complex ones after
- * tmvg_test_set_wait's poll_limit; 0: 2^22 polls, up to 4 us each), the results of
- * that call are not to be used, and the timeout is reported as that entry
- * point says.  The hook resets itself after that one launch; TMVG_SILENT_NONE
- * withdraws it. */
-enum { TMVG_SILENT_NONE = 0, TMVG_SILENT_PANEL = 1 };
+ * TMVG_SILENT_PRODUCT: one CTA of the next tensor-core product (an FP64 product
+ * from slices, or the FP32 factorisation's streamed update) loads no operands.
+ * The waits give up after about a second, the results of that call are not to be
+ * used, and the timeout is reported as that entry point says.  The hook resets
+ * itself after that one launch; TMVG_SILENT_NONE withdraws it. */
+enum { TMVG_SILENT_NONE = 0, TMVG_SILENT_PANEL = 1, TMVG_SILENT_PRODUCT = 2 };
 tmvg_status tmvg_test_set_silent(tmvg_handle h, int32_t what);
 
 /* ---- MultMM ----------------------------------------------------------
@@ -121,6 +121,9 @@ tmvg_status tmvg_test_set_silent(tmvg_handle h, int32_t what);
  * add = 1: C += alpha*A*B.  A and B may each be column-major (stepi == 1) or
  * row-major (stepj == 1): the CCC, CRC, RCC (and RRC) layouts; a row-major C
  * is computed as C^T = B^T A^T.  Operands must not overlap C.
+ * Asynchronous: should a bounded device-side wait run out, C is incomplete and
+ * the next call on the handle that synchronises (tmvg_synchronize, a solve, ...)
+ * returns TMVG_TIMEOUT; the _host form returns it itself.
  * Replaces: template void tmv::MultMM<add,double,double,double>
  *           (src/TMV_MultMM.cpp:405-477; declared
  *            include/tmv/TMV_MatrixArithFunc.h:55-58). */

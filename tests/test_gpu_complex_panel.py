@@ -70,7 +70,7 @@ def test_columns_of_ties(dev, n):
 
 def test_silent_peer_times_out_and_handle_recovers(dev):
     """One CTA of the first panel sends no candidate: the others give up after
-    2000 polls, the solve that follows reports TMVG_TIMEOUT, the interchanges
+    about a second, the solve that follows reports TMVG_TIMEOUT, the interchanges
     written are valid row numbers, and the next factorisation is right."""
     import torch
 
@@ -82,7 +82,6 @@ def test_silent_peer_times_out_and_handle_recovers(dev):
     b = rng.standard_normal((n, 2)) + 1j * rng.standard_normal((n, 2))
     A, B = linalg.colmajor(torch.from_numpy(a).to(dev)), linalg.colmajor(torch.from_numpy(b).to(dev))
     h = linalg.handle(dev.index or 0)
-    h.check(h.call("tmvg_test_set_wait", 2000, 0), "test_set_wait")
     h.check(h.call("tmvg_test_set_silent", 1), "test_set_silent")
     try:
         P = linalg.lu_decompose_z(A.t().clone().t())
@@ -90,7 +89,6 @@ def test_silent_peer_times_out_and_handle_recovers(dev):
         with pytest.raises(TmvgError) as ei:
             linalg.lu_ldiveq_z(A, torch.arange(n, device=dev), B.t().clone().t())
     finally:
-        h.check(h.call("tmvg_test_set_wait", 0, 0), "test_set_wait")
         h.check(h.call("tmvg_test_set_silent", 0), "test_set_silent")
     assert ei.value.status == 5  # TMVG_TIMEOUT
     assert ((p >= np.arange(n)) & (p < n)).all()

@@ -5,8 +5,10 @@
 
 namespace tmvg {
 
-// Polls of a bounded mbarrier wait before it reports a timeout.
-constexpr unsigned kTryWaitLimit = 1u << 22;
+// Polls of a bounded mbarrier wait before it reports a timeout: about a second (a
+// poll suspends the thread for up to 4 us).  A constant: as a kernel argument it
+// made the FP64 panels 1 to 2 % slower.
+constexpr unsigned kTryWaitLimit = 1u << 18;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p)
 {
@@ -33,10 +35,10 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes)
 }
 
 // Wait for the phase with the given parity to complete; false on timeout.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned limit = kTryWaitLimit)
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity)
 {
 #pragma unroll 1
-    for (unsigned spins = 0; spins < limit; ++spins) {
+    for (unsigned spins = 0; spins < kTryWaitLimit; ++spins) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -70,10 +72,10 @@ __device__ __forceinline__ void st_async16(uint32_t dst, const uint4& v, uint32_
 
 // Wait with cluster-scope acquire (pairs with release arrivals from other
 // CTAs of the cluster); false on timeout.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, unsigned limit = kTryWaitLimit)
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity)
 {
 #pragma unroll 1
-    for (unsigned spins = 0; spins < limit; ++spins) {
+    for (unsigned spins = 0; spins < kTryWaitLimit; ++spins) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"

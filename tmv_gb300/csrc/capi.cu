@@ -309,8 +309,7 @@ static tmvg_status lu_decompose_host(Context* c, int64_t n, T* A, int64_t sAi, i
     if (!st)
         st = check_cuda(c, cudaMemcpyAsync(P, dP.p, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, c->stream),
                         "lu: pivots d2h");
-    if (!st) st = check_cuda(c, cudaStreamSynchronize(c->stream), "lu sync");
-    return st;
+    return st ? st : collect_device_error(c, "lu");
 }
 
 // B := B / (P L U) (left) or B (P L U)^-1 (right) on host views; Div(dLU,
@@ -509,7 +508,7 @@ tmvg_status tmvg_set_stream(tmvg_handle h, void* stream)
 tmvg_status tmvg_synchronize(tmvg_handle h)
 {
     CTX_OR_BAIL(h);
-    return check_cuda(c, cudaStreamSynchronize(c->stream), "synchronize");
+    return collect_device_error(c, "synchronize");
 }
 
 const char* tmvg_last_error(tmvg_handle h)
@@ -536,7 +535,7 @@ tmvg_status tmvg_test_set_wait(tmvg_handle h, uint32_t poll_limit, int32_t skip_
 tmvg_status tmvg_test_set_silent(tmvg_handle h, int32_t what)
 {
     CTX_OR_BAIL(h);
-    if (what < TMVG_SILENT_NONE || what > TMVG_SILENT_PANEL)
+    if (what < TMVG_SILENT_NONE || what > TMVG_SILENT_PRODUCT)
         return set_error(c, TMVG_BAD_ARG, "test_set_silent: unknown part");
     c->test_silent = what;
     return TMVG_OK;
@@ -578,8 +577,7 @@ tmvg_status tmvg_multmm_f64_host(tmvg_handle h, int add, double alpha, int64_t m
                           Mat<const double>{dB.as<double>(), 1, k}, add ? 1.0 : 0.0,
                           Mat<double>{dC.as<double>(), 1, m});
     if (!st) st = d2h_matrix(c, C, dC.as<double>(), m, n, sCi, sCj, tmp.as<double>());
-    if (!st) st = check_cuda(c, cudaStreamSynchronize(c->stream), "multmm sync");
-    return st;
+    return st ? st : collect_device_error(c, "multmm");
 }
 
 tmvg_status tmvg_lu_decompose_f64(tmvg_handle h, int64_t n, double* A, int64_t lda, int64_t* P)
@@ -1186,7 +1184,7 @@ tmvg_status tmvg_lu_solve_bwd_f64(tmvg_handle h, int64_t n, const double* LU, in
                                       Mat<const double>{X, ldx, 1}, 0.0, Mat<double>{gA, 1, ldga});
         if (st) return st;
     }
-    return check_cuda(c, cudaStreamSynchronize(c->stream), "bwd sync");
+    return collect_device_error(c, "lu_solve_bwd");
 }
 
 tmvg_status tmvg_gemm_f32_tf32x3(tmvg_handle h, int64_t m, int64_t n, int64_t k, const float* A,

@@ -384,6 +384,7 @@ struct SlicedArgs {
     double* C;
     int64_t ldc;
     int64_t mt, nt;                  // tiles
+    int silent;                      // the CTA that loads nothing (failure-path test; -1: none)
     int* listed;                     // the tiles for the FP64 pipe: their count, then their numbers
 };
 
@@ -498,7 +499,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
     extern __shared__ uint8_t sl_smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(sl_smem_raw) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
-    __shared__ __align__(8) uint64_t full[kSlStages], empty[kSlStages], acc_full[GR], acc_empty[GR];
+    __shared__ __align__(8) uint64_t full[kSlStages], empty[kSlStages], acc_full[GR], acc_empty[GR], drained;
     __shared__ uint32_t s_tmem;
     __shared__ uint32_t s_ok[kMaxTilesPerCta / 32];
     __shared__ int s_open;
@@ -520,6 +521,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
             mbar_init(&acc_full[s], 1);
             mbar_init(&acc_empty[s], GW);
         }
+        mbar_init(&drained, 1);
         mbar_fence_init();
     }
     sl_fence_before();
@@ -567,7 +569,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
         if (lane == 0) {
             uint32_t it = 0;
             bool ok = true;
-            for (int i = 0; i < mine && ok; ++i) {
+            for (int i = 0; i < mine && ok && (int)blockIdx.x != g.silent; ++i) {
                 if (!sliced(i)) continue;
                 int64_t mi, ni;
                 sl_tile(g, blockIdx.x + (int64_t)i * gridDim.x, mi, ni);
@@ -629,9 +631,8 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant
             }
             if (!ok) atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
             // every product must be done before the tensor memory goes back
-            else
-                for (int s = 0; s < GR; ++s)
-                    if (ch[s] > 0) mbar_wait(&acc_full[s], (ch[s] - 1) & 1);
+            sl_commit(&drained);
+            mbar_wait(&drained, 0);
         }
     } else {
         // the warps of a tile: warp w of them drains lanes 32 (w % 4).. (rows of
@@ -916,7 +917,7 @@ static tmvg_status sliced_apply(Context* c, int64_t M, int64_t N, int64_t K, dou
     g.da = sa.digits, g.db = sb.digits, g.Kp = sa.Kp;
     g.C = C, g.ldc = ldc;
     g.mt = ceil_div(M, (int64_t)kSlM), g.nt = ceil_div(N, (int64_t)tn);
-    g.listed = listed;
+    g.listed = listed, g.silent = c->silenced(TMVG_SILENT_PRODUCT) ? 0 : -1;
     const unsigned grid = (unsigned)std::min<int64_t>(g.mt * g.nt, cap);
     auto kern = tn == 32 ? sliced_gemm_kernel<32> : sliced_gemm_kernel<kSlN>;
     const size_t smem = (size_t)kSlStages * (tn == 32 ? sl_stage_bytes<32>() : sl_stage_bytes<kSlN>()) + 1024;

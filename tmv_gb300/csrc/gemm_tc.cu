@@ -287,7 +287,7 @@ template <int KCH>
 __global__ void __launch_bounds__(kStThreads, 1)
 tf32x3_stream_kernel(const __grid_constant__ CUtensorMap mAhi, const __grid_constant__ CUtensorMap mAlo,
                      const __grid_constant__ CUtensorMap mBhi, const __grid_constant__ CUtensorMap mBlo,
-                     const __grid_constant__ CUtensorMap mC, int M, int N, int* err)
+                     const __grid_constant__ CUtensorMap mC, int M, int N, int* err, int silent)
 {
     extern __shared__ uint8_t st_smem_raw[];
     uint8_t* Bs = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(st_smem_raw) + 1023) &
@@ -295,7 +295,7 @@ tf32x3_stream_kernel(const __grid_constant__ CUtensorMap mAhi, const __grid_cons
     uint8_t* As = Bs + KCH * 2 * kStOp;                                       // [2][hi, lo]
     uint8_t* Cs = As + 2 * 2 * kStOp;                                         // [2][kStCBufs][32][128]
     __shared__ __align__(8) uint64_t full[2], empty[2], bfull, bempty, tfull[2], tempty[2], cfull[2][kStCBufs],
-        cempty[2][kStCBufs];
+        cempty[2][kStCBufs], drained;
     __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -314,6 +314,7 @@ tf32x3_stream_kernel(const __grid_constant__ CUtensorMap mAhi, const __grid_cons
         }
         mbar_init(&bfull, 1);
         mbar_init(&bempty, 1);
+        mbar_init(&drained, 1);
         for (int h = 0; h < 2; ++h)
             for (int q = 0; q < kStCBufs; ++q) {
                 mbar_init(&cfull[h][q], 1);
@@ -340,7 +341,7 @@ tf32x3_stream_kernel(const __grid_constant__ CUtensorMap mAhi, const __grid_cons
         if (lane == 0) {
             uint32_t it = 0, cols = 0;
             bool ok = true;
-            for (int i = 0, tr = r0, tc = c0; i < mine && ok; ++i, ++tr) {
+            for (int i = 0, tr = r0, tc = c0; i < mine && ok && (int)blockIdx.x != silent; ++i, ++tr) {
                 if (tr == mt) tr = 0, ++tc;
                 if (i == 0 || tr == 0) {
                     if (cols > 0) ok = mbar_wait(&bempty, (cols - 1) & 1);
@@ -401,7 +402,8 @@ tf32x3_stream_kernel(const __grid_constant__ CUtensorMap mAhi, const __grid_cons
             }
             if (!ok) atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
             // every product must be done before the tensor memory goes back
-            else if (mine > 0) mbar_wait(&tfull[(mine - 1) & 1], ((mine - 1) >> 1) & 1);
+            umma_commit(&drained);
+            mbar_wait(&drained, 0);
         }
     } else if (warp == 2) {
         if (lane == 0) {
@@ -591,7 +593,8 @@ static tmvg_status launch_stream(Context* c, const CUtensorMap* maps, int64_t m,
     const int64_t cap = max_ctas > 0 ? max_ctas : c->num_sms;
     cudaFuncSetAttribute(tf32x3_stream_kernel<KCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     tf32x3_stream_kernel<KCH><<<(unsigned)std::min(tiles, cap), kStThreads, smem, c->stream>>>(
-        maps[0], maps[1], maps[2], maps[3], maps[4], (int)m, (int)n, c->dflags);
+        maps[0], maps[1], maps[2], maps[3], maps[4], (int)m, (int)n, c->dflags,
+        c->silenced(TMVG_SILENT_PRODUCT) ? 0 : -1);
     ++c->launches;
     return check_cuda(c, cudaGetLastError(), "tf32x3 stream launch");
 }

@@ -591,11 +591,6 @@ __device__ __forceinline__ void reg2_update(T (&x)[NB], T lx, bool ux, T (&y)[NB
     }
 }
 
-// Polls of the panels' waits for their cluster's messages: about a second (a
-// poll suspends the thread for up to 4 us).  A constant: as a kernel argument
-// it made the FP64 panels 1 to 2 % slower.
-constexpr unsigned kPanelPolls = 1u << 18;
-
 template <typename T, int NB>
 __global__ void __launch_bounds__(kReg2Threads, 1)
 lu_panel_cluster_reg2_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int nb,
@@ -718,7 +713,7 @@ lu_panel_cluster_reg2_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t 
                         mbar_arrive_remote_release(cluster_addr(&mbar[par], lane));
                     }
                     // 3. wait for every CTA's record (bounded), reduce, pull rows
-                    const bool got = __all_sync(0xffffffffu, mbar_wait_cluster(&mbar[par], (uint32_t)((jj >> 1) & 1), kPanelPolls));
+                    const bool got = __all_sync(0xffffffffu, mbar_wait_cluster(&mbar[par], (uint32_t)((jj >> 1) & 1)));
                     if (!got) {
                         if (lane == 0) {
                             s_abort = 1;
@@ -1192,7 +1187,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             }
             if (warp == 0 && G > 1) {
                 // 4. every CTA's message (bounded wait), reduced here
-                const bool got = __all_sync(0xffffffffu, mbar_wait(&mbar[par], (uint32_t)((j >> 1) & 1), kPanelPolls));
+                const bool got = __all_sync(0xffffffffu, mbar_wait(&mbar[par], (uint32_t)((j >> 1) & 1)));
                 if (!got) {
                     if (lane == 0) {
                         s_abort = 1;
@@ -1207,7 +1202,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
             }
             if (kLongRcp && warp == kRcpWarp) {
                 // every candidate's reciprocal, beside warp 0's decision
-                const bool got = G == 1 || __all_sync(0xffffffffu, mbar_wait(&mbar[par], (uint32_t)((j >> 1) & 1), kPanelPolls));
+                const bool got = G == 1 || __all_sync(0xffffffffu, mbar_wait(&mbar[par], (uint32_t)((j >> 1) & 1)));
                 if (got && lane < (G > 1 ? G : nwarp)) {
                     const LeafMsg<T>& cm = G > 1 ? msg[par][lane] : wmsg[lane];
                     s_rcp[lane] = recip_rn(cm.head.pos != INT_MAX ? cm.leaf[0] : T(1));
@@ -1261,7 +1256,7 @@ lu_panel_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t n, int64_t k, int n
                 send_step = -1;
             }
             if (G > 1) {
-                if (!mbar_wait(&mbar_leaf, leaf_uses & 1u, kPanelPolls)) {
+                if (!mbar_wait(&mbar_leaf, leaf_uses & 1u)) {
                     if (tid == 0) atomicCAS(err, (int)kDevOk, (int)kDevTimeout);
                     s_abort = 1;  // every thread of the CTA reaches this
                 }

@@ -344,7 +344,7 @@ __device__ __forceinline__ double2 zfms(double2 a, double2 l, double2 u)
 template <int KB>
 __global__ void __launch_bounds__(kZPanelThreads)
 zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k, int kb, int64_t* __restrict__ P,
-                      int rpc, int* err, unsigned poll_limit, int silent)
+                      int rpc, int* err, int silent)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -386,7 +386,7 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
         __syncthreads();
         if (warp == 0) {
             if (lane < kZPanelCtas) mbar_arrive_remote_release(cluster_addr(&sh.met, lane));
-            const bool got = __all_sync(0xffffffffu, mbar_wait_cluster(&sh.met, met, poll_limit));
+            const bool got = __all_sync(0xffffffffu, mbar_wait_cluster(&sh.met, met));
             if (!got && lane == 0) give_up();
         }
         met ^= 1u;
@@ -483,7 +483,7 @@ zlu_panel_smem_kernel(int64_t n, double2* __restrict__ A, int64_t lda, int64_t k
             }
         }
         if (warp == 0) {
-            const bool got = __all_sync(0xffffffffu, mbar_wait_cluster(&sh.mbar[par], (uint32_t)((jj >> 1) & 1), poll_limit));
+            const bool got = __all_sync(0xffffffffu, mbar_wait_cluster(&sh.mbar[par], (uint32_t)((jj >> 1) & 1)));
             if (!got) {
                 if (lane == 0) give_up();
             } else {
@@ -912,7 +912,7 @@ static tmvg_status zlu_factor_blocked(Context* c, int64_t n, double2* A, int64_t
         ++c->launches;
         const int silent = c->silenced(TMVG_SILENT_PANEL) ? kZPanelCtas - 1 : -1;
         return check_cuda(c, cudaLaunchKernelEx(&cfg, zlu_panel_smem_kernel<KB>, n, A, lda, k, kb, P, rpc, c->dflags,
-                                                c->poll_limit ? c->poll_limit : kTryWaitLimit, silent),
+                                                silent),
                           "lu_z: panel launch");
     };
     auto swap = [&](int64_t c0, int64_t c1, int64_t k, int kb) {
