@@ -240,7 +240,9 @@ __device__ __forceinline__ T real_form(const T* __restrict__ z, int64_t si, int6
 
 // A published entry of the solution and the launch's epoch in one word that
 // is stored and loaded whole, so a consumer polls the value itself: no flag,
-// no fence, one L2 round trip.
+// no fence, one L2 round trip.  FP64: value and epoch, 8 bytes each.  FP32: both
+// in the second 8 bytes, the epoch above the value: neither kind ever reads as
+// the other's (an epoch is at least 1 and below 2^32), whatever the values.
 __device__ __forceinline__ void pub_store(void* words, int64_t at, double v, unsigned epoch)
 {
     asm volatile(
@@ -262,7 +264,7 @@ __device__ __forceinline__ bool pub_load(const void* words, int64_t at, unsigned
 }
 __device__ __forceinline__ void pub_store(void* words, int64_t at, float v, unsigned epoch)
 {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(static_cast<char*>(words) + 16 * at),
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(static_cast<char*>(words) + 16 * at + 8),
                  "l"(((unsigned long long)epoch << 32) | __float_as_uint(v))
                  : "memory");
 }
@@ -271,7 +273,7 @@ __device__ __forceinline__ bool pub_load(const void* words, int64_t at, unsigned
     unsigned long long x;
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];"
                  : "=l"(x)
-                 : "l"(static_cast<const char*>(words) + 16 * at)
+                 : "l"(static_cast<const char*>(words) + 16 * at + 8)
                  : "memory");
     v = __uint_as_float((unsigned)x);
     return (unsigned)(x >> 32) == epoch;
