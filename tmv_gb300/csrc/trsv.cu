@@ -153,16 +153,26 @@ tmvg_status lu_inv64(Context* c, int64_t n, const double* LU, int64_t ld, double
     return check_cuda(c, cudaGetLastError(), "inverse blocks");
 }
 
+__device__ __forceinline__ bool finite(double v) { return ((unsigned)__double2hiint(v) & 0x7ff00000u) != 0x7ff00000u; }
+__device__ __forceinline__ bool finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+
 // Y (w x cols, leading dimension ld) := D^-1 Y for one diagonal block from its
 // inverse: 64 rows x 8 columns per CTA, two entries per thread, corrected once,
 // y + D^-1 (b - D y) with y = D^-1 b, so that an ill-conditioned block costs no
 // accuracy (without it the residual of the inverse of a 65 x 65 matrix of
-// condition 1e10 grew 7-fold).  t is the block in the matrix: upper, or unit
-// lower; null: no correction.  Bound: the FP64 pipe.
+// condition 1e10 grew 7-fold, and that of a unit triangle with multipliers uniform in
+// (-1, 1) 5 to 20-fold).  t is the block in the matrix: upper, or unit lower.
+// Not `always`: only where an entry of the inverse exceeds kInvLarge.  Below it the
+// plain product's componentwise residual is that of a substitution (one block,
+// multipliers uniform in +-0.4, +-0.6, +-0.8, +-1: largest entry 2, 19, 180, 3100,
+// residual 0.97, 1.3, 2.0, 2.4 times the substitution's; unit lower blocks of random,
+// covariance and kernel matrices: largest entry 1 to 3.5, residual 1.0 to 1.1 times).
+// Bound: the FP64 pipe.
 constexpr int kApplyCols = 8;
+constexpr int kInvLarge = 0x40100000;  // 4.0 (upper half)
 __global__ void __launch_bounds__(256)
 apply_inv64_kernel(int w, int64_t cols, const double* __restrict__ dinv, bool upper, const double* __restrict__ t,
-                   int64_t ldt, double* Y, int64_t ld)
+                   int64_t ldt, double* Y, int64_t ld, bool always)
 {
     __shared__ double D[kTrsvBlock][kTrsvBlock + 1];
     __shared__ double y[kTrsvBlock][kApplyCols];
@@ -170,7 +180,9 @@ apply_inv64_kernel(int w, int64_t cols, const double* __restrict__ dinv, bool up
     const int64_t c0 = (int64_t)blockIdx.x * kApplyCols;
     for (int q = tid; q < kTrsvBlock * kTrsvBlock; q += 256) {
         const int rr = q / kTrsvBlock, cc = q % kTrsvBlock;
-        D[rr][cc] = rr < w && cc < w ? dinv[q] : 0.0;
+        const double d = rr < w && cc < w ? dinv[q] : 0.0;
+        always |= (__double2hiint(d) & 0x7fffffff) > kInvLarge;
+        D[rr][cc] = d;
     }
     double b[2], v[2];
 #pragma unroll
@@ -178,7 +190,7 @@ apply_inv64_kernel(int w, int64_t cols, const double* __restrict__ dinv, bool up
         b[e] = i < w && c0 + g + 4 * e < cols ? Y[i + (c0 + g + 4 * e) * ld] : 0.0;
         y[i][g + 4 * e] = b[e];
     }
-    __syncthreads();
+    const bool correct = __syncthreads_or(always);
     // entries beyond the diagonal take no part, whatever y holds there
     const int k0 = upper ? i & ~31 : 0, k1 = upper ? kTrsvBlock : (i | 31) + 1;
     auto times_inverse = [&] {
@@ -198,7 +210,7 @@ apply_inv64_kernel(int w, int64_t cols, const double* __restrict__ dinv, bool up
         __syncthreads();
     };
     times_inverse();
-    if (t) {
+    if (correct) {
         const double first[2] = {v[0], v[1]};
         share(first);
         double r[2] = {0.0, 0.0};
@@ -222,10 +234,10 @@ apply_inv64_kernel(int w, int64_t cols, const double* __restrict__ dinv, bool up
 }
 
 tmvg_status apply_inv64(Context* c, int w, int64_t cols, const double* dinv, bool upper, const double* t, int64_t ldt,
-                        double* Y, int64_t ld)
+                        double* Y, int64_t ld, bool always)
 {
     apply_inv64_kernel<<<(unsigned)ceil_div(cols, (int64_t)kApplyCols), 256, 0, c->stream>>>(w, cols, dinv, upper, t,
-                                                                                           ldt, Y, ld);
+                                                                                           ldt, Y, ld, always);
     ++c->launches;
     return check_cuda(c, cudaGetLastError(), "inverse block product");
 }
@@ -278,9 +290,6 @@ __device__ __forceinline__ bool pub_load(const void* words, int64_t at, unsigned
     v = __uint_as_float((unsigned)x);
     return (unsigned)(x >> 32) == epoch;
 }
-
-__device__ __forceinline__ bool finite(double v) { return ((unsigned)__double2hiint(v) & 0x7ff00000u) != 0x7ff00000u; }
-__device__ __forceinline__ bool finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
 
 // One CTA per (row block, group of NR right-hand sides); tickets hand the
 // pairs out block by block (all groups of block b before block b+1), and a

@@ -25,10 +25,11 @@ tmvg_status ztrsm_sync_free(Context* c, int64_t n, const double* z, int64_t tsi,
 
 // For the inverse: the inverted 64-row diagonal blocks of a packed LU factor
 // (row-major 64 x 64 each, in the context's buffer), and Y := D^-1 Y with one
-// of them (w rows; t: the block itself, upper or unit lower).
+// of them (w rows; t: the block itself, upper or unit lower; always: corrected
+// also where the block's inverse has no large entry).
 tmvg_status lu_inv64(Context* c, int64_t n, const double* LU, int64_t ld, double** dl, double** du);
 tmvg_status apply_inv64(Context* c, int w, int64_t cols, const double* dinv, bool upper, const double* t, int64_t ldt,
-                        double* Y, int64_t ld);
+                        double* Y, int64_t ld, bool always);
 
 // Repeated one-column solves with one triangle: invert its 128 x 128
 // diagonal blocks once (dinv: ceil(n/128)*128*128 elements, singular:
