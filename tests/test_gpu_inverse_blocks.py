@@ -1,5 +1,5 @@
 """The inverse from its factors where the 64-row diagonal blocks are hard: unit
-lower blocks with large multipliers."""
+lower blocks with large multipliers, and blocks whose own inverse is not finite."""
 import ctypes as C
 
 import numpy as np
@@ -50,3 +50,42 @@ def test_lower_blocks_with_large_multipliers(dev, n):
         return float((r / np.where(size > 0, size, 1.0)).max())
 
     assert residual(_inverse(dev, low)[:, cols]) <= 3 * residual(_substitute(low, cols))
+
+
+# (rows and columns of a 64-row block, and of two blocks)
+@pytest.mark.parametrize("n,i,j", [(40, 3, 9), (64, 0, 63), (150, 70, 100), (150, 130, 149), (700, 600, 630)])
+@pytest.mark.parametrize("size", [1e200, np.inf])
+def test_block_whose_inverse_overflows(dev, n, i, j, size):
+    """U = I but for two diagonal entries 1e-200 and U(i, j): x(i, j) overflows, all
+    other entries are finite (or, under an infinite U(i, j), what 0 times it
+    leaves), as the substitution finds them."""
+    up = np.eye(n)
+    up[i, i] = up[j, j] = 1e-200
+    up[i, j] = size
+    want = np.eye(n)
+    b0 = j // 64 * 64
+    with np.errstate(all="ignore"):
+        for k in reversed(range(n)):
+            want[k] = want[k] * (1.0 / up[k, k])
+            want[:k] -= up[:k, k:k + 1] * want[k]
+    got = _inverse(dev, up)
+    assert b0 <= i, "both in one block"
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    fin = np.isfinite(want)
+    assert np.array_equal(got[~fin & ~np.isnan(want)], want[~fin & ~np.isnan(want)])
+    assert (np.abs(got - want)[fin] <= 2.0 ** -50 * np.abs(want)[fin]).all()
+
+
+def test_lower_block_whose_inverse_overflows(dev):
+    """Multipliers of 1e160 twice in a row: one entry of L^-1 overflows, and 0 times
+    it fills its column, below by L and above by U = I; every other column is as the
+    substitution has it."""
+    n = 100
+    low = np.eye(n)
+    low[71, 70] = low[72, 71] = 1e160
+    with np.errstate(all="ignore"):
+        want = _substitute(low, np.arange(n))
+        assert np.isinf(want).sum() == 1
+        for k in reversed(range(n)):
+            want[:k] -= 0.0 * want[k]
+    assert np.array_equal(_inverse(dev, low), want, equal_nan=True)

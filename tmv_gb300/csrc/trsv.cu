@@ -167,7 +167,8 @@ __device__ __forceinline__ bool finite(float v) { return (__float_as_uint(v) & 0
 // multipliers uniform in +-0.4, +-0.6, +-0.8, +-1: largest entry 2, 19, 180, 3100,
 // residual 0.97, 1.3, 2.0, 2.4 times the substitution's; unit lower blocks of random,
 // covariance and kernel matrices: largest entry 1 to 3.5, residual 1.0 to 1.1 times).
-// Bound: the FP64 pipe.
+// Where the result is not finite the CTA's columns are substituted: D^-1 may
+// overflow where the solution does not.  Bound: the FP64 pipe.
 constexpr int kApplyCols = 8;
 constexpr int kInvLarge = 0x40100000;  // 4.0 (upper half)
 __global__ void __launch_bounds__(256)
@@ -227,6 +228,25 @@ apply_inv64_kernel(int w, int64_t cols, const double* __restrict__ dinv, bool up
         times_inverse();
 #pragma unroll
         for (int e = 0; e < 2; ++e) v[e] += first[e];
+    }
+    if (__syncthreads_or(!finite(v[0]) || !finite(v[1]))) {
+        for (int q = tid; q < kTrsvBlock * kTrsvBlock; q += 256) {
+            const int rr = q % kTrsvBlock, cc = q / kTrsvBlock;
+            D[rr][cc] = rr < w && cc < w ? t[rr + cc * ldt] : 0.0;
+        }
+        share(b);
+        for (int s = 0; s < w; ++s) {
+            const int k = upper ? w - 1 - s : s;
+            if (upper && tid < kApplyCols) y[k][tid] *= 1.0 / D[k][k];
+            __syncthreads();
+            if (i < w && (upper ? i < k : i > k)) {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) y[i][g + 4 * e] -= D[i][k] * y[k][g + 4 * e];
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) v[e] = y[i][g + 4 * e];
     }
 #pragma unroll
     for (int e = 0; e < 2; ++e)
