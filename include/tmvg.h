@@ -115,6 +115,16 @@ tmvg_status tmvg_test_set_wait(tmvg_handle h, uint32_t poll_limit, int32_t skip_
  * itself after that one launch; TMVG_SILENT_NONE withdraws it. */
 enum { TMVG_SILENT_NONE = 0, TMVG_SILENT_PANEL = 1, TMVG_SILENT_PRODUCT = 2 };
 tmvg_status tmvg_test_set_silent(tmvg_handle h, int32_t what);
+/* Test hook: until withdrawn (0) the handle's buffers named here cannot grow, as if
+ * the device's memory were used up. */
+enum {
+    TMVG_BUFFER_WORK = 1,   /* operands and permutations of a call */
+    TMVG_BUFFER_PANEL = 2,  /* scratch panels and operand splits of a factorisation */
+    TMVG_BUFFER_INV = 4,    /* inverted diagonal blocks of a solve */
+    TMVG_BUFFER_WORDS = 8,  /* published entries of a solve */
+    TMVG_BUFFER_POOL = 16   /* slices of a product */
+};
+tmvg_status tmvg_test_refuse_memory(tmvg_handle h, uint32_t buffers);
 
 /* ---- MultMM ----------------------------------------------------------
  * C (+)= alpha * A * B;  A m x k, B k x n, C m x n.  add = 0: C = alpha*A*B,

@@ -62,6 +62,7 @@ _SIGS = {
     "tmvg_probe_fp64_rate": (C.c_int, [vp, C.POINTER(dbl)]),
     "tmvg_test_set_wait": (C.c_int, [vp, C.c_uint32, C.c_int32]),
     "tmvg_test_set_silent": (C.c_int, [vp, C.c_int32]),
+    "tmvg_test_refuse_memory": (C.c_int, [vp, C.c_uint32]),
     "tmvg_timing_enable": (C.c_int, [vp, C.c_int]),
     "tmvg_timing_read": (C.c_int, [vp, C.c_int, C.POINTER(KernelTiming)]),
     "tmvg_multmm_f64": (C.c_int, [vp, C.c_int, dbl, i64, i64, i64, vp, i64, i64, vp, i64, i64,

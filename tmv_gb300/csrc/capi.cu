@@ -32,7 +32,7 @@ tmvg_status check_cuda(Context* c, cudaError_t e, const char* what)
     return set_error(c, TMVG_CUDA_ERROR, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-static void* grow(Context* c, void*& buf, size_t& have, size_t bytes)
+static void* grow(Context* c, void*& buf, size_t& have, size_t bytes, unsigned which = 0)
 {
     if (bytes <= have) return buf;
     if (buf) {
@@ -42,7 +42,7 @@ static void* grow(Context* c, void*& buf, size_t& have, size_t bytes)
         have = 0;
     }
     size_t want = bytes + bytes / 4 + 4096;
-    if (cudaMalloc(&buf, want) != cudaSuccess) {
+    if ((c->refuse & which) != 0 || cudaMalloc(&buf, want) != cudaSuccess) {
         cudaGetLastError();
         buf = nullptr;
         set_error(c, TMVG_OOM, "workspace allocation failed");
@@ -52,15 +52,18 @@ static void* grow(Context* c, void*& buf, size_t& have, size_t bytes)
     return buf;
 }
 
-void* workspace(Context* c, size_t bytes) { return grow(c, c->work, c->work_bytes, bytes); }
+void* workspace(Context* c, size_t bytes) { return grow(c, c->work, c->work_bytes, bytes, TMVG_BUFFER_WORK); }
 void* workspace2(Context* c, size_t bytes) { return grow(c, c->work2, c->work2_bytes, bytes); }
-void* workspace3(Context* c, size_t bytes) { return grow(c, c->work3, c->work3_bytes, bytes); }
+void* workspace3(Context* c, size_t bytes) { return grow(c, c->work3, c->work3_bytes, bytes, TMVG_BUFFER_PANEL); }
 void* perm_lists_buffer(Context* c, size_t bytes) { return grow(c, c->perm_lists, c->perm_lists_bytes, bytes); }
-void* trsv_dinv_buffer(Context* c, size_t bytes) { return grow(c, c->trsv_dinv, c->trsv_dinv_bytes, bytes); }
+void* trsv_dinv_buffer(Context* c, size_t bytes)
+{
+    return grow(c, c->trsv_dinv, c->trsv_dinv_bytes, bytes, TMVG_BUFFER_INV);
+}
 void* trsv_words_buffer(Context* c, size_t bytes)
 {
     const size_t had = c->trsv_words_bytes;
-    void* p = grow(c, c->trsv_words, c->trsv_words_bytes, bytes);
+    void* p = grow(c, c->trsv_words, c->trsv_words_bytes, bytes, TMVG_BUFFER_WORDS);
     // no word may hold an epoch before it is published
     if (p && c->trsv_words_bytes != had && cudaMemsetAsync(p, 0, c->trsv_words_bytes, c->stream) != cudaSuccess) {
         cudaGetLastError();
@@ -538,6 +541,13 @@ tmvg_status tmvg_test_set_silent(tmvg_handle h, int32_t what)
     if (what < TMVG_SILENT_NONE || what > TMVG_SILENT_PRODUCT)
         return set_error(c, TMVG_BAD_ARG, "test_set_silent: unknown part");
     c->test_silent = what;
+    return TMVG_OK;
+}
+
+tmvg_status tmvg_test_refuse_memory(tmvg_handle h, uint32_t buffers)
+{
+    CTX_OR_BAIL(h);
+    c->refuse = buffers;
     return TMVG_OK;
 }
 

@@ -129,6 +129,8 @@ struct Context {
     // flags are never published (reset after one launch).
     unsigned poll_limit = 0;
     int test_skip_blocks = 0;
+    // tmvg_test_refuse_memory: the buffers that cannot grow (TMVG_BUFFER_*).
+    unsigned refuse = 0;
     // tmvg_test_set_silent: the part that stays silent in the next launch that
     // has it (TMVG_SILENT_*).
     int test_silent = 0;

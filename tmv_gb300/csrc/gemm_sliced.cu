@@ -962,6 +962,7 @@ void* scratch_alloc(Context* c, size_t bytes, cudaStream_t s)
         cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
     }
     void* p = nullptr;
+    if (c->refuse & TMVG_BUFFER_POOL) return nullptr;
     if (cudaMallocFromPoolAsync(&p, bytes, c->pool, s) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;

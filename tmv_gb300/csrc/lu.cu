@@ -2476,7 +2476,8 @@ tmvg_status lu_factor(Context* c, int64_t n, T* A, int64_t lda, int64_t* P)
             const int nparts = (tc ? 6 : 0) + (reg ? 2 : 0);
             if (nparts > 0) {
                 unsigned char* w3 = (unsigned char*)workspace3(c, nparts * part);
-                if (!w3) return TMVG_OOM;
+                // (an FP64 step can do without its scratch panels)
+                if (!w3 && std::is_same<T, float>::value) return TMVG_OOM;
                 if (tc) {
                     for (int q = 0; q < 2; ++q) {
                         arena[q].Bhi = (float*)w3;
@@ -2486,7 +2487,7 @@ tmvg_status lu_factor(Context* c, int64_t n, T* A, int64_t lda, int64_t* P)
                     }
                     tc_any = true;
                 }
-                if (reg) {
+                if (reg && w3) {
                     Sbuf[0] = (T*)(w3 + (nparts - 2) * part);
                     Sbuf[1] = (T*)(w3 + (nparts - 1) * part);
                 }
@@ -2626,14 +2627,18 @@ tmvg_status lu_factor(Context* c, int64_t n, T* A, int64_t lda, int64_t* P)
 
 // Triangular solve of the pivoted right-hand sides: the single-launch
 // sync-free kernel (one CTA per 64-row block and group of right-hand sides)
-// up to 256 columns, the blocked product-based solve for more.
+// up to 256 columns, the blocked product-based solve for more and where the
+// kernel's buffers are not to be had.
 template <typename T>
 static tmvg_status tri_any(Context* c, int64_t n, const T* tri, int64_t tsi, int64_t tsj,
                            bool upper, bool unit, int64_t nrhs, T* B, int64_t bsi, int64_t bsj,
                            bool skip_zero)
 {
     if (nrhs <= 256 && ceil_div(n, (int64_t)64) * ceil_div(nrhs, (int64_t)4) <= kTrsvFlagCap)
-        return trsm_sync_free<T>(c, n, tri, tsi, tsj, upper, unit, nrhs, B, bsi, bsj, skip_zero);
+    {
+        const tmvg_status st = trsm_sync_free<T>(c, n, tri, tsi, tsj, upper, unit, nrhs, B, bsi, bsj, skip_zero);
+        if (st != TMVG_OOM) return st;
+    }
     return tri_solve<T>(c, n, tri, tsi, tsj, upper, unit, nrhs, B, bsi, bsj, skip_zero);
 }
 
@@ -2735,6 +2740,23 @@ __global__ void scatter_cols_kernel(int64_t n, const int* __restrict__ perm, con
     }
 }
 
+// Y := U^-1 L^-1 Y for Y = I, the diagonal blocks by substitution.
+template <typename T>
+static tmvg_status inverse_by_substitution(Context* c, int64_t n, const T* LU, int64_t lda, T* Y)
+{
+    tmvg_status st = TMVG_OK;
+    for (int64_t kb = 0; kb < n && !st; kb += kTriBlock) {
+        const int w = (int)std::min<int64_t>(kTriBlock, n - kb);
+        const int64_t cols = kb + w;
+        st = launch_tri_diag<T>(c, w, LU + kb + kb * lda, 1, lda, false, true, cols, Y + kb, 1, n, false);
+        if (!st && kb + w < n)
+            st = gemm<T>(c, n - kb - w, cols, w, T(-1), Mat<const T>{LU + (kb + w) + kb * lda, 1, lda},
+                         Mat<const T>{Y + kb, 1, n}, T(1), Mat<T>{Y + kb + w, 1, n});
+    }
+    if (!st) st = tri_solve<T>(c, n, LU, 1, lda, true, false, n, Y, 1, n, false);
+    return st;
+}
+
 // Y = U^-1 L^-1 into the dense n x n buffer Y (leading dimension n).
 // L^-1 is the unit-lower solve of the identity: column block c of L^-1 is
 // zero above row block c, so block step kb solves and updates only the
@@ -2746,7 +2768,8 @@ __global__ void scatter_cols_kernel(int64_t n, const int* __restrict__ perm, con
 // substitution took 80 us of every step.  The block column of the identity
 // stays on the FP64 pipe: it is triangular, and its tiles would not be sliced.
 // Pairs of upper blocks share one update of K = 128, whose time is that of
-// K = 64 (n = 1501: inverse 8.1 -> 2.7 ms).
+// K = 64 (n = 1501: inverse 8.1 -> 2.7 ms).  FP32, and FP64 without memory for the
+// blocks: by substitution.
 template <typename T>
 static tmvg_status inverse_unpermuted(Context* c, int64_t n, const T* LU, int64_t lda, T* Y)
 {
@@ -2758,6 +2781,7 @@ static tmvg_status inverse_unpermuted(Context* c, int64_t n, const T* LU, int64_
         constexpr int64_t W = kTriBlock;
         double *dl = nullptr, *du = nullptr;
         if (!st) st = lu_inv64(c, n, LU, lda, &dl, &du);
+        if (st == TMVG_OOM) return inverse_by_substitution<T>(c, n, LU, lda, Y);
         auto below = [&](int64_t kb, int w, int64_t c0, int64_t nc, bool fma_pipe) {
             return gemm<T>(c, n - kb - w, nc, w, T(-1), Mat<const T>{LU + (kb + w) + kb * lda, 1, lda},
                            Mat<const T>{Y + kb + c0 * n, 1, n}, T(1), Mat<T>{Y + kb + w + c0 * n, 1, n}, fma_pipe);
@@ -2790,16 +2814,7 @@ static tmvg_status inverse_unpermuted(Context* c, int64_t n, const T* LU, int64_
         }
         return st;
     } else {
-        for (int64_t kb = 0; kb < n && !st; kb += kTriBlock) {
-            const int w = (int)std::min<int64_t>(kTriBlock, n - kb);
-            const int64_t cols = kb + w;
-            st = launch_tri_diag<T>(c, w, LU + kb + kb * lda, 1, lda, false, true, cols, Y + kb, 1, n, false);
-            if (!st && kb + w < n)
-                st = gemm<T>(c, n - kb - w, cols, w, T(-1), Mat<const T>{LU + (kb + w) + kb * lda, 1, lda},
-                             Mat<const T>{Y + kb, 1, n}, T(1), Mat<T>{Y + kb + w, 1, n});
-        }
-        if (!st) st = tri_solve<T>(c, n, LU, 1, lda, true, false, n, Y, 1, n, false);
-        return st;
+        return st ? st : inverse_by_substitution<T>(c, n, LU, lda, Y);
     }
 }
 

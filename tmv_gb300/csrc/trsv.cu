@@ -620,12 +620,14 @@ tmvg_status trsm_sync_free(Context* c, int64_t n, const T* tri, int64_t tsi, int
     int* dsing = nullptr;
     if (nblk > 1 || !few) {
         tmvg_status st = inverse_blocks_buffer(c, nblk, &dinv, &dsing);
-        if (st) return st;
-        tri_inv64_kernel<T><<<(unsigned)nblk * kInvCtas, kInvThreads, 0, c->stream>>>(n, tri, tsi, tsj, unit, dinv,
-                                                                                   dsing);
-        ++c->launches;
-        st = check_cuda(c, cudaGetLastError(), "trsv inverse blocks");
-        if (st) return st;
+        if (st && !few) return st;
+        if (!st) {  // (few columns can do without)
+            tri_inv64_kernel<T><<<(unsigned)nblk * kInvCtas, kInvThreads, 0, c->stream>>>(n, tri, tsi, tsj, unit,
+                                                                                       dinv, dsing);
+            ++c->launches;
+            st = check_cuda(c, cudaGetLastError(), "trsv inverse blocks");
+            if (st) return st;
+        }
     }
     return launch_trsm<T, false>(c, n, tri, tsi, tsj, T(1), unit, nrhs, B, bsi, bsj, skip_zero, dinv, dsing, few);
 }

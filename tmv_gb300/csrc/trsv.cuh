@@ -11,6 +11,7 @@ constexpr int64_t kTrsvFlagCap = 65536;
 // B := T^-1 B for the lower (upper = false) or upper triangle of `tri`
 // (strides tsi, tsj; unit diagonal not read when unit), B n x nrhs with
 // strides; skip_zero as in tri_solve().  Best for nrhs <= 8.
+// TMVG_OOM (with B as it was) where its buffers are not to be had.
 template <typename T>
 tmvg_status trsm_sync_free(Context* c, int64_t n, const T* tri, int64_t tsi, int64_t tsj,
                            bool upper, bool unit, int64_t nrhs, T* B, int64_t bsi, int64_t bsj,
@@ -19,7 +20,8 @@ tmvg_status trsm_sync_free(Context* c, int64_t n, const T* tri, int64_t tsi, int
 // X := T^-1 X for the lower or upper triangle T(i, j) = z[i tsi + j tsj] of
 // complex entries (unit diagonal not read when unit; recip: 1 / T(j,j), 0 where
 // that is zero), X n x nrhs contiguous.  Records kDevRetry in the device error
-// word where the result is not finite or a T(j,j) is zero.
+// word where the result is not finite or a T(j,j) is zero.  TMVG_OOM (with X as
+// it was) where its buffers are not to be had.
 tmvg_status ztrsm_sync_free(Context* c, int64_t n, const double* z, int64_t tsi, int64_t tsj, bool upper, bool unit,
                             int64_t nrhs, double* X, const double2* recip);
 

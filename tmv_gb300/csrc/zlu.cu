@@ -1080,6 +1080,7 @@ zlu_solve_kernel(int64_t n, const double2* __restrict__ LU, int64_t lda, const i
 constexpr int kZSolveBlock = 64;
 constexpr int kZSolveCols = 4;
 constexpr int64_t kZSyncFreeRhs = 64;
+constexpr int64_t kZNoWorkspace = 128;  // systems below may be solved without any
 
 __global__ void zlu_gather_rows_kernel(int64_t n, int64_t nrhs, const int* __restrict__ perm,
                                        const double2* __restrict__ B, int64_t ldb, double2* __restrict__ X)
@@ -1266,13 +1267,15 @@ static tmvg_status zlu_ldiveq_blocked(Context* c, int64_t n, const double2* LU, 
     if (nrhs <= kZSyncFreeRhs) {
         st = ztrsm_sync_free(c, n, (const double*)LU, 1, lda, false, true, nrhs, (double*)X, dinv);
         if (!st) st = ztrsm_sync_free(c, n, (const double*)LU, 1, lda, true, false, nrhs, (double*)X, dinv);
-        if (st) return st;
-        zlu_copy_back_kernel<<<ge, 256, 0, c->stream>>>(n, nrhs, X, B, ldb, c->dflags);
-        ++c->launches;
-        if ((st = check_cuda(c, cudaGetLastError(), "lu_ldiveq_z: copy back"))) return st;
-        bool retry = false;
-        st = collect_device_error(c, "lu_ldiveq_z", &retry);
-        if (st || !retry) return st;
+        if (st && st != TMVG_OOM) return st;
+        bool retry = st == TMVG_OOM;  // (no memory for its buffers)
+        if (!retry) {
+            zlu_copy_back_kernel<<<ge, 256, 0, c->stream>>>(n, nrhs, X, B, ldb, c->dflags);
+            ++c->launches;
+            if ((st = check_cuda(c, cudaGetLastError(), "lu_ldiveq_z: copy back"))) return st;
+            st = collect_device_error(c, "lu_ldiveq_z", &retry);
+            if (st || !retry) return st;
+        }
         zlu_gather_rows_kernel<<<ge, 256, 0, c->stream>>>(n, nrhs, perm, B, ldb, X);
         ++c->launches;
         if ((st = check_cuda(c, cudaGetLastError(), "lu_ldiveq_z: gather"))) return st;
@@ -1313,7 +1316,11 @@ tmvg_status zlu_ldiveq(Context* c, int64_t n, const double2* LU, int64_t lda, co
     if (n < 0 || nrhs < 0 || lda < std::max<int64_t>(n, 1) || ldb < std::max<int64_t>(n, 1))
         return set_error(c, TMVG_BAD_ARG, "lu_ldiveq_z: bad sizes");
     if (n == 0 || nrhs == 0) return TMVG_OK;
-    if (n >= kZBlockedMin && n <= (int64_t)INT32_MAX) return zlu_ldiveq_blocked(c, n, LU, lda, P, nrhs, B, ldb);
+    if (n >= kZBlockedMin && n <= (int64_t)INT32_MAX) {
+        const tmvg_status st = zlu_ldiveq_blocked(c, n, LU, lda, P, nrhs, B, ldb);
+        // (a small system needs no workspace below)
+        if (st != TMVG_OOM || n >= kZNoWorkspace) return st;
+    }
     if (nrhs > 65535) return set_error(c, TMVG_UNSUPPORTED, "lu_ldiveq_z: too many right-hand sides");
     zlu_solve_kernel<<<(unsigned)nrhs, kZThreads, 0, c->stream>>>(n, LU, lda, P, B, ldb, c->dflags);
     ++c->launches;
@@ -1499,7 +1506,7 @@ tmvg_status zlu_rdiveq(Context* c, int64_t n, const double2* LU, int64_t lda, co
     const size_t o_dinv = al(sizeof(int) * n), o_x = o_dinv + al(sizeof(double2) * n);
     const int64_t most = std::min(nrows, kZSyncFreeRhs);
     unsigned char* ws = (unsigned char*)workspace(c, o_x + sizeof(double2) * (size_t)n * most);
-    if (!ws) return set_error(c, TMVG_OOM, "lu_rdiveq_z: workspace");
+    if (!ws) return serial(B, nrows);
     int* perm = (int*)ws;
     double2* dinv = (double2*)(ws + o_dinv);
     double2* X = (double2*)(ws + o_x);
@@ -1515,6 +1522,7 @@ tmvg_status zlu_rdiveq(Context* c, int64_t n, const double2* LU, int64_t lda, co
         if ((st = check_cuda(c, cudaGetLastError(), "lu_rdiveq_z: rows"))) return st;
         st = ztrsm_sync_free(c, n, (const double*)LU, lda, 1, false, false, nq, (double*)X, dinv);
         if (!st) st = ztrsm_sync_free(c, n, (const double*)LU, lda, 1, true, true, nq, (double*)X, dinv);
+        if (st == TMVG_OOM) return serial(B + q0, nrows - q0);
         if (st) return st;
         zlu_put_rows_kernel<<<ge, 256, 0, c->stream>>>(n, nq, perm, X, B + q0, ldb, c->dflags);
         ++c->launches;
