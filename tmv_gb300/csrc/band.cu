@@ -100,23 +100,32 @@ __device__ __forceinline__ double scale_by(double v, double x)
 // below 2^-68 before its rounding), then for the quotient one correction by
 // the exact remainder, for the reciprocal one by its own (Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000 processor",
-// 1990).  The value before the last rounding is within 2^-104 of the quotient,
-// and a quotient of two doubles is no nearer than about 2^-107 to a rounding
-// boundary: a wrong rounding would take a quotient in that last gap.  Divisors
-// just below a power of two put quotients there (1 / (1 - k u) = 1 + k u + k^2
-// u^2, halfway for odd k but for the last term), so those take the division
-// itself, as do operands or results near the ends of the range (the remainder
-// would not be exact).  Six operations for about ten (65536 general systems of
+// 1990).  y is not always the rounded reciprocal: near a tie it may be the other
+// neighbour, so |y - 1/b| <= 2^-54 (1 + 2^-14) for b in [1, 2).
+//
+// Why the last rounding is right (u = 2^-53; a, b, q = a / b scaled to [1, 2), B the
+// significand of b as an integer).  Both forms end in a value whose error is small
+// enough to matter only where q is next to a midpoint m of two doubles, and there
+// q - m = k / (2 B) ulps, k a nonzero integer (a quotient is never halfway): at least
+// u / b ulps.  Quotient: a y is off by q |y b - 1| < (1 + 2^-14) b u, less than an ulp
+// as long as b (1 + 2^-14) < 2, so q0 is one of the two doubles beside m, half an
+// ulp from q.  The remainder is then exact, and the corrected value is off by half
+// an ulp times |y b - 1| <= (1 + 2^-14) b u / 2: below u / b if b^2 (1 + 2^-14) < 4.
+// Reciprocal: 1 - b y is exact and the corrected value off by (y b - 1)^2 / b <=
+// (1 + 2^-14)^2 b u^2 / 4, a midpoint at least u^2 / b away: b (1 + 2^-14) < 2.  So divisors
+// with b >= 2 - 2^-13 take the division itself (there 1 / b is next to a midpoint in
+// earnest: 1 / (1 - k u) = 1 + k u + k^2 u^2), as do operands or results near the ends
+// of the range, where the remainder would not be exact.  Six operations for about ten (65536 general systems of
 // n = 1024 with lo = hi = 2, factor and solve: 10.6 -> 9.6 ms with the copy of
 // A saved).
 __device__ __forceinline__ bool mid_range(double x)
 {
     return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - 100u < 1846u;
 }
-// (the leading 20 bits of the significand are not all ones)
+// (the leading 13 bits of the significand are not all ones)
 __device__ __forceinline__ bool plain_divisor(double x)
 {
-    return mid_range(x) && (__double2hiint(x) & 0xfffff) != 0xfffff;
+    return mid_range(x) && (__double2hiint(x) & 0xfff80) != 0xfff80;
 }
 __device__ __forceinline__ double reciprocal_estimate(double b)
 {
