@@ -1006,6 +1006,8 @@ def run_reference(args) -> dict | None:
     if rank != 0:
         return None
     orc, kind, what = cpu_reference()
+    if kind != "reference":  # the oracle's restatement is no reference
+        return {"impl": "reference", "unavailable": "TMV 0.76 is not built on this machine (no TMV source tree)"}
     cores = os.cpu_count() or 1
     orc.set_threads(cores)
     n = args.n
