@@ -17,9 +17,10 @@
 // fused multiply-adds (values to rounding).
 //
 // Small matrices (n < 32) factor one column per step (pivot search in one
-// CTA, row interchange, scaling, rank-1 update over the grid) and solve one
-// CTA per right-hand side; larger ones factor by panels with look-ahead
-// (zlu_factor_blocked) and solve as real triangles (zlu_ldiveq_blocked).  The
+// CTA, row interchange, scaling, rank-1 update over the grid); larger ones factor
+// by panels with look-ahead (zlu_factor_blocked).  Small systems solve one CTA per
+// right-hand side (the line is in zlu_ldiveq), larger ones as real triangles
+// (zlu_ldiveq_blocked).  The
 // right solve (LU_RDivEq) substitutes short rows in TMV's order, one per CTA, and
 // solves longer ones as real triangles too.
 // Values agree with TMV's recursive factorisation to rounding; pivots are
@@ -1064,7 +1065,7 @@ zlu_solve_kernel(int64_t n, const double2* __restrict__ LU, int64_t lda, const i
 }
 
 // ---------------------------------------------------------------------------
-// Blocked left solve (n >= kZBlockedMin): B is gathered into a scratch copy in
+// Blocked left solve: B is gathered into a scratch copy in
 // the pivoted row order and, up to kZSyncFreeRhs columns, solved as a real
 // system by the sync-free solve (one launch per triangle; n = 2048 with 8
 // columns 1.2 ms, against 5.2 ms in 128 launches).  Where that finds a zero
@@ -1316,7 +1317,12 @@ tmvg_status zlu_ldiveq(Context* c, int64_t n, const double2* LU, int64_t lda, co
     if (n < 0 || nrhs < 0 || lda < std::max<int64_t>(n, 1) || ldb < std::max<int64_t>(n, 1))
         return set_error(c, TMVG_BAD_ARG, "lu_ldiveq_z: bad sizes");
     if (n == 0 || nrhs == 0) return TMVG_OK;
-    if (n >= kZBlockedMin && n <= (int64_t)INT32_MAX) {
+    // Below kZNoWorkspace unknowns a CTA per column, in TMV's order, where the
+    // blocked solve is no faster (us, this and the other): up to 64 columns below 48
+    // unknowns (33: 145 and 160, 40: 170 and 162 to 178, 48: 196 and 162); for more
+    // columns above 64 (65: 247 and 517, 127: 438 and 877; 33: 148 and 130, 64: 246 and 192).
+    const bool serial = nrhs <= kZSyncFreeRhs ? n < 48 : n < kZBlockedMin || (n > 64 && n < kZNoWorkspace);
+    if (!serial && n <= (int64_t)INT32_MAX) {
         const tmvg_status st = zlu_ldiveq_blocked(c, n, LU, lda, P, nrhs, B, ldb);
         // (a small system needs no workspace below)
         if (st != TMVG_OOM || n >= kZNoWorkspace) return st;
