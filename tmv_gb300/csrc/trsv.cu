@@ -613,12 +613,14 @@ tmvg_status trsm_sync_free(Context* c, int64_t n, const T* tri, int64_t tsi, int
         B = B + (n - 1) * bsi;
         bsi = -bsi;
     }
-    // The diagonal blocks are inverted first (all but the only one).
+    // The diagonal blocks are inverted first, but not an only one: there the
+    // substitution is on no chain (9 columns of n = 2: 116 us with the inverse, 69
+    // without; n = 32 118 and 90).
     const int64_t nblk = ceil_div(n, kTrsvBlock);
     const bool few = nrhs <= kTrsvFewRhs<T>;
     T* dinv = nullptr;
     int* dsing = nullptr;
-    if (nblk > 1 || !few) {
+    if (nblk > 1) {
         tmvg_status st = inverse_blocks_buffer(c, nblk, &dinv, &dsing);
         if (st && !few) return st;
         if (!st) {  // (few columns can do without)
