@@ -39,3 +39,18 @@ def test_left_and_right_solve(dev, n, nrhs):
     assert (np.abs(low @ (up @ x) - b[pa]) <= lim * (np.abs(low) @ (np.abs(up) @ np.abs(x)))).all()
     z = y[:, pa]  # y P^-1 ... (y P) L U = b^T
     assert (np.abs((z @ low) @ up - b.T) <= lim * (np.abs(z) @ np.abs(low) @ np.abs(up))).all()
+
+
+@pytest.mark.parametrize("n", [1, 2, 8, 33, 43, 44, 45, 64])
+def test_inverse(dev, n):
+    """Both sides of the inverse's line (44)."""
+    from tmv_gb300 import linalg
+
+    a, LU, P, low, up = _factor(dev, n, 70 + n)
+    y = linalg.lu_inverse(LU, P).cpu().numpy()
+    pa = np.arange(n)
+    for i, q in enumerate(P.cpu().numpy()):
+        pa[[i, q]] = pa[[q, i]]
+    z = y[:, pa]  # (P A)^-1: columns of U^-1 L^-1, each by two substitutions
+    size = np.abs(low) @ (np.abs(up) @ np.abs(z))
+    assert (np.abs(low @ (up @ z) - np.eye(n)) <= 4 * (n + 1) * 2.0 ** -53 * size).all()

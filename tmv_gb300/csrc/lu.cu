@@ -2780,6 +2780,10 @@ static tmvg_status inverse_unpermuted(Context* c, int64_t n, const T* LU, int64_
     if constexpr (std::is_same<T, double>::value) {
         constexpr int64_t W = kTriBlock;
         double *dl = nullptr, *du = nullptr;
+        // (below 44 unknowns the substitution is shorter than the blocks' launch and
+        // products: n = 8 59 us and 105, n = 33 103 and 125, n = 44 129 and 130, n = 56
+        // 182 and 142)
+        if (!st && n < 44) return inverse_by_substitution<T>(c, n, LU, lda, Y);
         if (!st) st = lu_inv64(c, n, LU, lda, &dl, &du);
         if (st == TMVG_OOM) return inverse_by_substitution<T>(c, n, LU, lda, Y);
         auto below = [&](int64_t kb, int w, int64_t c0, int64_t nc, bool fma_pipe) {
