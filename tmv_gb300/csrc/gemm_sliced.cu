@@ -420,19 +420,20 @@ __device__ __forceinline__ int sl_look(const SlicedArgs& g, int64_t mi, int64_t 
 template <int TN>
 __device__ __noinline__ bool sl_look_again(const SlicedArgs& g, int64_t mi, int64_t ni)
 {
-    constexpr int64_t kStep = 64;  // places between two votes
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q = lane >> 2, t = lane & 3;
     const bool work = warp < kSlEpiWarps / (kSlN / TN);
     const int64_t r0 = mi * kSlM + (warp & 3) * 32 + q;                 // rows r0 + 8 (0..3)
     const int64_t c0 = ni * TN + (int64_t)(warp >> 2) * kSlCols;        // columns
-    // (rows and columns outside read the last one's digits; they do not vote)
-    const uint16_t *pa[4], *pb[2];
+    // (rows and columns outside read the last one's digits; they do not vote.  A
+    // lane reads eight neighbouring places, which stand for the places the
+    // instruction would have it hold: the order of the sum is free)
+    const uint4 *pa[4], *pb[2];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) pa[u] = g.da + min(r0 + 8 * u, g.M - 1) * g.Kp + 2 * t;
+    for (int u = 0; u < 4; ++u) pa[u] = reinterpret_cast<const uint4*>(g.da + min(r0 + 8 * u, g.M - 1) * g.Kp) + t;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) pb[u] = g.db + min(c0 + 8 * u + q, g.N - 1) * g.Kp + 2 * t;
-    auto digits = [](const uint16_t* p) { return __ldg(reinterpret_cast<const uint32_t*>(p)) & 0x7fff7fffu; };
+    for (int u = 0; u < 2; ++u) pb[u] = reinterpret_cast<const uint4*>(g.db + min(c0 + 8 * u + q, g.N - 1) * g.Kp) + t;
+    constexpr uint32_t kAbs = 0x7fff7fffu;
     float sum[2][2][4] = {};
     // which of sum's elements need no more: bit 8 i + 4 j + e
     unsigned done = work ? 0u : 0xffffu;
@@ -447,27 +448,39 @@ __device__ __noinline__ bool sl_look_again(const SlicedArgs& g, int64_t mi, int6
                     __ldg(&g.eb[min(c, g.N - 1)]) == kZeroExp)
                     done |= 1u << (8 * i + 4 * j + e);
             }
-    for (int64_t k0 = 0; k0 < g.Kp; k0 += kStep) {
+    const int64_t steps = g.Kp / kSlK;
+    for (int64_t s0 = 0; s0 < steps; s0 += 2) {  // a vote every two
         if (__any_sync(0xffffffffu, done != 0xffffu)) {
-            for (int64_t k = k0; k < min(k0 + kStep, g.Kp); k += 16) {
-                uint32_t a[2][4], b[2][2];
+            uint4 av[2][4], bv[2][2];
 #pragma unroll
-                for (int i = 0; i < 2; ++i)
+            for (int h = 0; h < 2; ++h) {
+                const int64_t at = 4 * min(s0 + h, steps - 1);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) a[i][e] = digits(pa[2 * i + (e & 1)] + k + 8 * (e >> 1));
+                for (int u = 0; u < 4; ++u) av[h][u] = __ldg(pa[u] + at);
 #pragma unroll
-                for (int j = 0; j < 2; ++j)
+                for (int u = 0; u < 2; ++u) bv[h][u] = __ldg(pb[u] + at);
+            }
 #pragma unroll
-                    for (int e = 0; e < 2; ++e) b[j][e] = digits(pb[j] + k + 8 * e);
+            for (int h = 0; h < 2; ++h) {
+                if (s0 + h >= steps) break;
 #pragma unroll
-                for (int i = 0; i < 2; ++i)
+                for (int x = 0; x < 2; ++x)  // words x, y and then z, w: 16 places each
 #pragma unroll
-                    for (int j = 0; j < 2; ++j)
-                        asm volatile(
-                            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
-                            "{%8, %9}, {%0, %1, %2, %3};"
-                            : "+f"(sum[i][j][0]), "+f"(sum[i][j][1]), "+f"(sum[i][j][2]), "+f"(sum[i][j][3])
-                            : "r"(a[i][0]), "r"(a[i][1]), "r"(a[i][2]), "r"(a[i][3]), "r"(b[j][0]), "r"(b[j][1]));
+                    for (int i = 0; i < 2; ++i) {
+                        const uint4 &lo = av[h][2 * i], &hi = av[h][2 * i + 1];
+                        const uint32_t a[4] = {(x ? lo.z : lo.x) & kAbs, (x ? hi.z : hi.x) & kAbs,
+                                               (x ? lo.w : lo.y) & kAbs, (x ? hi.w : hi.y) & kAbs};
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {
+                            const uint32_t b0 = (x ? bv[h][j].z : bv[h][j].x) & kAbs;
+                            const uint32_t b1 = (x ? bv[h][j].w : bv[h][j].y) & kAbs;
+                            asm volatile(
+                                "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, "
+                                "%7}, {%8, %9}, {%0, %1, %2, %3};"
+                                : "+f"(sum[i][j][0]), "+f"(sum[i][j][1]), "+f"(sum[i][j][2]), "+f"(sum[i][j][3])
+                                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+                        }
+                    }
             }
 #pragma unroll
             for (int i = 0; i < 2; ++i)
@@ -807,7 +820,8 @@ sliced_rest_kernel(const __grid_constant__ SlicedArgs g)
     const int group = threadIdx.x / (kRestB * kRestB), gt = threadIdx.x % (kRestB * kRestB);
     RestBlock& sh = reinterpret_cast<RestBlock*>(rest_smem)[group];
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int64_t items = (int64_t)g.listed[0] * kSub;
+    const int listed = g.listed[0];
+    const int64_t items = (int64_t)listed * kSub;
     const int tx = gt % kRestB, ty = gt / kRestB;
     const bool ak = !Z && g.asj == 1, bk = g.bsi == 1;  // K contiguous
     auto a_at = [&](int t, int& r, int& k) { r = ak ? t / kRestK : t % kRestB, k = ak ? t % kRestK : t / kRestB; };
@@ -815,10 +829,14 @@ sliced_rest_kernel(const __grid_constant__ SlicedArgs g)
     auto sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(group) : "memory"); };
     for (int64_t it = (int64_t)group * gridDim.x + blockIdx.x; it < items; it += (int64_t)kRestGroups * gridDim.x) {
         int64_t mi, ni;
-        sl_tile(g, g.listed[1 + it / kSub], mi, ni);
-        const int sub = (int)(it % kSub);
-        const int64_t r0 = mi * kSlM + (sub % (kSlM / kRestB)) * kRestB, c0 = ni * TN + (sub / (kSlM / kRestB)) * kRestB;
-        if (r0 >= g.M || c0 >= g.N) continue;
+        // (one block of every tile after the other, the blocks in C first: they fall
+        // evenly on the CTAs)
+        sl_tile(g, g.listed[1 + it % listed], mi, ni);
+        const int sub = (int)(it / listed);
+        const int hb = (int)min((int64_t)(kSlM / kRestB), (g.M - mi * kSlM + kRestB - 1) / kRestB);
+        const int wb = (int)min((int64_t)(TN / kRestB), (g.N - ni * TN + kRestB - 1) / kRestB);
+        if (sub >= hb * wb) continue;
+        const int64_t r0 = mi * kSlM + (sub % hb) * kRestB, c0 = ni * TN + (sub / hb) * kRestB;
         double pa[kLoads], pb[kLoads], acc = 0.0;
         auto load = [&](int64_t k0) {
 #pragma unroll
