@@ -574,11 +574,10 @@ def batched_bench(dev, args, with_cpu: bool) -> dict:
 # byte of each kernel class, from one ncu capture of the class's main kernel
 # on the n = 8192 workload (commands and figures in profiles/):
 #   panel: lu_panel_leaf_kernel, k = 320: 2.08 MB / 4.03 MB
-#   trailing_update: the 3xTF32 update, k = 256: 432.1 MB / 495.7 MB (tf32x3_update_kernel;
-#   the streamed form reads and writes the same tiles)
+#   trailing_update: tf32x3_stream_kernel, k = 128: 459.4 MB / 512.0 MB
 #   tri_solve: trsv_pub_async_kernel: 140.4 MB / 138.5 MB
 # The traffic of a span is its algorithmic bytes times the ratio.
-NCU_TRAFFIC_PER_ALG_BYTE: dict = {"panel": 0.516, "trailing_update": 0.872, "tri_solve": 1.014}
+NCU_TRAFFIC_PER_ALG_BYTE: dict = {"panel": 0.516, "trailing_update": 0.897, "tri_solve": 1.014}
 
 KERNEL_NAMES = {
     "panel": "lu_panel_leaf_kernel (16-CTA cluster, 512 threads, one register-resident FP32 panel row "

@@ -95,9 +95,9 @@ int64_t tmvg_launch_count(tmvg_handle h);
  * and under the same clocks as the work.  Synchronises the stream. */
 tmvg_status tmvg_probe_fp64_rate(tmvg_handle h, double* tflops);
 /* Failure-path test hook, no counterpart in TMV.  poll_limit sets how many
- * polls the block-flag waits of the sync-free triangular solve (the solve of
- * up to 8 right-hand sides behind tmvg_tri_ldiveq_f64, tmvg_lu_ldiveq_f64 and
- * the FP64 solves) and of the mixed solve's streamed FP32 triangular solve
+ * polls the waits of the sync-free triangular solve (the solve of up to 256
+ * right-hand sides behind tmvg_tri_ldiveq_f64, tmvg_lu_ldiveq_f64 and the FP64
+ * solves, and the complex solves as real triangles) and of the mixed solve's streamed FP32 triangular solve
  * (n a multiple of 128) make before they give up (0 restores the default,
  * 2^24 polls with back-off).  skip_blocks > 0 makes the next such solve hand
  * its blocks out from ticket skip_blocks on, so the first blocks are never
@@ -182,7 +182,7 @@ tmvg_status tmvg_lu_decompose_f64_host(tmvg_handle h, int64_t n, double* A,
  * tmvg_lu_decompose_f64 and gives the same factors to rounding (it runs the
  * simplest schedule: the grid-barrier panel kernel, no look-ahead), but it
  * calls no cudaMalloc/cudaFree and needs no tmvg_handle: all scratch lives in
- * one static device array of 353,540 bytes (345 KiB) that every GPU loading
+ * one static device array of 337,156 bytes (329 KiB) that every GPU loading
  * this library holds until the process exits; each call looks up the array's
  * device address in the current context.  Runs on the current device and
  * the given cudaStream_t (NULL: legacy default stream) and synchronises that
@@ -295,8 +295,8 @@ tmvg_status tmvg_multmv_f64(tmvg_handle h, int add, double alpha, int64_t m,
  * Replaces: template void tmv::LU_Decompose(MatrixView<std::complex<double> >,
  *           ptrdiff_t*) (src/TMV_LUDecompose.cpp:514-559).
  * tmvg_lu_ldiveq_z64: B := (P L U)^-1 B, each column with TMV's vector
- * solves (zero entries skipped; a division by U(j,j) as TMV_Divide);
- * TMVG_SINGULAR when a zero U(j,j) meets a nonzero entry.  Synchronises.
+ * solves (zero entries skipped; a division by U(j,j) as TMV_Divide), from 48
+ * unknowns on as real triangles (values to rounding); TMVG_SINGULAR when a zero U(j,j) meets a nonzero entry.  Synchronises.
  * Replaces: template void tmv::LU_LDivEq(const GenMatrix<std::complex<double> >&,
  *           const ptrdiff_t*, MatrixView<std::complex<double> >)
  *           (src/TMV_LUDiv.cpp:186). */
@@ -306,7 +306,8 @@ tmvg_status tmvg_lu_ldiveq_z64(tmvg_handle h, int64_t n, const double* LU, int64
                                const int64_t* P, int64_t nrhs, double* B, int64_t ldb);
 /* B (nrows x n, column-major, leading dimension ldb) := B (P L U)^-1 with
  * TMV's row-oriented solves of the transposed factors (leading / trailing
- * zeros trimmed, a zero U(i,i) then TMVG_SINGULAR).  Synchronises.
+ * zeros trimmed, a zero U(i,i) then TMVG_SINGULAR), bit for bit up to n = 130;
+ * longer rows as real triangles (values to rounding).  Synchronises.
  * Replaces: template void tmv::LU_RDivEq(const GenMatrix<std::complex<double> >&,
  *           const ptrdiff_t*, MatrixView<std::complex<double> >)
  *           (src/TMV_LUDiv.cpp:370). */

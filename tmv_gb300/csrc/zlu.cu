@@ -1362,7 +1362,8 @@ __global__ void zlu_put_rows_kernel(int64_t n, int64_t nq, const int* __restrict
 // rounding; a zero U(i,i) or a value that is not finite sends the rows to the
 // substitution below, which decides as TMV does.  8 rows: n = 131 0.19 ms (4.9 with a thread per row),
 // 512 0.32 (75), 2048 1.3 (1232).  Up to kZRightSerial entries the bits of TMV's
-// order of operations are kept, which costs 0.5 ms at 130 entries.
+// order of operations are kept: that is promised to callers, and costs 0.3 ms at 130
+// entries (the real solves would be faster from about 50).
 constexpr int64_t kZRightSerial = 130;
 
 // One row of B per CTA: b := b (P L U)^-1 (LU_RDivEq, src/TMV_LUDiv.cpp:370-411:
