@@ -1015,6 +1015,10 @@ tmvg_status sliced_gemm(Context* c, int64_t M, int64_t N, int64_t K, double alph
 {
     // blocks of at most 256 MiB of digits per operand
     constexpr int64_t kMaxK = 16384;
+    // (blocks of K are added into C one after the other, each times alpha: an
+    // infinite alpha, or one that takes a partial sum out of range, would not give
+    // alpha times the sum)
+    if (K > kMaxK && !(std::fabs(alpha) <= 0x1p60)) return TMVG_UNSUPPORTED;
     const int64_t kb = std::min(K, kMaxK);
     const int64_t cap = std::max<int64_t>(kSlM, (((int64_t)1 << 28) / (2 * kSlices * (kb + kSlK))) / kSlM * kSlM);
     const int64_t mb = std::min(M, cap);

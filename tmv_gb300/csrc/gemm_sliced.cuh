@@ -25,7 +25,7 @@ bool sliced_wanted(Context* c, int64_t M, int64_t N, int64_t K);
 
 // C (M x N, column-major) = alpha A B + beta C (beta 0 or 1).  `max_ctas` bounds
 // the persistent grids (0: one CTA per SM).  TMVG_UNSUPPORTED (with nothing
-// launched) where the workspace is not to be had.
+// launched) where the workspace is not to be had, or a huge alpha meets a long K.
 // The left operand may be a complex matrix in its real form (zleft): A.p is the
 // complex data, A.si and A.sj its strides in complex elements, and the operand
 // is the 2m x 2k real matrix of 2 x 2 blocks (re, -im; im, re).  With B and C
