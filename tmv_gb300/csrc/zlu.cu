@@ -1248,6 +1248,8 @@ static tmvg_status zgemm_sub(Context* c, int64_t M, int64_t N, int K, const doub
     return check_cuda(c, cudaGetLastError(), "lu_ldiveq_z: product");
 }
 
+// TMVG_UNSUPPORTED, with B as it was, where the real solves decline and n is below
+// kZNoWorkspace.
 static tmvg_status zlu_ldiveq_blocked(Context* c, int64_t n, const double2* LU, int64_t lda, const int64_t* P,
                                       int64_t nrhs, double2* B, int64_t ldb)
 {
@@ -1277,6 +1279,7 @@ static tmvg_status zlu_ldiveq_blocked(Context* c, int64_t n, const double2* LU, 
             st = collect_device_error(c, "lu_ldiveq_z", &retry);
             if (st || !retry) return st;
         }
+        if (n < kZNoWorkspace) return TMVG_UNSUPPORTED;
         zlu_gather_rows_kernel<<<ge, 256, 0, c->stream>>>(n, nrhs, perm, B, ldb, X);
         ++c->launches;
         if ((st = check_cuda(c, cudaGetLastError(), "lu_ldiveq_z: gather"))) return st;
@@ -1324,8 +1327,10 @@ tmvg_status zlu_ldiveq(Context* c, int64_t n, const double2* LU, int64_t lda, co
     const bool serial = nrhs <= kZSyncFreeRhs ? n < 48 : n < kZBlockedMin || (n > 64 && n < kZNoWorkspace);
     if (!serial && n <= (int64_t)INT32_MAX) {
         const tmvg_status st = zlu_ldiveq_blocked(c, n, LU, lda, P, nrhs, B, ldb);
-        // (a small system needs no workspace below)
-        if (st != TMVG_OOM || n >= kZNoWorkspace) return st;
+        // a small system needs no workspace below, and where the real solves
+        // decline TMV's order decides (a column of zeros stays one, whatever the
+        // factors hold: the blocked solve's products would make 0 times infinity)
+        if (st != TMVG_UNSUPPORTED && (st != TMVG_OOM || n >= kZNoWorkspace)) return st;
     }
     if (nrhs > 65535) return set_error(c, TMVG_UNSUPPORTED, "lu_ldiveq_z: too many right-hand sides");
     zlu_solve_kernel<<<(unsigned)nrhs, kZThreads, 0, c->stream>>>(n, LU, lda, P, B, ldb, c->dflags);
